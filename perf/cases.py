@@ -270,3 +270,25 @@ def tolerance(case):
     if kind == "dbm":
         return {"rel": 1.5e-2, "max": 5e-2}                # 3.7e-3, 1.2e-2 seen (bias history of the top layer)
     return {"rel": 1e-3, "max": 0.15}                      # 2e-4, 3.5e-2 seen (CD-10 at 8192 x 8192)
+
+
+def exact(case, seed):
+    """What `run` returns, in 64 bits, for the kinds that draw nothing."""
+    kind, V, H, B = case["kind"], case["V"], case["H"], case["B"]
+    r = _Inputs(seed)
+
+    def layer(x, w, b):
+        w, b = (torch.from_numpy(np.ascontiguousarray(a)).cuda().double() for a in (w, b))
+        return torch.sigmoid(x @ w + b.view(1, -1))
+
+    if kind == "represent":
+        sizes = [V, H, case["H2"]]
+        params = [(r.weights(sizes[i], sizes[i + 1], 0.05), r.biases(sizes[i + 1], 0.5)) for i in range(2)]
+        low = layer(r.binary(V, B).double(), *params[0])
+        return [low, layer(low, *params[1])]
+    if kind == "infer":
+        w, bv, bh = r.weights(V, H, 0.05), r.biases(V, 0.5), r.biases(H, 0.5)
+        x = r.binary(V, case["batches"] * B).double()
+        h = layer(x, w, bh)
+        return h, float(((layer(h, w.T, bv) - x) ** 2).sum())
+    return None                                            # the others end in random draws
