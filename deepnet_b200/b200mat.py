@@ -1084,7 +1084,7 @@ def cuda_sync_threads():
 
 
 def set_gemm_path(path):
-    """0 auto, 1 tensor cores only, 2 CUDA cores only."""
+    """0 auto, 1 the tcgen05 kernel only, 2 CUDA cores only, 3 the one-launch kernel for small products only."""
     _lib.b200_set_gemm_path(ct.c_int(path))
 
 

@@ -90,6 +90,10 @@ int rewrite_f16_planes_if(const float* x, uint16_t* aux, int rows, long n, const
 int set_product_scatter(const float* match, float* const* out, int n, int cols);
 bool product_is_scattered(const float* out);
 int gemm_simt(const GemmProblem& g);
+// fp32-grade products of any alignment in one launch (gemm_small.cu); ERROR_UNSUPPORTED for term lists that are
+// not whole products (scaled half-precision planes, single parts).
+int gemm_small(const GemmProblem& g, bool ieee);
+int small_depth(const GemmProblem& g);      // slabs of K that one SM would walk in gemm_small; 0: a list it does not take
 // Returns ERROR_UNSUPPORTED when an operand is not addressable by TMA (leading
 // dimension not a multiple of 4 floats or base not 16-byte aligned).
 int gemm_tc(const GemmProblem& g);

@@ -8,7 +8,7 @@ using namespace b200;
 
 namespace {
 
-int g_path = 0;       // 0 auto, 1 tensor cores only, 2 CUDA cores only
+int g_path = 0;       // 0 auto; one kernel only: 1 tcgen05, 2 CUDA cores, 3 the one-launch kernel
 int g_dot_mode = 0;   // 0: fp32-grade (three TF32 terms), 1: single TF32 term
 constexpr long kTcMinWork = 1L << 21;  // below this many multiply-adds `dot` stays on CUDA cores
 
@@ -30,16 +30,25 @@ inline bool aux_shape_ok(const cudamat* aux, const cudamat* m) {
   return aux->on_device && aux->size[0] == aux_rows(m->size[0]) && aux->size[1] == m->size[1];
 }
 
+// The one-launch kernel (gemm_small.cu) against the tcgen05 one, by the slabs of 32 of K that an SM has to walk.
+// Measured (one launch against product + finishing launch): 4 slabs 10.9 against 15.1 us (500 x 100, K = 784), 8
+// slabs 17.8 against 23.6 (1024 x 256, K = 1024), 16 slabs 30.7 against 30.9 (1024 x 1024, two pairs of K = 256), 40
+// slabs 62 against 20 (512 x 100, K = 10 000).  Operands TMA cannot address stay here at any size (CUDA cores
+// took 13 times as long at 601 x 203, K = 1357).
+constexpr int kSmallDepth = 10;
+
 int run(const GemmProblem& g) {
   if (product_is_scattered(g.epi.out)) return gemm_tc(g);   // (fails loudly when the tensor-core kernel cannot take it)
   if (g_path == 2) return gemm_simt(g);
-  if (gemm_tc_supported(g)) {
-    const int r = gemm_tc(g);
-    // (a product with more operand pairs or tiles than one tensor-core launch carries)
-    if (r != ERROR_UNSUPPORTED || g_path == 1) return r;
-  } else if (g_path == 1) {
-    return ERROR_UNSUPPORTED;
-  }
+  if (g_path == 3) return gemm_small(g, false);
+  const bool tc = gemm_tc_supported(g);
+  const int depth = g_path == 0 ? small_depth(g) : 0;
+  int r = ERROR_UNSUPPORTED;
+  if (depth > 0 && (depth <= kSmallDepth || !tc)) r = gemm_small(g, false);
+  if (r != ERROR_UNSUPPORTED) return r;
+  // (unsupported: more operand pairs or tiles than one tensor-core launch carries)
+  if (tc) r = gemm_tc(g);
+  if (r != ERROR_UNSUPPORTED || g_path == 1) return r;
   return gemm_simt(g);
 }
 
@@ -324,8 +333,8 @@ struct b200_fused_gemm {
 
 extern "C" {
 
-// 0 auto (tensor cores when the operands are TMA-addressable), 1 tensor cores only
-// (ERROR_UNSUPPORTED otherwise), 2 CUDA cores only.
+// 0 auto (by size and alignment), 1 the tcgen05 kernel only (ERROR_UNSUPPORTED where TMA cannot address an
+// operand), 2 CUDA cores only, 3 the one-launch kernel only.
 int b200_set_gemm_path(int path) {
   g_path = path;
   return 0;
@@ -485,27 +494,34 @@ int dot(cudamat* mat1, cudamat* mat2, cudamat* target, float beta, float alpha) 
     g.pass[0].k = 0;
     return gemm_simt(g);
   }
-  const bool tc = g_path != 2 && gemm_tc_supported(g) && (g_path == 1 || (long)m * n * k >= kTcMinWork);
-  if (!tc) {
-    if (g_path == 1) return ERROR_UNSUPPORTED;
-    return gemm_simt(g);
-  }
-  if (g_dot_mode == 1) return gemm_tc(g);
   // fp32-grade: x = tf32(x) + lo with lo = x - tf32(x); lo.x + x.lo + x.x, small terms first,
   // every term a TF32 product (the kernel derives lo from the staged tile of x).  The cheaper
   // bfloat16 correction terms are a few times less accurate (2^-18 against 2^-20 per term),
   // which shows when a caller subtracts two nearly equal products, as the positive and
   // negative statistics are.
-  g.npass = 3;
+  GemmProblem f = g;
+  f.npass = 3;
   const int pa[3] = {kPartLo32, kPartX, kPartX}, pb[3] = {kPartX, kPartLo32, kPartX};
   for (int q = 0; q < 3; q++) {
-    g.pass[q].a = operand(mat1, pa[q]);
-    g.pass[q].b = operand(mat2, pb[q]);
-    g.pass[q].k = k;
-    g.pass[q].negate = 0;
+    f.pass[q].a = operand(mat1, pa[q]);
+    f.pass[q].b = operand(mat2, pb[q]);
+    f.pass[q].k = k;
+    f.pass[q].negate = 0;
   }
-  g.tf32_operands = 1;
-  return gemm_tc(g);
+  f.tf32_operands = 1;
+  if (g_path == 3 || (g_path == 0 && g_dot_mode != 1)) {
+    const int depth = small_depth(f);
+    if (g_path == 3 || (depth > 0 && (depth <= kSmallDepth || !gemm_tc_supported(f)))) {
+      const int r = gemm_small(f, true);
+      if (r != ERROR_UNSUPPORTED || g_path == 3) return r;
+    }
+  }
+  const bool tc = g_path != 2 && gemm_tc_supported(g) && (g_path == 1 || (long)m * n * k >= kTcMinWork);
+  if (!tc) {
+    if (g_path == 1) return ERROR_UNSUPPORTED;
+    return gemm_simt(g);
+  }
+  return gemm_tc(g_dot_mode == 1 ? g : f);
 }
 
 // deepnet/dbm.py:242,254 + deepnet/parameter.py:80-106 in one pass over the parameter:

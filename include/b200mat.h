@@ -312,7 +312,7 @@ int b200_sm_count(void);                  /* SMs in force (the device's, or the 
  * its copies deliver, so one of its bounded waits must run out (status word set, kernel returns).
  * No counterpart in the reference. */
 int b200_test_inject_stage_bytes(int extra_bytes);
-int b200_set_gemm_path(int path);         /* 0 auto, 1 tensor cores only, 2 CUDA cores only */
+int b200_set_gemm_path(int path);         /* 0 auto, 1 tcgen05 kernel only, 2 CUDA cores only, 3 one-launch kernel only */
 int b200_set_dot_precision(int mode);     /* 0 fp32-grade split TF32 (default), 1 one TF32 pass */
 /* Split-K of the tensor-core product: 0 (default) = cut the inner dimension into work items when the
  * output tiles alone would leave most SMs idle, 1 = never, n > 1 = always n splits.  No counterpart

@@ -572,3 +572,68 @@ def test_momentum_update_by_column_panels_equals_the_whole_update(cm, mode):
     for a, b in zip(out[0], out[1]):
         if a is not None:
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("ta,tb", [(0, 0), (1, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("m,n,k", [(1, 1, 1), (7, 5, 3), (64, 64, 32), (65, 63, 33), (127, 66, 129), (500, 100, 784), (300, 4, 1357),
+                                   (4, 257, 601)])
+def test_one_launch_product_in_all_layouts(cm, ta, tb, m, n, k):
+    """gemm_small.cu: edges of tiles and slabs, 16-byte and 4-byte copies, one to eight CTAs along K; two pairs of
+    matrices (the second negated, its left side exact), bias x column scale, beta.
+    Bound: 3 * 2^-23 per term from the split, 12 truncating additions (2^-23 each) per two slabs and one rounding (2^-24)
+    per two slabs, of sum |a||b|: below 2^-18 for k <= 2000."""
+    rng = np.random.default_rng(m * 7 + n * 3 + k)
+    A, A2 = rng.standard_normal((m, k)).astype(np.float32), (rng.random((m, k + 1)) < 0.4).astype(np.float32)
+    B, B2 = rng.standard_normal((k, n)).astype(np.float32), rng.standard_normal((k + 1, n)).astype(np.float32)
+    b, cs = rng.standard_normal((m, 1)).astype(np.float32), rng.random((1, n)).astype(np.float32)
+    old = rng.standard_normal((m, n)).astype(np.float32)
+    cm.set_gemm_path(3)
+    out = cm.CUDAMatrix(old)
+    P = cm.split_passes
+    cm.fused_gemm(P(make(cm, A, ta), make(cm, B, tb)) + P(make(cm, A2, tb), make(cm, B2, ta), negate=1, exact_a=True, terms="tf32"),
+                  out=out, bias=cm.CUDAMatrix(b), col_scale=cm.CUDAMatrix(cs), alpha=0.5, beta=2.0)
+    d = lambda x: x.astype(np.float64)
+    want = 0.5 * (d(A) @ d(B) - d(A2) @ d(B2)) + 2.0 * old + d(b) * cs
+    size = 0.5 * (np.abs(d(A)) @ np.abs(d(B)) + np.abs(d(A2)) @ np.abs(d(B2)))
+    assert (np.abs(get(out) - want) <= 2.0 ** -18 * size + 2.0 ** -22 * (2 * np.abs(old) + np.abs(b * cs) + 1e-30)).all()
+    got = get(cm.dot(make(cm, A, ta), make(cm, B, tb)))
+    assert (np.abs(got - d(A) @ d(B)) <= 2.0 ** -18 * (np.abs(d(A)) @ np.abs(d(B)))).all()
+
+
+@pytest.mark.parametrize("col0", [0, 3, 8])
+@pytest.mark.parametrize("m,n,k", [(65, 63, 33), (500, 100, 784), (127, 66, 2000)])
+def test_one_launch_product_draws_and_aux(cm, oracle, col0, m, n, k):
+    rng = np.random.default_rng(m + n + k)
+    W, X = (rng.standard_normal((k, m)) * 0.1).astype(np.float32), (rng.random((k, n)) < 0.3).astype(np.float32)
+    b = rng.standard_normal((m, 1)).astype(np.float32)
+    cm.set_gemm_path(3)
+    cm.CUDAMatrix.init_random(99)
+    oracle.EigenMatrix.init_random(99)
+    out, smp, out_aux, smp_aux = cm.empty((m, n)), cm.empty((m, n)), cm.empty_aux((m, n)), cm.empty_aux((m, n))
+    cm.set_rng_column_offset(col0)
+    try:
+        cm.fused_gemm(cm.split_passes(cm.CUDAMatrix(W).T, cm.CUDAMatrix(X), exact_b=True), out=out, sample=smp, out_aux=out_aux,
+                      sample_aux=smp_aux, bias=cm.CUDAMatrix(b), activation=1)
+    finally:
+        cm.set_rng_column_offset(0)
+    got = get(out)
+    assert relerr(got, 1 / (1 + np.exp(-(W.astype(np.float64).T @ X + b)))) < TOL
+    lo, bb = out_aux.planes()
+    np.testing.assert_array_equal(lo, bf16_round(got - tf32_trunc(got)))
+    np.testing.assert_array_equal(bb, bf16_round(got))
+    wide = np.zeros((m, col0 + n), np.float32)   # the draw of a shard is that of its columns of the global batch
+    wide[:, col0:] = got
+    want = get(oracle.EigenMatrix(wide).sample_bernoulli(target=oracle.empty(wide.shape)))[:, col0:]
+    np.testing.assert_array_equal(get(smp), want)
+    np.testing.assert_array_equal(smp_aux.planes()[1], want)
+
+
+@pytest.mark.parametrize("m,n,k", [(65, 63, 33), (100, 100, 1000)])
+def test_one_launch_dot_keeps_infinities(cm, m, n, k):
+    rng = np.random.default_rng(3)
+    A, B = rng.standard_normal((m, k)).astype(np.float32), rng.random((k, n)).astype(np.float32) + 0.5
+    A[3, 5], A[7, 9], A[7, 11], A[9, 2] = np.inf, np.inf, -np.inf, np.nan
+    got = get(cm.dot(cm.CUDAMatrix(A), cm.CUDAMatrix(B)))
+    assert np.isposinf(got[3]).all() and np.isnan(got[7]).all() and np.isnan(got[9]).all()
+    rest = np.delete(got, [3, 7, 9], axis=0)
+    assert np.isfinite(rest).all()
