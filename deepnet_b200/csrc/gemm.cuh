@@ -76,6 +76,7 @@ struct GemmProblem {
   // 1: part kPartX is read as TF32 (low 13 mantissa bits ignored), its meaning on the tensor
   // cores, which the CUDA-core kernel then reproduces; 0: kPartX is the full fp32 value.
   int tf32_operands;
+  int chunk_k = 0;   // products folded in tensor memory before they join the fp32 registers; 0: the kernel's own choice
   GemmPass pass[kMaxPass];
   GemmEpilogue epi;
 };
@@ -93,11 +94,13 @@ int gemm_simt(const GemmProblem& g);
 // fp32-grade products of any alignment in one launch (gemm_small.cu); ERROR_UNSUPPORTED for term lists that are
 // not whole products (scaled half-precision planes, single parts).
 int gemm_small(const GemmProblem& g, bool ieee);
+int recompute_nonfinite(const GemmProblem& g);   // non-finite entries of g.epi.out = alpha x the plain fp32 product
 int small_depth(const GemmProblem& g);      // slabs of K that one SM would walk in gemm_small; 0: a list it does not take
 // Returns ERROR_UNSUPPORTED when an operand is not addressable by TMA (leading
 // dimension not a multiple of 4 floats or base not 16-byte aligned).
 int gemm_tc(const GemmProblem& g);
 bool gemm_tc_supported(const GemmProblem& g);
+int gemm_tc_packed(const GemmProblem& g);   // the same behind a copy of the operands TMA cannot address
 
 #ifdef __CUDACC__
 // Applies the epilogue to one accumulator value and stores every requested output.

@@ -8,7 +8,7 @@ using namespace b200;
 
 namespace {
 
-int g_path = 0;       // 0 auto; one kernel only: 1 tcgen05, 2 CUDA cores, 3 the one-launch kernel
+int g_path = 0;       // 0 auto; one kernel only: 1 tcgen05, 2 CUDA cores, 3 the one-launch kernel, 4 tcgen05 behind aligned copies
 int g_dot_mode = 0;   // 0: fp32-grade (three TF32 terms), 1: single TF32 term
 constexpr long kTcMinWork = 1L << 21;  // below this many multiply-adds `dot` stays on CUDA cores
 
@@ -33,23 +33,27 @@ inline bool aux_shape_ok(const cudamat* aux, const cudamat* m) {
 // The one-launch kernel (gemm_small.cu) against the tcgen05 one, by the slabs of 32 of K that an SM has to walk.
 // Measured (one launch against product + finishing launch): 4 slabs 10.9 against 15.1 us (500 x 100, K = 784), 8
 // slabs 17.8 against 23.6 (1024 x 256, K = 1024), 16 slabs 30.7 against 30.9 (1024 x 1024, two pairs of K = 256), 40
-// slabs 62 against 20 (512 x 100, K = 10 000).  Operands TMA cannot address stay here at any size (CUDA cores
-// took 13 times as long at 601 x 203, K = 1357).
-constexpr int kSmallDepth = 10;
+// slabs 62 against 20 (512 x 100, K = 10 000).  Where the tcgen05 kernel needs aligned copies of its operands first
+// the line is the same: 8 slabs 21.7 against 26.8 us (1021 x 255, K = 1021), 11 slabs 27.1 against 28.8 (601 x
+// 203, K = 1357), 14 slabs 35.4 against 27.1 (1357 x 601, two pairs of K = 203).
+constexpr int kSmallDepth = 11;
 
 int run(const GemmProblem& g) {
   if (product_is_scattered(g.epi.out)) return gemm_tc(g);   // (fails loudly when the tensor-core kernel cannot take it)
   if (g_path == 2) return gemm_simt(g);
   if (g_path == 3) return gemm_small(g, false);
+  if (g_path == 4) return gemm_tc_packed(g);
   const bool tc = gemm_tc_supported(g);
   const int depth = g_path == 0 ? small_depth(g) : 0;
   int r = ERROR_UNSUPPORTED;
-  if (depth > 0 && (depth <= kSmallDepth || !tc)) r = gemm_small(g, false);
+  if (depth > 0 && depth <= kSmallDepth) r = gemm_small(g, false);
   if (r != ERROR_UNSUPPORTED) return r;
   // (unsupported: more operand pairs or tiles than one tensor-core launch carries)
   if (tc) r = gemm_tc(g);
+  else if (g_path == 0) r = gemm_tc_packed(g);
   if (r != ERROR_UNSUPPORTED || g_path == 1) return r;
-  return gemm_simt(g);
+  if (depth > 0) r = gemm_small(g, false);
+  return r != ERROR_UNSUPPORTED ? r : gemm_simt(g);
 }
 
 // hi may be null: the tensor core itself drops the low 13 mantissa bits of an fp32
@@ -334,7 +338,8 @@ struct b200_fused_gemm {
 extern "C" {
 
 // 0 auto (by size and alignment), 1 the tcgen05 kernel only (ERROR_UNSUPPORTED where TMA cannot address an
-// operand), 2 CUDA cores only, 3 the one-launch kernel only.
+// operand), 2 CUDA cores only, 3 the one-launch kernel only, 4 the
+// tcgen05 kernel behind aligned copies of its operands only.
 int b200_set_gemm_path(int path) {
   g_path = path;
   return 0;
@@ -511,11 +516,20 @@ int dot(cudamat* mat1, cudamat* mat2, cudamat* target, float beta, float alpha) 
   f.tf32_operands = 1;
   if (g_path == 3 || (g_path == 0 && g_dot_mode != 1)) {
     const int depth = small_depth(f);
-    if (g_path == 3 || (depth > 0 && (depth <= kSmallDepth || !gemm_tc_supported(f)))) {
+    const bool unaligned = !gemm_tc_supported(f);
+    // An infinity in an operand keeps its meaning where `dot` ran on CUDA cores before (operands TMA cannot address,
+    // little work): non-finite results are computed again in plain fp32.
+    if (g_path == 0 && unaligned && depth > kSmallDepth && beta == 0.0f) {
+      int r = gemm_tc_packed(f);
+      if (r == 0) r = recompute_nonfinite(f);
+      if (r != ERROR_UNSUPPORTED) return r;
+    }
+    if (g_path == 3 || (depth > 0 && (depth <= kSmallDepth || unaligned))) {
       const int r = gemm_small(f, true);
       if (r != ERROR_UNSUPPORTED || g_path == 3) return r;
     }
   }
+  if (g_path == 4) return gemm_tc_packed(f);
   const bool tc = g_path != 2 && gemm_tc_supported(g) && (g_path == 1 || (long)m * n * k >= kTcMinWork);
   if (!tc) {
     if (g_path == 1) return ERROR_UNSUPPORTED;

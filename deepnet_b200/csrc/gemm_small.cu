@@ -504,7 +504,32 @@ long cut_up(const GemmProblem& g, SmallParams& p) {
   return tiles * p.splits;
 }
 
+// Recomputes what came out non-finite (nothing, as a rule: one read of the result).
+__global__ void __launch_bounds__(256) k_recompute_nonfinite(const __grid_constant__ SmallParams p) {
+  grid_dependents_launch();
+  grid_dependency_wait();
+  const long items = (long)p.M * p.N;
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < items; i += (long)gridDim.x * blockDim.x) {
+    const int n = (int)(i / p.M), m = (int)(i - (long)n * p.M);
+    float* const at = p.e.out + (long)n * p.e.ldo + m;
+    if (!isfinite(*at)) *at = p.e.alpha * element_fp32(p, m, n);
+  }
+}
+
 }  // namespace
+
+int recompute_nonfinite(const GemmProblem& g) {
+  SmallParams p;
+  if (g.M <= 0 || g.N <= 0 || !gather_pairs(g, p)) return ERROR_UNSUPPORTED;
+  p.M = g.M;
+  p.N = g.N;
+  p.e = g.epi;
+  long blocks = ((long)g.M * g.N + 255) / 256;
+  if (blocks > (long)sm_count() * 8) blocks = (long)sm_count() * 8;
+  if (launch_dependent(k_recompute_nonfinite, dim3((unsigned)blocks), dim3(256), 0, stream(), p) != cudaSuccess)
+    return set_error(cudaGetErrorString(cudaGetLastError()));
+  return check_launch();
+}
 
 int small_depth(const GemmProblem& g) {
   SmallParams p;

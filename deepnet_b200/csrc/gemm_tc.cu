@@ -112,10 +112,10 @@ struct TcParams {
   long split_stride;       // floats between two partials
   int direct;              // 1: no group derives anything: the copies of both CTAs complete on the leader's `ready`
                            //    barrier and the converter warps stay out of the way
-  int store16;             // 1: the epilogue's only outputs are 16-bit planes (the draw's, or the result's two): every
-                           //    thread stores them straight to global memory (64 bytes per warp and column); no
-                           //    staging, barriers or TMA stores, whose latency otherwise keeps the epilogue warps
-                           //    from draining the next tile's first chunk in time
+  int direct_store;        // 1: every thread stores its results straight to global memory: where the epilogue's only
+                           //    outputs are 16-bit planes (64 bytes per warp and column; no staging, barriers or TMA
+                           //    stores, whose latency otherwise keeps the epilogue warps from draining the next
+                           //    tile's first chunk in time), and where columns do not start on 16 bytes
   GemmEpilogue epi;
   // Column panels of a plain result delivered to other GPUs (scatter_cols > 0): columns
   // [q * scatter_cols, (q + 1) * scatter_cols) go to scatter[q] (columns ldo apart, as epi.out) with
@@ -1009,7 +1009,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_gemm_tc(const __grid_constant
           }
           uint4 w = make_uint4(0, 0, 0, 0);
           if (draw) w = philox4x32_10((uint32_t)m, cblk0 + g4, key);
-          if (p.store16) {
+          if (p.direct_store) {
             uint16_t* const ob = reinterpret_cast<uint16_t*>(e.out_aux);
             uint16_t* const sb = reinterpret_cast<uint16_t*>(e.sample_aux);
             const long lda2 = 2L * e.ld_aux;
@@ -1017,6 +1017,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_gemm_tc(const __grid_constant
             for (int j = 0; j < 4; j++) {
               if (!row_ok || c0 + j >= pN) continue;
               const long word = (long)(c0 + j) * lda2 + m;
+              if (has_out) e.out[off + (long)(4 * g4 + j) * ldo] = x[j];
               if (has_aux) {
                 uint16_t lo16, b16;
                 if (e.aux_f16) {
@@ -1028,9 +1029,10 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_gemm_tc(const __grid_constant
                 ob[word] = lo16;
                 ob[word + e.ld_aux] = b16;
               }
-              if (has_smp_aux) {
+              if (draw) {
                 const bool on = word_to_uniform(pick_word(w, j)) < x[j];
-                sb[word + e.ld_aux] = (uint16_t)(on ? aux_one : 0);
+                if (has_smp) e.sample[off + (long)(4 * g4 + j) * ldo] = on ? 1.0f : 0.0f;
+                if (has_smp_aux) sb[word + e.ld_aux] = (uint16_t)(on ? aux_one : 0);
               }
             }
             continue;
@@ -1079,7 +1081,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_gemm_tc(const __grid_constant
 #pragma unroll
         for (int i = 0; i + 16 < COLS; i++) accum[i] = accum[i + 16];
         }
-        if (leader && !p.store16) tma_store_wait_all();   // results are in memory before the kernel can end
+        if (leader && !p.direct_store) tma_store_wait_all();   // results are in memory before the kernel can end
       }
 #ifdef B200_GEMM_TIMING
       t_epi += clock64() - t_e0;
@@ -1189,10 +1191,19 @@ bool make_map(CUtensorMap* out, const void* ptr, uint64_t d0, uint64_t d1, uint6
   return true;
 }
 
-// TMA needs a 16-byte aligned base and column stride.
+// TMA needs a 16-byte aligned base and column stride, of every matrix the term reads: x itself unless the part
+// comes from the aux matrix alone, and the aux matrix.
+inline bool reads_fp32(const GemmOperand& o) { return !(part_is_16bit(o.part) && o.aux); }
+inline bool fp32_tma_ok(const GemmOperand& o) { return (o.ld % 4 == 0) && (((uintptr_t)(o.ptr + o.row0) & 15) == 0); }
 inline bool tma_ok(const GemmOperand& o) {
-  return (o.ld % 4 == 0) && (((uintptr_t)(o.ptr + o.row0) & 15) == 0) &&
+  return (!reads_fp32(o) || fp32_tma_ok(o)) &&
          (!o.aux || (o.lda % 8 == 0 && ((uintptr_t)o.aux & 15) == 0 && o.row0 % 8 == 0));
+}
+// Activation epilogues store whole column segments with TMA when every output's columns start on 16 bytes (the
+// planes of an aux matrix do, its columns being a multiple of 8 floats).
+inline bool tma_outputs_ok(const GemmEpilogue& e) {
+  return e.ldo % 4 == 0 && e.ld_aux % 8 == 0 &&
+         (((uintptr_t)e.out | (uintptr_t)e.sample | (uintptr_t)e.out_aux | (uintptr_t)e.sample_aux) & 15) == 0;
 }
 
 // Shared-memory matrix descriptor, upper 32 bits: stride byte offset (bits 32-45, in
@@ -1358,13 +1369,6 @@ bool gemm_tc_supported(const GemmProblem& g) {
   }
   const GemmEpilogue& e = g.epi;
   if ((e.sample || e.sample_aux) && (e.col0 & 3)) return false;
-  // activation epilogues store whole column segments with TMA: 16-byte aligned columns (the
-  // planes of an aux matrix are, its columns being a multiple of 8 floats)
-  const bool plain = !e.bias && e.activation == 0 && !e.sample && !e.out_aux && !e.sample_aux && e.out;
-  if (!plain) {
-    if (e.ldo % 4 != 0 || e.ld_aux % 8 != 0) return false;
-    if (((uintptr_t)e.out | (uintptr_t)e.sample | (uintptr_t)e.out_aux | (uintptr_t)e.sample_aux) & 15) return false;
-  }
   return encode_fn() != nullptr;
 }
 
@@ -1400,6 +1404,104 @@ int set_product_scatter(const float* match, float* const* out, int n, int cols) 
 }
 
 bool product_is_scattered(const float* out) { return g_scatter_n > 0 && out != nullptr && out == g_scatter_match; }
+
+// Copies of fp32 operands whose columns TMA cannot address (leading dimension not a multiple of four floats, base
+// not on 16 bytes), one launch for all of a product: columns start on 16 bytes in the copy.  Bound by memory: 8
+// bytes per element.
+constexpr int kMaxPack = 2 * kMaxGroups;
+struct PackJob {
+  const float* src;
+  float* dst;
+  int rows, cols, ld, ldp;
+  long first;              // first quad (four rows of a column) of this matrix in the launch's list
+};
+struct PackJobs {
+  PackJob job[kMaxPack];
+  int n;
+  long total;
+};
+static __global__ void __launch_bounds__(256) k_pack_operands(const __grid_constant__ PackJobs p) {
+  grid_dependents_launch();
+  grid_dependency_wait();
+  const long nth = (long)gridDim.x * blockDim.x;
+  int j = 0;
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < p.total; i += nth) {
+    while (j + 1 < p.n && i >= p.job[j + 1].first) j++;
+    const PackJob& b = p.job[j];
+    const long e = i - b.first;
+    const int quads = b.ldp >> 2;
+    const int c = (int)(e / quads), r = (int)(e - (long)c * quads) << 2;
+    const float* src = b.src + (long)c * b.ld + r;
+    float4 v;
+    v.x = src[0];
+    v.y = r + 1 < b.rows ? src[1] : 0.0f;
+    v.z = r + 2 < b.rows ? src[2] : 0.0f;
+    v.w = r + 3 < b.rows ? src[3] : 0.0f;
+    *reinterpret_cast<float4*>(b.dst + (long)c * b.ldp + r) = v;
+  }
+}
+
+// gemm_tc behind a copy of the operands that TMA cannot address.  These products ran on CUDA cores before, which
+// add in fp32 with rounding: short chunks keep the error where it was (relative, K = 4095: logistic 9.6e-7 with
+// chunks of 128, 2.2e-6 with 2048, 1.1e-6 on CUDA cores), and cost nothing here (4095 x 255, K = 4095: 87 us against
+// 2947).
+int gemm_tc_packed(const GemmProblem& g) {
+  GemmProblem f = g;
+  f.chunk_k = g.epi.activation == 1 ? 128 : 32;
+  PackJobs p;
+  p.n = 0;
+  p.total = 0;
+  for (int q = 0; q < g.npass; q++) {
+    for (int o = 0; o < 2; o++) {
+      const GemmOperand& s = o ? g.pass[q].b : g.pass[q].a;
+      if (!reads_fp32(s) || fp32_tma_ok(s)) continue;
+      if (s.row0 != 0 || g.pass[q].k <= 0) return ERROR_UNSUPPORTED;
+      const int across = o ? g.N : g.M;
+      const bool kmajor = o ? !s.trans : s.trans != 0;
+      const int rows = kmajor ? g.pass[q].k : across, cols = kmajor ? across : g.pass[q].k;
+      int at = 0;
+      while (at < p.n && p.job[at].src != s.ptr) at++;
+      if (at < p.n) {
+        if (p.job[at].rows != rows || p.job[at].cols != cols || p.job[at].ld != s.ld) return ERROR_UNSUPPORTED;
+        continue;
+      }
+      if (p.n == kMaxPack) return ERROR_UNSUPPORTED;
+      PackJob& b = p.job[p.n++];
+      b.src = s.ptr;
+      b.rows = rows;
+      b.cols = cols;
+      b.ld = s.ld;
+      b.ldp = (rows + 3) & ~3;
+      b.first = p.total;
+      p.total += (long)(b.ldp >> 2) * cols;
+    }
+  }
+  if (p.n) {
+    float* ws = (float*)workspace(4, (size_t)p.total * 16);
+    if (!ws) return CUDA_ERROR;
+    for (int j = 0; j < p.n; j++) p.job[j].dst = ws + 4 * p.job[j].first;
+    // every term over a copied matrix names the copy, also where it reads the aux matrix alone: the terms over one
+    // pair of matrices share their staged tiles
+    for (int q = 0; q < f.npass; q++)
+      for (int o = 0; o < 2; o++) {
+        GemmOperand& s = o ? f.pass[q].b : f.pass[q].a;
+        for (int j = 0; j < p.n; j++)
+          if (p.job[j].src == s.ptr) {
+            s.ptr = p.job[j].dst;
+            s.ld = p.job[j].ldp;
+            break;
+          }
+      }
+  }
+  if (!gemm_tc_supported(f)) return ERROR_UNSUPPORTED;
+  if (p.n) {
+    long blocks = (p.total + 255) / 256;
+    if (blocks > (long)sm_count() * 8) blocks = (long)sm_count() * 8;
+    if (launch_dependent(k_pack_operands, dim3((unsigned)blocks), dim3(256), 0, stream(), p) != cudaSuccess)
+      return set_error(cudaGetErrorString(cudaGetLastError()));
+  }
+  return gemm_tc(f);
+}
 
 int gemm_tc(const GemmProblem& g) {
 #ifdef B200_HOST_TIMING
@@ -1583,7 +1685,7 @@ int gemm_tc(const GemmProblem& g) {
   // at 512, 1.3e-6 at 1024, 2.9e-6 at 2048, 6e-6 at 4096; the bar is 1e-5).  Long chunks cover
   // the tile epilogue: the issuer runs two chunks ahead of the epilogue warps, which are busy for
   // 40-50 us per tile while the products of a tile take about 100 us.
-  const int ck = chunk_k >= 16 ? chunk_k : (g.epi.activation == 1 ? 2048 : 128);
+  const int ck = chunk_k >= 16 ? chunk_k : g.chunk_k > 0 ? g.chunk_k : (g.epi.activation == 1 ? 2048 : 128);
   p.chunk_iters = ck / bk < 1 ? 1 : ck / bk;
 
   // Split-K: a product whose tiles would occupy less than half of the SMs and whose inner dimension
@@ -1653,9 +1755,10 @@ int gemm_tc(const GemmProblem& g) {
     const char* sv = getenv("B200_EPI_STORE16");
     store16_mode = sv ? atoi(sv) : 1;
   }
-  p.store16 = store16_mode != 0 && !epi_is_plain(epi) && !e.out && !e.sample && (e.out_aux || e.sample_aux);
+  p.direct_store = !epi_is_plain(epi) &&
+                   (!tma_outputs_ok(e) || (store16_mode != 0 && !e.out && !e.sample && (e.out_aux || e.sample_aux)));
   for (int i = 0; i < kOutArrays; i++) p.out_map[i] = -1;
-  if (!epi_is_plain(epi)) {
+  if (!epi_is_plain(epi) && !p.direct_store) {
     // outputs of the activation epilogues, stored as boxes of 128 rows x 4 columns: M x N floats
     // with columns ldo apart, or one bfloat16 plane of an aux matrix (columns 2 ld_aux bfloat16
     // apart, plane 1 starting ld_aux bfloat16 into the column)

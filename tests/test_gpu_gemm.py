@@ -637,3 +637,45 @@ def test_one_launch_dot_keeps_infinities(cm, m, n, k):
     assert np.isposinf(got[3]).all() and np.isnan(got[7]).all() and np.isnan(got[9]).all()
     rest = np.delete(got, [3, 7, 9], axis=0)
     assert np.isfinite(rest).all()
+
+
+@pytest.mark.parametrize("ta,tb", [(0, 0), (1, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("m,n,k", [(129, 65, 33), (501, 301, 1027), (257, 259, 130)])
+def test_product_behind_aligned_copies(cm, oracle, ta, tb, m, n, k):
+    """Operands TMA cannot address through the tcgen05 kernel: copies of the operands, results stored without TMA;
+    against float64, and the draw against the oracle on the kernel's own probabilities."""
+    rng = np.random.default_rng(m + n + k)
+    A, B = (rng.standard_normal((m, k)) * 0.1).astype(np.float32), rng.standard_normal((k, n)).astype(np.float32)
+    b = rng.standard_normal((m, 1)).astype(np.float32)
+    d = lambda x: x.astype(np.float64)
+    cm.set_gemm_path(4)
+    P = cm.split_passes
+    a_, b_ = make(cm, A, ta), make(cm, B, tb)
+    out = cm.empty((m, n))
+    cm.fused_gemm(P(a_, b_, terms="tf32") + P(a_, b_, negate=1), out=out, alpha=0.5)
+    size = np.abs(d(A)) @ np.abs(d(B))
+    assert (np.abs(get(out)) <= 2.0 ** -17 * size).all()     # the difference of two forms, 2^-18 of sum |a||b| each
+    cm.CUDAMatrix.init_random(5)
+    oracle.EigenMatrix.init_random(5)
+    smp, out_aux, smp_aux = cm.empty((m, n)), cm.empty_aux((m, n)), cm.empty_aux((m, n))
+    cm.fused_gemm(P(a_, b_), out=out, sample=smp, out_aux=out_aux, sample_aux=smp_aux, bias=cm.CUDAMatrix(b), activation=1)
+    got = get(out)
+    assert relerr(got, 1 / (1 + np.exp(-(d(A) @ d(B) + b)))) < TOL
+    lo, bb = out_aux.planes()
+    np.testing.assert_array_equal(lo, bf16_round(got - tf32_trunc(got)))
+    np.testing.assert_array_equal(bb, bf16_round(got))
+    want = get(oracle.EigenMatrix(got).sample_bernoulli(target=oracle.empty((m, n))))
+    np.testing.assert_array_equal(get(smp), want)
+    np.testing.assert_array_equal(smp_aux.planes()[1], want)
+    assert cm.read_status() == 0
+
+
+def test_big_unaligned_dot_keeps_infinities(cm):
+    rng = np.random.default_rng(3)
+    m, n, k = 1501, 301, 1501     # deep enough for the tcgen05 kernel
+    A, B = rng.standard_normal((m, k)).astype(np.float32), rng.random((k, n)).astype(np.float32) + 0.5
+    want = A.astype(np.float64) @ B
+    A[3, 5], A[9, 2] = np.inf, np.nan
+    got = get(cm.dot(cm.CUDAMatrix(A), cm.CUDAMatrix(B)))
+    assert np.isposinf(got[3]).all() and np.isnan(got[9]).all()
+    assert relerr(np.delete(got, [3, 9], axis=0), np.delete(want, [3, 9], axis=0)) < TOL
