@@ -179,11 +179,15 @@ struct Stager {
   }
 };
 
-// x = hi + lo.  `round` is 0x1000: hi rounded to TF32, lo of 12 significant bits at most; or 0 for an exact operand,
-// which is read as the tensor core reads it (low 13 bits dropped).
-__device__ __forceinline__ void split_parts(float x, uint32_t round, uint32_t& hi, uint32_t& lo) {
-  hi = (__float_as_uint(x) + round) & 0xffffe000u;
-  lo = __float_as_uint(x - __uint_as_float(hi));
+// x = hi + lo, hi rounded to TF32, lo of 12 significant bits at most.  An exact operand is used as it is: the tensor
+// core drops the low 13 bits.
+template <bool kExact>
+__device__ __forceinline__ void split_parts(float x, uint32_t& hi, uint32_t& lo) {
+  hi = __float_as_uint(x);
+  if (!kExact) {
+    hi = (hi + 0x1000u) & 0xffffe000u;
+    lo = __float_as_uint(x - __uint_as_float(hi));
+  }
 }
 
 // Half a slab of one operand for a warp: x[i][c] = element of row 4g + i at k = 8t + 4 * half + c.  `tile` points
@@ -196,6 +200,40 @@ __device__ __forceinline__ void read_half(const float* tile, float (&x)[4][4]) {
     const float4 v = *reinterpret_cast<const float4*>(tile + i * (kKMajor ? SK : SM_T));
     if (kKMajor) { x[i][0] = v.x; x[i][1] = v.y; x[i][2] = v.z; x[i][3] = v.w; }
     else { x[0][i] = v.x; x[1][i] = v.y; x[2][i] = v.z; x[3][i] = v.w; }
+  }
+}
+
+// Half a slab for a warp: its 32 x 32 outputs over 16 values of K.  One instance per pair of directions and of
+// exact operands: with the directions read at run time the two ways of a fragment into its registers met in moves.
+// mma slots: rows g, g + 8 of product i = rows 4g + 2i, 4g + 2i + 1; column g of product n = column 4g + n; k slots
+// t, t + 4 = the lane's k values 2j, 2j + 1.
+template <bool kAK, bool kBK, bool kEA, bool kEB>
+__device__ __forceinline__ void half_slab(const float* ta, const float* tb, float (&part)[2][4][4]) {
+  float xa[4][4], xb[4][4];
+  read_half<kAK>(ta, xa);
+  read_half<kBK>(tb, xb);
+#pragma unroll
+  for (int j = 0; j < 2; j++) {
+    uint32_t ah[2][4], al[2][4], bh[4][2], bl[4][2];
+#pragma unroll
+    for (int n = 0; n < 4; n++)
+#pragma unroll
+      for (int c = 0; c < 2; c++) split_parts<kEB>(xb[n][2 * j + c], bh[n][c], bl[n][c]);
+#pragma unroll
+    for (int i = 0; i < 2; i++) {
+#pragma unroll
+      for (int c = 0; c < 4; c++) split_parts<kEA>(xa[2 * i + (c & 1)][2 * j + (c >> 1)], ah[i][c], al[i][c]);
+      if (!kEA) {
+#pragma unroll
+        for (int n = 0; n < 4; n++) mma_tf32_16x8x8(part[i][n], al[i], bh[n]);
+      }
+      if (!kEB) {
+#pragma unroll
+        for (int n = 0; n < 4; n++) mma_tf32_16x8x8(part[i][n], ah[i], bl[n]);
+      }
+#pragma unroll
+      for (int n = 0; n < 4; n++) mma_tf32_16x8x8(part[i][n], ah[i], bh[n]);
+    }
   }
 }
 
@@ -254,7 +292,7 @@ __global__ void __launch_bounds__(kSmallThreads, 2) k_gemm_small(const __grid_co
   const int g = (threadIdx.x & 31) >> 2, t = threadIdx.x & 3;
   int offa = 0, offb = 0;       // where the lane's fragments start in a tile
   int q = -1, qnext = first;
-  bool ak = false, bk = false, ea = false, eb = false;
+  int form = 0;                 // directions and exact operands of the pair
   float sign = 1.0f;
 #pragma unroll 1
   for (int s = first; s < last; s++) {
@@ -267,50 +305,21 @@ __global__ void __launch_bounds__(kSmallThreads, 2) k_gemm_small(const __grid_co
         qnext = q + 1 < p.npairs ? p.pair[q + 1].slab0 : p.slabs;
       } while (s >= qnext);
       const SmallPair& pr = p.pair[q];
-      ak = pr.a.kmajor;
-      bk = pr.b.kmajor;
-      ea = pr.a.exact;
-      eb = pr.b.exact;
+      const bool ak = pr.a.kmajor, bk = pr.b.kmajor;
+      form = (ak ? 8 : 0) + (bk ? 4 : 0) + (pr.a.exact ? 2 : 0) + (pr.b.exact ? 1 : 0);
       sign = pr.negate ? -1.0f : 1.0f;
       offa = ak ? at_k(wm + 4 * g, 8 * t + 4 * half) : at_m(8 * t + 4 * half, wm + 4 * g);
       offb = kTileFloats + (bk ? at_k(wn + 4 * g, 8 * t + 4 * half) : at_m(8 * t + 4 * half, wn + 4 * g));
     }
     const float* sa = smem + (size_t)((s - first) % kStages) * (2 * kTileFloats);
-    const uint32_t ra = ea ? 0u : 0x1000u, rb = eb ? 0u : 0x1000u;
-    float xa[4][4], xb[4][4];
-    if (ak) read_half<true>(sa + offa, xa);
-    else read_half<false>(sa + offa, xa);
-    if (bk) read_half<true>(sa + offb, xb);
-    else read_half<false>(sa + offb, xb);
-#pragma unroll
-    for (int j = 0; j < 2; j++) {
-      // mma slots: rows g, g + 8 of product i = rows 4g + 2i, 4g + 2i + 1; column g of product n = column 4g + n;
-      // k slots t, t + 4 = the lane's k values 2j, 2j + 1
-      uint32_t ah[2][4], al[2][4], bh[4][2], bl[4][2];
-#pragma unroll
-      for (int i = 0; i < 2; i++)
-#pragma unroll
-        for (int c = 0; c < 4; c++) split_parts(xa[2 * i + (c & 1)][2 * j + (c >> 1)], ra, ah[i][c], al[i][c]);
-#pragma unroll
-      for (int n = 0; n < 4; n++)
-#pragma unroll
-        for (int c = 0; c < 2; c++) split_parts(xb[n][2 * j + c], rb, bh[n][c], bl[n][c]);
-      if (!ea) {
-#pragma unroll
-        for (int i = 0; i < 2; i++)
-#pragma unroll
-          for (int n = 0; n < 4; n++) mma_tf32_16x8x8(part[i][n], al[i], bh[n]);
-      }
-      if (!eb) {
-#pragma unroll
-        for (int i = 0; i < 2; i++)
-#pragma unroll
-          for (int n = 0; n < 4; n++) mma_tf32_16x8x8(part[i][n], ah[i], bl[n]);
-      }
-#pragma unroll
-      for (int i = 0; i < 2; i++)
-#pragma unroll
-        for (int n = 0; n < 4; n++) mma_tf32_16x8x8(part[i][n], ah[i], bh[n]);
+    const float *ta = sa + offa, *tb = sa + offb;
+    switch (form) {
+#define B200_HALF_SLAB(F) case F: half_slab<((F) & 8) != 0, ((F) & 4) != 0, ((F) & 2) != 0, ((F) & 1) != 0>(ta, tb, part); break;
+      B200_HALF_SLAB(0) B200_HALF_SLAB(1) B200_HALF_SLAB(2) B200_HALF_SLAB(3)
+      B200_HALF_SLAB(4) B200_HALF_SLAB(5) B200_HALF_SLAB(6) B200_HALF_SLAB(7)
+      B200_HALF_SLAB(8) B200_HALF_SLAB(9) B200_HALF_SLAB(10) B200_HALF_SLAB(11)
+      B200_HALF_SLAB(12) B200_HALF_SLAB(13) B200_HALF_SLAB(14) B200_HALF_SLAB(15)
+#undef B200_HALF_SLAB
     }
     // into the running sum after two slabs, and where the sign may change or the share ends
     if (((s - first) & 1) || s + 1 == last || s + 1 == qnext) {
