@@ -12,8 +12,8 @@ probabilities, deepnet/ais.py:158), not the sample.  `exact_log_z` is deepnet/ai
 (`ExactZ_binary_binary`): the sum over all 2^V visible configurations with the hidden units
 summed out analytically.
 
-On b200mat the two products of a step go through `fused_gemm` (bias and the schedule factor in
-the epilogue); `fused=False` keeps the reference's call-by-call form, which the CPU restatement
+On b200mat a step of the binary RBM is two fused products (bias, schedule factor, logistic and draw in the
+epilogue) around one kernel for the importance weights and the hidden draw; `fused=False` keeps the reference's call-by-call form, which the CPU restatement
 runs too.  Both forms consume the random stream identically (two sampling calls per step).
 """
 import numpy as np
@@ -46,14 +46,13 @@ def ais_binary_rbm(cm, weight, hidden_bias, visible_bias, num_chains, schedule, 
     v_state.sample_bernoulli(target=v_sample)
     w_ais = cm.CUDAMatrix(np.zeros((1, B), np.float32))
     w_aux = w.split_bf16(cm.empty_aux((V, H))) if fused else None
-    for i in range(1, len(schedule)):
+    if fused:   # all steps from C: two products and one kernel each
+        cm.ais_binary_steps(w, w_aux, a, b, v_state, v_sample, h_state, h_sample, w_ais, schedule)
+    for i in range(1, 0 if fused else len(schedule)):
         s_prev, s = float(schedule[i - 1]), float(schedule[i])
         # hidden pre-activation W'v + a (deepnet/ais.py:153-154)
-        if fused:
-            cm.fused_gemm(cm.split_passes(w.T, v_sample, exact_b=True, a_aux=w_aux), out=h_state, bias=a)
-        else:
-            cm.dot(w.T, v_sample, target=h_state)
-            h_state.add_col_vec(a)
+        cm.dot(w.T, v_sample, target=h_state)
+        h_state.add_col_vec(a)
         # importance weight (deepnet/ais.py:156-162)
         h_state.mult(s_prev, target=h_temp)
         h_state.mult(s)
@@ -65,11 +64,8 @@ def ais_binary_rbm(cm, weight, hidden_bias, visible_bias, num_chains, schedule, 
         # Gibbs sweep at inverse temperature s (deepnet/ais.py:164-170)
         cm.sigmoid(h_state)
         h_state.sample_bernoulli(target=h_sample)
-        if fused:
-            cm.fused_gemm(cm.split_passes(w, h_sample, exact_b=True, a_aux=w_aux), out=v_state, bias=b)
-        else:
-            cm.dot(w, h_sample, target=v_state)
-            v_state.add_col_vec(b)
+        cm.dot(w, h_sample, target=v_state)
+        v_state.add_col_vec(b)
         v_state.mult(s)
         cm.sigmoid(v_state)
         v_state.sample_bernoulli(target=v_sample)

@@ -616,3 +616,108 @@ int momentum_update(cudamat* w, cudamat* delta, cudamat* grad, cudamat* suff, cu
 }
 
 }  // extern "C"
+
+namespace {
+
+__device__ __forceinline__ float log_1_plus_exp(float x) { return x > 0 ? x + log1pf(expf(-x)) : log1pf(expf(x)); }
+
+// What an annealing step does between its two products (deepnet/ais.py:156-166), one block per chain: with x the
+// hidden pre-activations W'v + a,
+//   w += sum_j [log(1 + exp(s x_j)) - log(1 + exp(s0 x_j))] + ds b'v,   h ~ Bernoulli(sigmoid(s x))
+// and, by the first block, the visible bias of the next product, s b.  Nine calls of the matrix API otherwise.
+// Latency bound (500 x 100: 200 KB).
+__global__ void __launch_bounds__(256) k_ais_hidden(const float* x, const float* b, const float* v, float* w, float* h,
+                                                    float* sb, int H, int V, int col0, float s0, float s, float ds,
+                                                    PhiloxKey key) {
+  __shared__ float red[2][8];
+  grid_dependents_launch();
+  grid_dependency_wait();
+  const int c = blockIdx.x, gc = c + col0;
+  float gain = 0.0f, bv = 0.0f;
+  for (int j = threadIdx.x; j < H; j += 256) {
+    const float t = x[(long)c * H + j], ts = t * s;
+    gain += log_1_plus_exp(ts) - log_1_plus_exp(t * s0);
+    const uint4 r = philox4x32_10((uint32_t)j, (uint32_t)(gc >> 2), key);
+    h[(long)c * H + j] = word_to_uniform(pick_word(r, gc & 3)) < sigmoid_accurate(ts) ? 1.0f : 0.0f;
+  }
+  for (int i = threadIdx.x; i < V; i += 256) {
+    bv = fmaf(b[i], v[(long)c * V + i], bv);
+    if (c == 0) sb[i] = s * b[i];
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    gain += __shfl_xor_sync(0xffffffffu, gain, o);
+    bv += __shfl_xor_sync(0xffffffffu, bv, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    red[0][threadIdx.x >> 5] = gain;
+    red[1][threadIdx.x >> 5] = bv;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    for (int i = 1; i < 8; i++) {
+      gain += red[0][i];
+      bv += red[1][i];
+    }
+    w[c] = (w[c] + gain) + ds * bv;
+  }
+}
+
+}  // namespace
+
+// The annealing steps 1 .. n - 1 of `schedule` for a binary RBM (deepnet/ais.py:152-170), three launches a step, issued
+// from here: w V x H (w_aux its bfloat16 parts), a H x 1, b V x 1, v_state / v_sample V x B, h_pre / h_sample H x B,
+// sb V x 1 scratch, weights 1 x B (added to).  Two sampling calls a step, in the order of the reference's calls.
+extern "C" int ais_binary_steps(rnd_struct* rnd_state, cudamat* w, cudamat* w_aux, cudamat* a, cudamat* b, cudamat* v_state,
+                                cudamat* v_sample, cudamat* h_pre, cudamat* h_sample, cudamat* sb, cudamat* weights,
+                                const double* schedule, int n) {
+  if (!rnd_state || !schedule) return ERROR_GENERIC;
+  cudamat* all[10] = {w, w_aux, a, b, v_state, v_sample, h_pre, h_sample, sb, weights};
+  for (int i = 0; i < 10; i++) {
+    if (!all[i]->on_device) return ERROR_NOT_ON_DEVICE;
+    if (all[i]->is_trans) return ERROR_TRANSPOSED;
+  }
+  const int V = w->size[0], H = w->size[1], B = v_state->size[1];
+  if (!aux_shape_ok(w_aux, w) || numel(a) != H || numel(b) != V || numel(sb) != V || numel(weights) != B ||
+      v_state->size[0] != V || !same_shape(v_state, v_sample) || h_pre->size[0] != H || h_pre->size[1] != B ||
+      !same_shape(h_pre, h_sample))
+    return ERROR_INCOMPATIBLE_DIMENSIONS;
+  if ((long)V * H * B == 0) return 0;
+  cudamat wt = *w;
+  wt.is_trans = 1;
+  b200_fused_gemm up = {}, down = {};
+  // the samples are exact: lo16(w) . b16(x) and w . x
+  auto product = [](b200_fused_gemm& f, cudamat* m, cudamat* aux, cudamat* x) {
+    f.npass = 2;
+    f.alpha = 1.0f;
+    for (int q = 0; q < 2; q++) {
+      f.pass[q].a = m;
+      f.pass[q].b = x;
+      f.pass[q].a_aux = aux;
+      f.pass[q].a_part = q ? kPartX : kPartLo16;
+      f.pass[q].b_part = q ? kPartX : kPartB16;
+    }
+  };
+  product(up, &wt, w_aux, v_sample);
+  up.bias = a;
+  up.out = h_pre;
+  product(down, w, w_aux, h_sample);
+  down.bias = sb;
+  down.activation = 1;
+  down.out = v_state;
+  down.sample = v_sample;
+  for (int i = 1; i < n; i++) {
+    int err = fused_gemm(rnd_state, &up);
+    if (err) return err;
+    const float s0 = (float)schedule[i - 1], s = (float)schedule[i];
+    const PhiloxKey key = make_philox_key(rnd_state->seed, rnd_state->calls++);
+    if (launch_dependent(k_ais_hidden, dim3((unsigned)B), dim3(256), 0, stream(), h_pre->data_device, b->data_device,
+                         v_state->data_device, weights->data_device, h_sample->data_device, sb->data_device, H, V, rng_col0(),
+                         s0, s, (float)(schedule[i] - schedule[i - 1]), key) != cudaSuccess)
+      return set_error(cudaGetErrorString(cudaGetLastError()));
+    down.alpha = s;
+    err = fused_gemm(rnd_state, &down);
+    if (err) return err;
+  }
+  return check_launch();
+}

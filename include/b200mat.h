@@ -312,6 +312,11 @@ int b200_sm_count(void);                  /* SMs in force (the device's, or the 
  * its copies deliver, so one of its bounded waits must run out (status word set, kernel returns).
  * No counterpart in the reference. */
 int b200_test_inject_stage_bytes(int extra_bytes);
+/* All steps of an annealing schedule (n inverse temperatures) of a binary RBM's partition function estimate
+ * (deepnet/ais.py:152-170): w V x H and its aux, biases a (H) and b (V), chain states, sb (V) scratch, weights 1 x B added to. */
+int ais_binary_steps(rnd_struct* rnd_state, cudamat* w, cudamat* w_aux, cudamat* a, cudamat* b, cudamat* v_state,
+                     cudamat* v_sample, cudamat* h_pre, cudamat* h_sample, cudamat* sb, cudamat* weights,
+                     const double* schedule, int n);
 int b200_set_gemm_path(int path);         /* 0 auto, 1 tcgen05 kernel only, 2 CUDA cores only, 3 one-launch kernel only */
 int b200_set_dot_precision(int mode);     /* 0 fp32-grade split TF32 (default), 1 one TF32 pass */
 /* Split-K of the tensor-core product: 0 (default) = cut the inner dimension into work items when the
