@@ -1154,6 +1154,26 @@ class Event(object):
             pass
 
 
+def ais_binary_steps(w, w_aux, a, b, v_state, v_sample, h_pre, h_sample, weights, schedule):
+    """Every step of the annealing schedule for a binary RBM (see `ais.ais_binary_rbm`), issued from C."""
+    steps = np.ascontiguousarray(schedule, np.float64).reshape(-1)
+    scaled_bias = empty(b.shape)
+    _check(_lib.ais_binary_steps(CUDAMatrix.rnd_state_p, w.p_mat, w_aux.p_mat, a.p_mat, b.p_mat, v_state.p_mat,
+                                 v_sample.p_mat, h_pre.p_mat, h_sample.p_mat, scaled_bias.p_mat, weights.p_mat,
+                                 steps.ctypes.data_as(ct.POINTER(ct.c_double)), ct.c_int(len(steps))))
+
+
+def copy_to_rows(mat, rows):
+    """The matrix as (columns x rows) into `rows`, a C-contiguous float32 host array of that shape: the memory of a
+    column-major matrix is that of its transpose row by row, so nothing is rearranged or copied twice."""
+    if rows.dtype != np.float32 or not rows.flags.c_contiguous or rows.shape != (mat.mat.size[1], mat.mat.size[0]):
+        raise CUDAMatException("copy_to_rows needs a C-contiguous float32 array of the transposed shape")
+    view = cudamat()
+    ct.memmove(ct.byref(view), ct.byref(mat.mat), ct.sizeof(view))
+    view.data_host = rows.ctypes.data_as(ct.POINTER(ct.c_float))
+    _check(_lib.copy_to_host(ct.byref(view)))
+
+
 def host_alloc(shape):
     """Returns (array, ptr): a pinned float32 Fortran-order host array; free with host_free(ptr)."""
     n = int(np.prod(shape))

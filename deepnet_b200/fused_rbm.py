@@ -459,7 +459,7 @@ class FusedRBM(LossReadback):
         cm, B, W, P = self.cm, self.B, self.W, self.cm.split_passes
         Wa = None if self.f16 else self.W_aux     # the bfloat16 parts exist only in that form of the aux
         n = data.shape[1] // B
-        rep = np.zeros((n * B, self.H), np.float32)
+        rep = np.empty((n * B, self.H), np.float32)
         err = 0.0
         soft = self.visible == REPLICATED_SOFTMAX
         for b in range(n):
@@ -479,7 +479,7 @@ class FusedRBM(LossReadback):
                 else:
                     cm.fused_gemm(down, out=self.v_neg, bias=self.bv, activation=self._act(self.visible))
                     cm._check(cm._lib.add_sq_diff(self.v_neg.p_mat, v0.p_mat, self.loss_acc.p_mat))
-            rep[b * B:(b + 1) * B, :] = np.array(self.h_pos.asarray()).T
+            cm.copy_to_rows(self.h_pos, rep[b * B:(b + 1) * B])
         if input_recon:
             err = self.read_loss()
             return rep, err
