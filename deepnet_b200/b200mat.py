@@ -805,7 +805,7 @@ def _build_fused_gemm(passes, out=None, sample=None, bias=None, col_scale=None, 
 (OP_FUSED_GEMM, OP_SUM_AXIS, OP_ADD_SUM_AXIS, OP_ROW_SUM_DIFF, OP_ADD_SQ_DIFF, OP_MOMENTUM_UPDATE, OP_SPLIT_F16,
  OP_SPLIT_BF16, OP_ALLREDUCE, OP_SOFTMAX_SCALED, OP_SAMPLE_MULTINOMIAL, OP_DIV_BY_ROW, OP_ADD_SCALAR, OP_ASSIGN_SCALAR,
  OP_COPY, OP_SAMPLE_BERNOULLI, OP_SOFTMAX_SAMPLE, OP_MOMENTUM_UPDATE_COLUMNS, OP_ALLREDUCE_BEGIN, OP_ALLREDUCE_END,
- OP_SM_LIMIT, OP_DP_PEER_UPDATE) = range(22)
+ OP_SM_LIMIT, OP_DP_PEER_UPDATE, OP_RBM_BIAS_UPDATE) = range(23)
 
 
 class _Op(ct.Structure):
@@ -840,6 +840,11 @@ class Immediate(object):
 
     def momentum_update(self, w, delta, grad, suff, inv_batch, momentum, eps, l2=0.0, l1=0.0, w_aux=None, w_scale=None):
         w.momentum_update(delta, grad, suff, inv_batch, momentum, eps, l2=l2, l1=l1, w_aux=w_aux, w_scale=w_scale)
+
+    def rbm_bias_update(self, v_pos, v_neg, h_pos, h_neg, suff, b, db, sq_acc, inv_batch, momentum, eps):
+        _check(_lib.rbm_bias_update(v_pos.p_mat, v_neg.p_mat, h_pos.p_mat, h_neg.p_mat, suff.p_mat, b.p_mat, db.p_mat,
+                                    sq_acc.p_mat if sq_acc is not None else None, ct.c_float(inv_batch),
+                                    ct.c_float(momentum), ct.c_float(eps)))
 
     def momentum_update_columns(self, w, delta, grad, suff, col0, ncols, inv_batch, momentum, eps, l2=0.0, l1=0.0,
                                 w_aux=None, w_scale=None):
@@ -943,6 +948,9 @@ class Program(object):
 
     def momentum_update(self, w, delta, grad, suff, inv_batch, momentum, eps, l2=0.0, l1=0.0, w_aux=None, w_scale=None):
         return self._add(OP_MOMENTUM_UPDATE, (w, delta, grad, suff, w_aux, w_scale), (), (inv_batch, momentum, eps, l2, l1))
+
+    def rbm_bias_update(self, v_pos, v_neg, h_pos, h_neg, suff, b, db, sq_acc, inv_batch, momentum, eps):
+        return self._add(OP_RBM_BIAS_UPDATE, (v_pos, v_neg, h_pos, h_neg, suff, b, db, sq_acc), (), (inv_batch, momentum, eps))
 
     def momentum_update_columns(self, w, delta, grad, suff, col0, ncols, inv_batch, momentum, eps, l2=0.0, l1=0.0,
                                 w_aux=None, w_scale=None):

@@ -26,6 +26,8 @@ int dp_allreduce_end(int slot);
 int b200_set_sm_limit(int sms);
 int dp_peer_update(cudamat* w, cudamat* delta, cudamat* w_aux, cudamat* w_scale, cudamat* pack, cudamat* b, cudamat* db,
                    float inv_batch, float mom_b, float eps_b, float mom_w, float eps_w, float l2, float l1);
+int rbm_bias_update(cudamat* v_pos, cudamat* v_neg, cudamat* h_pos, cudamat* h_neg, cudamat* suff, cudamat* b, cudamat* db,
+                    cudamat* sq_acc, float inv_batch, float momentum, float eps);
 int split_f16(cudamat* x, cudamat* aux, cudamat* exp_dev, int exp_const);
 int split_bf16(cudamat* x, cudamat* aux);
 int dp_allreduce(cudamat* mat);
@@ -62,6 +64,7 @@ enum {
   B200_OP_ALLREDUCE_END = 19,     // i0 slot
   B200_OP_SM_LIMIT = 20,          // i0 SMs the following kernels size their grids for (0 = all)
   B200_OP_DP_PEER_UPDATE = 21,    // m0 w, m1 delta, m2 w_aux?, m3 w_scale?, m4 pack, m5 b, m6 db; f0 inv_batch, f1 mom_b, f2 eps_b, f3 mom_w, f4 eps_w, f5 l2, f6 l1
+  B200_OP_RBM_BIAS_UPDATE = 22,   // m0 v_pos, m1 v_neg, m2 h_pos, m3 h_neg, m4 suff, m5 b, m6 db, m7 sq_acc?; f0 inv_batch, f1 momentum, f2 eps
   B200_OP_COUNT
 };
 
@@ -107,6 +110,9 @@ extern "C" int b200_run_program(rnd_struct* rnd_state, b200_op* ops, int n, int*
       case B200_OP_SM_LIMIT: err = b200_set_sm_limit(o.i0); break;
       case B200_OP_DP_PEER_UPDATE:
         err = dp_peer_update(o.m[0], o.m[1], o.m[2], o.m[3], o.m[4], o.m[5], o.m[6], o.f0, o.f1, o.f2, o.f3, o.f4, o.f5, o.f6);
+        break;
+      case B200_OP_RBM_BIAS_UPDATE:
+        err = rbm_bias_update(o.m[0], o.m[1], o.m[2], o.m[3], o.m[4], o.m[5], o.m[6], o.m[7], o.f0, o.f1, o.f2);
         break;
       default: break;
     }

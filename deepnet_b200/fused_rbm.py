@@ -246,10 +246,18 @@ class FusedRBM(LossReadback):
                 prog.set_floats(op, f0=sc["inv_b"], f1=emom, f2=eeps, f3=l2, f4=l1)
         prog.run()
 
-    def _issue_updates(self, X, sc, wb, w_scale=None):
+    def _issue_updates(self, X, sc, wb, w_scale=None, bias=None):
         """All-reduce of the packed statistics, then the two updates (biases are not regularised,
-        deepnet/dbm.py:249).  Returns the operations whose scalars follow the schedules."""
+        deepnet/dbm.py:249).  Returns the operations whose scalars follow the schedules.  bias (one rank): (v_pos, v_neg,
+        loss accumulator or None), the visible states whose row sums are still to be taken: bias
+        statistics, bias update and error are then one operation."""
         V, H = self.V, self.H
+        if bias is not None:
+            ub = self._op(X, "bias_tail", 0, 8.0 * (V + H) * self.B, "rbm_bias_update", bias[0], bias[1], self.h_pos, self.h_neg,
+                          self.suff_b, self.b, self.db, bias[2], sc["inv_b"], sc["mom"], sc["eps"])
+            uw = self._op(X, "update_W", 0, 6 * wb, "momentum_update", self.W, self.dW, None, self.suff_W, sc["inv_b"],
+                          sc["emom"], sc["eeps"], l2=sc["l2"], l1=sc["l1"], w_aux=self.W_aux, w_scale=w_scale)
+            return ub, uw
         if self.dp_peer:
             # exchange + update of every parameter in one pass over peer memory (no NCCL)
             u = self._op(X, "peer_update", 0, 6 * wb, "dp_peer_update", self.W, self.dW, self.W_aux, w_scale, self.pack,
@@ -277,6 +285,7 @@ class FusedRBM(LossReadback):
         if sa and self._given_aux is None:
             self._op(X, "split", 0, 2 * vb, "split_bf16", v0, v0a)
         h_samp_aux, v_neg_aux = (self.h_samp_aux, self.v_neg_aux) if sa else (None, None)
+        tail = self.world_size == 1 and not self.dp_peer     # statistics stay here: biases in one operation
         # positive phase: h0 = sigmoid(W' v0 + b_h), and its Bernoulli sample
         self._op(X, "gemm_up", gf, 2.5 * hb, "fused_gemm",
                  P(W.T, v0, exact_b=exact, a_aux=Wa, b_aux=v0a if sa else None),
@@ -289,7 +298,7 @@ class FusedRBM(LossReadback):
                      out_aux=None if draw_v else v_neg_aux, sample=self.v_samp if draw_v else None,
                      sample_aux=self.v_samp_aux if (draw_v and sa) else None, bias=self.bv,
                      activation=self._act(self.visible))
-            if i == 0:
+            if i == 0 and not (tail and k == 1):   # (after a single step the tail reads the same states)
                 self._op(X, "sq_err", 0, 2 * vb, "sq_diff", self.v_neg, v0, self.loss_acc)
             # the hidden means are only read after the last step (statistics); before that the draw suffices
             up = (P(W.T, self.v_samp, exact_b=True, a_aux=Wa, b_aux=self.v_samp_aux if sa else None) if draw_v
@@ -302,6 +311,8 @@ class FusedRBM(LossReadback):
         pos = P(v0, self.h_pos.T, exact_a=exact, terms="tf32")
         neg = P(self.v_neg, self.h_neg.T, negate=1, terms="tf32")
         self._op(X, "gemm_stats", 2 * gf, wb, "fused_gemm", pos + neg, out=self.suff_W)
+        if tail:
+            return self._issue_updates(X, sc, wb, bias=(v0, self.v_neg, self.loss_acc if k == 1 else None))
         self._op(X, "row_sum", 0, 2 * vb, "row_sum_diff", v0, self.v_neg, self.suff_bv)
         self._op(X, "row_sum", 0, 2 * hb, "row_sum_diff", self.h_pos, self.h_neg, self.suff_bh)
         return self._issue_updates(X, sc, wb)
@@ -437,6 +448,8 @@ class FusedRBM(LossReadback):
         pos = P(self.v0n, self.h_pos.T, terms="tf32")
         neg = P(self.v_negn, self.h_neg.T, negate=1, terms="tf32")
         self._op(X, "gemm_stats", 2 * gf, wb, "fused_gemm", pos + neg, out=self.suff_W)
+        if self.world_size == 1 and not self.dp_peer:
+            return self._issue_updates(X, sc, wb, bias=(self.v0n, self.v_negn, None))
         self._op(X, "row_sum", 0, 2 * vb, "row_sum_diff", self.v0n, self.v_negn, self.suff_bv)
         self._op(X, "row_sum", 0, 2 * hb, "row_sum_diff", self.h_pos, self.h_neg, self.suff_bh)
         return self._issue_updates(X, sc, wb)

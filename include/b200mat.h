@@ -317,6 +317,10 @@ int b200_test_inject_stage_bytes(int extra_bytes);
 int ais_binary_steps(rnd_struct* rnd_state, cudamat* w, cudamat* w_aux, cudamat* a, cudamat* b, cudamat* v_state,
                      cudamat* v_sample, cudamat* h_pre, cudamat* h_sample, cudamat* sb, cudamat* weights,
                      const double* schedule, int n);
+/* Bias statistics, bias update and (sq_acc, optional) squared reconstruction error of an RBM with packed biases
+ * [visible | hidden] in one launch (deepnet/layer.py:202-213, parameter.py:80-106, logistic_layer.py:48-52). */
+int rbm_bias_update(cudamat* v_pos, cudamat* v_neg, cudamat* h_pos, cudamat* h_neg, cudamat* suff, cudamat* b, cudamat* db,
+                    cudamat* sq_acc, float inv_batch, float momentum, float eps);
 int b200_set_gemm_path(int path);         /* 0 auto, 1 tcgen05 kernel only, 2 CUDA cores only, 3 one-launch kernel only */
 int b200_set_dot_precision(int mode);     /* 0 fp32-grade split TF32 (default), 1 one TF32 pass */
 /* Split-K of the tensor-core product: 0 (default) = cut the inner dimension into work items when the
@@ -384,7 +388,7 @@ int dp_wait(int timeout_ms);
  * 5 momentum_update, 6 split_f16, 7 split_bf16, 8 dp_allreduce, 9 softmax_scaled, 10 sample_multinomial,
  * 11 div_by_row_vec, 12 add_scalar, 13 assign_scalar, 14 copy_on_device, 15 sample_bernoulli,
  * 16 softmax_sample, 17 momentum_update_columns, 18 dp_allreduce_begin, 19 dp_allreduce_end,
- * 20 b200_set_sm_limit, 21 dp_peer_update); m[], i0.., f0.. are its arguments in declaration order (matrices, then integers,
+ * 20 b200_set_sm_limit, 21 dp_peer_update, 22 rbm_bias_update); m[], i0.., f0.. are its arguments in declaration order (matrices, then integers,
  * then floats; gemm for kind 0).  Stops at the first failure: returns its code, *failed_at its index. */
 struct b200_fused_gemm;
 typedef struct b200_op {

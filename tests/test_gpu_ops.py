@@ -272,3 +272,27 @@ def test_single_launch_statistics_after_a_shutdown(cm):
         assert abs(float(get(acc)[0, 0]) - sq) < 1e-5 * sq
         cm.cublas_shutdown()
         cm.cublas_init()
+
+
+@pytest.mark.parametrize("with_error", [True, False])
+@pytest.mark.parametrize("V,H,B", [(1, 1, 1), (33, 31, 7), (784, 500, 100), (65, 200, 1024), (40, 33, 1025)])
+def test_bias_tail_matches_the_separate_operations(cm, with_error, V, H, B):
+    """Row sums of pos - neg (bound: one rounding of 2^-24 per addition, of sum |pos - neg|), the bias update bit for bit on
+    those sums, the squared error (each square rounded once, sums of up to four in fp32: 2^-22), twice in a row."""
+    rng = np.random.default_rng(V + H + B)
+    mats = [rng.random((n, B)).astype(np.float32) for n in (V, V, H, H)]
+    dev = [cm.CUDAMatrix(m) for m in mats]
+    b, db = (rng.standard_normal((V + H, 1)).astype(np.float32) for _ in range(2))
+    gb, gdb, suff, acc = cm.CUDAMatrix(b), cm.CUDAMatrix(db), cm.empty((V + H, 1)), cm.empty((1, 1))
+    wb, wdb = cm.CUDAMatrix(b), cm.CUDAMatrix(db)
+    d = [m.astype(np.float64) for m in mats]
+    diff = np.concatenate([d[0] - d[1], d[2] - d[3]])
+    for turn in range(1, 3):
+        cm.Immediate().rbm_bias_update(*dev, suff, gb, gdb, acc if with_error else None, 1.0 / B, 0.9, 0.1)
+        s = get(suff)
+        assert (np.abs(s[:, 0] - diff.sum(1)) <= (B + 2) * 2.0 ** -24 * np.abs(diff).sum(1) + 1e-30).all()
+        wb.momentum_update(wdb, None, cm.CUDAMatrix(s), 1.0 / B, 0.9, 0.1)
+        np.testing.assert_array_equal(get(gb), get(wb))
+        np.testing.assert_array_equal(get(gdb), get(wdb))
+        want = turn * ((d[0] - d[1]) ** 2).sum() if with_error else 0.0
+        assert abs(get(acc)[0, 0] - want) <= 2.0 ** -21 * want
