@@ -85,6 +85,8 @@ __device__ __forceinline__ void block_argmax(float& v, int& i, float* sv, int* s
 __global__ void __launch_bounds__(256) k_colsum(const float* __restrict__ m, float* __restrict__ t, int h, int w,
                                                 float mult, float beta) {
   __shared__ float smem[32];
+  grid_dependents_launch();
+  grid_dependency_wait();
   for (int c = blockIdx.x; c < w; c += gridDim.x) {
     const float* col = m + (long)c * h;
     float s = 0;
@@ -110,6 +112,8 @@ __global__ void __launch_bounds__(32 * kRowLanes) k_rowsum(const float* __restri
                                                            int h, int w, int cols_per_split, float mult, float beta,
                                                            bool final_pass) {
   __shared__ float smem[kRowLanes][33];
+  grid_dependents_launch();
+  grid_dependency_wait();
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int r = blockIdx.x * 32 + tx;
   const int c0 = blockIdx.y * cols_per_split;
@@ -143,6 +147,8 @@ __global__ void __launch_bounds__(32 * kRowLanes) k_rowsum4(const float* __restr
                                                             int h, int w, int cols_per_split, float mult, float beta,
                                                             bool final_pass) {
   __shared__ float4 smem[kRowLanes][33];
+  grid_dependents_launch();
+  grid_dependency_wait();
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int r = (blockIdx.x * 32 + tx) * 4;
   const int c0 = blockIdx.y * cols_per_split;
@@ -189,6 +195,8 @@ __global__ void __launch_bounds__(32 * kRowLanes) k_rowsum4(const float* __restr
 }
 __global__ void __launch_bounds__(256) k_rowsum_finish(const float* __restrict__ part, float* __restrict__ t, int h,
                                                        int splits, float mult, float beta) {
+  grid_dependents_launch();
+  grid_dependency_wait();
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
   if (r >= h) return;
   float tot = 0;
@@ -353,7 +361,7 @@ int launch_axis_sum(const float* m, int h, int w, int axis, float* t, float mult
   if ((long)h * w == 0) return 0;
   if (axis == 0) {
     int blocks = w < sm_count() * 8 ? w : sm_count() * 8;
-    k_colsum<<<blocks, 256, 0, stream()>>>(m, t, h, w, mult, beta);
+    (void)launch_dependent(k_colsum, dim3((unsigned)blocks), dim3(256), 0, stream(), m, t, h, w, mult, beta);
     return check_launch();
   }
   const bool vec4 = (h % 4 == 0) && (((uintptr_t)m | (uintptr_t)t) & 15) == 0;
@@ -373,12 +381,13 @@ int launch_axis_sum(const float* m, int h, int w, int axis, float* t, float mult
   }
   const bool final_pass = splits == 1;
   if (vec4)
-    k_rowsum4<<<dim3(bx, splits), 32 * kRowLanes, 0, stream()>>>(m, dst, h, w, cps, final_pass ? mult : 1.0f,
-                                                                final_pass ? beta : 0.0f, final_pass);
+    (void)launch_dependent(k_rowsum4, dim3(bx, splits), dim3(32 * kRowLanes), 0, stream(), m, dst, h, w, cps,
+                           final_pass ? mult : 1.0f, final_pass ? beta : 0.0f, final_pass);
   else
-    k_rowsum<<<dim3(bx, splits), 32 * kRowLanes, 0, stream()>>>(m, dst, h, w, cps, final_pass ? mult : 1.0f,
-                                                               final_pass ? beta : 0.0f, final_pass);
-  if (!final_pass) k_rowsum_finish<<<(h + 255) / 256, 256, 0, stream()>>>(dst, t, h, splits, mult, beta);
+    (void)launch_dependent(k_rowsum, dim3(bx, splits), dim3(32 * kRowLanes), 0, stream(), m, dst, h, w, cps,
+                           final_pass ? mult : 1.0f, final_pass ? beta : 0.0f, final_pass);
+  if (!final_pass)
+    (void)launch_dependent(k_rowsum_finish, dim3((h + 255) / 256), dim3(256), 0, stream(), dst, t, h, splits, mult, beta);
   return check_launch();
 }
 
