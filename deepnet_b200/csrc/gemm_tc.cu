@@ -1323,7 +1323,8 @@ int launch_tc(TcParams& p) {
 
 // Split-K: the partial products of the splits are summed in split order (the same bits every run)
 // and the epilogue runs once per element, on CUDA cores: one thread per row and block of four
-// columns, which share one Philox block exactly as the tensor-core epilogue assigns them.
+// columns, which share one Philox block exactly as the tensor-core epilogue assigns them.  Bound by the latency of
+// the partials' reads (L2): sixteen are in flight per thread.
 __global__ void __launch_bounds__(256) k_splitk_finish(const float* __restrict__ part, int splits, long stride, int M,
                                                        int N, const GemmEpilogue e) {
   grid_dependents_launch();
@@ -1333,17 +1334,33 @@ __global__ void __launch_bounds__(256) k_splitk_finish(const float* __restrict__
   const bool draw = e.sample != nullptr || e.sample_aux != nullptr;
   for (long it = (long)blockIdx.x * blockDim.x + threadIdx.x; it < items; it += (long)gridDim.x * blockDim.x) {
     const int b = (int)(it / M), m = (int)(it - (long)b * M);
+    const int n0 = 4 * b, ncols = min(4, N - n0);
+    const float* src = part + (long)n0 * M + m;
+    long at[4];
+    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+    for (int j = 0; j < 4; j++) at[j] = (long)min(j, ncols - 1) * M;   // (a column past the last repeats it)
+    int sp = 0;
+    for (; sp + 4 <= splits; sp += 4) {
+      float v[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) v[i][j] = src[(long)(sp + i) * stride + at[j]];
+#pragma unroll
+      for (int i = 0; i < 4; i++)
+#pragma unroll
+        for (int j = 0; j < 4; j++) acc[j] += v[i][j];
+    }
+    for (; sp < splits; sp++) {
+#pragma unroll
+      for (int j = 0; j < 4; j++) acc[j] += src[(long)sp * stride + at[j]];
+    }
     uint4 w = make_uint4(0, 0, 0, 0);
     if (draw) w = philox4x32_10((uint32_t)m, (uint32_t)(b + (e.col0 >> 2)), e.key);
 #pragma unroll
-    for (int j = 0; j < 4; j++) {
-      const int n = 4 * b + j;
-      if (n >= N) break;
-      const float* src = part + (long)n * M + m;
-      float acc = 0.0f;
-      for (int sp = 0; sp < splits; sp++) acc += src[(long)sp * stride];
-      epilogue_store(e, acc, m, n, word_to_uniform(pick_word(w, j)));
-    }
+    for (int j = 0; j < 4; j++)
+      if (j < ncols) epilogue_store(e, acc[j], m, n0 + j, word_to_uniform(pick_word(w, j)));
   }
 }
 
