@@ -268,12 +268,21 @@ __global__ void __launch_bounds__(256) k_softmax(const float* m, float* t, int h
   }
 }
 
+// A counter per reduction group, zero between calls (the last block resets it).
+unsigned* ticket_counters(int n) {
+  return (unsigned*)workspace_zeroed(3, (size_t)(n < 4096 ? 4096 : n) * sizeof(unsigned));
+}
+
 // ---- scalar reductions --------------------------------------------------------
-// mode 0: sum a; 1: sum a*a; 2: sum a*b; 3: sum (a-b)^2.  Stage 1 writes one double per
-// block, stage 2 (one block) folds them.
-__global__ void __launch_bounds__(256) k_scalar_partial(const float* __restrict__ a, const float* __restrict__ b,
-                                                        long n, int mode, double* __restrict__ part) {
+// mode 0: sum a; 1: sum a*a; 2: sum a*b; 3: sum (a-b)^2.  Every block leaves a double, the one that finishes last
+// folds them in a fixed order and stores the result into pinned host memory: one launch and no copy before the
+// host's wait (two launches and a copy before: the call is on the critical path of whoever reads a norm every update).
+__global__ void __launch_bounds__(256) k_scalar(const float* __restrict__ a, const float* __restrict__ b, long n, int mode,
+                                                double* __restrict__ part, unsigned* counter, double* out) {
   __shared__ double smem[32];
+  __shared__ bool is_last;
+  grid_dependents_launch();
+  grid_dependency_wait();
   const long tid = (long)blockIdx.x * blockDim.x + threadIdx.x, nth = (long)gridDim.x * blockDim.x;
   double s = 0;
   long start = 0;
@@ -319,17 +328,20 @@ __global__ void __launch_bounds__(256) k_scalar_partial(const float* __restrict_
     }
   }
   s = block_sum(s, smem);
-  if (threadIdx.x == 0) part[blockIdx.x] = s;
-}
-__global__ void __launch_bounds__(256) k_scalar_final(const double* __restrict__ part, int nparts,
-                                                      double* __restrict__ out, float* acc) {
-  __shared__ double smem[32];
-  double s = 0;
-  for (int i = threadIdx.x; i < nparts; i += blockDim.x) s += part[i];
-  s = block_sum(s, smem);
   if (threadIdx.x == 0) {
-    if (out) *out = s;
-    if (acc) *acc += (float)s;
+    part[blockIdx.x] = s;
+    __threadfence();
+    is_last = atomicAdd(counter, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!is_last) return;
+  __threadfence();
+  double t = 0;
+  for (int i = threadIdx.x; i < (int)gridDim.x; i += blockDim.x) t += __ldcg(part + i);
+  t = block_sum(t, smem);
+  if (threadIdx.x == 0) {
+    *out = t;
+    *counter = 0u;
   }
 }
 
@@ -342,13 +354,22 @@ int scalar_reduce(cudamat* a, cudamat* b, int mode, double* result) {
   if (blocks < 1) blocks = 1;
   double* part = (double*)workspace(1, (size_t)(blocks + 1) * sizeof(double));
   if (!part) return CUDA_ERROR;
-  k_scalar_partial<<<blocks, 256, 0, stream()>>>(a->data_device, b ? b->data_device : nullptr, n, mode, part + 1);
-  k_scalar_final<<<1, 256, 0, stream()>>>(part + 1, blocks, part, nullptr);
+  unsigned* counter = ticket_counters(1);
+  if (!counter) return CUDA_ERROR;
+  // eight bytes of pinned memory for the life of the process (one scalar is read at a time: the workspaces above are
+  // the library's, not the caller's, too)
+  static double* host = nullptr;
+  if (!host && cudaHostAlloc((void**)&host, sizeof(double), cudaHostAllocPortable) != cudaSuccess) {
+    host = nullptr;
+    return set_error("pinned allocation for a scalar result failed");
+  }
+  if (launch_dependent(k_scalar, dim3((unsigned)blocks), dim3(256), 0, stream(), a->data_device, b ? b->data_device : nullptr, n,
+                       mode, part + 1, counter, host) != cudaSuccess)
+    return set_error(cudaGetErrorString(cudaGetLastError()));
   int err = check_launch();
   if (err) return err;
-  if (cudaMemcpyAsync(result, part, sizeof(double), cudaMemcpyDeviceToHost, stream()) != cudaSuccess)
-    return set_error("scalar readback failed");
   if (cudaStreamSynchronize(stream()) != cudaSuccess) return set_error(cudaGetErrorString(cudaGetLastError()));
+  *result = *(volatile double*)host;
   return 0;
 }
 
@@ -607,11 +628,6 @@ extern "C" int add_sum_by_axis_noalloc(cudamat* mat, cudamat* target, int axis, 
 // let the block that finishes last fold the partial results, in a fixed order (the same bits
 // every run): no second launch, which at the small configurations costs more than the sums.
 namespace {
-
-// A counter per reduction group, zero between calls (the last block resets it).
-unsigned* ticket_counters(int n) {
-  return (unsigned*)workspace_zeroed(3, (size_t)(n < 4096 ? 4096 : n) * sizeof(unsigned));
-}
 
 // out[r] = sum_c a[r, c] - sum_c b[r, c].  Block = 32 row lanes x 8 column lanes, kVec rows per
 // lane (4 with 128-bit loads); blockIdx.y splits the columns.
