@@ -152,10 +152,9 @@ struct Stager {
         }
       } else {
         const int in_k = k < K ? 4 : 0;
-        const int t = threadIdx.x;
 #pragma unroll
-        for (int i = 0; i < 8; i++) {
-          cp4(tile + 4u * (uint32_t)at_k((t >> 5) + 8 * i, t & 31), s, 8 * i < left ? in_k : 0);
+        for (int i = 0; i < 8; i++) {     // 8 rows on: r / 4 grows by 2 (its bit 0 is the first row's own)
+          cp4(tile + (dst ^ (((2u * i) & 7u) * 16u)) + i * (8 * SK * 4), s, 8 * i < left ? in_k : 0);
           s += step;
         }
       }
@@ -167,10 +166,9 @@ struct Stager {
         s += step;
       }
     } else {
-      const int t = threadIdx.x;
 #pragma unroll
-      for (int i = 0; i < 8; i++) {
-        cp4(tile + 4u * (uint32_t)at_m((t >> 6) + 4 * i, t & 63), s, (left > 0 && k + 4 * i < K) ? 4 : 0);
+      for (int i = 0; i < 8; i++) {       // 4 values of k on: k / 8 is i / 2 (the first k is below 4)
+        cp4(tile + (dst ^ ((i >> 1) * 32u)) + i * (4 * SM_T * 4), s, (left > 0 && k + 4 * i < K) ? 4 : 0);
         s += step;
       }
     }

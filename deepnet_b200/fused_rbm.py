@@ -255,6 +255,8 @@ class FusedRBM(LossReadback):
         if bias is not None:
             ub = self._op(X, "bias_tail", 0, 8.0 * (V + H) * self.B, "rbm_bias_update", bias[0], bias[1], self.h_pos, self.h_neg,
                           self.suff_b, self.b, self.db, bias[2], sc["inv_b"], sc["mom"], sc["eps"])
+            if self.B > 1024:      # past that the operation is made of its separate launches
+                self.kernel_launches += 3 if bias[2] is not None else 2
             uw = self._op(X, "update_W", 0, 6 * wb, "momentum_update", self.W, self.dW, None, self.suff_W, sc["inv_b"],
                           sc["emom"], sc["eeps"], l2=sc["l2"], l1=sc["l1"], w_aux=self.W_aux, w_scale=w_scale)
             return ub, uw
