@@ -76,7 +76,7 @@ struct GemmProblem {
   // 1: part kPartX is read as TF32 (low 13 mantissa bits ignored), its meaning on the tensor
   // cores, which the CUDA-core kernel then reproduces; 0: kPartX is the full fp32 value.
   int tf32_operands;
-  int chunk_k = 0;   // products folded in tensor memory before they join the fp32 registers; 0: the kernel's own choice
+  int odd = 0;       // 1: some operand is a copy of a matrix TMA cannot address
   GemmPass pass[kMaxPass];
   GemmEpilogue epi;
 };

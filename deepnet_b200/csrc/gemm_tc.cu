@@ -1199,6 +1199,9 @@ inline bool tma_ok(const GemmOperand& o) {
   return (!reads_fp32(o) || fp32_tma_ok(o)) &&
          (!o.aux || (o.lda % 8 == 0 && ((uintptr_t)o.aux & 15) == 0 && o.row0 % 8 == 0));
 }
+inline bool plain_result(const GemmEpilogue& e) {
+  return !e.bias && e.activation == 0 && !e.sample && !e.out_aux && !e.sample_aux && e.out;
+}
 // Activation epilogues store whole column segments with TMA when every output's columns start on 16 bytes (the
 // planes of an aux matrix do, its columns being a multiple of 8 floats).
 inline bool tma_outputs_ok(const GemmEpilogue& e) {
@@ -1464,7 +1467,7 @@ static __global__ void __launch_bounds__(256) k_pack_operands(const __grid_const
 // 2947).
 int gemm_tc_packed(const GemmProblem& g) {
   GemmProblem f = g;
-  f.chunk_k = g.epi.activation == 1 ? 128 : 32;
+  f.odd = 1;
   PackJobs p;
   p.n = 0;
   p.total = 0;
@@ -1702,7 +1705,11 @@ int gemm_tc(const GemmProblem& g) {
   // at 512, 1.3e-6 at 1024, 2.9e-6 at 2048, 6e-6 at 4096; the bar is 1e-5).  Long chunks cover
   // the tile epilogue: the issuer runs two chunks ahead of the epilogue warps, which are busy for
   // 40-50 us per tile while the products of a tile take about 100 us.
-  const int ck = chunk_k >= 16 ? chunk_k : g.chunk_k > 0 ? g.chunk_k : (g.epi.activation == 1 ? 2048 : 128);
+  // Matrices TMA could not have addressed as fp32 (planes of odd matrices, copied operands, odd results) ran on CUDA
+  // cores before, which round every addition: short chunks keep their error where it was.
+  bool odd = g.odd != 0 || (!plain_result(g.epi) && !tma_outputs_ok(g.epi));
+  for (int q = 0; q < g.npass; q++) odd = odd || !fp32_tma_ok(g.pass[q].a) || !fp32_tma_ok(g.pass[q].b);
+  const int ck = chunk_k >= 16 ? chunk_k : odd ? (g.epi.activation == 1 ? 128 : 32) : (g.epi.activation == 1 ? 2048 : 128);
   p.chunk_iters = ck / bk < 1 ? 1 : ck / bk;
 
   // Split-K: a product whose tiles would occupy less than half of the SMs and whose inner dimension

@@ -679,3 +679,26 @@ def test_big_unaligned_dot_keeps_infinities(cm):
     got = get(cm.dot(cm.CUDAMatrix(A), cm.CUDAMatrix(B)))
     assert np.isposinf(got[3]).all() and np.isnan(got[9]).all()
     assert relerr(np.delete(got, [3, 9], axis=0), np.delete(want, [3, 9], axis=0)) < TOL
+
+
+@pytest.mark.parametrize("ta,tb", [(0, 0), (1, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("m,n,k", [(129, 67, 131), (501, 301, 1027)])
+def test_scaled_half_precision_product_of_odd_matrices(cm, ta, tb, m, n, k):
+    """Planes of matrices whose fp32 columns TMA cannot address (the planes' columns start on 16 bytes); results of any
+    alignment.  Bound 1e-6 of the largest entry, as for even sizes."""
+    rng = np.random.default_rng(16)
+    A, B = (rng.standard_normal((m, k)) * 0.03).astype(np.float32), rng.random((k, n)).astype(np.float32)
+    cm.set_gemm_path(1)
+    ga, gb = (cm.CUDAMatrix(np.asfortranarray(x.T if t else x)) for x, t in ((A, ta), (B, tb)))
+    scale = cm.f16_scale_state(np.abs(A).max())
+    xa = ga.split_f16(cm.empty_aux(ga.shape), exp_dev=scale.slice(0, 1))
+    xb = gb.split_f16(cm.empty_aux(gb.shape), exp_const=14)
+    out, bias = cm.empty((m, n)), cm.CUDAMatrix(rng.standard_normal((m, 1)).astype(np.float32))
+    kw = dict(out=out, scale_exp=scale.slice(0, 1), scale_exp_const=14)
+    passes = cm.f16_passes(ga.T if ta else ga, xa, gb.T if tb else gb, xb)
+    cm.fused_gemm(passes, **kw)
+    want = A.astype(np.float64) @ B.astype(np.float64)
+    assert relerr(get(out), want) < 1e-6
+    cm.fused_gemm(passes, bias=bias, activation=1, **kw)
+    assert relerr(get(out), 1 / (1 + np.exp(-(want + get(bias))))) < 1e-6
+    assert cm.read_status() == 0
