@@ -31,11 +31,11 @@ inline bool aux_shape_ok(const cudamat* aux, const cudamat* m) {
 }
 
 // The one-launch kernel (gemm_small.cu) against the tcgen05 one, by the slabs of 32 of K that an SM has to walk.
-// Measured (one launch against product + finishing launch): 4 slabs 10.9 against 15.1 us (500 x 100, K = 784), 8
-// slabs 17.8 against 23.6 (1024 x 256, K = 1024), 16 slabs 30.7 against 30.9 (1024 x 1024, two pairs of K = 256), 40
+// Measured (one launch against product + finishing launch): 4 slabs 10.0 against 15.1 us (500 x 100, K = 784), 8
+// slabs 15.5 against 23.6 (1024 x 256, K = 1024), 16 slabs 28.8 against 30.9 (1024 x 1024, two pairs of K = 256), 40
 // slabs 62 against 20 (512 x 100, K = 10 000).  Where the tcgen05 kernel needs aligned copies of its operands first
-// the line is the same: 8 slabs 21.7 against 26.8 us (1021 x 255, K = 1021), 11 slabs 27.1 against 28.8 (601 x
-// 203, K = 1357), 14 slabs 35.4 against 27.1 (1357 x 601, two pairs of K = 203).
+// the line is the same: 8 slabs 21.7 against 26.8 us (1021 x 255, K = 1021), 11 slabs 24.2 against 26.1 (601 x
+// 203, K = 1357), 14 slabs 32.7 against 28.9 (1357 x 601, two pairs of K = 203).
 constexpr int kSmallDepth = 11;
 
 int run(const GemmProblem& g) {

@@ -23,10 +23,10 @@
 //
 // Bound by instruction issue (the split of the operands and the copies, not the products): a slab takes an SM
 // 0.9 us with two CTAs on it, 1.4 us with one.  Measured, with the error against 64 bits of a logistic layer:
-//   500 x 100, K = 784       15.1 us (tcgen05 product + finishing launch, 2.0e-7) -> 10.9 us (5.5e-8)
-//   784 x 500, 2 x K = 100   19.2 us                                               -> 13.6 us
-//   1024 x 256, K = 1024     23.6 us                                               -> 17.8 us
-//   601 x 203, K = 1357      350 us (CUDA cores)                                   -> 27 us
+//   500 x 100, K = 784       15.1 us (tcgen05 product + finishing launch, 2.0e-7) -> 10.0 us (5.5e-8)
+//   784 x 500, 2 x K = 100   19.2 us                                               -> 12.8 us
+//   1024 x 256, K = 1024     23.6 us                                               -> 15.5 us
+//   601 x 203, K = 1357      519 us (CUDA cores, 2.4e-7)                           -> 24.2 us (6.0e-8)
 #include "gemm.cuh"
 
 namespace b200 {
