@@ -93,7 +93,12 @@ bool product_is_scattered(const float* out);
 int gemm_simt(const GemmProblem& g);
 // fp32-grade products of any alignment in one launch (gemm_small.cu); ERROR_UNSUPPORTED for term lists that are
 // not whole products (scaled half-precision planes, single parts).
-int gemm_small(const GemmProblem& g, bool ieee);
+enum SmallForm {
+  kSmallSplit,   // split TF32
+  kSmallIeee,    // the same, non-finite results computed again in plain fp32
+  kSmallFp32     // fp32 multiply-adds of the full operands (one pair of matrices)
+};
+int gemm_small(const GemmProblem& g, SmallForm form);
 int recompute_nonfinite(const GemmProblem& g);   // non-finite entries of g.epi.out = alpha x the plain fp32 product
 int small_depth(const GemmProblem& g);      // slabs of K that one SM would walk in gemm_small; 0: a list it does not take
 // Returns ERROR_UNSUPPORTED when an operand is not addressable by TMA (leading

@@ -10,7 +10,7 @@ namespace {
 
 int g_path = 0;       // 0 auto; one kernel only: 1 tcgen05, 2 CUDA cores, 3 the one-launch kernel, 4 tcgen05 behind aligned copies
 int g_dot_mode = 0;   // 0: fp32-grade (three TF32 terms), 1: single TF32 term
-constexpr long kTcMinWork = 1L << 21;  // below this many multiply-adds `dot` stays on CUDA cores
+constexpr long kTcMinWork = 1L << 21;  // below this many multiply-adds `dot` multiplies full fp32 operands
 
 inline int lead(const cudamat* m) { return m->is_trans ? m->size[1] : m->size[0]; }
 inline int nonlead(const cudamat* m) { return m->is_trans ? m->size[0] : m->size[1]; }
@@ -38,21 +38,37 @@ inline bool aux_shape_ok(const cudamat* aux, const cudamat* m) {
 // 203, K = 1357), 14 slabs 32.7 against 28.9 (1357 x 601, two pairs of K = 203).
 constexpr int kSmallDepth = 11;
 
+// `dot` on operands TMA cannot address and `dot` of little work multiply full fp32 operands with rounding adds (k_gemm_simt,
+// and in one launch gemm_small's fp32 form): a 0/1 selection returns the selected entries bit for bit, integer
+// products below 2^24 are exact, an infinity keeps its meaning.  Split TF32 holds 22 or 23 bits of an operand, which shows
+// while K is short.  Relative error against float64, 201 x 101 outputs, normal operands (0/1 against normal):
+//   K       k_gemm_simt         one launch, fp32    one launch, split   split, aligned copies
+//   1       2.5e-8  (0)         2.5e-8  (0)         7.9e-8  (2.9e-8)    4.0e-7  (1.2e-7)
+//   16      7.3e-8  (3.6e-8)    7.3e-8  (3.6e-8)    1.4e-7  (6.2e-8)    4.0e-7  (1.4e-7)
+//   100     1.8e-7  (7.9e-8)    1.0e-7  (5.9e-8)    2.4e-7  (9.4e-8)    4.3e-7  (1.5e-7)
+//   400     3.6e-7  (1.4e-7)    1.4e-7  (7.5e-8)    2.4e-7  (1.0e-7)    4.3e-7  (1.6e-7)
+//   600     4.5e-7  (1.8e-7)    1.3e-7  (8.2e-8)    2.4e-7  (1.1e-7)    4.3e-7  (1.6e-7)
+//   4001    1.1e-6  (4.4e-7)    2.9e-7  (1.3e-7)    2.6e-7  (1.2e-7)    4.5e-7  (1.9e-7)
+// The fp32 form costs what the split costs to within a fifth (us): 201 x 101, K = 1001: 183.6 / 10.8 / 9.8 / 14.8; 1021 x
+// 255, K = 1021: 191 / 22.7 / 20.0 / 26.6.  From K = 600 on the split behind aligned copies is no less exact than
+// k_gemm_simt was on random operands, and deeper products take it (2047 x 511, K = 2047: 433 / 149 / 127 / 46).
+constexpr int kPackedDotK = 600;
+
 int run(const GemmProblem& g) {
   if (product_is_scattered(g.epi.out)) return gemm_tc(g);   // (fails loudly when the tensor-core kernel cannot take it)
   if (g_path == 2) return gemm_simt(g);
-  if (g_path == 3) return gemm_small(g, false);
+  if (g_path == 3) return gemm_small(g, kSmallSplit);
   if (g_path == 4) return gemm_tc_packed(g);
   const bool tc = gemm_tc_supported(g);
   const int depth = g_path == 0 ? small_depth(g) : 0;
   int r = ERROR_UNSUPPORTED;
-  if (depth > 0 && depth <= kSmallDepth) r = gemm_small(g, false);
+  if (depth > 0 && depth <= kSmallDepth) r = gemm_small(g, kSmallSplit);
   if (r != ERROR_UNSUPPORTED) return r;
   // (unsupported: more operand pairs or tiles than one tensor-core launch carries)
   if (tc) r = gemm_tc(g);
   else if (g_path == 0) r = gemm_tc_packed(g);
   if (r != ERROR_UNSUPPORTED || g_path == 1) return r;
-  if (depth > 0) r = gemm_small(g, false);
+  if (depth > 0) r = gemm_small(g, kSmallSplit);
   return r != ERROR_UNSUPPORTED ? r : gemm_simt(g);
 }
 
@@ -654,26 +670,23 @@ int dot(cudamat* mat1, cudamat* mat2, cudamat* target, float beta, float alpha) 
     f.pass[q].negate = 0;
   }
   f.tf32_operands = 1;
-  if (g_path == 3 || (g_path == 0 && g_dot_mode != 1)) {
-    const int depth = small_depth(f);
-    const bool unaligned = !gemm_tc_supported(f);
-    // An infinity in an operand keeps its meaning where `dot` ran on CUDA cores before (operands TMA cannot address,
-    // little work): non-finite results are computed again in plain fp32.
-    if (g_path == 0 && unaligned && depth > kSmallDepth && beta == 0.0f) {
+  if (g_path == 2) return gemm_simt(g);
+  if (g_path == 4) return gemm_tc_packed(f);
+  const bool tc = gemm_tc_supported(g);
+  if (g_path == 1) return tc ? gemm_tc(g_dot_mode == 1 ? g : f) : ERROR_UNSUPPORTED;
+  // Operands TMA cannot address and little work: fp32 multiply-adds of the full operands.
+  if (!tc || (long)m * n * k < kTcMinWork) {
+    if (g_path == 0 && !tc && k >= kPackedDotK && g_dot_mode != 1 && beta == 0.0f && small_depth(f) > kSmallDepth) {
       int r = gemm_tc_packed(f);
       if (r == 0) r = recompute_nonfinite(f);
       if (r != ERROR_UNSUPPORTED) return r;
     }
-    if (g_path == 3 || (depth > 0 && (depth <= kSmallDepth || unaligned))) {
-      const int r = gemm_small(f, true);
-      if (r != ERROR_UNSUPPORTED || g_path == 3) return r;
-    }
+    const int r = gemm_small(f, kSmallFp32);
+    return r != ERROR_UNSUPPORTED || g_path == 3 ? r : gemm_simt(g);
   }
-  if (g_path == 4) return gemm_tc_packed(f);
-  const bool tc = g_path != 2 && gemm_tc_supported(g) && (g_path == 1 || (long)m * n * k >= kTcMinWork);
-  if (!tc) {
-    if (g_path == 1) return ERROR_UNSUPPORTED;
-    return gemm_simt(g);
+  if (g_path == 3 || (g_dot_mode != 1 && small_depth(f) <= kSmallDepth)) {
+    const int r = gemm_small(f, kSmallIeee);
+    if (r != ERROR_UNSUPPORTED || g_path == 3) return r;
   }
   return gemm_tc(g_dot_mode == 1 ? g : f);
 }

@@ -9,9 +9,13 @@
 // 4g .. 4g + 3 and k = 8t .. 8t + 7 and every fragment read is 16 bytes, without bank conflicts behind the
 // swizzles below.
 // The parts are made in registers: hi = x rounded to TF32 (11 significant bits), lo = x - hi (exact, at
-// most 12 bits), and a . b = lo.hi + hi.lo + hi.hi on mma.sync TF32: 2^-22 per term at worst.
+// most 12 bits, of which the tensor core reads 11), and a . b = lo.hi + hi.lo + hi.hi on mma.sync TF32:
+// 2^-21 per term at worst (lo.lo is left out: 2^-22, and a bit of either lo: 2^-23 each).
 // The tensor core truncates when it accumulates: after two slabs its accumulator is added to
 // the running sum with ordinary rounding and starts over.
+// The other form of the kernel multiplies full fp32 operands on CUDA cores from the same staged tiles: `dot` where
+// every bit of a short product counts.  A lane keeps the 4 x 8 outputs that its mma products end in; a slab takes
+// up to a fifth longer (500 x 100, K = 784: 11.2 us against 10.0; 1024 x 256, K = 1024: 20.3 against 16.7).
 //
 // Few tiles and a long K are cut along K over the CTAs of a thread-block cluster (2, 4 or 8): each
 // leaves its partial tile in its own shared memory, and every CTA of the cluster sums one share of
@@ -235,6 +239,38 @@ __device__ __forceinline__ void half_slab(const float* ta, const float* tb, floa
   }
 }
 
+// Half a slab of full fp32 multiply-adds: the lane's 4 rows x 8 columns (the ones its mma products end in) over 16
+// values of K, in order.  `rows` and `cols`: the lane's first row and column in the tile.  12 reads of 16 bytes,
+// without bank conflicts, to 128 multiply-adds.
+template <bool kAK, bool kBK>
+__device__ __forceinline__ void half_slab_fp32(const float* sa, const float* sb, int rows, int cols, int half,
+                                               float (&acc)[2][4][4]) {
+#pragma unroll
+  for (int kc = 0; kc < 4; kc++) {
+    const int k = 16 * half + 4 * kc;
+    float a[4][4], b[8][4];      // [row][k], [column][k]
+    read_half<kAK>(sa + (kAK ? at_k(rows, k) : at_m(k, rows)), a);
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      float x[4][4];
+      read_half<kBK>(sb + (kBK ? at_k(cols + 4 * h, k) : at_m(k, cols + 4 * h)), x);
+#pragma unroll
+      for (int n = 0; n < 4; n++)
+#pragma unroll
+        for (int c = 0; c < 4; c++) b[4 * h + n][c] = x[n][c];
+    }
+#pragma unroll
+    for (int c = 0; c < 4; c++)
+#pragma unroll
+      for (int r = 0; r < 4; r++)
+#pragma unroll
+        for (int n = 0; n < 8; n++) {
+          float& s = acc[r >> 1][n & 3][2 * (r & 1) + (n >> 2)];
+          s = fmaf(a[r][c], b[n][c], s);
+        }
+  }
+}
+
 // The sum of one output element as a chain of fp32 multiply-adds.
 __device__ __noinline__ float element_fp32(const SmallParams& p, int m, int n) {
   float acc = 0.0f;
@@ -251,6 +287,7 @@ __device__ __noinline__ float element_fp32(const SmallParams& p, int m, int n) {
 
 // Two CTAs per SM: with one, the next product's CTAs could not become resident before this one's end, and the
 // dependent launch would hide nothing (500 x 100, K = 784: 15.8 us at one CTA per SM and no spills, 10.9 at two).
+template <bool kFp32>
 __global__ void __launch_bounds__(kSmallThreads, 2) k_gemm_small(const __grid_constant__ SmallParams p) {
   extern __shared__ float4 smem4[];
   float* const smem = reinterpret_cast<float*>(smem4);
@@ -310,6 +347,16 @@ __global__ void __launch_bounds__(kSmallThreads, 2) k_gemm_small(const __grid_co
       offb = kTileFloats + (bk ? at_k(wn + 4 * g, 8 * t + 4 * half) : at_m(8 * t + 4 * half, wn + 4 * g));
     }
     const float* sa = smem + (size_t)((s - first) % kStages) * (2 * kTileFloats);
+    if constexpr (kFp32) {   // (one pair, not negated)
+      const float* sb = sa + kTileFloats;
+      switch (form >> 2) {
+        case 0: half_slab_fp32<false, false>(sa, sb, wm + 4 * g, wn + 8 * t, half, acc); break;
+        case 1: half_slab_fp32<false, true>(sa, sb, wm + 4 * g, wn + 8 * t, half, acc); break;
+        case 2: half_slab_fp32<true, false>(sa, sb, wm + 4 * g, wn + 8 * t, half, acc); break;
+        case 3: half_slab_fp32<true, true>(sa, sb, wm + 4 * g, wn + 8 * t, half, acc); break;
+      }
+      continue;
+    }
     const float *ta = sa + offa, *tb = sa + offb;
     switch (form) {
 #define B200_HALF_SLAB(F) case F: half_slab<((F) & 8) != 0, ((F) & 4) != 0, ((F) & 2) != 0, ((F) & 1) != 0>(ta, tb, part); break;
@@ -399,7 +446,7 @@ __global__ void __launch_bounds__(kSmallThreads, 2) k_gemm_small(const __grid_co
       }
     }
     const int ncols = min(4, p.N - n);
-    if (p.ieee) {
+    if (!kFp32 && p.ieee) {
 #pragma unroll
       for (int j = 0; j < 4; j++)
         if (j < ncols && !isfinite(x[j])) x[j] = element_fp32(p, m, n + j);
@@ -548,20 +595,23 @@ int small_depth(const GemmProblem& g) {
 
 // ieee: results that come out non-finite are computed again in plain fp32, so that an infinity in an operand
 // means what it means there (its low part is not a number).
-int gemm_small(const GemmProblem& g, bool ieee) {
+int gemm_small(const GemmProblem& g, SmallForm form) {
   SmallParams p;
   if (g.M <= 0 || g.N <= 0 || !gather_pairs(g, p)) return ERROR_UNSUPPORTED;
-  p.ieee = ieee;
+  const bool fp32 = form == kSmallFp32;
+  if (fp32 && (p.npairs != 1 || p.pair[0].negate)) return ERROR_UNSUPPORTED;
+  p.ieee = form == kSmallIeee;
   p.e = g.epi;
   const long ctas = cut_up(g, p);
   if (ctas > 0x7fffffffL) return ERROR_UNSUPPORTED;
-  static bool attr_set[64] = {false};
+  static bool attr_set[2][64] = {{false}};
+  void (*const kernel)(SmallParams) = fp32 ? k_gemm_small<true> : k_gemm_small<false>;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return set_error("cudaGetDevice failed");
-  if (!attr_set[dev]) {   // (setting it twice from two threads does no harm)
-    if (cudaFuncSetAttribute(k_gemm_small, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem) != cudaSuccess)
+  if (!attr_set[fp32][dev]) {   // (setting it twice from two threads does no harm)
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem) != cudaSuccess)
       return set_error("cudaFuncSetAttribute(max dynamic shared memory) failed");
-    attr_set[dev] = true;
+    attr_set[fp32][dev] = true;
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)ctas);
@@ -577,7 +627,7 @@ int gemm_small(const GemmProblem& g, bool ieee) {
   at[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = dependent_launch_enabled() ? 2 : 1;
-  if (cudaLaunchKernelEx(&cfg, k_gemm_small, p) != cudaSuccess) return set_error(cudaGetErrorString(cudaGetLastError()));
+  if (cudaLaunchKernelEx(&cfg, kernel, p) != cudaSuccess) return set_error(cudaGetErrorString(cudaGetLastError()));
   return check_launch();
 }
 

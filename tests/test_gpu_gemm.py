@@ -702,3 +702,29 @@ def test_scaled_half_precision_product_of_odd_matrices(cm, ta, tb, m, n, k):
     cm.fused_gemm(passes, bias=bias, activation=1, **kw)
     assert relerr(get(out), 1 / (1 + np.exp(-(want + get(bias))))) < 1e-6
     assert cm.read_status() == 0
+
+
+@pytest.mark.parametrize("ta,tb", [(0, 0), (1, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("m,n,k", [(7, 5, 1), (65, 67, 4), (64, 128, 16), (100, 101, 64), (201, 101, 100), (33, 31, 257), (2049, 513, 63),
+                                   (61, 29, 1357), (4, 100, 4096)])
+def test_dot_of_full_operands_keeps_their_bits(cm, ta, tb, m, n, k):
+    """Operands TMA cannot address, and little work on any: fp32 multiply-adds.  A selection returns the selected entries,
+    sums of integer products below 2^24 are exact in any order, and the error against float64 is no larger than
+    k_gemm_simt's, which adds one term after the other (a chain cut into shares and added up is shorter)."""
+    rng = np.random.default_rng(m + n + k)
+    d = lambda x: x.astype(np.float64)
+    dot = lambda a, b: get(cm.dot(make(cm, a, ta), make(cm, b, tb)))
+    B = rng.standard_normal((k, n)).astype(np.float32)
+    pick = rng.integers(0, k, m)
+    A = np.zeros((m, k), np.float32)
+    A[np.arange(m), pick] = 1.0
+    np.testing.assert_array_equal(dot(A, B), B[pick])
+    top = int((2 ** 24 / k) ** 0.5)      # k * top^2 <= 2^24
+    A, C = (rng.integers(0, top + 1, s).astype(np.float32) for s in ((m, k), (k, n)))
+    np.testing.assert_array_equal(dot(A, C), d(A) @ d(C))
+    A = rng.standard_normal((m, k)).astype(np.float32)
+    want = d(A) @ d(B)
+    auto = np.linalg.norm(dot(A, B) - want)
+    cm.set_gemm_path(2)
+    assert auto <= 1.02 * np.linalg.norm(dot(A, B) - want)
+    assert cm.read_status() == 0
