@@ -63,7 +63,8 @@ struct SmallParams {
   SmallPair pair[kMaxPairs];
   int npairs, slabs, splits;
   int M, N, tiles_m;
-  int ieee;            // recompute non-finite results in plain fp32 (`dot` keeps the meaning of inf)
+  int ieee;            // non-finite results are computed again: in plain fp32 (`dot` keeps the meaning of inf), else as
+                       // the tcgen05 kernel's parts give them
   GemmEpilogue e;
 };
 
@@ -276,10 +277,29 @@ __device__ __noinline__ float element_fp32(const SmallParams& p, int m, int n) {
   float acc = 0.0f;
   for (int q = 0; q < p.npairs; q++) {
     const SmallPair& pr = p.pair[q];
-    for (int k = 0; k < pr.k; k++) {
+    for (int k = 0; k < pr.k && !isnan(acc); k++) {   // (NaN stays)
       const float a = pr.a.kmajor ? pr.a.p[(long)m * pr.a.ld + k] : pr.a.p[(long)k * pr.a.ld + m];
       const float b = pr.b.kmajor ? pr.b.p[(long)n * pr.b.ld + k] : pr.b.p[(long)k * pr.b.ld + n];
       acc = fmaf(pr.negate ? -a : a, b, acc);
+    }
+  }
+  return acc;
+}
+
+// The same of the parts as the tcgen05 kernel takes them, by truncation: an operand so near the largest float that it
+// rounds to an infinity stays finite, an infinity (whose low part is not a number) gives NaN.
+__device__ __noinline__ float element_truncated(const SmallParams& p, int m, int n) {
+  float acc = 0.0f;
+  for (int q = 0; q < p.npairs; q++) {
+    const SmallPair& pr = p.pair[q];
+    for (int k = 0; k < pr.k && !isnan(acc); k++) {
+      const float a = pr.a.kmajor ? pr.a.p[(long)m * pr.a.ld + k] : pr.a.p[(long)k * pr.a.ld + m];
+      const float b = pr.b.kmajor ? pr.b.p[(long)n * pr.b.ld + k] : pr.b.p[(long)k * pr.b.ld + n];
+      const float ah = __uint_as_float(__float_as_uint(a) & 0xffffe000u), bh = __uint_as_float(__float_as_uint(b) & 0xffffe000u);
+      const float s = pr.negate ? -1.0f : 1.0f;
+      if (!pr.a.exact) acc = fmaf(s * (a - ah), bh, acc);
+      if (!pr.b.exact) acc = fmaf(s * ah, b - bh, acc);
+      acc = fmaf(s * ah, bh, acc);
     }
   }
   return acc;
@@ -446,10 +466,10 @@ __global__ void __launch_bounds__(kSmallThreads, 2) k_gemm_small(const __grid_co
       }
     }
     const int ncols = min(4, p.N - n);
-    if (!kFp32 && p.ieee) {
+    if (!kFp32) {
 #pragma unroll
       for (int j = 0; j < 4; j++)
-        if (j < ncols && !isfinite(x[j])) x[j] = element_fp32(p, m, n + j);
+        if (j < ncols && !isfinite(x[j])) x[j] = p.ieee ? element_fp32(p, m, n + j) : element_truncated(p, m, n + j);
     }
     const long off = (long)n * e.ldo + m;
 #pragma unroll

@@ -728,3 +728,28 @@ def test_dot_of_full_operands_keeps_their_bits(cm, ta, tb, m, n, k):
     cm.set_gemm_path(2)
     assert auto <= 1.02 * np.linalg.norm(dot(A, B) - want)
     assert cm.read_status() == 0
+
+
+@pytest.mark.parametrize("m,n,k", [(64, 64, 64), (65, 63, 33), (500, 100, 784)])
+def test_operands_near_the_largest_float_stay_finite(cm, m, n, k):
+    """Rounded to TF32 these would become infinities (and, times a zero, not a number); what the tcgen05 kernel reads is
+    their truncation, which is finite.  An infinity gives NaN there, its low part being none."""
+    top = np.finfo(np.float32).max
+    rng = np.random.default_rng(m)
+    W = (rng.standard_normal((k, m)) * 0.1).astype(np.float32)
+    X = (rng.random((k, n)) < 0.4).astype(np.float32)
+    W[1, ::3], W[2, 1::3] = -top, top
+    X[1:3, ::2], X[1:3, 1::2] = 0.0, 1.0
+    X[2, :] *= 1.0 - X[1, :] * (np.arange(n) % 4 == 1)
+    zero = cm.empty((m, 1))
+    w, x = cm.CUDAMatrix(W), cm.CUDAMatrix(X)
+    for kw in (dict(exact_b=True), dict(terms="tf32")):
+        out = cm.empty((m, n))
+        cm.fused_gemm(cm.split_passes(w.T, x, **kw), out=out, bias=zero, activation=1)
+        with np.errstate(over="ignore"):
+            want = 1 / (1 + np.exp(-(W.astype(np.float64).T @ X)))
+        np.testing.assert_allclose(get(out), want, rtol=1e-5, atol=1e-30)
+    W[0, 5] = np.inf
+    out = cm.empty((m, n))
+    cm.fused_gemm(cm.split_passes(cm.CUDAMatrix(W).T, x, exact_b=True), out=out, bias=zero, activation=1)
+    assert np.isnan(get(out)[5]).all() and np.isfinite(np.delete(get(out), 5, axis=0)).all()
