@@ -233,7 +233,7 @@ __global__ void __launch_bounds__(32 * kTailLanes) k_bias_tail(TailLayer v, Tail
       }
 #pragma unroll
       for (int i = 0; i < 4; i++) s += d[i];
-      e += (double)((d[0] * d[0] + d[1] * d[1]) + (d[2] * d[2] + d[3] * d[3]));
+      e += ((double)d[0] * d[0] + (double)d[1] * d[1]) + ((double)d[2] * d[2] + (double)d[3] * d[3]);
     }
     for (; c < cases; c += kTailLanes) {
       const long o = (long)c * l.rows + r;

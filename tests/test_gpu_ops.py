@@ -296,3 +296,17 @@ def test_bias_tail_matches_the_separate_operations(cm, with_error, V, H, B):
         np.testing.assert_array_equal(get(gdb), get(wdb))
         want = turn * ((d[0] - d[1]) ** 2).sum() if with_error else 0.0
         assert abs(get(acc)[0, 0] - want) <= 2.0 ** -21 * want
+
+
+@pytest.mark.parametrize("V,B", [(33, 32), (65, 97), (784, 100)])
+def test_bias_tail_adds_squares_in_double(cm, V, B):
+    """Differences whose squares all round the same way in fp32 (four of them, added in fp32, lose three half-units): the error
+    is the sum in 64 bits rounded once, also on a minibatch whose columns do not start on 16 bytes."""
+    d = np.array([0.7862465977668762, 0.6392413377761841, 0.27659112215042114, 0.9504463076591492], np.float32)
+    x = np.broadcast_to(d[(np.arange(B) // 8) % 4][None, :], (V, B)).astype(np.float32)
+    data = cm.CUDAMatrix(np.concatenate([np.zeros((V, 1), np.float32), x], axis=1))
+    zero, h = cm.CUDAMatrix(np.zeros((V, B), np.float32)), cm.CUDAMatrix(np.zeros((5, B), np.float32))
+    suff, b, db = (cm.empty((V + 5, 1)) for _ in range(3))
+    acc = cm.empty((1, 1))
+    cm.Immediate().rbm_bias_update(data.slice(1, B + 1), zero, h, h, suff, b, db, acc, 1.0 / B, 0.5, 0.1)
+    assert get(acc)[0, 0] == np.float32((x.astype(np.float64) ** 2).sum())
