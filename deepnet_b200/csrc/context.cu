@@ -18,13 +18,32 @@ static int g_sm_count = 0;
 static int g_col0 = 0;
 static int* g_status = nullptr;
 static char g_err[512] = "";
-static void* g_ws[8] = {nullptr};
-static size_t g_ws_bytes[8] = {0};
-static bool g_ws_fresh[8] = {false};   // allocated since it was last cleared (workspace_zeroed)
 static std::mutex g_mu;
+
+// Scratch of the streams the library has run on: calls on two streams that nobody orders share none.  The first entry is
+// the library's own stream's.  When the others are all taken, a further stream takes over the one that was selected
+// longest ago, once the device has finished what may still use it; the memory stays (a captured graph may name it).
+constexpr int kWorkspaces = 8, kScratchStreams = 8;
+struct Scratch {
+  unsigned long long stream;    // cudaStreamGetId, 0: not taken
+  unsigned long selected;
+  void* p[kWorkspaces];
+  size_t bytes[kWorkspaces];
+  bool fresh[kWorkspaces];      // allocated since it was last cleared (workspace_zeroed)
+};
+static Scratch g_scratch[kScratchStreams];
+static Scratch* g_ws = g_scratch;   // the current stream's
 
 static int g_dependent_launch = -1;        // programmatic dependent launch of the hot kernels: -1 = read the environment
 static uint32_t g_wait_limit = 1u << 24;   // iterations of a bounded device-side wait: ~1-2 s
+
+// Handles are used again after a stream is destroyed, ids are not.
+static unsigned long long stream_id(cudaStream_t s) {
+  unsigned long long id = 0;
+  if (cudaStreamGetId(s, &id) == cudaSuccess) return id + 1;
+  cudaGetLastError();
+  return ~(unsigned long long)(uintptr_t)s;
+}
 
 // Creates the library stream and the device status word.  A failure (a device with no memory left,
 // a context in an error state) is recorded and leaves the library uninitialised: stream() then
@@ -56,6 +75,8 @@ static void ensure_init() {
   }
   g_status = status;
   g_own_stream = true;
+  g_ws = g_scratch;
+  g_ws->stream = stream_id(s);
   g_stream = s;   // published last: a non-null stream means the library is usable
 }
 
@@ -103,40 +124,64 @@ int check_launch() {
   return check_launch_any_stream();
 }
 
+// Makes the scratch of `s` the current one.
+static int select_scratch(cudaStream_t s) {
+  static unsigned long clock = 0;
+  const unsigned long long id = stream_id(s);
+  Scratch* take = nullptr;
+  for (int i = 0; i < kScratchStreams && !take; i++)
+    if (g_scratch[i].stream == id) take = &g_scratch[i];
+  if (!take) {
+    take = &g_scratch[1];
+    for (int i = 2; i < kScratchStreams; i++)
+      if (g_scratch[i].selected < take->selected) take = &g_scratch[i];
+    bool used = false;
+    for (int i = 0; i < kWorkspaces; i++) used = used || take->p[i];
+    if (used && cudaDeviceSynchronize() != cudaSuccess) return set_error(cudaGetErrorString(cudaGetLastError()));
+    take->stream = id;
+  }
+  take->selected = ++clock;
+  g_ws = take;
+  return 0;
+}
+
 void* workspace(int slot, size_t bytes) {
   ensure_init();
-  if (slot < 0 || slot >= 8) return nullptr;
-  if (g_ws_bytes[slot] >= bytes && g_ws[slot]) return g_ws[slot];
-  if (g_ws[slot]) {
+  if (slot < 0 || slot >= kWorkspaces) return nullptr;
+  Scratch& ws = *g_ws;
+  if (ws.bytes[slot] >= bytes && ws.p[slot]) return ws.p[slot];
+  if (ws.p[slot]) {
     cudaStreamSynchronize(g_stream);
-    cudaFree(g_ws[slot]);
-    g_ws[slot] = nullptr;
-    g_ws_bytes[slot] = 0;
+    cudaFree(ws.p[slot]);
+    ws.p[slot] = nullptr;
+    ws.bytes[slot] = 0;
   }
   size_t want = bytes + bytes / 4 + 256;
-  if (cudaMalloc(&g_ws[slot], want) != cudaSuccess) {
+  if (cudaMalloc(&ws.p[slot], want) != cudaSuccess) {
     cudaGetLastError();
-    if (cudaMalloc(&g_ws[slot], bytes) != cudaSuccess) {
+    if (cudaMalloc(&ws.p[slot], bytes) != cudaSuccess) {
+      cudaGetLastError();
+      ws.p[slot] = nullptr;
       set_error("workspace allocation failed");
       return nullptr;
     }
     want = bytes;
   }
-  g_ws_bytes[slot] = want;
-  g_ws_fresh[slot] = true;
-  return g_ws[slot];
+  ws.bytes[slot] = want;
+  ws.fresh[slot] = true;
+  return ws.p[slot];
 }
 
 // The same, all zero when first handed out (and again after it had to grow): counters that their
 // users leave at zero between calls.
 void* workspace_zeroed(int slot, size_t bytes) {
   void* p = workspace(slot, bytes);
-  if (p && g_ws_fresh[slot]) {
-    if (cudaMemsetAsync(p, 0, g_ws_bytes[slot], g_stream) != cudaSuccess) {
+  if (p && g_ws->fresh[slot]) {
+    if (cudaMemsetAsync(p, 0, g_ws->bytes[slot], g_stream) != cudaSuccess) {
       set_error("workspace clear failed");
       return nullptr;
     }
-    g_ws_fresh[slot] = false;
+    g_ws->fresh[slot] = false;
   }
   return p;
 }
@@ -194,12 +239,14 @@ int b200_set_wait_limit(unsigned int iterations) {
 
 int cublas_shutdown() {
   if (!g_stream) return 0;
-  cudaStreamSynchronize(g_stream);
-  for (int i = 0; i < 8; i++) {
-    if (g_ws[i]) cudaFree(g_ws[i]);
-    g_ws[i] = nullptr;
-    g_ws_bytes[i] = 0;
-    g_ws_fresh[i] = false;
+  cudaDeviceSynchronize();
+  for (Scratch& ws : g_scratch) {
+    for (int i = 0; i < kWorkspaces; i++) {
+      if (ws.p[i]) cudaFree(ws.p[i]);
+      ws.p[i] = nullptr;
+      ws.bytes[i] = 0;
+      ws.fresh[i] = false;
+    }
   }
   return 0;
 }
@@ -233,6 +280,11 @@ int b200_set_stream(void* s) {
   ensure_init();
   static cudaStream_t own = nullptr;
   if (g_own_stream) own = g_stream;
+  const cudaStream_t next = s ? (cudaStream_t)s : own;
+  if (next) {
+    const int err = select_scratch(next);
+    if (err) return err;
+  }
   if (s) {
     g_stream = (cudaStream_t)s;
     g_own_stream = false;

@@ -290,7 +290,8 @@ int add_sq_diff(cudamat* a, cudamat* b, cudamat* acc);
 
 /* Library control. */
 int b200_device_count(void);
-int b200_set_stream(void* cuda_stream);   /* NULL restores the library's own stream */
+int b200_set_stream(void* cuda_stream);   /* NULL restores the library's own stream; scratch is kept per stream, for up to
+                                           * eight of them: a ninth waits for the device, then takes one over */
 void* b200_get_stream(void);
 void* b200_event_create(void);            /* CUDA events recorded on the library stream */
 int b200_event_record(void* ev);

@@ -6,6 +6,7 @@ Tolerance: 1e-5 of the largest magnitude of the exact result (the bound the path
 meet on activations and gradients); the single-pass TF32 mode is checked at 2e-3."""
 import numpy as np
 import pytest
+import torch
 
 pytestmark = pytest.mark.gpu
 
@@ -753,3 +754,37 @@ def test_operands_near_the_largest_float_stay_finite(cm, m, n, k):
     out = cm.empty((m, n))
     cm.fused_gemm(cm.split_passes(cm.CUDAMatrix(W).T, x, exact_b=True), out=out, bias=zero, activation=1)
     assert np.isnan(get(out)[5]).all() and np.isfinite(np.delete(get(out), 5, axis=0)).all()
+
+
+def test_unordered_streams_share_no_scratch(cm):
+    """Products behind aligned copies, cut along K, and row sums on streams that nobody orders, more of them than the library
+    keeps scratch for: every result has the bits of the same call alone."""
+    rng = np.random.default_rng(12)
+    m, n, k = 1501, 301, 1501
+    mats = [cm.CUDAMatrix(rng.standard_normal((m, k)).astype(np.float32)) for _ in range(3)]
+    b = cm.CUDAMatrix(rng.standard_normal((k, n)).astype(np.float32))
+
+    def issue(i, out, sums):
+        cm.dot(mats[i % 3], b, target=out)
+        cm._check(cm._lib.sum_by_axis(mats[i % 3].p_mat, sums.p_mat, 1))
+        cm.fused_gemm(cm.split_passes(mats[(i + 1) % 3], b), out=out, beta=1.0)
+
+    want = []
+    for i in range(3):
+        out, sums = cm.empty((m, n)), cm.empty((m, 1))
+        issue(i, out, sums)
+        want.append((get(out), get(sums)))
+    for nstreams, turns in ((2, 24), (11, 33)):
+        streams = [torch.cuda.Stream() for _ in range(nstreams)]
+        outs = [(cm.empty((m, n)), cm.empty((m, 1))) for _ in range(turns)]
+        cm.cuda_sync_threads()
+        try:
+            for t in range(turns):
+                cm._check(cm._lib.b200_set_stream(streams[t % nstreams].cuda_stream))
+                issue(t, *outs[t])
+        finally:
+            cm._lib.b200_set_stream(None)
+        torch.cuda.synchronize()
+        for t in range(turns):
+            for got, w in zip(outs[t], want[t % 3]):
+                np.testing.assert_array_equal(get(got), w)
