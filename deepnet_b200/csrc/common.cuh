@@ -46,6 +46,8 @@ int sm_count();                        // SMs of the current device
 int check_launch();                    // cudaGetLastError -> 0 or CUDA_ERROR (message kept); CUDA_ERROR when the library failed to initialise
 int check_launch_any_stream();         // the same for entry points that also run without the library stream
 int set_error(const char* msg);        // records msg, returns CUDA_ERROR
+void clear_error();                    // forgets the recorded text: the caller has another way to go
+bool stream_capturing();               // the library stream is being captured: nothing may be allocated
 int rng_col0();                        // first global column of this process's minibatch shard
 void* workspace(int slot, size_t bytes);  // grow-only cached device scratch of the current stream, slot 0..7
 void* workspace_zeroed(int slot, size_t bytes);  // the same, cleared when first handed out or regrown (counters left at zero by their users)

@@ -33,6 +33,7 @@ struct Scratch {
 };
 static Scratch g_scratch[kScratchStreams];
 static Scratch* g_ws = g_scratch;   // the current stream's
+static size_t g_scratch_limit = ~(size_t)0;   // largest scratch a call gets (b200_test_limit_scratch)
 
 static int g_dependent_launch = -1;        // programmatic dependent launch of the hot kernels: -1 = read the environment
 static uint32_t g_wait_limit = 1u << 24;   // iterations of a bounded device-side wait: ~1-2 s
@@ -114,6 +115,15 @@ int set_error(const char* msg) {
   return CUDA_ERROR;
 }
 
+void clear_error() { g_err[0] = 0; }
+
+bool stream_capturing() {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(stream(), &st) == cudaSuccess) return st != cudaStreamCaptureStatusNone;
+  cudaGetLastError();
+  return true;
+}
+
 int check_launch_any_stream() {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return set_error(cudaGetErrorString(e));
@@ -149,6 +159,10 @@ void* workspace(int slot, size_t bytes) {
   ensure_init();
   if (slot < 0 || slot >= kWorkspaces) return nullptr;
   Scratch& ws = *g_ws;
+  if (bytes > g_scratch_limit) {
+    set_error("workspace allocation failed");
+    return nullptr;
+  }
   if (ws.bytes[slot] >= bytes && ws.p[slot]) return ws.p[slot];
   if (ws.p[slot]) {
     cudaStreamSynchronize(g_stream);
@@ -229,6 +243,12 @@ int b200_set_sm_limit(int sms) {
 // default, B200_DEPENDENT_LAUNCH=0 or this call with 0 turns it off.  No counterpart in the reference.
 int b200_set_dependent_launch(int on) {
   g_dependent_launch = on ? 1 : 0;
+  return 0;
+}
+
+// Scratch beyond `bytes` is refused from now on, as by a device without memory (0: no limit).
+int b200_test_limit_scratch(size_t bytes) {
+  g_scratch_limit = bytes ? bytes : ~(size_t)0;
   return 0;
 }
 

@@ -1497,8 +1497,13 @@ int gemm_tc_packed(const GemmProblem& g) {
     }
   }
   if (p.n) {
-    float* ws = (float*)workspace(4, (size_t)p.total * 16);
-    if (!ws) return CUDA_ERROR;
+    // Other kernels take these products without scratch: in a capture, which must not allocate and whose graph must not
+    // name memory that a later call may replace, and where the device has no memory left.
+    float* ws = stream_capturing() ? nullptr : (float*)workspace(4, (size_t)p.total * 16);
+    if (!ws) {
+      clear_error();
+      return ERROR_UNSUPPORTED;
+    }
     for (int j = 0; j < p.n; j++) p.job[j].dst = ws + 4 * p.job[j].first;
     // every term over a copied matrix names the copy, also where it reads the aux matrix alone: the terms over one
     // pair of matrices share their staged tiles
@@ -1740,9 +1745,16 @@ int gemm_tc(const GemmProblem& g) {
       want = g_split_mode < min_ki ? g_split_mode : min_ki;
     }
     if (scatter) want = 1;   // a partial is not a result: the panels go out whole
+    float* ws = nullptr;
     if (want > 1) {
-      float* ws = (float*)workspace(2, (size_t)want * g.M * g.N * sizeof(float));
-      if (!ws) return CUDA_ERROR;
+      if (!odd || !stream_capturing()) ws = (float*)workspace(2, (size_t)want * g.M * g.N * sizeof(float));
+      if (!ws) {   // (products of odd matrices did without scratch on CUDA cores: uncut they do so here)
+        if (!odd) return CUDA_ERROR;
+        clear_error();
+        want = 1;
+      }
+    }
+    if (want > 1) {
       p.splits = want;
       p.split_stride = (long)g.M * g.N;
       GemmEpilogue& pe = p.epi;       // the kernel stores raw partials; g.epi runs in the finishing kernel

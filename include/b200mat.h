@@ -313,6 +313,8 @@ int b200_sm_count(void);                  /* SMs in force (the device's, or the 
  * its copies deliver, so one of its bounded waits must run out (status word set, kernel returns).
  * No counterpart in the reference. */
 int b200_test_inject_stage_bytes(int extra_bytes);
+/* Test hook: scratch beyond `bytes` is refused, as by a device without memory (0: no limit). */
+int b200_test_limit_scratch(size_t bytes);
 /* All steps of an annealing schedule (n inverse temperatures) of a binary RBM's partition function estimate
  * (deepnet/ais.py:152-170): w V x H and its aux, biases a (H) and b (V), chain states, sb (V) scratch, weights 1 x B added to. */
 int ais_binary_steps(rnd_struct* rnd_state, cudamat* w, cudamat* w_aux, cudamat* a, cudamat* b, cudamat* v_state,

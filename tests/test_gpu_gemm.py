@@ -4,6 +4,8 @@ and the fused epilogue (bias, logistic, Bernoulli draw, TF32 split, negated pass
 
 Tolerance: 1e-5 of the largest magnitude of the exact result (the bound the path must
 meet on activations and gradients); the single-pass TF32 mode is checked at 2e-3."""
+import ctypes as ct
+
 import numpy as np
 import pytest
 import torch
@@ -788,3 +790,75 @@ def test_unordered_streams_share_no_scratch(cm):
         for t in range(turns):
             for got, w in zip(outs[t], want[t % 3]):
                 np.testing.assert_array_equal(get(got), w)
+
+
+class _Captured(object):
+    """The library's calls inside the block, recorded on a stream of torch's as a graph."""
+
+    def __init__(self, cm):
+        self.cm, self.stream, self.graph = cm, torch.cuda.Stream(), torch.cuda.CUDAGraph()
+
+    def __enter__(self):
+        self.cm.cuda_sync_threads()
+        self.cm._lib.b200_set_stream(self.stream.cuda_stream)
+        self.ctx = torch.cuda.graph(self.graph, stream=self.stream)
+        self.ctx.__enter__()
+        return self
+
+    def __exit__(self, *exc):
+        try:
+            return self.ctx.__exit__(*exc)
+        finally:
+            self.cm._lib.b200_set_stream(None)
+
+    def replay(self):
+        self.graph.replay()
+        torch.cuda.synchronize()
+
+
+def test_products_of_odd_matrices_can_be_captured(cm):
+    """They used no scratch while CUDA cores ran them: a capture that comes before any other use of the library's
+    scratch records them, and the graph reads no memory that a later call may replace."""
+    rng = np.random.default_rng(8)
+    m, n, k = 1501, 301, 1501
+    A, B = (rng.standard_normal((m, k)) * 0.1).astype(np.float32), (rng.random((k, n)) < 0.4).astype(np.float32)
+    a, b, bias = cm.CUDAMatrix(A), cm.CUDAMatrix(B), cm.empty((m, 1))
+    aux_a, aux_b = a.split_f16(cm.empty_aux((m, k)), exp_const=14), b.split_f16(cm.empty_aux((k, n)), exp_const=14)
+    outs = [cm.empty((m, n)) for _ in range(3)]
+    torch.zeros(1, device="cuda")
+    cm.cublas_shutdown()                     # (hands the scratch back)
+    cm.cublas_init()
+    with _Captured(cm) as graph:
+        cm.dot(a, b, target=outs[0])
+        cm.fused_gemm(cm.split_passes(a, b, exact_b=True), out=outs[1], bias=bias, activation=1)
+        cm.fused_gemm(cm.f16_passes(a, aux_a, b, aux_b), out=outs[2], scale_exp_const=28)
+    A2 = (A * 0.5).astype(np.float32)
+    a.overwrite(A2)
+    a.split_f16(aux_a, exp_const=14)
+    big = cm.empty((3001, 3001))
+    cm.dot(big, big)                         # the scratch of a larger product
+    cm.cuda_sync_threads()
+    graph.replay()
+    want = A2.astype(np.float64) @ B
+    for got, w in zip(outs, (want, 1 / (1 + np.exp(-want)), want)):
+        assert relerr(get(got), w) < TOL
+
+
+def test_products_of_odd_matrices_do_without_scratch(cm):
+    """A device without memory for scratch: products that CUDA cores ran without any still give their results."""
+    rng = np.random.default_rng(8)
+    m, n, k = 1501, 301, 1501
+    A, B = (rng.standard_normal((m, k)) * 0.1).astype(np.float32), (rng.random((k, n)) < 0.4).astype(np.float32)
+    a, b, bias = cm.CUDAMatrix(A), cm.CUDAMatrix(B), cm.empty((m, 1))
+    aux_a, aux_b = a.split_f16(cm.empty_aux((m, k)), exp_const=14), b.split_f16(cm.empty_aux((k, n)), exp_const=14)
+    outs = [cm.empty((m, n)) for _ in range(3)]
+    cm._lib.b200_test_limit_scratch(ct.c_size_t(1024))
+    try:
+        cm.dot(a, b, target=outs[0])
+        cm.fused_gemm(cm.split_passes(a, b, exact_b=True), out=outs[1], bias=bias, activation=1)
+        cm.fused_gemm(cm.f16_passes(a, aux_a, b, aux_b), out=outs[2], scale_exp_const=28)
+    finally:
+        cm._lib.b200_test_limit_scratch(ct.c_size_t(0))
+    want = A.astype(np.float64) @ B
+    for got, w in zip(outs, (want, 1 / (1 + np.exp(-want)), want)):
+        assert relerr(get(got), w) < TOL
