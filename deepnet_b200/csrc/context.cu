@@ -260,6 +260,7 @@ int b200_set_wait_limit(unsigned int iterations) {
 int cublas_shutdown() {
   if (!g_stream) return 0;
   cudaDeviceSynchronize();
+  free_scalar_words();
   for (Scratch& ws : g_scratch) {
     for (int i = 0; i < kWorkspaces; i++) {
       if (ws.p[i]) cudaFree(ws.p[i]);

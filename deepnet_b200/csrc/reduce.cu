@@ -3,6 +3,7 @@
 // (cudamat/cudamat.cu:1148-1258, 1733-1759, 2104-2118, 2192-2240; the axis sums replace
 // the reference's GEMV with a ones vector, cudamat/cudamat.py:724-748,1546-1577).
 // Warp-shuffle trees inside a block; HBM-bound: 4 bytes read per input element.
+#include <condition_variable>
 #include <mutex>
 
 #include "common.cuh"
@@ -345,6 +346,17 @@ __global__ void __launch_bounds__(256) k_scalar(const float* __restrict__ a, con
   }
 }
 
+// Where a result arrives in pinned host memory: a word of its own for every call under way, so that host threads inside
+// a reduction at the same time each read theirs.  Scratch and launch are one step under the lock (two calls on a stream
+// then run one after the other), the wait is outside.  A call beyond the 32nd waits for a word.
+constexpr int kScalarWords = 32;
+struct ScalarWords {
+  std::mutex mu;
+  std::condition_variable freed;
+  double* words = nullptr;
+  uint32_t busy = 0;
+} g_scalars;
+
 int scalar_reduce(cudamat* a, cudamat* b, int mode, double* result) {
   if (!a->on_device || (b && !b->on_device)) return ERROR_NOT_ON_DEVICE;
   const long n = numel(a);
@@ -352,30 +364,47 @@ int scalar_reduce(cudamat* a, cudamat* b, int mode, double* result) {
   const int cap = sm_count() * 8;
   if (blocks > cap) blocks = cap;
   if (blocks < 1) blocks = 1;
+  ScalarWords& s = g_scalars;
+  std::unique_lock<std::mutex> lock(s.mu);
+  s.freed.wait(lock, [&] { return ~s.busy != 0u; });
   double* part = (double*)workspace(1, (size_t)(blocks + 1) * sizeof(double));
   if (!part) return CUDA_ERROR;
   unsigned* counter = ticket_counters(1);
   if (!counter) return CUDA_ERROR;
-  // eight bytes of pinned memory for the life of the process (one scalar is read at a time: the workspaces above are
-  // the library's, not the caller's, too)
-  static double* host = nullptr;
-  if (!host && cudaHostAlloc((void**)&host, sizeof(double), cudaHostAllocPortable) != cudaSuccess) {
-    host = nullptr;
+  if (!s.words && cudaHostAlloc((void**)&s.words, kScalarWords * sizeof(double), cudaHostAllocPortable) != cudaSuccess) {
+    cudaGetLastError();
+    s.words = nullptr;
     return set_error("pinned allocation for a scalar result failed");
   }
-  if (launch_dependent(k_scalar, dim3((unsigned)blocks), dim3(256), 0, stream(), a->data_device, b ? b->data_device : nullptr, n,
-                       mode, part + 1, counter, host) != cudaSuccess)
+  const int w = __builtin_ctz(~s.busy);
+  double* const host = s.words + w;
+  const cudaStream_t st = stream();
+  if (launch_dependent(k_scalar, dim3((unsigned)blocks), dim3(256), 0, st, a->data_device, b ? b->data_device : nullptr, n, mode,
+                       part + 1, counter, host) != cudaSuccess)
     return set_error(cudaGetErrorString(cudaGetLastError()));
   int err = check_launch();
   if (err) return err;
-  if (cudaStreamSynchronize(stream()) != cudaSuccess) return set_error(cudaGetErrorString(cudaGetLastError()));
-  *result = *(volatile double*)host;
-  return 0;
+  s.busy |= 1u << w;
+  lock.unlock();
+  const bool done = cudaStreamSynchronize(st) == cudaSuccess;
+  if (done) *result = *(volatile double*)host;
+  lock.lock();
+  s.busy &= ~(1u << w);
+  lock.unlock();
+  s.freed.notify_one();
+  return done ? 0 : set_error(cudaGetErrorString(cudaGetLastError()));
 }
 
 }  // namespace
 
 namespace b200 {
+
+void free_scalar_words() {
+  std::lock_guard<std::mutex> lock(g_scalars.mu);
+  if (g_scalars.busy || !g_scalars.words) return;
+  cudaFreeHost(g_scalars.words);
+  g_scalars.words = nullptr;
+}
 
 // target (h or w entries) = beta*target + mult * sum along `axis` of the stored matrix.
 int launch_axis_sum(const float* m, int h, int w, int axis, float* t, float mult, float beta) {

@@ -2,6 +2,8 @@
 boundary.  Integer/0-1 work (random words, Bernoulli thresholds, arg-max one-hots) is
 bit-exact; floating point within the tolerances of cudamat/test_cudamat.py (1e-4
 elementwise, 1e-3 sums) or tighter."""
+import threading
+
 import numpy as np
 import pytest
 
@@ -310,3 +312,27 @@ def test_bias_tail_adds_squares_in_double(cm, V, B):
     acc = cm.empty((1, 1))
     cm.Immediate().rbm_bias_update(data.slice(1, B + 1), zero, h, h, suff, b, db, acc, 1.0 / B, 0.5, 0.1)
     assert get(acc)[0, 0] == np.float32((x.astype(np.float64) ** 2).sum())
+
+
+def test_threads_read_their_own_scalars(cm):
+    """Host threads inside a scalar reduction at the same time, more of them than there are result words, after results on
+    another thread and a shutdown: every call returns its own matrix's value."""
+    rng = np.random.default_rng(4)
+    mats = [cm.CUDAMatrix((rng.random((n, 3)) * (i + 1)).astype(np.float32)) for i, n in enumerate([1, 5, 700, 33000] * 10)]
+    want = [m.euclid_norm() for m in mats]
+    for _ in range(2):
+        wrong = []
+
+        def work(i):
+            for _ in range(50):
+                if mats[i].euclid_norm() != want[i]:
+                    wrong.append(i)
+
+        threads = [threading.Thread(target=work, args=(i,)) for i in range(len(mats))]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert not wrong
+        cm.cublas_shutdown()
+        cm.cublas_init()
