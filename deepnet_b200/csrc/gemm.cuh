@@ -100,6 +100,7 @@ enum SmallForm {
 };
 int gemm_small(const GemmProblem& g, SmallForm form);
 int recompute_nonfinite(const GemmProblem& g);   // non-finite entries of g.epi.out = alpha x the plain fp32 product
+bool small_beats_tc(const GemmProblem& g);  // one launch is the faster one, on operands the tcgen05 kernel takes as they are
 int small_depth(const GemmProblem& g);      // slabs of K that one SM would walk in gemm_small; 0: a list it does not take
 // Returns ERROR_UNSUPPORTED when an operand is not addressable by TMA (leading
 // dimension not a multiple of 4 floats or base not 16-byte aligned).

@@ -30,12 +30,10 @@ inline bool aux_shape_ok(const cudamat* aux, const cudamat* m) {
   return aux->on_device && aux->size[0] == aux_rows(m->size[0]) && aux->size[1] == m->size[1];
 }
 
-// The one-launch kernel (gemm_small.cu) against the tcgen05 one, by the slabs of 32 of K that an SM has to walk.
-// Measured (one launch against product + finishing launch): 4 slabs 10.0 against 15.1 us (500 x 100, K = 784), 8
-// slabs 15.5 against 23.6 (1024 x 256, K = 1024), 16 slabs 28.8 against 30.9 (1024 x 1024, two pairs of K = 256), 40
-// slabs 62 against 20 (512 x 100, K = 10 000).  Where the tcgen05 kernel needs aligned copies of its operands first
-// the line is the same: 8 slabs 21.7 against 26.8 us (1021 x 255, K = 1021), 11 slabs 24.2 against 26.1 (601 x
-// 203, K = 1357), 14 slabs 32.7 against 28.9 (1357 x 601, two pairs of K = 203).
+// Where the tcgen05 kernel needs aligned copies of its operands first: the one-launch kernel (gemm_small.cu) up to so many
+// slabs of 32 of K that an SM has to walk.  Measured (one launch against copies + product + finish): 8 slabs 20.0 against
+// 26.6 us (1021 x 255, K = 1021), 11 slabs 25.1 against 26.3 (601 x 203, K = 1357), 14 slabs 32.7 against 28.9 (1357 x 601,
+// two pairs of K = 203).
 constexpr int kSmallDepth = 11;
 
 // `dot` on operands TMA cannot address and `dot` of little work multiply full fp32 operands with rounding adds (k_gemm_simt,
@@ -62,7 +60,7 @@ int run(const GemmProblem& g) {
   const bool tc = gemm_tc_supported(g);
   const int depth = g_path == 0 ? small_depth(g) : 0;
   int r = ERROR_UNSUPPORTED;
-  if (depth > 0 && depth <= kSmallDepth) r = gemm_small(g, kSmallSplit);
+  if (depth > 0 && (tc ? small_beats_tc(g) : depth <= kSmallDepth)) r = gemm_small(g, kSmallSplit);
   if (r != ERROR_UNSUPPORTED) return r;
   // (unsupported: more operand pairs or tiles than one tensor-core launch carries)
   if (tc) r = gemm_tc(g);
@@ -684,7 +682,7 @@ int dot(cudamat* mat1, cudamat* mat2, cudamat* target, float beta, float alpha) 
     const int r = gemm_small(f, kSmallFp32);
     return r != ERROR_UNSUPPORTED || g_path == 3 ? r : gemm_simt(g);
   }
-  if (g_path == 3 || (g_dot_mode != 1 && small_depth(f) <= kSmallDepth)) {
+  if (g_path == 3 || (g_dot_mode != 1 && small_beats_tc(f))) {
     const int r = gemm_small(f, kSmallIeee);
     if (r != ERROR_UNSUPPORTED || g_path == 3) return r;
   }

@@ -25,12 +25,14 @@
 // need TMA's alignment (or a pass through shared memory), and setting up tensor memory, barriers and
 // roles costs more than these products compute.
 //
-// Bound by instruction issue (the split of the operands and the copies, not the products): a slab takes an SM
-// 0.9 us with two CTAs on it, 1.4 us with one.  Measured, with the error against 64 bits of a logistic layer:
+// Bound by instruction issue (the split of the operands and the copies, not the products): a CTA walks a slab in
+// 1.05 us (two terms) or 1.35 (three) alone on its SM, in 1.1 or 1.5 beside another.  Measured, with the error against 64 bits of a logistic layer:
 //   500 x 100, K = 784       15.1 us (tcgen05 product + finishing launch, 2.0e-7) -> 10.0 us (5.5e-8)
 //   784 x 500, 2 x K = 100   19.2 us                                               -> 12.8 us
 //   1024 x 256, K = 1024     23.6 us                                               -> 15.5 us
 //   601 x 203, K = 1357      519 us (CUDA cores, 2.4e-7)                           -> 24.2 us (6.0e-8)
+#include <initializer_list>
+
 #include "gemm.cuh"
 
 namespace b200 {
@@ -578,6 +580,48 @@ long cut_up(const GemmProblem& g, SmallParams& p) {
   return tiles * p.splits;
 }
 
+int allow_shared_memory() {
+  static bool attr_set[64] = {false};
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return set_error("cudaGetDevice failed");
+  if (!attr_set[dev]) {   // (setting it twice from two threads does no harm)
+    for (void (*kernel)(SmallParams) : {k_gemm_small<true>, k_gemm_small<false>})
+      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem) != cudaSuccess)
+        return set_error("cudaFuncSetAttribute(max dynamic shared memory) failed");
+    attr_set[dev] = true;
+  }
+  return 0;
+}
+
+// CTAs of clusters of `splits` that are resident at the same time (two per SM, less what the clusters leave over in every
+// group of SMs that shares them: 296 CTAs in clusters of four took two waves).
+long resident_ctas(int splits) {
+  static long room[9] = {0};   // (computed twice by two threads: the same value)
+  const long all = 2L * sm_count();
+  if (splits == 1) return all;
+  if (!room[splits]) {
+    if (allow_shared_memory()) return all;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)splits);
+    cfg.blockDim = dim3(kSmallThreads);
+    cfg.dynamicSmemBytes = kSmallSmem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)splits;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, k_gemm_small<false>, &cfg) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      return all;
+    }
+    room[splits] = (long)n * splits;
+  }
+  return room[splits] < all ? room[splits] : all;
+}
+
 // Recomputes what came out non-finite (nothing, as a rule: one read of the result).
 __global__ void __launch_bounds__(256) k_recompute_nonfinite(const __grid_constant__ SmallParams p) {
   grid_dependents_launch();
@@ -613,6 +657,48 @@ int small_depth(const GemmProblem& g) {
   return depth < (1 << 30) ? (int)depth : 1 << 30;
 }
 
+// Whether one launch is faster than the tcgen05 kernel on operands that both take: both sides estimated in us, from
+// about 150 products of 64 x 32 to 4096 x 1024 outputs and K from 16 to 4096.  The line is not one depth: the tcgen05
+// kernel spends 13 us on a plain product of many tiles where this one goes through several waves (2048 x 2048, two pairs of
+// K = 32: 14.9 against 27.1 us at 8 slabs an SM), 39 us on an activation of short K (1024 x 1024, K = 128: 39.5 against
+// 12.2), and cuts a long K over more CTAs (500 x 100, K = 2800: 16.9 against 18.1).
+bool small_beats_tc(const GemmProblem& g) {
+  SmallParams p;
+  if (g.M <= 0 || g.N <= 0 || !gather_pairs(g, p)) return false;
+  const GemmEpilogue& e = g.epi;
+  const bool act = e.bias || e.activation != 0 || e.sample || e.out_aux || e.sample_aux;
+  const long ctas = cut_up(g, p);
+  const int sms = sm_count();
+  // here: a start and an end per wave of two CTAs per SM, and the walk over K; a rows-major operand's slab takes 0.1 more
+  const long room = resident_ctas(p.splits);
+  const float waves = (float)((ctas + room - 1) / room);
+  float walk = 0.0f;
+  int shortest = 1 << 30;
+  for (int q = 0; q < p.npairs; q++) {
+    const SmallPair& s = p.pair[q];
+    const int slabs = (s.k + SK - 1) / SK, terms = 3 - (s.a.exact != 0) - (s.b.exact != 0);
+    const float per_slab = ctas > sms ? 0.3f + 0.41f * terms : 0.45f + 0.3f * terms;
+    walk += slabs * (per_slab + 0.1f * ((s.a.kmajor ? 0 : 1) + (s.b.kmajor ? 0 : 1)));
+    shortest = slabs < shortest ? slabs : shortest;
+  }
+  const float one = waves * ((act ? 6.5f : 5.0f) + walk / p.splits);
+  // there: tiles of 128 rows x up to 256 columns; K is cut (and a second launch finishes) when the tiles fill less than half
+  // of the SMs and every pair has 8 slabs
+  const bool wide = g.N > 128;
+  const long tc_ctas = wide && g.M > 128 ? 2L * ((g.M + 255) / 256) * ((g.N + 255) / 256)
+                                         : (long)((g.M + 127) / 128) * (wide ? (g.N + 255) / 256 : 1);
+  const float n = (float)p.slabs;
+  float tc;
+  if (tc_ctas * 2 <= sms && shortest >= 8) {
+    tc = wide ? (act ? 18.3f : 19.5f) + 0.13f * n : (act ? 9.8f : 11.3f) + 0.07f * n;
+    const float second = wide ? 5.0f - 0.08f * n : 4.0f - 0.03f * n;   // of another pair, hidden behind a long K
+    if (p.npairs > 1 && second > 0.0f) tc += second;
+  } else {
+    tc = act ? (wide ? 39.0f : 17.0f) + 0.3f * n : (wide ? 12.0f : 7.5f) + 0.87f * n;
+  }
+  return one < tc + 1.0f;
+}
+
 // ieee: results that come out non-finite are computed again in plain fp32, so that an infinity in an operand
 // means what it means there (its low part is not a number).
 int gemm_small(const GemmProblem& g, SmallForm form) {
@@ -624,15 +710,9 @@ int gemm_small(const GemmProblem& g, SmallForm form) {
   p.e = g.epi;
   const long ctas = cut_up(g, p);
   if (ctas > 0x7fffffffL) return ERROR_UNSUPPORTED;
-  static bool attr_set[2][64] = {{false}};
   void (*const kernel)(SmallParams) = fp32 ? k_gemm_small<true> : k_gemm_small<false>;
-  int dev = 0;
-  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return set_error("cudaGetDevice failed");
-  if (!attr_set[fp32][dev]) {   // (setting it twice from two threads does no harm)
-    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmallSmem) != cudaSuccess)
-      return set_error("cudaFuncSetAttribute(max dynamic shared memory) failed");
-    attr_set[fp32][dev] = true;
-  }
+  const int err = allow_shared_memory();
+  if (err) return err;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)ctas);
   cfg.blockDim = dim3(kSmallThreads);

@@ -862,3 +862,20 @@ def test_products_of_odd_matrices_do_without_scratch(cm):
     want = A.astype(np.float64) @ B
     for got, w in zip(outs, (want, 1 / (1 + np.exp(-want)), want)):
         assert relerr(get(got), w) < TOL
+
+
+@pytest.mark.parametrize("m,n,k,kernel", [(500, 100, 784, 3), (784, 500, 352, 3), (500, 100, 2800, 1), (2048, 2048, 32, 1),
+                                          (4096, 1024, 64, 1)])
+def test_statistics_take_the_kernel_measured_faster(cm, m, n, k, kernel):
+    """Differences of two outer products: the automatic choice gives the bits of the kernel that was measured faster."""
+    rng = np.random.default_rng(k)
+    A, B, C, D = ((rng.standard_normal(s)).astype(np.float32) for s in ((m, k), (k, n), (m, k), (k, n)))
+    passes = (cm.split_passes(cm.CUDAMatrix(A), cm.CUDAMatrix(B), terms="tf32") +
+              cm.split_passes(cm.CUDAMatrix(C), cm.CUDAMatrix(D), negate=1, terms="tf32"))
+    got = []
+    for path in (0, kernel):
+        cm.set_gemm_path(path)
+        out = cm.empty((m, n))
+        cm.fused_gemm(passes, out=out)
+        got.append(get(out))
+    np.testing.assert_array_equal(got[0], got[1])
