@@ -96,7 +96,8 @@ int gemm_simt(const GemmProblem& g);
 enum SmallForm {
   kSmallSplit,   // split TF32
   kSmallIeee,    // the same, non-finite results computed again in plain fp32
-  kSmallFp32     // fp32 multiply-adds of the full operands (one pair of matrices)
+  kSmallFp32,    // fp32 multiply-adds of the full operands (one pair of matrices)
+  kSmallFp32Parts   // the same for a list of parts: an infinity, whose low part is not a number, gives NaN
 };
 int gemm_small(const GemmProblem& g, SmallForm form);
 int recompute_nonfinite(const GemmProblem& g);   // non-finite entries of g.epi.out = alpha x the plain fp32 product

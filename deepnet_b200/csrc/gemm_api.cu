@@ -52,6 +52,34 @@ constexpr int kSmallDepth = 11;
 // k_gemm_simt was on random operands, and deeper products take it (2047 x 511, K = 2047: 433 / 149 / 127 / 46).
 constexpr int kPackedDotK = 600;
 
+// TF32 terms of odd matrices that the tcgen05 kernel's truncating adds do not suit: chunks of 32 keep the error of long sums
+// below that of k_gemm_simt, which ran them and rounds every addition, but not that of short ones, nor, ever, with an exact
+// operand (0/1).  They take one launch, a short single pair in its fp32 form.  Relative error against float64:
+//                                      k_gemm_simt  copies, tcgen05  one launch, split  one launch, fp32
+//   one pair, K = 64                   3.7e-7       4.3e-7           2.5e-7             1.1e-7
+//   the same, positive operands        2.7e-7       3.7e-7           2.3e-7             0.7e-7
+//   positive operands, K = 400         3.8e-7       3.7e-7           2.0e-7             0.6e-7
+//   0/1 and positive operand, K = 65   8.0e-8       1.2e-7           8.4e-8             4.2e-8
+//   the same, K = 801                  8.0e-8       1.2e-7           9.0e-8             1.05e-7   (an ulp: 1.2e-7)
+//   difference of two of K = 32        1.9e-6       2.0e-6           0.6e-6
+//   difference of two of K = 64        2.7e-6       2.2e-6           1.5e-6
+enum { kAnyLength, kOneLaunchFp32, kOneLaunch };
+int short_tf32(const GemmProblem& g) {
+  long k = 0;
+  int pairs = 0, low = 0;
+  for (int q = 0; q < g.npass; q++) {
+    const int pa = g.pass[q].a.part, pb = g.pass[q].b.part;
+    if (pa == kPartX && pb == kPartX) {
+      k += g.pass[q].k;
+      pairs++;
+    }
+    if (pa == kPartLo32 || pb == kPartLo32) low++;
+  }
+  if (!low) return kAnyLength;
+  if (pairs == 1 && k < 400) return kOneLaunchFp32;
+  return k < 128 || (pairs == 1 && low == 1) ? kOneLaunch : kAnyLength;
+}
+
 int run(const GemmProblem& g) {
   if (product_is_scattered(g.epi.out)) return gemm_tc(g);   // (fails loudly when the tensor-core kernel cannot take it)
   if (g_path == 2) return gemm_simt(g);
@@ -60,7 +88,10 @@ int run(const GemmProblem& g) {
   const bool tc = gemm_tc_supported(g);
   const int depth = g_path == 0 ? small_depth(g) : 0;
   int r = ERROR_UNSUPPORTED;
-  if (depth > 0 && (tc ? small_beats_tc(g) : depth <= kSmallDepth)) r = gemm_small(g, kSmallSplit);
+  const int tf32 = tc || !depth ? kAnyLength : short_tf32(g);
+  if (tf32 == kOneLaunchFp32) r = gemm_small(g, kSmallFp32Parts);
+  if (r != ERROR_UNSUPPORTED) return r;
+  if (depth > 0 && (tc ? small_beats_tc(g) : depth <= kSmallDepth || tf32 != kAnyLength)) r = gemm_small(g, kSmallSplit);
   if (r != ERROR_UNSUPPORTED) return r;
   // (unsupported: more operand pairs or tiles than one tensor-core launch carries)
   if (tc) r = gemm_tc(g);

@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(kSmallThreads, 2) k_gemm_small(const __grid_co
       }
     }
     const int ncols = min(4, p.N - n);
-    if (!kFp32) {
+    if (!kFp32 || !p.ieee) {
 #pragma unroll
       for (int j = 0; j < 4; j++)
         if (j < ncols && !isfinite(x[j])) x[j] = p.ieee ? element_fp32(p, m, n + j) : element_truncated(p, m, n + j);
@@ -704,9 +704,9 @@ bool small_beats_tc(const GemmProblem& g) {
 int gemm_small(const GemmProblem& g, SmallForm form) {
   SmallParams p;
   if (g.M <= 0 || g.N <= 0 || !gather_pairs(g, p)) return ERROR_UNSUPPORTED;
-  const bool fp32 = form == kSmallFp32;
+  const bool fp32 = form == kSmallFp32 || form == kSmallFp32Parts;
   if (fp32 && (p.npairs != 1 || p.pair[0].negate)) return ERROR_UNSUPPORTED;
-  p.ieee = form == kSmallIeee;
+  p.ieee = form == kSmallIeee || form == kSmallFp32;
   p.e = g.epi;
   const long ctas = cut_up(g, p);
   if (ctas > 0x7fffffffL) return ERROR_UNSUPPORTED;

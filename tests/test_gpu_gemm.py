@@ -879,3 +879,26 @@ def test_statistics_take_the_kernel_measured_faster(cm, m, n, k, kernel):
         cm.fused_gemm(passes, out=out)
         got.append(get(out))
     np.testing.assert_array_equal(got[0], got[1])
+
+
+@pytest.mark.parametrize("exact", [False, True])
+@pytest.mark.parametrize("m,n,k", [(2047, 2047, 96), (1025, 4095, 65), (2047, 2047, 399), (1025, 1023, 801)])
+def test_tf32_products_of_odd_matrices_lose_no_bits(cm, exact, m, n, k):
+    """TF32 products of odd matrices, deeper than one launch is given for its speed: their error against float64 is no larger
+    than that of the CUDA-core kernel on the same terms (1 %: chance), but for long sums with a 0/1 side,
+    which lie below an ulp of the result in every form.  An infinity's low part is not a number."""
+    rng = np.random.default_rng(k)
+    A = ((rng.random((m, k)) < 0.2) if exact else rng.standard_normal((m, k))).astype(np.float32)
+    B = rng.random((k, n)).astype(np.float32)
+    want = A.astype(np.float64) @ B
+    err = []
+    for path in (0, 2):
+        cm.set_gemm_path(path)
+        out = cm.empty((m, n))
+        cm.fused_gemm(cm.split_passes(cm.CUDAMatrix(A), cm.CUDAMatrix(B), exact_a=exact, terms="tf32"), out=out)
+        err.append(np.linalg.norm(get(out) - want))
+    assert err[0] <= (1.01 * err[1] if k < 400 or not exact else 2.0 ** -23 * np.linalg.norm(want))
+    cm.set_gemm_path(0)
+    B[3, 4] = np.inf
+    cm.fused_gemm(cm.split_passes(cm.CUDAMatrix(A), cm.CUDAMatrix(B), exact_a=exact, terms="tf32"), out=out)
+    assert np.isnan(get(out)[:, 4]).all() and np.isfinite(np.delete(get(out), 4, axis=1)).all()
