@@ -1092,7 +1092,8 @@ def cuda_sync_threads():
 
 
 def set_gemm_path(path):
-    """0 auto, 1 the tcgen05 kernel only, 2 CUDA cores only, 3 the one-launch kernel for small products only."""
+    """0 auto; one kernel only: 1 tcgen05, 2 CUDA cores, 3 the one-launch kernel for small products, 4 tcgen05 behind aligned
+    copies of its operands."""
     _lib.b200_set_gemm_path(ct.c_int(path))
 
 

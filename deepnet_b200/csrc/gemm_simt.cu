@@ -1,6 +1,6 @@
-// fp32 CUDA-core product for operands the tensor-core path cannot address (leading
-// dimensions that are not multiples of 4 floats, unaligned views) and for tiny
-// problems.  64x64 output tile, 16-deep slices in shared memory, 4x4 outputs per
+// fp32 CUDA-core product of any term list: what no other kernel takes (lists that are not whole products, more
+// operand pairs than one launch carries, an empty inner dimension), and the plain form the others are
+// compared with (b200_set_gemm_path(2)).  64x64 output tile, 16-deep slices in shared memory, 4x4 outputs per
 // thread, every edge bounds-checked.  Same pass list and epilogue as the tcgen05 kernel.
 #include "gemm.cuh"
 

@@ -162,8 +162,9 @@ int copy_transpose(cudamat* source, cudamat* target);                           
 int normlimit_by_axis(cudamat* mat, cudamat* target, int axis, float norm);                 /* cudamat.cu:1289 (axis 0 only, as there) */
 
 /* ---- matrix product: cudamat/cudamat.cu:1671-1696 (cublasSgemm) ---------------------- */
-/* target = beta * target + alpha * op(mat1) . op(mat2); tcgen05 split-TF32 when the
- * operands are TMA-addressable (leading dimension a multiple of 4, 16-byte aligned). */
+/* target = beta * target + alpha * op(mat1) . op(mat2).  Split TF32 on the tensor cores when the operands are
+ * TMA-addressable (leading dimension a multiple of 4, 16-byte aligned) and m n k >= 2^21, or behind aligned
+ * copies for deep products from k = 600 on; full fp32 multiply-adds otherwise (selections exact bit for bit). */
 int dot(cudamat* mat1, cudamat* mat2, cudamat* target, float beta, float alpha);
 
 /* ================= additions: no counterpart in the reference ======================== */
@@ -290,8 +291,8 @@ int add_sq_diff(cudamat* a, cudamat* b, cudamat* acc);
 
 /* Library control. */
 int b200_device_count(void);
-int b200_set_stream(void* cuda_stream);   /* NULL restores the library's own stream; scratch is kept per stream, for up to
-                                           * eight of them: a ninth waits for the device, then takes one over */
+int b200_set_stream(void* cuda_stream);   /* NULL restores the library's own stream; scratch is kept per stream, for that
+                                           * one and seven more: the next waits for the device, then takes one over */
 void* b200_get_stream(void);
 void* b200_event_create(void);            /* CUDA events recorded on the library stream */
 int b200_event_record(void* ev);
@@ -324,7 +325,8 @@ int ais_binary_steps(rnd_struct* rnd_state, cudamat* w, cudamat* w_aux, cudamat*
  * [visible | hidden] in one launch (deepnet/layer.py:202-213, parameter.py:80-106, logistic_layer.py:48-52). */
 int rbm_bias_update(cudamat* v_pos, cudamat* v_neg, cudamat* h_pos, cudamat* h_neg, cudamat* suff, cudamat* b, cudamat* db,
                     cudamat* sq_acc, float inv_batch, float momentum, float eps);
-int b200_set_gemm_path(int path);         /* 0 auto, 1 tcgen05 kernel only, 2 CUDA cores only, 3 one-launch kernel only */
+int b200_set_gemm_path(int path);         /* 0 auto; one kernel only: 1 tcgen05, 2 CUDA cores, 3 one launch, 4 tcgen05 behind
+                                           * aligned copies of its operands */
 int b200_set_dot_precision(int mode);     /* 0 fp32-grade split TF32 (default), 1 one TF32 pass */
 /* Split-K of the tensor-core product: 0 (default) = cut the inner dimension into work items when the
  * output tiles alone would leave most SMs idle, 1 = never, n > 1 = always n splits.  No counterpart
