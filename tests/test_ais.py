@@ -72,6 +72,43 @@ def test_ais_at_layer_sizes_of_the_reference_models(cm):
     assert abs(log_z - want) < 0.5
 
 
+@pytest.mark.gpu
+@pytest.mark.parametrize("col0", [0, 3])
+@pytest.mark.parametrize("V,H,B", [(301, 517, 5), (17, 33, 203), (260, 255, 1)])
+def test_annealing_steps_match_the_call_by_call_form(cm, col0, V, H, B):
+    """The steps issued from C against the reference's calls on the device, chain by chain: layers of more than one pass of a
+    block and odd ones, nonzero biases, a shard whose first column is not a multiple of four.  Both consume one random
+    stream; a draw may differ where two correct probabilities straddle its uniform, about one in 10^7."""
+    w, a, b = small_rbm(V=V, H=H, scale=0.1, seed=V)
+    schedule = np.linspace(0.0, 1.0, 8)
+    cm.set_rng_column_offset(col0)
+    try:
+        got, want = (ais.ais_binary_rbm(cm, w, a, b, B, schedule, seed=9, fused=fused) for fused in (True, False))
+    finally:
+        cm.set_rng_column_offset(0)
+    # bound: fp32 sums of V + H terms a step, whose sizes are those of the log weights' own parts
+    np.testing.assert_allclose(got[1], want[1], rtol=0, atol=1e-4 * np.abs(want[1]).max() + 1e-3)
+    assert cm.CUDAMatrix.rnd_state.calls == 1 + 2 * (len(schedule) - 1)
+
+
+@pytest.mark.gpu
+def test_annealing_steps_refuse_shapes_that_do_not_fit(cm):
+    cm.CUDAMatrix.init_random(1)
+    V, H, B = 12, 8, 5
+    good = dict(w=(V, H), a=(H, 1), b=(V, 1), v_state=(V, B), v_sample=(V, B), h_pre=(H, B), h_sample=(H, B), weights=(1, B))
+
+    def call(**shapes):
+        m = {k: cm.empty(s) for k, s in dict(good, **shapes).items()}
+        cm.ais_binary_steps(m["w"], m["w"].split_bf16(cm.empty_aux(m["w"].shape)), m["a"], m["b"], m["v_state"], m["v_sample"],
+                            m["h_pre"], m["h_sample"], m["weights"], [0.0, 0.5, 1.0])
+
+    call()
+    for name, shape in (("w", (V, H + 1)), ("a", (H + 1, 1)), ("b", (V + 1, 1)), ("v_state", (V + 1, B)), ("v_sample", (V, B + 1)),
+                        ("h_pre", (H, B + 1)), ("h_sample", (H + 1, B)), ("weights", (1, B - 1))):
+        with pytest.raises(cm.CUDAMatException):
+            call(**{name: shape})
+
+
 def small_rs_rbm(V=30, H=8, seed=4):
     rng = np.random.default_rng(seed)
     return ((rng.standard_normal((V, H)) * 0.3).astype(np.float32), (rng.standard_normal(H) * 0.1).astype(np.float32),

@@ -583,7 +583,7 @@ def test_momentum_update_by_column_panels_equals_the_whole_update(cm, mode):
 def test_one_launch_product_in_all_layouts(cm, ta, tb, m, n, k):
     """gemm_small.cu: edges of tiles and slabs, 16-byte and 4-byte copies, one to eight CTAs along K; two pairs of
     matrices (the second negated, its left side exact), bias x column scale, beta.
-    Bound: 3 * 2^-23 per term from the split, 12 truncating additions (2^-23 each) per two slabs and one rounding (2^-24)
+    Bound: 2^-21 per term from the split, 12 truncating additions (2^-23 each) per two slabs and one rounding (2^-24)
     per two slabs, of sum |a||b|: below 2^-18 for k <= 2000."""
     rng = np.random.default_rng(m * 7 + n * 3 + k)
     A, A2 = rng.standard_normal((m, k)).astype(np.float32), (rng.random((m, k + 1)) < 0.4).astype(np.float32)
@@ -902,3 +902,37 @@ def test_tf32_products_of_odd_matrices_lose_no_bits(cm, exact, m, n, k):
     B[3, 4] = np.inf
     cm.fused_gemm(cm.split_passes(cm.CUDAMatrix(A), cm.CUDAMatrix(B), exact_a=exact, terms="tf32"), out=out)
     assert np.isnan(get(out)[:, 4]).all() and np.isfinite(np.delete(get(out), 4, axis=1)).all()
+
+
+@pytest.mark.parametrize("ta,tb", [(0, 0), (1, 0), (0, 1), (1, 1)])
+@pytest.mark.parametrize("m,n,k", [(129, 65, 33), (257, 259, 130), (1501, 301, 1501)])
+def test_plain_product_behind_aligned_copies(cm, ta, tb, m, n, k):
+    """One product, not the difference of two of the same copies: against float64.  Bound: 2^-20 per term and chunks of 32
+    whose adds truncate, of sum |a||b| (below 2^-18 at any K)."""
+    rng = np.random.default_rng(m + n + k)
+    A, B = rng.standard_normal((m, k)).astype(np.float32), rng.standard_normal((k, n)).astype(np.float32)
+    d = lambda x: x.astype(np.float64)
+    cm.set_gemm_path(4)
+    out = cm.empty((m, n))
+    cm.fused_gemm(cm.split_passes(make(cm, A, ta), make(cm, B, tb), terms="tf32"), out=out, alpha=0.5)
+    assert (np.abs(get(out) - 0.5 * (d(A) @ d(B))) <= 2.0 ** -18 * 0.5 * (np.abs(d(A)) @ np.abs(d(B)))).all()
+    got = get(cm.dot(make(cm, A, ta), make(cm, B, tb), 3.0))
+    assert (np.abs(got - 3.0 * (d(A) @ d(B))) <= 2.0 ** -18 * 3.0 * (np.abs(d(A)) @ np.abs(d(B)))).all()
+
+
+@pytest.mark.parametrize("alpha", [1.0, -0.5])
+@pytest.mark.parametrize("ta,tb", [(0, 0), (1, 0), (0, 1), (1, 1)])
+def test_deep_unaligned_dot_keeps_infinities_in_all_layouts(cm, ta, tb, alpha):
+    """Behind aligned copies (K of 600 and more): what came out non-finite is computed again from the operands themselves."""
+    rng = np.random.default_rng(3)
+    m, n, k = 1501, 301, 1501
+    A, B = rng.standard_normal((m, k)).astype(np.float32), rng.random((k, n)).astype(np.float32) + 0.5
+    want = alpha * (A.astype(np.float64) @ B)
+    A[3, 5], A[9, 2] = np.inf, np.nan
+    B[1000, 7] = np.float32(np.inf)
+    got = get(cm.dot(make(cm, A, ta), make(cm, B, tb), alpha))
+    rest = np.delete(np.arange(m), [3, 9])
+    assert (got[3, np.arange(n) != 7] == alpha * np.inf).all() and np.isnan(got[9]).all()
+    np.testing.assert_array_equal(got[rest, 7], np.sign(alpha * A[rest, 1000]) * np.inf)
+    cols = np.delete(np.arange(n), 7)
+    assert relerr(got[np.ix_(rest, cols)], want[np.ix_(rest, cols)]) < TOL

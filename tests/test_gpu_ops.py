@@ -336,3 +336,19 @@ def test_threads_read_their_own_scalars(cm):
         assert not wrong
         cm.cublas_shutdown()
         cm.cublas_init()
+
+
+@pytest.mark.parametrize("shape", [(1, 1), (255, 1), (256, 1), (257, 3), (1000, 37), (4096, 301)])
+def test_scalar_reductions_after_a_squared_difference(cm, shape):
+    """One block to as many as there are, each fold by the block that ends last, on counters that add_sq_diff used before."""
+    rng = np.random.default_rng(shape[0])
+    a, b = (rng.standard_normal(shape).astype(np.float32) for _ in range(2))
+    ga, gb, acc = cm.CUDAMatrix(a), cm.CUDAMatrix(b), cm.empty((1, 1))
+    a, b = a.astype(np.float64), b.astype(np.float64)
+    for turn in range(1, 4):
+        cm.Immediate().sq_diff(ga, gb, acc)
+        assert abs(ga.euclid_norm() - np.sqrt((a * a).sum())) <= 1e-6 * np.sqrt((a * a).sum())
+        cm.Immediate().sq_diff(ga, gb, acc)
+        assert abs(cm.vdot(ga, gb) - (a * b).sum()) <= 1e-6 * np.abs(a * b).sum()
+        want = 2 * turn * ((a - b) ** 2).sum()
+        assert abs(get(acc)[0, 0] - want) <= 1e-6 * want
