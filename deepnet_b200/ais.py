@@ -39,7 +39,9 @@ def ais_binary_rbm(cm, weight, hidden_bias, visible_bias, num_chains, schedule, 
     cm.CUDAMatrix.init_random(seed)
     B = num_chains
     v_state, v_sample = cm.empty((V, B)), cm.empty((V, B))
-    h_state, h_temp, h_deriv, h_sample = cm.empty((H, B)), cm.empty((H, B)), cm.empty((H, B)), cm.empty((H, B))
+    h_state, h_sample = cm.empty((H, B)), cm.empty((H, B))
+    if not fused:
+        h_temp, h_deriv = cm.empty((H, B)), cm.empty((H, B))
     # chains start from the uniform model: state = sigmoid(0), one Bernoulli draw (deepnet/ais.py:146-148)
     v_state.assign(0)
     cm.sigmoid(v_state)
