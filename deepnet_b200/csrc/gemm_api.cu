@@ -86,18 +86,20 @@ int run(const GemmProblem& g) {
   if (g_path == 3) return gemm_small(g, kSmallSplit);
   if (g_path == 4) return gemm_tc_packed(g);
   const bool tc = gemm_tc_supported(g);
-  const int depth = g_path == 0 ? small_depth(g) : 0;
   int r = ERROR_UNSUPPORTED;
-  const int tf32 = tc || !depth ? kAnyLength : short_tf32(g);
-  if (tf32 == kOneLaunchFp32) r = gemm_small(g, kSmallFp32Parts);
-  if (r != ERROR_UNSUPPORTED) return r;
-  if (depth > 0 && (tc ? small_beats_tc(g) : depth <= kSmallDepth || tf32 != kAnyLength)) r = gemm_small(g, kSmallSplit);
+  if (g_path == 0 && tc) {
+    if (small_beats_tc(g)) r = gemm_small(g, kSmallSplit);
+  } else if (g_path == 0) {
+    const int tf32 = short_tf32(g), depth = small_depth(g);
+    if (tf32 == kOneLaunchFp32) r = gemm_small(g, kSmallFp32Parts);
+    if (r == ERROR_UNSUPPORTED && depth > 0 && (depth <= kSmallDepth || tf32 != kAnyLength)) r = gemm_small(g, kSmallSplit);
+  }
   if (r != ERROR_UNSUPPORTED) return r;
   // (unsupported: more operand pairs or tiles than one tensor-core launch carries)
   if (tc) r = gemm_tc(g);
   else if (g_path == 0) r = gemm_tc_packed(g);
   if (r != ERROR_UNSUPPORTED || g_path == 1) return r;
-  if (depth > 0) r = gemm_small(g, kSmallSplit);
+  r = gemm_small(g, kSmallSplit);
   return r != ERROR_UNSUPPORTED ? r : gemm_simt(g);
 }
 

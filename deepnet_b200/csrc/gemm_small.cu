@@ -468,7 +468,7 @@ __global__ void __launch_bounds__(kSmallThreads, 2) k_gemm_small(const __grid_co
       }
     }
     const int ncols = min(4, p.N - n);
-    if (!kFp32 || !p.ieee) {
+    if ((!kFp32 || !p.ieee) && !isfinite((x[0] + x[1]) + (x[2] + x[3]))) {   // (a finite sum has finite terms)
 #pragma unroll
       for (int j = 0; j < 4; j++)
         if (j < ncols && !isfinite(x[j])) x[j] = p.ieee ? element_fp32(p, m, n + j) : element_truncated(p, m, n + j);
