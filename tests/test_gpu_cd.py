@@ -293,6 +293,32 @@ def test_fused_softmax_ops_match_the_call_sequence(cm, oracle):
     assert cm.CUDAMatrix.rnd_state.calls == B
 
 
+@pytest.mark.parametrize("V", [512, 513, 4096, 4097, 9001])
+def test_multinomial_draws_equal_the_call_sequence_at_any_vocabulary(cm, V):
+    """Words that a bound rules out are passed over without their logarithm: the counts stay those of the per-document
+    loop, word for word, also with words of probability zero, one dominant word, one usable word and none."""
+    rng = np.random.default_rng(V)
+    B = 5
+    p = rng.random((V, B)).astype(np.float32) ** 8
+    p[rng.random((V, B)) < 0.3] = 0.0
+    p[V - 1, 1] = 50.0 * p[:, 1].sum()
+    p[:, 2] = 0.0
+    p[V // 2, 2] = 3.0
+    p[:, 3] = 0.0
+    lens = np.array([[40, 7, 9, 5, 1]], np.float32)
+    cm.CUDAMatrix.init_random(8)
+    lay = dbm.ReplicatedSoftmaxLayer(cm, "v", V, dbm.Hyperparams(sample_input=True), is_input=True)
+    lay.AllocateMemory(B)
+    lay.state.assign(cm.CUDAMatrix(p))
+    lay.NN.assign(cm.CUDAMatrix(lens))
+    cm.CUDAMatrix.init_random(8)
+    lay.Sample()
+    cm.CUDAMatrix.init_random(8)
+    fused = get(cm.CUDAMatrix(p).sample_multinomial(cm.CUDAMatrix(lens), cm.empty((V, B))))
+    np.testing.assert_array_equal(fused, get(lay.sample))
+    np.testing.assert_array_equal(fused.sum(axis=0), lens.ravel())
+
+
 @pytest.mark.parametrize("scale", [0.02, 1.0])
 def test_fused_engine_replicated_softmax_matches_oracle(cm, oracle, scale):
     # config 2 at 1/50 size and at its full size (10 000 words, 512 hidden units, documents of about
