@@ -109,6 +109,18 @@ int gemm_tc(const GemmProblem& g);
 bool gemm_tc_supported(const GemmProblem& g);
 int gemm_tc_packed(const GemmProblem& g);   // the same behind a copy of the operands TMA cannot address
 
+// The annealing steps 1 .. n - 1 of a binary RBM in one launch (chains.cu); ERROR_UNSUPPORTED where single products are the
+// faster way.  The chains start from 0/1 states.
+struct AisChains {
+  const float *w, *a, *b;
+  float *v_state, *v_sample, *h_pre, *h_sample, *sb, *weights;
+  int V, H, B;
+  const double* schedule;
+  int n;
+  unsigned long long seed, call0;
+};
+int ais_chains(const AisChains& a);
+
 #ifdef __CUDACC__
 // Applies the epilogue to one accumulator value and stores every requested output.
 // `u` is the uniform of this element (only read when e.sample != null).

@@ -867,6 +867,14 @@ extern "C" int ais_binary_steps(rnd_struct* rnd_state, cudamat* w, cudamat* w_au
       !same_shape(h_pre, h_sample))
     return ERROR_INCOMPATIBLE_DIMENSIONS;
   if ((long)V * H * B == 0) return 0;
+  if (g_path == 0) {
+    const AisChains c = {w->data_device, a->data_device, b->data_device, v_state->data_device, v_sample->data_device,
+                         h_pre->data_device, h_sample->data_device, sb->data_device, weights->data_device,
+                         V, H, B, schedule, n, rnd_state->seed, rnd_state->calls};
+    const int err = ais_chains(c);
+    if (err == 0) rnd_state->calls += 2ull * (n - 1);
+    if (err != ERROR_UNSUPPORTED) return err;
+  }
   cudamat wt = *w;
   wt.is_trans = 1;
   b200_fused_gemm up = {}, down = {};

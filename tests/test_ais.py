@@ -92,6 +92,27 @@ def test_annealing_steps_match_the_call_by_call_form(cm, col0, V, H, B):
 
 
 @pytest.mark.gpu
+@pytest.mark.parametrize("V,H,B,steps", [(784, 500, 100, 20), (64, 9, 1, 4), (97, 128, 33, 300), (1024, 129, 37, 5), (5, 3, 2, 3)])
+def test_annealing_in_one_launch_matches_the_products(cm, V, H, B, steps):
+    """All steps in one launch against three launches a step (the products on CUDA cores), chain by chain: columns left in
+    global memory, whole and ragged quads of rows, fewer hidden units than blocks, more temperatures than travel with a launch.
+    One chain may go elsewhere, where a draw's uniform falls between two correct probabilities."""
+    w, a, b = small_rbm(V=V, H=H, scale=0.05, seed=V)
+    schedule = np.linspace(0.0, 1.0, steps + 1)
+    got = ais.ais_binary_rbm(cm, w, a, b, B, schedule, seed=9)
+    calls = cm.CUDAMatrix.rnd_state.calls
+    cm.set_gemm_path(2)
+    try:
+        want = ais.ais_binary_rbm(cm, w, a, b, B, schedule, seed=9)
+    finally:
+        cm.set_gemm_path(0)
+    # bound: the log weights of the other form are fp32 sums over `steps` of fp32 sums of V + H terms
+    assert (np.abs(got[1] - want[1]) > 1e-4 * np.abs(want[1]).max() + 1e-3).sum() <= 1
+    assert calls == cm.CUDAMatrix.rnd_state.calls == 1 + 2 * steps
+    assert cm.read_status() == 0
+
+
+@pytest.mark.gpu
 def test_annealing_steps_refuse_shapes_that_do_not_fit(cm):
     cm.CUDAMatrix.init_random(1)
     V, H, B = 12, 8, 5
