@@ -805,7 +805,8 @@ def _build_fused_gemm(passes, out=None, sample=None, bias=None, col_scale=None, 
 (OP_FUSED_GEMM, OP_SUM_AXIS, OP_ADD_SUM_AXIS, OP_ROW_SUM_DIFF, OP_ADD_SQ_DIFF, OP_MOMENTUM_UPDATE, OP_SPLIT_F16,
  OP_SPLIT_BF16, OP_ALLREDUCE, OP_SOFTMAX_SCALED, OP_SAMPLE_MULTINOMIAL, OP_DIV_BY_ROW, OP_ADD_SCALAR, OP_ASSIGN_SCALAR,
  OP_COPY, OP_SAMPLE_BERNOULLI, OP_SOFTMAX_SAMPLE, OP_MOMENTUM_UPDATE_COLUMNS, OP_ALLREDUCE_BEGIN, OP_ALLREDUCE_END,
- OP_SM_LIMIT, OP_DP_PEER_UPDATE, OP_RBM_BIAS_UPDATE) = range(23)
+ OP_SM_LIMIT, OP_DP_PEER_UPDATE, OP_RBM_BIAS_UPDATE, OP_SOFTMAX_RECONSTRUCTION,
+ OP_DOCUMENT_LENGTHS) = range(25)
 
 
 class _Op(ct.Structure):
@@ -879,6 +880,15 @@ class Immediate(object):
 
     def softmax_scaled(self, mat, scale, target):
         mat.softmax_scaled(scale, target)
+
+    def softmax_reconstruction(self, pre, nn, state, norm, data=None, acc=None):
+        """state = nn softmax(pre), norm = state / nn; with data: acc += sum (norm - data)^2."""
+        p = lambda m: m.p_mat if m is not None else None
+        _check(_lib.softmax_reconstruction(pre.p_mat, nn.p_mat, state.p_mat, norm.p_mat, p(data), p(acc)))
+
+    def document_lengths(self, counts, nn, norm, tiny):
+        """nn = column sums of counts + tiny, norm = counts / nn."""
+        _check(_lib.document_lengths(counts.p_mat, nn.p_mat, norm.p_mat, ct.c_float(tiny)))
 
     def sample_multinomial(self, probs, nn, target, max_draws=1000):
         probs.sample_multinomial(nn, target, max_draws)
@@ -981,6 +991,12 @@ class Program(object):
 
     def softmax_scaled(self, mat, scale, target):
         return self._add(OP_SOFTMAX_SCALED, (mat, scale, target))
+
+    def softmax_reconstruction(self, pre, nn, state, norm, data=None, acc=None):
+        return self._add(OP_SOFTMAX_RECONSTRUCTION, (pre, nn, state, norm, data, acc))
+
+    def document_lengths(self, counts, nn, norm, tiny):
+        return self._add(OP_DOCUMENT_LENGTHS, (counts, nn, norm), (), (tiny,))
 
     def sample_multinomial(self, probs, nn, target, max_draws=1000):
         return self._add(OP_SAMPLE_MULTINOMIAL, (probs, nn, target), (max_draws,))

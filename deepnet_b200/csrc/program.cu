@@ -31,6 +31,8 @@ int rbm_bias_update(cudamat* v_pos, cudamat* v_neg, cudamat* h_pos, cudamat* h_n
 int split_f16(cudamat* x, cudamat* aux, cudamat* exp_dev, int exp_const);
 int split_bf16(cudamat* x, cudamat* aux);
 int dp_allreduce(cudamat* mat);
+int softmax_reconstruction(cudamat* pre, cudamat* nn, cudamat* state, cudamat* norm, cudamat* data, cudamat* acc);
+int document_lengths(cudamat* counts, cudamat* nn, cudamat* norm, float tiny);
 int softmax_scaled(cudamat* mat, cudamat* scale, cudamat* target);
 int sample_multinomial(rnd_struct* rnd_state, cudamat* probs, cudamat* nn, cudamat* target, int max_draws);
 int div_by_row_vec(cudamat* mat, cudamat* vec, cudamat* target);
@@ -65,6 +67,8 @@ enum {
   B200_OP_SM_LIMIT = 20,          // i0 SMs the following kernels size their grids for (0 = all)
   B200_OP_DP_PEER_UPDATE = 21,    // m0 w, m1 delta, m2 w_aux?, m3 w_scale?, m4 pack, m5 b, m6 db; f0 inv_batch, f1 mom_b, f2 eps_b, f3 mom_w, f4 eps_w, f5 l2, f6 l1
   B200_OP_RBM_BIAS_UPDATE = 22,   // m0 v_pos, m1 v_neg, m2 h_pos, m3 h_neg, m4 suff, m5 b, m6 db, m7 sq_acc?; f0 inv_batch, f1 momentum, f2 eps
+  B200_OP_SOFTMAX_RECONSTRUCTION = 23,   // m0 pre, m1 nn, m2 state, m3 norm, m4 data?, m5 acc?
+  B200_OP_DOCUMENT_LENGTHS = 24,  // m0 counts, m1 nn, m2 norm, f0 tiny
   B200_OP_COUNT
 };
 
@@ -114,6 +118,8 @@ extern "C" int b200_run_program(rnd_struct* rnd_state, b200_op* ops, int n, int*
       case B200_OP_RBM_BIAS_UPDATE:
         err = rbm_bias_update(o.m[0], o.m[1], o.m[2], o.m[3], o.m[4], o.m[5], o.m[6], o.m[7], o.f0, o.f1, o.f2);
         break;
+      case B200_OP_SOFTMAX_RECONSTRUCTION: err = softmax_reconstruction(o.m[0], o.m[1], o.m[2], o.m[3], o.m[4], o.m[5]); break;
+      case B200_OP_DOCUMENT_LENGTHS: err = document_lengths(o.m[0], o.m[1], o.m[2], o.f0); break;
       default: break;
     }
     if (err) {

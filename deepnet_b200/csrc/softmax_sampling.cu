@@ -58,6 +58,143 @@ __global__ void __launch_bounds__(256) k_softmax_scaled(const float* m, const fl
   }
 }
 
+// One block of up to 1024 threads per column, the column in registers: kPer values a thread, read once.  Bound by the
+// latency of that read and of the block's sums: a few columns of some thousand words do not fill the device.
+constexpr int kColumnMax = 16 * 1024;      // longest column kept in registers
+template <typename F>
+__device__ __forceinline__ float block_fold(float v, float* red, float none, F f) {
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = f(v, __shfl_xor_sync(0xffffffffu, v, o));
+  __syncthreads();               // (red is free: what it held has been read)
+  if (lane == 0) red[wid] = v;
+  __syncthreads();
+  v = lane < nw ? red[lane] : none;
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v = f(v, __shfl_xor_sync(0xffffffffu, v, o));
+  return v;
+}
+__device__ __forceinline__ float add_f(float a, float b) { return a + b; }
+
+// state = scale softmax(m) by columns; with norm: norm = state / scale; with acc: *acc += sum (norm - data)^2, the columns'
+// errors added in column order by the block that finishes last.
+template <int kPer>
+__global__ void __launch_bounds__(1024) k_softmax_columns(const float* __restrict__ m, const float* __restrict__ scale, float* state,
+                                                          float* norm, const float* data, double* part, unsigned* counter,
+                                                          float* acc, int h, int w) {
+  __shared__ float red[32];
+  __shared__ double dred[32];
+  __shared__ bool is_last;
+  grid_dependents_launch();
+  grid_dependency_wait();
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+  for (int c = blockIdx.x; c < w; c += gridDim.x) {
+    const long at = (long)c * h;
+    float x[kPer], mx = -INFINITY;
+#pragma unroll
+    for (int i = 0; i < kPer; i++) {
+      const int r = threadIdx.x + i * (int)blockDim.x;
+      x[i] = r < h ? m[at + r] : -INFINITY;
+    }
+#pragma unroll
+    for (int i = 0; i < kPer; i++) mx = fmaxf(mx, x[i]);
+    mx = block_fold(mx, red, -INFINITY, fmaxf);
+    float s = 0.0f;
+#pragma unroll
+    for (int i = 0; i < kPer; i++) {
+      const int r = threadIdx.x + i * (int)blockDim.x;
+      x[i] = r < h ? expf(x[i] - mx) : 0.0f;
+      s += x[i];
+    }
+    s = block_fold(s, red, 0.0f, add_f);
+    const float n = scale[c], f = n / s;   // NN / sum, then one multiply per element (mult_by_row)
+    double e = 0.0;
+#pragma unroll
+    for (int i = 0; i < kPer; i++) {
+      const int r = threadIdx.x + i * (int)blockDim.x;
+      if (r >= h) continue;
+      x[i] *= f;
+      state[at + r] = x[i];
+      if (norm) {
+        const float y = x[i] / n;
+        norm[at + r] = y;
+        if (acc) {
+          const float d = y - data[at + r];
+          e += (double)d * d;
+        }
+      }
+    }
+    if (acc) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+      __syncthreads();
+      if (lane == 0) dred[wid] = e;
+      __syncthreads();
+      if (threadIdx.x == 0) {
+        double t = 0.0;
+        for (int i = 0; i < nw; i++) t += dred[i];
+        part[c] = t;
+      }
+    }
+  }
+  if (!acc) return;
+  if (threadIdx.x == 0) {
+    __threadfence();
+    is_last = atomicAdd(counter, 1u) == gridDim.x - 1;
+  }
+  __syncthreads();
+  if (!is_last || wid != 0) return;
+  __threadfence();
+  double t = 0.0;
+  for (int i = lane; i < w; i += 32) t += __ldcg(part + i);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+  if (lane == 0) {
+    *acc += (float)t;
+    *counter = 0u;
+  }
+}
+
+// nn = column sums + tiny, norm = v / nn
+template <int kPer>
+__global__ void __launch_bounds__(1024) k_document_lengths(const float* __restrict__ v, float tiny, float* nn, float* norm, int h,
+                                                           int w) {
+  __shared__ float red[32];
+  grid_dependents_launch();
+  grid_dependency_wait();
+  for (int c = blockIdx.x; c < w; c += gridDim.x) {
+    const long at = (long)c * h;
+    float x[kPer], s = 0.0f;
+#pragma unroll
+    for (int i = 0; i < kPer; i++) {
+      const int r = threadIdx.x + i * (int)blockDim.x;
+      x[i] = r < h ? v[at + r] : 0.0f;
+    }
+#pragma unroll
+    for (int i = 0; i < kPer; i++) s += x[i];
+    s = block_fold(s, red, 0.0f, add_f) + tiny;
+    if (threadIdx.x == 0) nn[c] = s;
+#pragma unroll
+    for (int i = 0; i < kPer; i++) {
+      const int r = threadIdx.x + i * (int)blockDim.x;
+      if (r < h) norm[at + r] = x[i] / s;
+    }
+  }
+}
+
+// Threads and blocks for columns of h values: four a thread up to 4096, then sixteen.
+void column_grid(int h, int w, int& threads, int& blocks, bool& four) {
+  four = h <= 4096;
+  threads = ((h + (four ? 4 : 16) - 1) / (four ? 4 : 16) + 31) & ~31;
+  blocks = w < sm_count() * 8 ? w : sm_count() * 8;
+}
+
+__global__ void __launch_bounds__(256) k_zero(float* x, long n) {
+  grid_dependents_launch();
+  grid_dependency_wait();
+  for (long i = (long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (long)gridDim.x * blockDim.x) x[i] = 0.0f;
+}
+
 // grid = (draw groups, documents); a block races 4 draws (the 4 words of one Philox block) of
 // one document over all words.
 __global__ void __launch_bounds__(256) k_sample_multinomial(const float* __restrict__ probs,
@@ -347,6 +484,11 @@ __global__ void __launch_bounds__(256) k_sample_energy_softmax(const float* __re
 
 extern "C" {
 
+int sum_by_axis(cudamat* mat, cudamat* target, int axis);
+int add_scalar(cudamat* mat, float alpha, cudamat* target);
+int div_by_row_vec(cudamat* mat, cudamat* vec, cudamat* target);
+int add_sq_diff(cudamat* a, cudamat* b, cudamat* acc);
+
 // target[:, j] = scale[j] * softmax(mat[:, j]); scale is 1 x cols (the document lengths NN).
 int softmax_scaled(cudamat* mat, cudamat* scale, cudamat* target) {
   if (!mat->on_device || !scale->on_device || !target->on_device) return ERROR_NOT_ON_DEVICE;
@@ -354,8 +496,72 @@ int softmax_scaled(cudamat* mat, cudamat* scale, cudamat* target) {
   if (!same_shape(mat, target) || numel(scale) != mat->size[1]) return ERROR_INCOMPATIBLE_DIMENSIONS;
   const int h = mat->size[0], w = mat->size[1];
   if ((long)h * w == 0) return 0;
+  if (h <= kColumnMax) {
+    int threads, blocks;
+    bool four;
+    column_grid(h, w, threads, blocks, four);
+    (void)launch_dependent(four ? k_softmax_columns<4> : k_softmax_columns<16>, dim3(blocks), dim3(threads), 0, stream(),
+                           mat->data_device, scale->data_device, target->data_device, nullptr, nullptr, nullptr, nullptr, nullptr, h, w);
+    return check_launch();
+  }
   (void)launch_dependent(k_softmax_scaled, dim3(w < sm_count() * 8 ? w : sm_count() * 8), dim3(256), 0, stream(), mat->data_device,
                          scale->data_device, target->data_device, h, w);
+  return check_launch();
+}
+
+// The visible layer of a replicated softmax from its pre-activations (deepnet/replicated_softmax_layer.py:12-21,128-135):
+// state = nn softmax(pre), norm = state / nn (what the statistics take) and, with data and acc, acc += sum (norm -
+// data)^2.  Three launches as separate calls: 20 + 4 + 7 us at 10 000 x 100.
+int softmax_reconstruction(cudamat* pre, cudamat* nn, cudamat* state, cudamat* norm, cudamat* data, cudamat* acc) {
+  if (!pre->on_device || !nn->on_device || !state->on_device || !norm->on_device) return ERROR_NOT_ON_DEVICE;
+  if ((data && !data->on_device) || (acc && !acc->on_device)) return ERROR_NOT_ON_DEVICE;
+  if (pre->is_trans || state->is_trans || norm->is_trans || (data && data->is_trans)) return ERROR_TRANSPOSED;
+  if (!same_shape(pre, state) || !same_shape(pre, norm) || numel(nn) != pre->size[1] || (!data != !acc) ||
+      (data && (!same_shape(pre, data) || numel(acc) < 1)))
+    return ERROR_INCOMPATIBLE_DIMENSIONS;
+  const int h = pre->size[0], w = pre->size[1];
+  if ((long)h * w == 0) return 0;
+  if (h > kColumnMax) {
+    int err = softmax_scaled(pre, nn, state);
+    if (!err) err = div_by_row_vec(state, nn, norm);
+    return err || !acc ? err : add_sq_diff(norm, data, acc);
+  }
+  double* part = nullptr;
+  unsigned* counter = nullptr;
+  if (acc) {
+    part = (double*)workspace(1, (size_t)w * sizeof(double));
+    counter = (unsigned*)workspace_zeroed(3, 4096 * sizeof(unsigned));   // (the first counter: add_sq_diff's, zero between calls)
+    if (!part || !counter) return CUDA_ERROR;
+  }
+  int threads, blocks;
+  bool four;
+  column_grid(h, w, threads, blocks, four);
+  if (launch_dependent(four ? k_softmax_columns<4> : k_softmax_columns<16>, dim3(blocks), dim3(threads), 0, stream(),
+                       pre->data_device, nn->data_device, state->data_device, norm->data_device, data ? data->data_device : nullptr,
+                       part, counter, acc ? acc->data_device : nullptr, h, w) != cudaSuccess)
+    return set_error(cudaGetErrorString(cudaGetLastError()));
+  return check_launch();
+}
+
+// What a replicated softmax takes of its word counts (deepnet/replicated_softmax_layer.py, deepnet/edge.py:225-228): nn = column
+// sums + tiny, norm = counts / nn.  Three launches as separate calls.
+int document_lengths(cudamat* counts, cudamat* nn, cudamat* norm, float tiny) {
+  if (!counts->on_device || !nn->on_device || !norm->on_device) return ERROR_NOT_ON_DEVICE;
+  if (counts->is_trans || norm->is_trans) return ERROR_TRANSPOSED;
+  if (!same_shape(counts, norm) || numel(nn) != counts->size[1]) return ERROR_INCOMPATIBLE_DIMENSIONS;
+  const int h = counts->size[0], w = counts->size[1];
+  if ((long)h * w == 0) return 0;
+  if (h > kColumnMax) {
+    int err = sum_by_axis(counts, nn, 0);
+    if (!err) err = add_scalar(nn, tiny, nn);
+    return err ? err : div_by_row_vec(counts, nn, norm);
+  }
+  int threads, blocks;
+  bool four;
+  column_grid(h, w, threads, blocks, four);
+  if (launch_dependent(four ? k_document_lengths<4> : k_document_lengths<16>, dim3(blocks), dim3(threads), 0, stream(),
+                       counts->data_device, tiny, nn->data_device, norm->data_device, h, w) != cudaSuccess)
+    return set_error(cudaGetErrorString(cudaGetLastError()));
   return check_launch();
 }
 
@@ -368,8 +574,11 @@ int sample_multinomial(rnd_struct* rnd_state, cudamat* probs, cudamat* nn, cudam
   if (max_draws < 1) return ERROR_UNSUPPORTED;
   const int h = probs->size[0], w = probs->size[1];
   if ((long)h * w == 0) return 0;
-  if (cudaMemsetAsync(target->data_device, 0, (size_t)h * w * sizeof(float), stream()) != cudaSuccess)
-    return set_error("cudaMemsetAsync failed");
+  // (a kernel, not a memset: the launches around it stay dependent)
+  const long n = (long)h * w, zb = (n + 1023) / 1024;
+  if (launch_dependent(k_zero, dim3((unsigned)(zb < sm_count() * 8L ? zb : sm_count() * 8L)), dim3(256), 0, stream(), target->data_device, n) !=
+      cudaSuccess)
+    return set_error(cudaGetErrorString(cudaGetLastError()));
   const unsigned long long call0 = rnd_state->calls;
   rnd_state->calls += (unsigned long long)w;
   int groups = (max_draws + 3) / 4 + 1;

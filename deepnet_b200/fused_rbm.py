@@ -180,8 +180,8 @@ class FusedRBM(LossReadback):
         """deepnet/dbm.py:217-222: the visible layer feeds a draw upward instead of its means."""
         return bool(self.hyp.sample_input) and self.hyp.sample_input_after <= step
 
-    # launches behind one operation of the vocabulary (row and column sums: partial + finishing launch)
-    _LAUNCHES = dict(sum=2, add_sums=2, sm_limit=0, allreduce_end=0)
+    # launches behind one operation of the vocabulary (the draws' counts start from zero)
+    _LAUNCHES = dict(sample_multinomial=2, sm_limit=0, allreduce_end=0)
 
     def _op(self, X, name, flops, nbytes, method, *args, **kw):
         """Names one operation of the step to the executor X (`Immediate` or a recording `Program`);
@@ -426,9 +426,7 @@ class FusedRBM(LossReadback):
         vb, hb, wb = 4.0 * V * B, 4.0 * H * B, 4.0 * V * H
         v0 = data                                              # integer counts: exact in TF32
         # GetData: NN = column sums + tiny; v0n = data / NN for the statistics
-        self._op(X, "col_sum", 0, vb, "sum", v0, 0, self.NN)
-        self._op(X, "add_scalar", 0, 8.0 * B, "add_scalar", self.NN, self.tiny)
-        self._op(X, "div_by_row", 0, 2 * vb, "div_by_row", v0, self.NN, self.v0n)
+        self._op(X, "document_lengths", 0, 2 * vb, "document_lengths", v0, self.NN, self.v0n, self.tiny)
         # positive phase: hidden bias is scaled by the document length (deepnet/dbm.py:101-104)
         self._op(X, "gemm_up", gf, 2 * hb, "fused_gemm", P(W.T, v0, exact_b=True, a_aux=Wa), out=self.h_pos,
                  sample=self.h_samp, bias=self.bh, col_scale=self.NN, activation=1)
@@ -436,10 +434,10 @@ class FusedRBM(LossReadback):
             # visible: NN * softmax(W h + b_v)
             self._op(X, "gemm_down", gf, vb, "fused_gemm", P(W, self.h_samp, exact_b=True, a_aux=Wa), out=self.v_act,
                      bias=self.bv, activation=0)
-            self._op(X, "softmax", 0, 2 * vb, "softmax_scaled", self.v_act, self.NN, self.v_neg)
-            self._op(X, "div_by_row", 0, 2 * vb, "div_by_row", self.v_neg, self.NN, self.v_negn)
-            if i == 0:   # squared error between state / NN and the counts (replicated_softmax_layer.py:128-135)
-                self._op(X, "sq_err", 0, 2 * vb, "sq_diff", self.v_negn, v0, self.loss_acc)
+            # ... its statistics' form, and the squared error between state / NN and the counts
+            # (replicated_softmax_layer.py:128-135)
+            self._op(X, "softmax", 0, (4 if i == 0 else 3) * vb, "softmax_reconstruction", self.v_act, self.NN, self.v_neg,
+                     self.v_negn, v0 if i == 0 else None, self.loss_acc if i == 0 else None)
             if draw_v:   # word counts drawn from the softmax feed upward
                 self._op(X, "multinomial", 0, 2 * vb, "sample_multinomial", self.v_neg, self.NN, self.v_samp)
                 up = P(W.T, self.v_samp, exact_b=True, a_aux=Wa)

@@ -278,6 +278,8 @@ int softmax_sample(rnd_struct* rnd_state, cudamat* pre, cudamat* bias, cudamat* 
 
 /* target[:, j] = scale[j] * softmax(mat[:, j]): the six calls of
  * deepnet/replicated_softmax_layer.py:12-21 (max, add_row_mult, exp, sum, divide, mult_by_row). */
+int softmax_reconstruction(cudamat* pre, cudamat* nn, cudamat* state, cudamat* norm, cudamat* data, cudamat* acc);   /* state = nn softmax(pre), norm = state / nn; data and acc (or neither): acc += sum (norm - data)^2 */
+int document_lengths(cudamat* counts, cudamat* nn, cudamat* norm, float tiny);   /* nn = column sums + tiny, norm = counts / nn */
 int softmax_scaled(cudamat* mat, cudamat* scale, cudamat* target);
 
 /* target[:, i] = word counts of int(nn[i]) (at most max_draws) exponential-race draws from the
@@ -393,8 +395,9 @@ int dp_wait(int timeout_ms);
  * 5 momentum_update, 6 split_f16, 7 split_bf16, 8 dp_allreduce, 9 softmax_scaled, 10 sample_multinomial,
  * 11 div_by_row_vec, 12 add_scalar, 13 assign_scalar, 14 copy_on_device, 15 sample_bernoulli,
  * 16 softmax_sample, 17 momentum_update_columns, 18 dp_allreduce_begin, 19 dp_allreduce_end,
- * 20 b200_set_sm_limit, 21 dp_peer_update, 22 rbm_bias_update); m[], i0.., f0.. are its arguments in declaration order (matrices, then integers,
- * then floats; gemm for kind 0).  Stops at the first failure: returns its code, *failed_at its index. */
+ * 20 b200_set_sm_limit, 21 dp_peer_update, 22 rbm_bias_update,
+ * 23 softmax_reconstruction, 24 document_lengths); m[], i0.., f0.. are its arguments in declaration order (matrices, then
+ * integers, then floats; gemm for kind 0).  Stops at the first failure: returns its code, *failed_at its index. */
 struct b200_fused_gemm;
 typedef struct b200_op {
   int kind;

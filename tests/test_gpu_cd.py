@@ -596,3 +596,31 @@ def test_loss_read_back_behind_the_updates(cm):
             got.append(eng.loss_end(3 & 1))
     assert got == want
     assert cm.read_status() == 0
+
+
+@pytest.mark.parametrize("V", [1, 100, 4096, 4097, 10001, 16384, 16385])
+def test_softmax_columns_match_their_definition(cm, V):
+    """Whole columns in registers (4 or 16 values a thread) and, past 16384 rows, the calls one by one: state, its normalised form,
+    the error and the document lengths against float64.  Bound: a sum of V positive fp32 terms and a handful of roundings."""
+    rng = np.random.default_rng(V)
+    B = 7
+    pre = (3 * rng.standard_normal((V, B))).astype(np.float32)
+    counts = rng.poisson(2.0, (V, B)).astype(np.float32)
+    counts[0] += 1
+    m = {n: cm.empty((V, B)) for n in ("state", "norm", "v0n")}
+    nn, loss = cm.empty((1, B)), cm.empty((1, 1))
+    X, data = cm.Immediate(), cm.CUDAMatrix(counts)
+    X.document_lengths(data, nn, m["v0n"], 1e-10)
+    X.softmax_reconstruction(cm.CUDAMatrix(pre), nn, m["state"], m["norm"], data, loss)
+    lengths = counts.astype(np.float64).sum(axis=0)
+    np.testing.assert_array_equal(get(nn)[0], lengths.astype(np.float32))        # sums of small integers are exact
+    np.testing.assert_allclose(get(m["v0n"]), counts / lengths, rtol=1e-6)
+    e = np.exp(pre.astype(np.float64) - pre.max(axis=0))
+    p = e / e.sum(axis=0)
+    np.testing.assert_allclose(get(m["norm"]), p, rtol=1e-5, atol=1e-12)
+    np.testing.assert_allclose(get(m["state"]), p * lengths, rtol=1e-5, atol=1e-12)
+    np.testing.assert_allclose(get(loss)[0, 0], ((p - counts) ** 2).sum(), rtol=1e-5)
+    X.softmax_reconstruction(cm.CUDAMatrix(pre), nn, m["state"], m["norm"])
+    np.testing.assert_allclose(get(m["norm"]), p, rtol=1e-5, atol=1e-12)
+    again = get(cm.CUDAMatrix(pre).softmax_scaled(nn, target=cm.empty((V, B))))
+    np.testing.assert_array_equal(again, get(m["state"]))
