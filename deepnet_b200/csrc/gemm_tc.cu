@@ -1528,6 +1528,58 @@ int gemm_tc_packed(const GemmProblem& g) {
   return gemm_tc(f);
 }
 
+// Split-K: how many parts of K for tiles that would occupy `ctas` SMs and an inner dimension of `min_ki` k-blocks.
+static int splits_of(int ctas, int min_ki) {
+  if (ctas * 2 > sm_count()) return 1;
+  int want = sm_count() / ctas;
+  if (want > min_ki / 4) want = min_ki / 4;
+  return want > 32 ? 32 : (want < 1 ? 1 : want);
+}
+
+// Columns of a tile.  One CTA per 128 rows up to N = 128.  Wider products share 256 x 256 tiles between two CTAs, which runs
+// the tensor pipe at its rate, where the tiles fill the device; a product of few tiles is bound by what surrounds them, and
+// narrower tiles of a single CTA come off better: the epilogue of 128 accumulator columns per thread takes 19 000 clocks
+// for a partial tile and as many for an activation, that of 64 takes 3900 and 18 600, of 32 1900 and 8600.  Clocks of a
+// k-block: 1060, 960, 840.  Measured, 256 / 128 / 64 columns, us with the finishing launch:
+//   4096 x 256, K = 1024      30.3 / 25.4 / 25.8       2048 x 512, K = 2048    36.4 / 34.8 / 42.1
+//   1024 x 256, K = 4096      29.8 / 21.8 / 27.0       500 x 2048, K = 784     27.8 / 21.5 / 19.7
+//   1000 x 2048, K = 500      34.5 / 28.0 / 30.7       1024 x 4096, two pairs of K = 256, plain   28.9 / 39.9 / 67.3
+// Products on 16-bit planes alone (the big models' own) and odd matrices keep the wide tiles.
+static int tile_columns(const GemmProblem& g) {
+  if (g.N <= 64) return 64;
+  if (g.N <= 128) return 128;
+  if (g_split_mode != 0 || g.odd || g.M <= BM || product_is_scattered(g.epi.out)) return 256;
+  int slabs = 0, min_ki = 1 << 30;
+  for (int q = 0; q < g.npass; q++) {
+    const GemmPass& t = g.pass[q];
+    if (part_is_f16(t.a.part)) return 256;
+    if (q > 0 && same_operand(t.a, g.pass[q - 1].a) && same_operand(t.b, g.pass[q - 1].b) && t.k == g.pass[q - 1].k) continue;
+    const int ki = (t.k + 31) / 32;
+    slabs += ki;
+    min_ki = ki < min_ki ? ki : min_ki;
+  }
+  const bool plain = plain_result(g.epi);
+  const int sms = sm_count();
+  int best = 256;
+  float best_clocks = 0.0f;
+  for (int bn = 256; bn >= 64; bn /= 2) {
+    const long ctas = bn == 256 ? 2L * ((g.M + 255) / 256) * ((g.N + 255) / 256) : (long)((g.M + BM - 1) / BM) * ((g.N + bn - 1) / bn);
+    const int splits = ctas < sms && min_ki >= 8 ? splits_of((int)ctas, min_ki) : 1;
+    const float waves = (float)((ctas * splits + sms - 1) / sms), depth = (float)slabs / splits;
+    const float block = bn == 256 ? 1060.0f : (bn == 128 ? 960.0f : 840.0f);
+    const float tile = splits > 1 ? (bn == 256 ? 18900.0f : (bn == 128 ? 3900.0f : 1900.0f)) + 10000.0f + 1200.0f * splits
+                       : plain    ? (bn == 256 ? 14200.0f : (bn == 128 ? 10000.0f : 7800.0f))
+                                  : (bn == 256 ? 20000.0f : (bn == 128 ? 18600.0f : 8600.0f));
+    const float clocks = 5000.0f + waves * (depth * block + tile);
+    // (a narrower tile has to come out ahead by what the estimate is good for)
+    if (bn == 256 || clocks < 0.95f * best_clocks) {
+      best = bn;
+      best_clocks = clocks;
+    }
+  }
+  return best;
+}
+
 int gemm_tc(const GemmProblem& g) {
 #ifdef B200_HOST_TIMING
   const double t_begin = HostTimes::now();
@@ -1535,7 +1587,7 @@ int gemm_tc(const GemmProblem& g) {
   const bool scatter = g_scatter_n > 0 && g.epi.out != nullptr && g.epi.out == g_scatter_match;
   if (!gemm_tc_supported(g))
     return scatter ? set_error("a product whose result is scattered to peers must run on the tensor cores") : ERROR_UNSUPPORTED;
-  const int BN = g.N > 128 ? 256 : (g.N > 64 ? 128 : 64);
+  const int BN = tile_columns(g);
   static int pair_mode = -1;   // B200_GEMM_2CTA=0 keeps one CTA per tile
   static int chunk_k = 0;
   if (pair_mode < 0) {
@@ -1714,7 +1766,11 @@ int gemm_tc(const GemmProblem& g) {
   // cores before, which round every addition: short chunks keep their error where it was.
   bool odd = g.odd != 0 || (!plain_result(g.epi) && !tma_outputs_ok(g.epi));
   for (int q = 0; q < g.npass; q++) odd = odd || !fp32_tma_ok(g.pass[q].a) || !fp32_tma_ok(g.pass[q].b);
-  const int ck = chunk_k >= 16 ? chunk_k : odd ? (g.epi.activation == 1 ? 128 : 32) : (g.epi.activation == 1 ? 2048 : 128);
+  // Tiles narrower than the widest are the ones that were cut along K more often, into shorter sums: 128 products keep their
+  // error where it was or below (500 x 2048, K = 784 behind a logistic: 4.2e-7 as cut wide tiles, 6.3e-7 with 2048), and the
+  // drain of 32 or 64 columns fits between two chunks.
+  const bool narrow = BN < 256 && g.N > 128;
+  const int ck = chunk_k >= 16 ? chunk_k : narrow && !odd ? 128 : odd ? (g.epi.activation == 1 ? 128 : 32) : (g.epi.activation == 1 ? 2048 : 128);
   p.chunk_iters = ck / bk < 1 ? 1 : ck / bk;
 
   // Split-K: a product whose tiles would occupy less than half of the SMs and whose inner dimension
@@ -1736,11 +1792,7 @@ int gemm_tc(const GemmProblem& g) {
       min_ki_to_split = mv ? atoi(mv) : 8;
     }
     if (g_split_mode == 0) {
-      if (ctas * 2 <= sm_count() && min_ki >= min_ki_to_split) {
-        want = sm_count() / ctas;
-        if (want > min_ki / 4) want = min_ki / 4;
-        if (want > 32) want = 32;
-      }
+      if (min_ki >= min_ki_to_split) want = splits_of(ctas, min_ki);
     } else if (g_split_mode > 1) {
       want = g_split_mode < min_ki ? g_split_mode : min_ki;
     }
@@ -1792,7 +1844,9 @@ int gemm_tc(const GemmProblem& g) {
     store16_mode = sv ? atoi(sv) : 1;
   }
   p.direct_store = !epi_is_plain(epi) &&
-                   (!tma_outputs_ok(e) || (store16_mode != 0 && !e.out && !e.sample && (e.out_aux || e.sample_aux)));
+                   (!tma_outputs_ok(e) || (store16_mode != 0 && !e.out && !e.sample && (e.out_aux || e.sample_aux)) ||
+                    // a CTA with one tile has no next one whose first chunk waits: 18 600 clocks against 26 500 staged
+                    (BN == 128 && g.N > 128 && (long)((g.M + BM - 1) / BM) * ((g.N + BN - 1) / BN) <= sm_count()));
   for (int i = 0; i < kOutArrays; i++) p.out_map[i] = -1;
   if (!epi_is_plain(epi) && !p.direct_store) {
     // outputs of the activation epilogues, stored as boxes of 128 rows x 4 columns: M x N floats

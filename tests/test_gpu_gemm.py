@@ -936,3 +936,37 @@ def test_deep_unaligned_dot_keeps_infinities_in_all_layouts(cm, ta, tb, alpha):
     np.testing.assert_array_equal(got[rest, 7], np.sign(alpha * A[rest, 1000]) * np.inf)
     cols = np.delete(np.arange(n), 7)
     assert relerr(got[np.ix_(rest, cols)], want[np.ix_(rest, cols)]) < TOL
+
+
+@pytest.mark.parametrize("M,N,K,two_pairs", [(4096, 256, 1024, False), (1024, 256, 4096, False), (500, 2048, 784, False),
+                                             (1000, 2044, 500, False), (1000, 132, 260, False), (132, 1000, 300, True),
+                                             (260, 516, 256, True)])
+def test_narrow_tiles_of_products_of_few_tiles(cm, M, N, K, two_pairs):
+    """Products whose 256-column tiles leave the device idle take tiles of 128 or 64 columns of a single CTA: ragged rows and
+    columns of either width, cut along K and not, against float64.  Bound: sums of K products in chunks of 128 (2048 behind
+    the logistic) at 2^-18 a term, 1e-5 of the largest result."""
+    rng = np.random.default_rng(M + N)
+    w = [(rng.standard_normal((K, M)) * 0.05).astype(np.float32) for _ in range(1 + two_pairs)]
+    x = [rng.random((K, N)).astype(np.float32) for _ in range(1 + two_pairs)]
+    b = rng.standard_normal((M, 1)).astype(np.float32)
+    passes = []
+    for wi, xi in zip(w, x):
+        passes += cm.split_passes(cm.CUDAMatrix(wi).T, cm.CUDAMatrix(xi))
+    out, sample, plain = cm.empty((M, N)), cm.empty((M, N)), cm.empty((M, N))
+    cm.CUDAMatrix.init_random(3)
+    cm.set_gemm_path(1)
+    try:
+        cm.fused_gemm(passes, out=out, sample=sample, bias=cm.CUDAMatrix(b), activation=1)
+        cm.fused_gemm(passes, out=plain)
+    finally:
+        cm.set_gemm_path(0)
+    pre = sum(wi.T.astype(np.float64) @ xi for wi, xi in zip(w, x))
+    want = 1 / (1 + np.exp(-(pre + b)))
+    got, draws = np.array(out.asarray()), np.array(sample.asarray())
+    assert np.abs(got - want).max() < 1e-5
+    assert np.abs(np.array(plain.asarray()) - pre).max() < 1e-5 * np.abs(pre).max()
+    again, unit = cm.empty((M, N)), cm.CUDAMatrix(got)
+    cm.CUDAMatrix.init_random(3)
+    unit.sample_bernoulli(target=again)                       # the same stream on the same probabilities
+    np.testing.assert_array_equal(draws, np.array(again.asarray()))
+    assert cm.read_status() == 0
