@@ -61,6 +61,11 @@ class _FusedGemm(ct.Structure):
                 ("scale_exp_const", ct.c_int), ("aux_f16", ct.c_int), ("aux_exp", ct.c_int)]
 
 
+class _BiasLayers(ct.Structure):
+    _fields_ = ([(n, ct.POINTER(cudamat) * 4) for n in ("pos", "neg", "suff", "b", "db")] +
+                [("sq_acc", ct.POINTER(cudamat)), ("layers", ct.c_int)])
+
+
 _lib.get_last_cuda_error.restype = ct.c_char_p
 _lib.euclid_norm.restype = ct.c_float
 _lib.vdot.restype = ct.c_float
@@ -766,6 +771,17 @@ def fused_gemm(passes, out=None, sample=None, bias=None, col_scale=None, activat
     _check(_lib.fused_gemm(CUDAMatrix.rnd_state_p, ct.byref(f)))
 
 
+def _build_bias_layers(layers, sq_acc):
+    t = _BiasLayers()
+    t.layers = len(layers)
+    for i, mats in enumerate(layers):
+        for name, m in zip(("pos", "neg", "suff", "b", "db"), mats):
+            getattr(t, name)[i] = m.p_mat
+    if sq_acc is not None:
+        t.sq_acc = sq_acc.p_mat
+    return t
+
+
 def _build_fused_gemm(passes, out=None, sample=None, bias=None, col_scale=None, activation=0, alpha=1.0, beta=0.0,
                       out_aux=None, sample_aux=None, scale_exp=None, scale_exp_const=0, aux_f16=False, aux_exp=0):
     """The argument block of `fused_gemm` (it points into the matrices' handles: keep them alive)."""
@@ -806,7 +822,7 @@ def _build_fused_gemm(passes, out=None, sample=None, bias=None, col_scale=None, 
  OP_SPLIT_BF16, OP_ALLREDUCE, OP_SOFTMAX_SCALED, OP_SAMPLE_MULTINOMIAL, OP_DIV_BY_ROW, OP_ADD_SCALAR, OP_ASSIGN_SCALAR,
  OP_COPY, OP_SAMPLE_BERNOULLI, OP_SOFTMAX_SAMPLE, OP_MOMENTUM_UPDATE_COLUMNS, OP_ALLREDUCE_BEGIN, OP_ALLREDUCE_END,
  OP_SM_LIMIT, OP_DP_PEER_UPDATE, OP_RBM_BIAS_UPDATE, OP_SOFTMAX_RECONSTRUCTION,
- OP_DOCUMENT_LENGTHS) = range(25)
+ OP_DOCUMENT_LENGTHS, OP_BIAS_UPDATES, OP_UPDATE_ALL) = range(27)
 
 
 class _Op(ct.Structure):
@@ -841,6 +857,16 @@ class Immediate(object):
 
     def momentum_update(self, w, delta, grad, suff, inv_batch, momentum, eps, l2=0.0, l1=0.0, w_aux=None, w_scale=None):
         w.momentum_update(delta, grad, suff, inv_batch, momentum, eps, l2=l2, l1=l1, w_aux=w_aux, w_scale=w_scale)
+
+    def bias_updates(self, layers, inv_batch, momentum, eps, sq_acc=None):
+        """Statistics and update of the biases of up to four layers (pos, neg, suff, b, db)."""
+        _check(_lib.bias_updates(ct.byref(_build_bias_layers(layers, sq_acc)), ct.c_float(inv_batch), ct.c_float(momentum),
+                                 ct.c_float(eps)))
+
+    def update_all(self, layers, w, delta, suff, w_aux, inv_batch, mom_b, eps_b, mom_w, eps_w, l2=0.0, l1=0.0, sq_acc=None):
+        """`bias_updates` of the layers and `momentum_update` of w with its bfloat16 parts, in one launch."""
+        _check(_lib.update_all(ct.byref(_build_bias_layers(layers, sq_acc)), w.p_mat, delta.p_mat, suff.p_mat, w_aux.p_mat,
+                               *(ct.c_float(x) for x in (inv_batch, mom_b, eps_b, mom_w, eps_w, l2, l1))))
 
     def rbm_bias_update(self, v_pos, v_neg, h_pos, h_neg, suff, b, db, sq_acc, inv_batch, momentum, eps):
         _check(_lib.rbm_bias_update(v_pos.p_mat, v_neg.p_mat, h_pos.p_mat, h_neg.p_mat, suff.p_mat, b.p_mat, db.p_mat,
@@ -932,7 +958,7 @@ class Program(object):
         for name, v in zip(("f0", "f1", "f2", "f3", "f4", "f5", "f6", "f7"), floats):
             setattr(op, name, float(v))
         if gemm is not None:
-            op.gemm = ct.pointer(gemm)
+            op.gemm = ct.cast(ct.pointer(gemm), ct.POINTER(_FusedGemm))
             self._keep.append(gemm)
         self._ops.append(op)
         self._arr = None
@@ -958,6 +984,19 @@ class Program(object):
 
     def momentum_update(self, w, delta, grad, suff, inv_batch, momentum, eps, l2=0.0, l1=0.0, w_aux=None, w_scale=None):
         return self._add(OP_MOMENTUM_UPDATE, (w, delta, grad, suff, w_aux, w_scale), (), (inv_batch, momentum, eps, l2, l1))
+
+    def bias_updates(self, layers, inv_batch, momentum, eps, sq_acc=None):
+        for mats in layers:
+            self._keep.extend(mats)
+        self._keep.append(sq_acc)
+        return self._add(OP_BIAS_UPDATES, (), (), (inv_batch, momentum, eps), gemm=_build_bias_layers(layers, sq_acc))
+
+    def update_all(self, layers, w, delta, suff, w_aux, inv_batch, mom_b, eps_b, mom_w, eps_w, l2=0.0, l1=0.0, sq_acc=None):
+        for mats in layers:
+            self._keep.extend(mats)
+        self._keep.append(sq_acc)
+        return self._add(OP_UPDATE_ALL, (w, delta, suff, w_aux), (), (inv_batch, mom_b, eps_b, mom_w, eps_w, l2, l1),
+                         gemm=_build_bias_layers(layers, sq_acc))
 
     def rbm_bias_update(self, v_pos, v_neg, h_pos, h_neg, suff, b, db, sq_acc, inv_batch, momentum, eps):
         return self._add(OP_RBM_BIAS_UPDATE, (v_pos, v_neg, h_pos, h_neg, suff, b, db, sq_acc), (), (inv_batch, momentum, eps))

@@ -227,30 +227,37 @@ __device__ __forceinline__ void update_one(float& w, float& d, float g, float su
   w = __fadd_rn(w, __fmul_rn(d, neps));
 }
 
-// What ends a CD update beside the weights, in one launch: for every unit r of the two layers
+// What ends an update beside the weights, in one launch: for every unit r of up to four layers
 //   suff[r] = sum_c pos[r, c] - neg[r, c]   (deepnet/layer.py:202-213), then the parameter update of the biases,
-// and, with `acc`, acc[0] += sum (v_pos - v_neg)^2, the reconstruction error of deepnet/logistic_layer.py:48-52 (the
-// visible rows are being read anyway).  A block owns 32 rows whole (8 lanes of columns, folded in order), so the sums
+// and, with `acc`, acc[0] += sum (pos - neg)^2 of the first, the reconstruction error of deepnet/logistic_layer.py:48-52
+// (the visible rows are being read anyway).  A block owns 32 rows whole (8 lanes of columns, folded in order), so the sums
 // need no second pass; the error's partial sums (doubles) are folded by the block that finishes last, in order.
 // Latency bound at the sizes it is used for.  Four launches before: 784 + 500 units, 100 cases: 10.6 -> 4 us.
 constexpr int kTailLanes = 8;
+constexpr int kTailLayers = 4;
 struct TailLayer {
   const float *pos, *neg;
-  int rows;
+  float *suff, *b, *db;
+  int rows, block0;        // first block
 };
-__global__ void __launch_bounds__(32 * kTailLanes) k_bias_tail(TailLayer v, TailLayer h, float* suff, float* b, float* db,
-                                                               int cases, int vblocks, double* part, unsigned* counter,
-                                                               float* acc, float ninv_batch, float momentum, float neps) {
+struct TailArgs {
+  TailLayer l[kTailLayers];
+  int layers, cases;
+  double* part;
+  unsigned* counter;
+  float *acc, ninv_batch, momentum, neps;
+};
+__device__ __forceinline__ void bias_tail(const TailArgs& a) {
   __shared__ float sums[kTailLanes][33];
   __shared__ double sq[kTailLanes];
   __shared__ bool is_last;
-  grid_dependents_launch();
-  grid_dependency_wait();
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const bool visible = (int)blockIdx.x < vblocks;
-  const TailLayer l = visible ? v : h;
-  const int r0 = 32 * (visible ? (int)blockIdx.x : (int)blockIdx.x - vblocks), r = r0 + tx;
-  const bool err = visible && acc != nullptr;
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, cases = a.cases;
+  int which = 0;
+  while (which + 1 < a.layers && (int)blockIdx.x >= a.l[which + 1].block0) which++;
+  const TailLayer l = a.l[which];
+  const int r = 32 * ((int)blockIdx.x - l.block0) + tx;
+  const bool err = which == 0 && a.acc != nullptr;
+  const int err_blocks = (a.l[0].rows + 31) / 32;
   float s = 0.0f;
   double e = 0.0;
   if (r < l.rows) {
@@ -284,32 +291,36 @@ __global__ void __launch_bounds__(32 * kTailLanes) k_bias_tail(TailLayer v, Tail
     float t = 0.0f;
 #pragma unroll
     for (int j = 0; j < kTailLanes; j++) t += sums[j][tx];
-    const long at = (visible ? 0 : (long)v.rows) + r;
-    suff[at] = t;
-    float w = b[at], d = db[at];
-    update_one(w, d, 0.0f, t, ninv_batch, momentum, neps, 0.0f, 0.0f);
-    b[at] = w;
-    db[at] = d;
+    l.suff[r] = t;
+    float w = l.b[r], d = l.db[r];
+    update_one(w, d, 0.0f, t, a.ninv_batch, a.momentum, a.neps, 0.0f, 0.0f);
+    l.b[r] = w;
+    l.db[r] = d;
   }
   if (!err) return;
   if (threadIdx.x == 0) {
     double t = 0.0;
     for (int j = 0; j < kTailLanes; j++) t += sq[j];
-    part[blockIdx.x] = t;
+    a.part[blockIdx.x] = t;
     __threadfence();
-    is_last = atomicAdd(counter, 1u) == (unsigned)(vblocks - 1);
+    is_last = atomicAdd(a.counter, 1u) == (unsigned)(err_blocks - 1);
   }
   __syncthreads();
   if (!is_last || ty != 0) return;
   __threadfence();
   double t = 0.0;
-  for (int i = tx; i < vblocks; i += 32) t += __ldcg(part + i);
+  for (int i = tx; i < err_blocks; i += 32) t += __ldcg(a.part + i);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
   if (tx == 0) {
-    *acc += (float)t;
-    *counter = 0u;
+    *a.acc += (float)t;
+    *a.counter = 0u;
   }
+}
+__global__ void __launch_bounds__(32 * kTailLanes) k_bias_tail(const __grid_constant__ TailArgs a) {
+  grid_dependents_launch();
+  grid_dependency_wait();
+  bias_tail(a);
 }
 
 // One block walks all cases of its 32 rows: past this many cases the launches that also split the cases are faster.
@@ -324,8 +335,74 @@ int momentum_update(cudamat* w, cudamat* delta, cudamat* grad, cudamat* suff, cu
                     float inv_batch, float momentum, float eps, float l2, float l1);
 }
 
-// Bias statistics (positive minus negative), bias update and, with sq_acc, the squared reconstruction error of an RBM
-// whose biases, histories and statistics are packed [visible | hidden]; one launch up to kTailCases cases.
+// Bias statistics (positive minus negative) and bias update of up to four layers and, with sq_acc, the squared
+// difference of the first layer's states.
+struct b200_bias_layers {
+  cudamat *pos[kTailLayers], *neg[kTailLayers], *suff[kTailLayers], *b[kTailLayers], *db[kTailLayers];
+  cudamat* sq_acc;
+  int layers;
+};
+// Checks the layers; blocks: of the one launch, 0 where the sums take launches of their own.
+static int plan_bias_tail(b200_bias_layers* t, float inv_batch, float momentum, float eps, TailArgs& a, int& blocks) {
+  blocks = 0;
+  if (!t || t->layers < 1 || t->layers > kTailLayers) return ERROR_UNSUPPORTED;
+  const int n = t->layers;
+  bool empty = false;
+  for (int i = 0; i < n; i++) {
+    for (cudamat* m : {t->pos[i], t->neg[i], t->suff[i], t->b[i], t->db[i]}) {
+      if (!m) return ERROR_GENERIC;
+      if (!m->on_device) return ERROR_NOT_ON_DEVICE;
+      if (m->is_trans) return ERROR_TRANSPOSED;
+    }
+    const long rows = t->pos[i]->size[0];
+    if (!same_shape(t->pos[i], t->neg[i]) || t->pos[i]->size[1] != t->pos[0]->size[1] || numel(t->suff[i]) != rows ||
+        numel(t->b[i]) != rows || numel(t->db[i]) != rows)
+      return ERROR_INCOMPATIBLE_DIMENSIONS;
+    empty = empty || rows == 0;
+  }
+  if (t->sq_acc && !t->sq_acc->on_device) return ERROR_NOT_ON_DEVICE;
+  if (t->sq_acc && numel(t->sq_acc) < 1) return ERROR_INCOMPATIBLE_DIMENSIONS;
+  a.cases = t->pos[0]->size[1];
+  if (a.cases > kTailCases || a.cases == 0 || empty) return 0;
+  a.layers = n;
+  for (int i = 0; i < n; i++) {
+    a.l[i] = {t->pos[i]->data_device, t->neg[i]->data_device, t->suff[i]->data_device, t->b[i]->data_device,
+              t->db[i]->data_device, t->pos[i]->size[0], blocks};
+    blocks += (a.l[i].rows + 31) / 32;
+  }
+  a.part = nullptr;
+  a.counter = nullptr;
+  a.acc = nullptr;
+  a.ninv_batch = -inv_batch;
+  a.momentum = momentum;
+  a.neps = -eps;
+  if (t->sq_acc) {
+    a.acc = t->sq_acc->data_device;
+    a.part = (double*)workspace(1, (size_t)((a.l[0].rows + 31) / 32 + 1) * sizeof(double));
+    a.counter = (unsigned*)workspace_zeroed(3, 4096 * sizeof(unsigned));   // (the first counter: add_sq_diff's, zero between calls)
+    if (!a.part || !a.counter) return CUDA_ERROR;
+  }
+  return 0;
+}
+extern "C" int bias_updates(b200_bias_layers* t, float inv_batch, float momentum, float eps) {
+  TailArgs a;
+  int blocks = 0;
+  int err = plan_bias_tail(t, inv_batch, momentum, eps, a, blocks);
+  if (err) return err;
+  if (blocks == 0) {
+    const int n = t->layers;
+    err = t->sq_acc ? add_sq_diff(t->neg[0], t->pos[0], t->sq_acc) : 0;
+    for (int i = 0; i < n && !err; i++) err = row_sum_diff(t->pos[i], t->neg[i], t->suff[i]);
+    for (int i = 0; i < n && !err; i++)
+      err = momentum_update(t->b[i], t->db[i], nullptr, t->suff[i], nullptr, nullptr, inv_batch, momentum, eps, 0.0f, 0.0f);
+    return err;
+  }
+  if (launch_dependent(k_bias_tail, dim3((unsigned)blocks), dim3(32 * kTailLanes), 0, stream(), a) != cudaSuccess)
+    return set_error(cudaGetErrorString(cudaGetLastError()));
+  return check_launch();
+}
+
+// The same for an RBM whose biases, histories and statistics are packed [visible | hidden].
 extern "C" int rbm_bias_update(cudamat* v_pos, cudamat* v_neg, cudamat* h_pos, cudamat* h_neg, cudamat* suff, cudamat* b,
                                cudamat* db, cudamat* sq_acc, float inv_batch, float momentum, float eps) {
   cudamat* all[7] = {v_pos, v_neg, h_pos, h_neg, suff, b, db};
@@ -333,36 +410,18 @@ extern "C" int rbm_bias_update(cudamat* v_pos, cudamat* v_neg, cudamat* h_pos, c
     if (!all[i]->on_device) return ERROR_NOT_ON_DEVICE;
     if (all[i]->is_trans) return ERROR_TRANSPOSED;
   }
-  if (sq_acc && !sq_acc->on_device) return ERROR_NOT_ON_DEVICE;
-  const int V = v_pos->size[0], H = h_pos->size[0], B = v_pos->size[1];
-  if (!same_shape(v_pos, v_neg) || !same_shape(h_pos, h_neg) || h_pos->size[1] != B || numel(suff) != (long)V + H ||
-      !same_shape(suff, b) || !same_shape(suff, db) || (sq_acc && numel(sq_acc) < 1))
-    return ERROR_INCOMPATIBLE_DIMENSIONS;
-  if (B > kTailCases || (long)V * H * B == 0) {
-    cudamat sv = *suff, sh = *suff;
-    sv.size[0] = V;
-    sh.size[0] = H;
-    sv.size[1] = sh.size[1] = 1;
-    sh.data_device += V;
-    int err = sq_acc ? add_sq_diff(v_neg, v_pos, sq_acc) : 0;
-    if (!err) err = row_sum_diff(v_pos, v_neg, &sv);
-    if (!err) err = row_sum_diff(h_pos, h_neg, &sh);
-    return err ? err : momentum_update(b, db, nullptr, suff, nullptr, nullptr, inv_batch, momentum, eps, 0.0f, 0.0f);
+  const int V = v_pos->size[0], H = h_pos->size[0];
+  if (numel(suff) != (long)V + H || !same_shape(suff, b) || !same_shape(suff, db)) return ERROR_INCOMPATIBLE_DIMENSIONS;
+  cudamat half[6];       // suff, b, db of either layer
+  for (int i = 0; i < 3; i++) {
+    half[i] = half[3 + i] = *all[4 + i];
+    half[i].size[0] = V;
+    half[3 + i].size[0] = H;
+    half[i].size[1] = half[3 + i].size[1] = 1;
+    half[3 + i].data_device += V;
   }
-  const int vblocks = (V + 31) / 32, hblocks = (H + 31) / 32;
-  double* part = nullptr;
-  unsigned* counter = nullptr;
-  if (sq_acc) {
-    part = (double*)workspace(1, (size_t)(vblocks + 1) * sizeof(double));
-    counter = (unsigned*)workspace_zeroed(3, 4096 * sizeof(unsigned));   // (the first counter: add_sq_diff's, zero between calls)
-    if (!part || !counter) return CUDA_ERROR;
-  }
-  const TailLayer lv = {v_pos->data_device, v_neg->data_device, V}, lh = {h_pos->data_device, h_neg->data_device, H};
-  if (launch_dependent(k_bias_tail, dim3((unsigned)(vblocks + hblocks)), dim3(32 * kTailLanes), 0, stream(), lv, lh,
-                       suff->data_device, b->data_device, db->data_device, B, vblocks, part, counter,
-                       sq_acc ? sq_acc->data_device : nullptr, -inv_batch, momentum, -eps) != cudaSuccess)
-    return set_error(cudaGetErrorString(cudaGetLastError()));
-  return check_launch();
+  b200_bias_layers t = {{v_pos, h_pos}, {v_neg, h_neg}, {half, half + 3}, {half + 1, half + 4}, {half + 2, half + 5}, sq_acc, 2};
+  return bias_updates(&t, inv_batch, momentum, eps);
 }
 
 namespace {
@@ -375,12 +434,10 @@ namespace {
 // pass (k_split_f16) rewrite the aux with a new exponent.  One pass over the weights in the
 // common case: 24 bytes per weight instead of 28.
 template <bool kHasGrad, int kAux>
-__global__ void __launch_bounds__(256) k_update(float* w, float* delta, float* grad, const float* suff,
-                                                uint16_t* w_aux, float* scale, int rows, int lda, long n, bool vec,
-                                                float ninv_batch, float momentum, float neps, float l2, float l1) {
-  grid_dependents_launch();
-  grid_dependency_wait();
-  const long tid = (long)blockIdx.x * blockDim.x + threadIdx.x, nth = (long)gridDim.x * blockDim.x;
+__device__ __forceinline__ void update_weights(float* w, float* delta, float* grad, const float* suff, uint16_t* w_aux,
+                                               float* scale, int rows, int lda, long n, bool vec, float ninv_batch,
+                                               float momentum, float neps, float l2, float l1, int block, int blocks) {
+  const long tid = (long)block * blockDim.x + threadIdx.x, nth = (long)blocks * blockDim.x;
   float wmax = 0.0f;
   const float f16_scale = kAux == 2 ? exp2f(scale[0]) : 1.0f;
   if (vec) {   // n % 4 == 0, and with an aux rows % 4 == 0: four consecutive elements share a column
@@ -443,6 +500,38 @@ __global__ void __launch_bounds__(256) k_update(float* w, float* delta, float* g
     const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(wmax));
     if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<unsigned*>(scale) + 2, m);
   }
+}
+
+template <bool kHasGrad, int kAux>
+__global__ void __launch_bounds__(256) k_update(float* w, float* delta, float* grad, const float* suff,
+                                                uint16_t* w_aux, float* scale, int rows, int lda, long n, bool vec,
+                                                float ninv_batch, float momentum, float neps, float l2, float l1) {
+  grid_dependents_launch();
+  grid_dependency_wait();
+  update_weights<kHasGrad, kAux>(w, delta, grad, suff, w_aux, scale, rows, lda, n, vec, ninv_batch, momentum, neps, l2, l1,
+                                 (int)blockIdx.x, (int)gridDim.x);
+}
+
+// The biases' blocks and the weights' in one launch: neither needs the other, and one after the other the first, bound by
+// latency, stood before the second, bound by memory.
+struct UpdateArgs {
+  float *w, *delta;
+  const float* suff;
+  uint16_t* w_aux;
+  int rows, lda;
+  long n;
+  bool vec;
+  float ninv_batch, momentum, neps, l2, l1;
+};
+__global__ void __launch_bounds__(256) k_update_all(const __grid_constant__ TailArgs a, const __grid_constant__ UpdateArgs u,
+                                                    int tail_blocks) {
+  grid_dependents_launch();
+  grid_dependency_wait();
+  if ((int)blockIdx.x < tail_blocks)
+    bias_tail(a);
+  else
+    update_weights<false, 1>(u.w, u.delta, nullptr, u.suff, u.w_aux, nullptr, u.rows, u.lda, u.n, u.vec, u.ninv_batch, u.momentum,
+                             u.neps, u.l2, u.l1, (int)blockIdx.x - tail_blocks, (int)gridDim.x - tail_blocks);
 }
 
 // After an update in scaled half-precision form.  The exponent wanted for the new parameter puts
@@ -797,6 +886,31 @@ int momentum_update_columns(cudamat* w, cudamat* delta, cudamat* grad, cudamat* 
 int momentum_update(cudamat* w, cudamat* delta, cudamat* grad, cudamat* suff, cudamat* w_aux, cudamat* w_scale,
                     float inv_batch, float momentum, float eps, float l2, float l1) {
   return momentum_update_columns(w, delta, grad, suff, w_aux, w_scale, 0, w->size[1], inv_batch, momentum, eps, l2, l1);
+}
+
+// bias_updates and momentum_update of a weight matrix with its bfloat16 parts, in one launch where the biases take one.
+int update_all(b200_bias_layers* t, cudamat* w, cudamat* delta, cudamat* suff, cudamat* w_aux, float inv_batch, float mom_b,
+               float eps_b, float mom_w, float eps_w, float l2, float l1) {
+  if (!w->on_device || !delta->on_device || !suff->on_device || !w_aux->on_device) return ERROR_NOT_ON_DEVICE;
+  if (w->is_trans || delta->is_trans || suff->is_trans) return ERROR_TRANSPOSED;
+  if (!same_shape(w, delta) || !same_shape(w, suff) || !aux_shape_ok(w_aux, w)) return ERROR_INCOMPATIBLE_DIMENSIONS;
+  TailArgs a;
+  int tail = 0;
+  int err = plan_bias_tail(t, inv_batch, mom_b, eps_b, a, tail);
+  if (err) return err;
+  const long n = numel(w);
+  if (tail == 0 || n == 0) {
+    err = bias_updates(t, inv_batch, mom_b, eps_b);
+    return err ? err : momentum_update(w, delta, nullptr, suff, w_aux, nullptr, inv_batch, mom_w, eps_w, l2, l1);
+  }
+  UpdateArgs u = {w->data_device, delta->data_device, suff->data_device, reinterpret_cast<uint16_t*>(w_aux->data_device),
+                  w->size[0], aux_rows(w->size[0]), n, false, -inv_batch, mom_w, -eps_w, l2, l1};
+  u.vec = (((uintptr_t)u.w | (uintptr_t)u.delta | (uintptr_t)u.suff | (uintptr_t)u.w_aux) & 15) == 0 && u.rows % 4 == 0;
+  long blocks = ((u.vec ? n / 4 : n) + 255) / 256;
+  if (blocks > (long)sm_count() * 8) blocks = (long)sm_count() * 8;
+  if (launch_dependent(k_update_all, dim3((unsigned)(tail + blocks)), dim3(256), 0, stream(), a, u, tail) != cudaSuccess)
+    return set_error(cudaGetErrorString(cudaGetLastError()));
+  return check_launch();
 }
 
 }  // extern "C"

@@ -80,10 +80,11 @@ class FusedDBM(LossReadback):
             self.kernel_launches = 0
             handles = self._issue(prog, self._batch, gibbs, step == 0, mom, eps, l2, l1)
             rec = self._programs[key] = (prog, handles, self.kernel_launches)
-        prog, (bias_ops, weight_ops), self.kernel_launches = rec
+        prog, (bias_ops, weight_ops, first), self.kernel_launches = rec
         ct.memmove(ct.byref(self._batch.mat), ct.byref(data.mat), ct.sizeof(data.mat))
         self._batch.mat.owns_data = 0
         self._batch_owner = data
+        prog.set_floats(first, f1=mom, f2=eps, f3=mom, f4=eps, f5=l2, f6=l1)
         for i in bias_ops:
             prog.set_floats(i, f1=mom, f2=eps)
         for i in weight_ops:
@@ -116,23 +117,24 @@ class FusedDBM(LossReadback):
                 below = None if j == 0 else ((neg[0], False) if j == 1 else (ns[j - 1], True))
                 above = (ns[j + 1], True) if j < L - 1 else None
                 self._update_layer(X, j, below, above, neg[j], ns[j] if j > 0 else None)
-        # ---- statistics pos - neg and updates: bias statistics are row sums of pos - neg, one launch
-        # a layer (the visible positive state is the data)
-        for j in range(L):
-            X.row_sum_diff(data if j == 0 else pos[j], neg[j], self.suff_b[j])
+        # ---- statistics pos - neg and updates (the visible positive state is the data)
         for i in range(L - 1):
             # the difference of two nearly equal products: TF32 correction terms; the data are exact
             P = cm.split_passes
             p = P(data if i == 0 else pos[i], pos[i + 1].T, exact_a=(i == 0), terms="tf32")
             n = P(neg[i], neg[i + 1].T, negate=1, terms="tf32")
             X.fused_gemm(p + n, out=self.suff_W[i])
-        self.kernel_launches += (L - 1) + L + 1 + (L - 1) + (2 * L if first_step else 0)
+        self.kernel_launches += (L - 1) + 1 + (L - 1) + (2 * L if first_step else 0)
         inv_b = 1.0 / self.B
-        bias_ops = [X.momentum_update(self.b[j], self.db[j], None, self.suff_b[j], inv_b, mom, eps) for j in range(L)]
+        layers = [(data if j == 0 else pos[j], neg[j], self.suff_b[j], self.b[j], self.db[j]) for j in range(L)]
+        # the first four layers' biases go with the first weights (past 1024 cases in launches of their own)
+        first = X.update_all(layers[:4], self.W[0], self.dW[0], self.suff_W[0], self.W_aux[0], inv_b, mom, eps, mom, eps, l2=l2,
+                             l1=l1)
+        bias_ops = [X.bias_updates(layers[j:j + 4], inv_b, mom, eps) for j in range(4, L, 4)]
         weight_ops = [X.momentum_update(self.W[i], self.dW[i], None, self.suff_W[i], inv_b, mom, eps, l2=l2, l1=l1,
-                                        w_aux=self.W_aux[i]) for i in range(L - 1)]
-        self.kernel_launches += 2 * L - 1
-        return bias_ops, weight_ops
+                                        w_aux=self.W_aux[i]) for i in range(1, L - 1)]
+        self.kernel_launches += (len(bias_ops) if self.B <= 1024 else 2 * L) + L - 1
+        return bias_ops, weight_ops, first
 
     def read_loss(self, reset=True):
         v = float(np.array(self.loss_acc.asarray())[0, 0])

@@ -238,7 +238,7 @@ class FusedRBM(LossReadback):
                 ct.memmove(ct.byref(view.mat), ct.byref(m.mat), ct.sizeof(m.mat))
                 view.mat.owns_data = 0
         self._batch_owner = (data, data_aux)
-        if isinstance(ub, tuple):       # the peer-memory update: one operation carries every scalar
+        if isinstance(ub, tuple):       # one operation carries every scalar
             prog.set_floats(ub[1], f0=sc["inv_b"], f1=mom, f2=eps, f3=emom, f4=eeps, f5=l2, f6=l1)
         else:
             prog.set_floats(ub, f0=sc["inv_b"], f1=mom, f2=eps)
@@ -250,16 +250,16 @@ class FusedRBM(LossReadback):
         """All-reduce of the packed statistics, then the two updates (biases are not regularised,
         deepnet/dbm.py:249).  Returns the operations whose scalars follow the schedules.  bias (one rank): (v_pos, v_neg,
         loss accumulator or None), the visible states whose row sums are still to be taken: bias
-        statistics, bias update and error are then one operation."""
+        statistics, error and both updates are then one operation."""
         V, H = self.V, self.H
         if bias is not None:
-            ub = self._op(X, "bias_tail", 0, 8.0 * (V + H) * self.B, "rbm_bias_update", bias[0], bias[1], self.h_pos, self.h_neg,
-                          self.suff_b, self.b, self.db, bias[2], sc["inv_b"], sc["mom"], sc["eps"])
+            layers = [(bias[0], bias[1], self.suff_bv, self.bv, self.dbv), (self.h_pos, self.h_neg, self.suff_bh, self.bh, self.dbh)]
+            u = self._op(X, "update", 0, 8.0 * (V + H) * self.B + 6 * wb, "update_all", layers, self.W, self.dW, self.suff_W,
+                         self.W_aux, sc["inv_b"], sc["mom"], sc["eps"], sc["emom"], sc["eeps"], l2=sc["l2"], l1=sc["l1"],
+                         sq_acc=bias[2])
             if self.B > 1024:      # past that the operation is made of its separate launches
-                self.kernel_launches += 3 if bias[2] is not None else 2
-            uw = self._op(X, "update_W", 0, 6 * wb, "momentum_update", self.W, self.dW, None, self.suff_W, sc["inv_b"],
-                          sc["emom"], sc["eeps"], l2=sc["l2"], l1=sc["l1"], w_aux=self.W_aux, w_scale=w_scale)
-            return ub, uw
+                self.kernel_launches += 5 if bias[2] is not None else 4
+            return ("update", u), None
         if self.dp_peer:
             # exchange + update of every parameter in one pass over peer memory (no NCCL)
             u = self._op(X, "peer_update", 0, 6 * wb, "dp_peer_update", self.W, self.dW, self.W_aux, w_scale, self.pack,

@@ -323,6 +323,16 @@ int b200_test_limit_scratch(size_t bytes);
 int ais_binary_steps(rnd_struct* rnd_state, cudamat* w, cudamat* w_aux, cudamat* a, cudamat* b, cudamat* v_state,
                      cudamat* v_sample, cudamat* h_pre, cudamat* h_sample, cudamat* sb, cudamat* weights,
                      const double* schedule, int n);
+/* Bias statistics (suff = row sums of pos - neg) and bias update of up to four layers in one launch; sq_acc (optional) += squared
+ * difference of the first layer's states.  update_all: the same and momentum_update of a weight matrix with its bfloat16
+ * parts, in one launch. */
+typedef struct b200_bias_layers {
+  cudamat *pos[4], *neg[4], *suff[4], *b[4], *db[4], *sq_acc;
+  int layers;
+} b200_bias_layers;
+int bias_updates(b200_bias_layers* t, float inv_batch, float momentum, float eps);
+int update_all(b200_bias_layers* t, cudamat* w, cudamat* delta, cudamat* suff, cudamat* w_aux, float inv_batch, float mom_b,
+               float eps_b, float mom_w, float eps_w, float l2, float l1);
 /* Bias statistics, bias update and (sq_acc, optional) squared reconstruction error of an RBM with packed biases
  * [visible | hidden] in one launch (deepnet/layer.py:202-213, parameter.py:80-106, logistic_layer.py:48-52). */
 int rbm_bias_update(cudamat* v_pos, cudamat* v_neg, cudamat* h_pos, cudamat* h_neg, cudamat* suff, cudamat* b, cudamat* db,
@@ -396,8 +406,8 @@ int dp_wait(int timeout_ms);
  * 11 div_by_row_vec, 12 add_scalar, 13 assign_scalar, 14 copy_on_device, 15 sample_bernoulli,
  * 16 softmax_sample, 17 momentum_update_columns, 18 dp_allreduce_begin, 19 dp_allreduce_end,
  * 20 b200_set_sm_limit, 21 dp_peer_update, 22 rbm_bias_update,
- * 23 softmax_reconstruction, 24 document_lengths); m[], i0.., f0.. are its arguments in declaration order (matrices, then
- * integers, then floats; gemm for kind 0).  Stops at the first failure: returns its code, *failed_at its index. */
+ * 23 softmax_reconstruction, 24 document_lengths, 25 bias_updates, 26 update_all); m[], i0.., f0.. are its arguments in declaration order (matrices, then
+ * integers, then floats; gemm for kind 0, and pointing to the b200_bias_layers of 25 and 26).  Stops at the first failure: returns its code, *failed_at its index. */
 struct b200_fused_gemm;
 typedef struct b200_op {
   int kind;

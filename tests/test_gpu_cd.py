@@ -624,3 +624,36 @@ def test_softmax_columns_match_their_definition(cm, V):
     np.testing.assert_allclose(get(m["norm"]), p, rtol=1e-5, atol=1e-12)
     again = get(cm.CUDAMatrix(pre).softmax_scaled(nn, target=cm.empty((V, B))))
     np.testing.assert_array_equal(again, get(m["state"]))
+
+
+@pytest.mark.parametrize("sizes,B", [((784, 500), 100), ((33, 1, 64), 7), ((5, 31, 32, 129), 1024), ((40, 30), 1025)])
+@pytest.mark.parametrize("rows", [64, 37])
+def test_updates_in_one_launch_match_the_separate_calls(cm, sizes, B, rows):
+    """Biases of two to four layers (whole and ragged blocks of rows, past the cases one launch takes) and a weight matrix of
+    whole and odd columns: bit for bit what the separate calls give, whose sums over at most 1024 cases differ only in order:
+    1e-5 of the largest sum."""
+    rng = np.random.default_rng(B)
+    f = lambda *s: rng.standard_normal(s).astype(np.float32)
+    host = [(f(n, B), f(n, B), f(n, 1), f(n, 1)) for n in sizes]
+    w, d, g = f(rows, 50), f(rows, 50), f(rows, 50)
+    X = cm.Immediate()
+    results = []
+    for fused in (True, False):
+        layers = [(cm.CUDAMatrix(p), cm.CUDAMatrix(n), cm.empty((p.shape[0], 1)), cm.CUDAMatrix(b), cm.CUDAMatrix(db))
+                  for p, n, b, db in host]
+        W, D, S, acc = cm.CUDAMatrix(w), cm.CUDAMatrix(d), cm.CUDAMatrix(g), cm.empty((1, 1))
+        aux = W.split_bf16(cm.empty_aux((rows, 50)))
+        if fused:
+            X.update_all(layers, W, D, S, aux, 1.0 / B, 0.5, 0.1, 0.9, 0.2, l2=1e-3, l1=1e-4, sq_acc=acc)
+        else:
+            X.sq_diff(layers[0][0], layers[0][1], acc)
+            for p, n, s, b, db in layers:
+                X.row_sum_diff(p, n, s)
+                X.momentum_update(b, db, None, s, 1.0 / B, 0.5, 0.1)
+            X.momentum_update(W, D, None, S, 1.0 / B, 0.9, 0.2, l2=1e-3, l1=1e-4, w_aux=aux)
+        results.append(([get(m) for m in (W, D, aux)], [get(m) for l in layers for m in l[2:]], float(get(acc)[0, 0])))
+    for a, b in zip(results[0][0], results[1][0]):
+        np.testing.assert_array_equal(a.view(np.uint32), b.view(np.uint32))
+    for a, b in zip(results[0][1], results[1][1]):
+        assert np.abs(a - b).max() <= 1e-5 * max(1.0, np.abs(b).max())
+    assert abs(results[0][2] - results[1][2]) <= 1e-6 * results[1][2]
