@@ -1227,15 +1227,42 @@ def ais_binary_steps(w, w_aux, a, b, v_state, v_sample, h_pre, h_sample, weights
                                  steps.ctypes.data_as(ct.POINTER(ct.c_double)), ct.c_int(len(steps))))
 
 
+def _rows_pointer(mat, rows):
+    if rows.dtype != np.float32 or not rows.flags.c_contiguous or rows.shape != (mat.mat.size[1], mat.mat.size[0]):
+        raise CUDAMatException("copy_to_rows needs a C-contiguous float32 array of the transposed shape")
+    return rows.ctypes.data_as(ct.POINTER(ct.c_float))
+
+
 def copy_to_rows(mat, rows):
     """The matrix as (columns x rows) into `rows`, a C-contiguous float32 host array of that shape: the memory of a
     column-major matrix is that of its transpose row by row, so nothing is rearranged or copied twice."""
-    if rows.dtype != np.float32 or not rows.flags.c_contiguous or rows.shape != (mat.mat.size[1], mat.mat.size[0]):
-        raise CUDAMatException("copy_to_rows needs a C-contiguous float32 array of the transposed shape")
+    ptr = _rows_pointer(mat, rows)
     view = cudamat()
     ct.memmove(ct.byref(view), ct.byref(mat.mat), ct.sizeof(view))
-    view.data_host = rows.ctypes.data_as(ct.POINTER(ct.c_float))
+    view.data_host = ptr
     _check(_lib.copy_to_host(ct.byref(view)))
+
+
+class RowsOut(object):
+    """`copy_to_rows` behind the work that produces the matrices: `with RowsOut() as out: out.add(mat, rows)`.  Work enqueued
+    after an `add` may rewrite the matrix of the `add` before it; the rows are there when the block ends."""
+
+    def __enter__(self):
+        self.held = bool(_lib.b200_rows_begin())
+        return self
+
+    def add(self, mat, rows):
+        if self.held:
+            _check(_lib.b200_rows_add(mat.p_mat, _rows_pointer(mat, rows)))
+        else:
+            copy_to_rows(mat, rows)
+
+    def __exit__(self, kind, *_):
+        if self.held:
+            self.held = False
+            err = _lib.b200_rows_end()
+            if kind is None:
+                _check(err)
 
 
 def host_alloc(shape):

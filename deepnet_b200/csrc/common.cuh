@@ -51,6 +51,7 @@ bool stream_capturing();               // the library stream is being captured: 
 int rng_col0();                        // first global column of this process's minibatch shard
 void* workspace(int slot, size_t bytes);  // grow-only cached device scratch of the current stream, slot 0..7
 void* workspace_zeroed(int slot, size_t bytes);  // the same, cleared when first handed out or regrown (counters left at zero by their users)
+void free_rows_staging();              // staging area of results written out, at shutdown
 void free_scalar_words();              // pinned words of the scalar reductions, at shutdown
 int* status_word();                    // device int: non-zero after a bounded wait gave up
 bool initialised();                    // the library stream and status word exist (tries to create them)

@@ -261,6 +261,7 @@ int cublas_shutdown() {
   if (!g_stream) return 0;
   cudaDeviceSynchronize();
   free_scalar_words();
+  free_rows_staging();
   for (Scratch& ws : g_scratch) {
     for (int i = 0; i < kWorkspaces; i++) {
       if (ws.p[i]) cudaFree(ws.p[i]);

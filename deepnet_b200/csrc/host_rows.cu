@@ -1,0 +1,192 @@
+// Results written out to ordinary (pageable) host memory behind the work that produces them.
+//
+// A device-to-host copy into pageable memory goes through the driver's own pinned buffer on the calling thread, which meanwhile
+// issues nothing: 110 us a megabyte, most of a minibatch's time where representations are written out
+// (deepnet/extract_rbm_representation.py).  Here the copy lands in pinned pieces on a stream of its own and a few threads
+// carry the pieces to where they belong, while the caller goes on to the next minibatch.
+// One staging area per process (4 MB and four threads, made on first use, given back by cublas_shutdown): whoever
+// begins while another thread holds it is told so and copies the plain way.
+#include <condition_variable>
+#include <cstring>
+#include <deque>
+#include <mutex>
+#include <thread>
+#include <vector>
+
+#include "common.cuh"
+
+using namespace b200;
+
+namespace {
+
+constexpr int kPieces = 16, kCarriers = 4;
+constexpr size_t kPieceBytes = 256 * 1024;
+
+struct RowsStaging {
+  std::mutex mu;
+  std::condition_variable work, freed;
+  struct Job {
+    int piece;
+    float* dst;
+    size_t bytes;
+  };
+  std::deque<Job> jobs;
+  std::vector<std::thread> carriers;
+  char* pinned = nullptr;
+  cudaEvent_t landed[kPieces] = {nullptr}, ready = nullptr, done[2] = {nullptr, nullptr};
+  cudaStream_t copies = nullptr;
+  bool free_piece[kPieces];
+  int device = 0, in_flight = 0, adds = 0;
+  bool held = false, stop = false, made = false, failed = false;
+
+  void carry() {
+    cudaSetDevice(device);
+    std::unique_lock<std::mutex> lock(mu);
+    for (;;) {
+      work.wait(lock, [&] { return stop || !jobs.empty(); });
+      if (jobs.empty()) return;
+      const Job j = jobs.front();
+      jobs.pop_front();
+      lock.unlock();
+      const bool ok = cudaEventSynchronize(landed[j.piece]) == cudaSuccess;
+      if (ok) memcpy(j.dst, pinned + j.piece * kPieceBytes, j.bytes);
+      lock.lock();
+      failed |= !ok;
+      free_piece[j.piece] = true;
+      in_flight--;
+      freed.notify_all();
+    }
+  }
+  void give_back() {
+    {
+      std::lock_guard<std::mutex> lock(mu);
+      stop = true;
+    }
+    work.notify_all();
+    for (std::thread& t : carriers) t.join();
+    carriers.clear();
+    if (pinned) cudaFreeHost(pinned);
+    pinned = nullptr;
+    for (cudaEvent_t* e : {&ready, &done[0], &done[1]}) {
+      if (*e) cudaEventDestroy(*e);
+      *e = nullptr;
+    }
+    for (cudaEvent_t& e : landed) {
+      if (e) cudaEventDestroy(e);
+      e = nullptr;
+    }
+    if (copies) cudaStreamDestroy(copies);
+    copies = nullptr;
+    made = stop = false;
+  }
+  bool make() {
+    bool ok = cudaGetDevice(&device) == cudaSuccess && cudaMallocHost((void**)&pinned, kPieces * kPieceBytes) == cudaSuccess &&
+              cudaStreamCreateWithFlags(&copies, cudaStreamNonBlocking) == cudaSuccess;
+    for (cudaEvent_t* e : {&ready, &done[0], &done[1]}) ok = ok && cudaEventCreateWithFlags(e, cudaEventDisableTiming) == cudaSuccess;
+    for (cudaEvent_t& e : landed) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
+    for (bool& f : free_piece) f = true;
+    try {
+      for (int i = 0; ok && i < kCarriers; i++) carriers.emplace_back([this] { carry(); });
+    } catch (...) {
+      ok = false;
+    }
+    made = true;
+    if (!ok) {
+      cudaGetLastError();
+      give_back();
+    }
+    return ok;
+  }
+};
+// (never destroyed: the threads of a process that skips cublas_shutdown outlive its static objects)
+RowsStaging& staging() {
+  static RowsStaging* s = new RowsStaging;
+  return *s;
+}
+std::mutex g_holder;     // guards `held` and the making of the staging area
+
+}  // namespace
+
+namespace b200 {
+void free_rows_staging() {
+  std::lock_guard<std::mutex> lock(g_holder);
+  RowsStaging& s = staging();
+  if (s.made && !s.held) s.give_back();
+}
+}  // namespace b200
+
+extern "C" {
+
+// 1: the staging area is the caller's until b200_rows_end; 0: it is taken, or cannot be had (copy the plain way).
+int b200_rows_begin(void) {
+  if (!initialised() || stream_capturing()) return 0;
+  std::lock_guard<std::mutex> lock(g_holder);
+  RowsStaging& s = staging();
+  int device = -1;
+  if (s.held || cudaGetDevice(&device) != cudaSuccess || (s.made && s.device != device)) return 0;
+  if (!s.made && !s.make()) return 0;
+  s.held = true;
+  s.failed = false;
+  s.adds = 0;
+  return 1;
+}
+
+// The matrix into `dst` (numel floats), behind the work enqueued so far.  Work enqueued after this call may rewrite the matrix
+// of the call before; this one's only after the next call or b200_rows_end.
+int b200_rows_add(cudamat* src, float* dst) {
+  RowsStaging& s = staging();
+  if (!s.held) return ERROR_GENERIC;
+  if (!src->on_device) return ERROR_NOT_ON_DEVICE;
+  if (cudaEventRecord(s.ready, stream()) != cudaSuccess || cudaStreamWaitEvent(s.copies, s.ready, 0) != cudaSuccess)
+    return set_error(cudaGetErrorString(cudaGetLastError()));
+  const size_t bytes = (size_t)numel(src) * sizeof(float);
+  for (size_t at = 0; at < bytes; at += kPieceBytes) {
+    const size_t n = bytes - at < kPieceBytes ? bytes - at : kPieceBytes;
+    int piece = -1;
+    {
+      std::unique_lock<std::mutex> lock(s.mu);
+      s.freed.wait(lock, [&] {
+        for (piece = 0; piece < kPieces; piece++)
+          if (s.free_piece[piece]) return true;
+        return false;
+      });
+      s.free_piece[piece] = false;
+    }
+    const bool ok = cudaMemcpyAsync(s.pinned + piece * kPieceBytes, (const char*)src->data_device + at, n, cudaMemcpyDeviceToHost,
+                                    s.copies) == cudaSuccess &&
+                    cudaEventRecord(s.landed[piece], s.copies) == cudaSuccess;
+    std::lock_guard<std::mutex> lock(s.mu);
+    if (!ok) {
+      s.free_piece[piece] = true;
+      s.failed = true;
+      return set_error(cudaGetErrorString(cudaGetLastError()));
+    }
+    s.jobs.push_back({piece, (float*)((char*)dst + at), n});
+    s.in_flight++;
+    s.work.notify_one();
+  }
+  // the matrix of the call before has been read once this stream is past its copies
+  if (s.adds > 0 && cudaStreamWaitEvent(stream(), s.done[(s.adds - 1) & 1], 0) != cudaSuccess)
+    return set_error(cudaGetErrorString(cudaGetLastError()));
+  if (cudaEventRecord(s.done[s.adds & 1], s.copies) != cudaSuccess) return set_error(cudaGetErrorString(cudaGetLastError()));
+  s.adds++;
+  return 0;
+}
+
+// Returns when everything added is where it belongs.
+int b200_rows_end(void) {
+  RowsStaging& s = staging();
+  if (!s.held) return ERROR_GENERIC;
+  bool failed;
+  {
+    std::unique_lock<std::mutex> lock(s.mu);
+    s.freed.wait(lock, [&] { return s.in_flight == 0; });
+    failed = s.failed;
+  }
+  if (s.adds > 0 && cudaStreamWaitEvent(stream(), s.done[(s.adds - 1) & 1], 0) != cudaSuccess) failed = true;
+  std::lock_guard<std::mutex> lock(g_holder);
+  s.held = false;
+  return failed ? set_error("a copy to the host failed") : 0;
+}
+
+}  // extern "C"

@@ -138,6 +138,7 @@ class FusedRBM(LossReadback):
             self.v_samp = z(V, B)
             self.v_act = z(V, B)                  # W h + b_v before the softmax
             self.tiny = 1e-10
+        self._h_out = None                        # second buffer of representations being written out
         self._sched = Parameter(cm, self.hyp)
         self._esched = Parameter(cm, self.ehyp)
         self.kernel_launches = 0
@@ -475,24 +476,28 @@ class FusedRBM(LossReadback):
         rep = np.empty((n * B, self.H), np.float32)
         err = 0.0
         soft = self.visible == REPLICATED_SOFTMAX
-        for b in range(n):
-            v0 = data.slice(b * B, (b + 1) * B)
-            if soft:
-                v0.sum(axis=0, target=self.NN)
-                self.NN.add(self.tiny)
-            cm.fused_gemm(P(W.T, v0, exact_b=soft or self.binary_data, a_aux=Wa), out=self.h_pos, bias=self.bh, activation=1,
-                          col_scale=self.NN if soft else None)
-            if input_recon:
-                down = P(W, self.h_pos, a_aux=Wa)
+        if n > 1 and self._h_out is None:
+            self._h_out = cm.empty((self.H, B))
+        with cm.RowsOut() as out:
+            for b in range(n):
+                v0 = data.slice(b * B, (b + 1) * B)
+                h = self.h_pos if (n - 1 - b) % 2 == 0 else self._h_out    # one is on its way to the host, the last stays
                 if soft:
-                    cm.fused_gemm(down, out=self.v_act, bias=self.bv, activation=0)
-                    self.v_act.softmax_scaled(self.NN, target=self.v_neg)
-                    self.v_neg.div_by_row(self.NN, target=self.v_negn)
-                    cm._check(cm._lib.add_sq_diff(self.v_negn.p_mat, v0.p_mat, self.loss_acc.p_mat))
-                else:
-                    cm.fused_gemm(down, out=self.v_neg, bias=self.bv, activation=self._act(self.visible))
-                    cm._check(cm._lib.add_sq_diff(self.v_neg.p_mat, v0.p_mat, self.loss_acc.p_mat))
-            cm.copy_to_rows(self.h_pos, rep[b * B:(b + 1) * B])
+                    v0.sum(axis=0, target=self.NN)
+                    self.NN.add(self.tiny)
+                cm.fused_gemm(P(W.T, v0, exact_b=soft or self.binary_data, a_aux=Wa), out=h, bias=self.bh, activation=1,
+                              col_scale=self.NN if soft else None)
+                if input_recon:
+                    down = P(W, h, a_aux=Wa)
+                    if soft:
+                        cm.fused_gemm(down, out=self.v_act, bias=self.bv, activation=0)
+                        self.v_act.softmax_scaled(self.NN, target=self.v_neg)
+                        self.v_neg.div_by_row(self.NN, target=self.v_negn)
+                        cm._check(cm._lib.add_sq_diff(self.v_negn.p_mat, v0.p_mat, self.loss_acc.p_mat))
+                    else:
+                        cm.fused_gemm(down, out=self.v_neg, bias=self.bv, activation=self._act(self.visible))
+                        cm._check(cm._lib.add_sq_diff(self.v_neg.p_mat, v0.p_mat, self.loss_acc.p_mat))
+                out.add(h, rep[b * B:(b + 1) * B])
         if input_recon:
             err = self.read_loss()
             return rep, err

@@ -323,6 +323,11 @@ int b200_test_limit_scratch(size_t bytes);
 int ais_binary_steps(rnd_struct* rnd_state, cudamat* w, cudamat* w_aux, cudamat* a, cudamat* b, cudamat* v_state,
                      cudamat* v_sample, cudamat* h_pre, cudamat* h_sample, cudamat* sb, cudamat* weights,
                      const double* schedule, int n);
+/* Results into ordinary host memory behind the work that produces them: begin (0: not to be had, copy_to_host instead), add a
+ * matrix at a time (the one before may be rewritten by work enqueued after), end returns when all is there. */
+int b200_rows_begin(void);
+int b200_rows_add(cudamat* src, float* dst);
+int b200_rows_end(void);
 /* Bias statistics (suff = row sums of pos - neg) and bias update of up to four layers in one launch; sq_acc (optional) += squared
  * difference of the first layer's states.  update_all: the same and momentum_update of a weight matrix with its bfloat16
  * parts, in one launch. */

@@ -657,3 +657,23 @@ def test_updates_in_one_launch_match_the_separate_calls(cm, sizes, B, rows):
     for a, b in zip(results[0][1], results[1][1]):
         assert np.abs(a - b).max() <= 1e-5 * max(1.0, np.abs(b).max())
     assert abs(results[0][2] - results[1][2]) <= 1e-6 * results[1][2]
+
+
+def test_representations_leave_while_the_next_minibatch_is_computed(cm):
+    """Several pieces a minibatch and a ragged last one, an even and an odd number of minibatches, and the staging area taken by
+    someone else (plain copies): the rows are the products', bit for bit."""
+    rng = np.random.default_rng(4)
+    V, H, B = 300, 701, 250
+    w = (rng.standard_normal((V, H)) * 0.05).astype(np.float32)
+    eng = FusedRBM(cm, V, H, B, w, dbm.Hyperparams(), binary_data=True, seed=1)
+    for n in (4, 3, 1):
+        x = (rng.random((V, n * B)) < 0.3).astype(np.float32)
+        data = cm.CUDAMatrix(x)
+        with cm.RowsOut() as taken:
+            assert taken.held
+            want = eng.Inference(data)
+        got = eng.Inference(data)
+        np.testing.assert_array_equal(got, want)
+        np.testing.assert_array_equal(get(eng.h_pos).T, got[(n - 1) * B:])
+        assert np.abs(got - 1 / (1 + np.exp(-(x.T.astype(np.float64) @ w)))).max() < 1e-5
+    assert cm.read_status() == 0
