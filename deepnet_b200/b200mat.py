@@ -753,8 +753,8 @@ def correct_preds(mat, p, target=None, cutoff=0.5):
 
 
 def fused_gemm(passes, out=None, sample=None, bias=None, col_scale=None, activation=0, alpha=1.0, beta=0.0,
-               out_aux=None, sample_aux=None, scale_exp=None, scale_exp_const=0, aux_f16=False, aux_exp=0):
-    """out = act(alpha * sum_p (+/-) a_p . b_p + beta * out + bias (x) col_scale) in one kernel.
+               out_aux=None, sample_aux=None, scale_exp=None, scale_exp_const=0, aux_f16=False, aux_exp=0, add=None):
+    """out = act(alpha * sum_p (+/-) a_p . b_p + beta * out + add + bias (x) col_scale) in one kernel.
 
     `passes` is a list of (a, b) or (a, b, negate); a and b are fp32 matrices, `.T` views, or
     parts of them (`lo32(x)`, `lo16(x)`, `b16(x)`, see `split_passes`); both operands of a
@@ -768,7 +768,7 @@ def fused_gemm(passes, out=None, sample=None, bias=None, col_scale=None, activat
     """
     f = _build_fused_gemm(passes, out, sample, bias, col_scale, activation, alpha, beta, out_aux, sample_aux, scale_exp,
                           scale_exp_const, aux_f16, aux_exp)
-    _check(_lib.fused_gemm(CUDAMatrix.rnd_state_p, ct.byref(f)))
+    _check(_lib.fused_gemm_add(CUDAMatrix.rnd_state_p, ct.byref(f), add.p_mat if add is not None else None))
 
 
 def _build_bias_layers(layers, sq_acc):
@@ -968,7 +968,8 @@ class Program(object):
         for p in passes:
             self._keep.extend([p[0], p[1]])
         self._keep.extend(v for v in kw.values() if isinstance(v, CUDAMatrix))
-        return self._add(OP_FUSED_GEMM, gemm=_build_fused_gemm(passes, **kw))
+        add = kw.pop("add", None)
+        return self._add(OP_FUSED_GEMM, (add,), gemm=_build_fused_gemm(passes, **kw))
 
     def sum(self, mat, axis, target):
         return self._add(OP_SUM_AXIS, (mat, target), (axis,))

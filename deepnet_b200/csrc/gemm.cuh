@@ -76,6 +76,7 @@ struct GemmProblem {
   // 1: part kPartX is read as TF32 (low 13 mantissa bits ignored), its meaning on the tensor
   // cores, which the CUDA-core kernel then reproduces; 0: kPartX is the full fp32 value.
   int tf32_operands;
+  const float* prior = nullptr;   // what beta multiplies instead of epi.out (gemm_small only), columns ldo apart
   int odd = 0;       // 1: some operand is a copy of a matrix TMA cannot address
   GemmPass pass[kMaxPass];
   GemmEpilogue epi;

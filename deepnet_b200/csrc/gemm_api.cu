@@ -81,6 +81,18 @@ int short_tf32(const GemmProblem& g) {
 }
 
 int run(const GemmProblem& g) {
+  if (g.prior) {
+    // the one-launch kernel reads another matrix there; for the others, whose products are long, it is copied to the output
+    if (g_path == 3 || (g_path == 0 && (gemm_tc_supported(g) ? small_beats_tc(g) : small_depth(g) <= kSmallDepth))) {
+      const int r = gemm_small(g, kSmallSplit);
+      if (r != ERROR_UNSUPPORTED) return r;
+    }
+    if (cudaMemcpyAsync(g.epi.out, g.prior, (size_t)g.M * g.N * sizeof(float), cudaMemcpyDeviceToDevice, stream()) != cudaSuccess)
+      return set_error(cudaGetErrorString(cudaGetLastError()));
+    GemmProblem copied = g;
+    copied.prior = nullptr;
+    return run(copied);
+  }
   if (product_is_scattered(g.epi.out)) return gemm_tc(g);   // (fails loudly when the tensor-core kernel cannot take it)
   if (g_path == 2) return gemm_simt(g);
   if (g_path == 3) return gemm_small(g, kSmallSplit);
@@ -661,7 +673,9 @@ int split_f16(cudamat* x, cudamat* aux, cudamat* exp_dev, int exp_const) {
   return check_launch();
 }
 
-int fused_gemm(rnd_struct* rnd_state, b200_fused_gemm* f) {
+// The same with add (M x N, or null) added to every output before the activation (beta 0, out given): what a layer gets from a
+// neighbour that stands still is multiplied once.
+int fused_gemm_add(rnd_struct* rnd_state, b200_fused_gemm* f, cudamat* add) {
   if (f->npass <= 0 || f->npass > kMaxPass) return ERROR_UNSUPPORTED;
   GemmProblem g;
   g.npass = f->npass;
@@ -722,6 +736,14 @@ int fused_gemm(rnd_struct* rnd_state, b200_fused_gemm* f) {
   if (f->sample) e.sample = f->sample->data_device;
   if (f->sample_aux) e.sample_aux = f->sample_aux->data_device;
   if (e.beta != 0.0f && !e.out) return ERROR_UNSUPPORTED;
+  if (add) {
+    if (!add->on_device) return ERROR_NOT_ON_DEVICE;
+    if (add->is_trans) return ERROR_TRANSPOSED;
+    if (add->size[0] != g.M || add->size[1] != g.N) return ERROR_INCOMPATIBLE_DIMENSIONS;
+    if (e.beta != 0.0f || !e.out) return ERROR_UNSUPPORTED;
+    e.beta = 1.0f;
+    if (add->data_device != e.out) g.prior = add->data_device;
+  }
   if (f->bias) {
     if (!f->bias->on_device) return ERROR_NOT_ON_DEVICE;
     if (numel(f->bias) != g.M) return ERROR_INCOMPATIBLE_DIMENSIONS;
@@ -740,6 +762,7 @@ int fused_gemm(rnd_struct* rnd_state, b200_fused_gemm* f) {
   }
   return run(g);
 }
+int fused_gemm(rnd_struct* rnd_state, b200_fused_gemm* f) { return fused_gemm_add(rnd_state, f, nullptr); }
 
 // cudamat/cudamat.cu:1671-1696: target = beta * target + alpha * op(mat1) . op(mat2).
 int dot(cudamat* mat1, cudamat* mat2, cudamat* target, float beta, float alpha) {

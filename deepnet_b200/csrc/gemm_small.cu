@@ -67,6 +67,7 @@ struct SmallParams {
   int M, N, tiles_m;
   int ieee;            // non-finite results are computed again: in plain fp32 (`dot` keeps the meaning of inf), else as
                        // the tcgen05 kernel's parts give them
+  const float* prior;  // what beta multiplies
   GemmEpilogue e;
 };
 
@@ -477,7 +478,7 @@ __global__ void __launch_bounds__(kSmallThreads, 2) k_gemm_small(const __grid_co
 #pragma unroll
     for (int j = 0; j < 4; j++) {
       x[j] *= alpha;
-      if (e.beta != 0.0f && j < ncols) x[j] += e.beta * e.out[off + (long)j * e.ldo];
+      if (e.beta != 0.0f && j < ncols) x[j] += e.beta * p.prior[off + (long)j * e.ldo];
       if (e.bias) x[j] += (e.col_scale && j < ncols) ? bias * e.col_scale[n + j] : bias;
       if (e.activation == 1) x[j] = sigmoid_accurate(x[j]);
     }
@@ -708,6 +709,7 @@ int gemm_small(const GemmProblem& g, SmallForm form) {
   if (fp32 && (p.npairs != 1 || p.pair[0].negate)) return ERROR_UNSUPPORTED;
   p.ieee = form == kSmallIeee || form == kSmallFp32;
   p.e = g.epi;
+  p.prior = g.prior ? g.prior : g.epi.out;
   const long ctas = cut_up(g, p);
   if (ctas > 0x7fffffffL) return ERROR_UNSUPPORTED;
   void (*const kernel)(SmallParams) = fp32 ? k_gemm_small<true> : k_gemm_small<false>;

@@ -13,7 +13,7 @@ struct b200_fused_gemm;
 struct b200_bias_layers;
 
 extern "C" {
-int fused_gemm(rnd_struct* rnd_state, b200_fused_gemm* f);
+int fused_gemm_add(rnd_struct* rnd_state, b200_fused_gemm* f, cudamat* add);
 int sum_by_axis(cudamat* mat, cudamat* target, int axis);
 int add_sum_by_axis(cudamat* mat, cudamat* target, int axis, float mult);
 int row_sum_diff(cudamat* a, cudamat* b, cudamat* target);
@@ -48,7 +48,7 @@ int softmax_sample(rnd_struct* rnd_state, cudamat* pre, cudamat* bias, cudamat* 
 }
 
 enum {
-  B200_OP_FUSED_GEMM = 0,      // gemm
+  B200_OP_FUSED_GEMM = 0,      // gemm, m0 add?
   B200_OP_SUM_AXIS = 1,        // m0 mat, m1 target, i0 axis
   B200_OP_ADD_SUM_AXIS = 2,    // m0 mat, m1 target, i0 axis, f0 mult
   B200_OP_ROW_SUM_DIFF = 3,    // m0 a, m1 b, m2 target
@@ -93,7 +93,7 @@ extern "C" int b200_run_program(rnd_struct* rnd_state, b200_op* ops, int n, int*
     b200_op& o = ops[i];
     int err = ERROR_UNSUPPORTED;
     switch (o.kind) {
-      case B200_OP_FUSED_GEMM: err = fused_gemm(rnd_state, o.gemm); break;
+      case B200_OP_FUSED_GEMM: err = fused_gemm_add(rnd_state, o.gemm, o.m[0]); break;
       case B200_OP_SUM_AXIS: err = sum_by_axis(o.m[0], o.m[1], o.i0); break;
       case B200_OP_ADD_SUM_AXIS: err = add_sum_by_axis(o.m[0], o.m[1], o.i0, o.f0); break;
       case B200_OP_ROW_SUM_DIFF: err = row_sum_diff(o.m[0], o.m[1], o.m[2]); break;

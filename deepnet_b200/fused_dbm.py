@@ -40,6 +40,7 @@ class FusedDBM(LossReadback):
         self.pos = [z(n, B) for n in sizes]
         self.neg = [z(n, B) for n in sizes]
         self.neg_sample = [z(n, B) for n in sizes]
+        self.from_data = z(sizes[1], B)           # W[0]' data of the positive phase
         self.loss_acc = z(1, 1)
         self._sched = Parameter(cm, hyperparams)
         self.kernel_launches = 0
@@ -49,8 +50,8 @@ class FusedDBM(LossReadback):
         self._programs = {}
         self._batch = cm.CUDAMatrix._from_mat(cm.cudamat())
 
-    def _update_layer(self, X, j, below, above, out, sample):
-        """state_j = sigmoid(W[j-1]' below + W[j] above + b_j) (deepnet/dbm.py:82-105), optional draw.
+    def _update_layer(self, X, j, below, above, out, sample, add=None):
+        """state_j = sigmoid(W[j-1]' below + W[j] above + add + b_j) (deepnet/dbm.py:82-105), optional draw.
         below / above = (state, exact): exact states (0/1) have no low part."""
         P = self.cm.split_passes
         passes = []
@@ -58,7 +59,7 @@ class FusedDBM(LossReadback):
             passes += P(self.W[j - 1].T, below[0], exact_b=below[1], a_aux=self.W_aux[j - 1])
         if above is not None:
             passes += P(self.W[j], above[0], exact_b=above[1], a_aux=self.W_aux[j])
-        X.fused_gemm(passes, out=out, sample=sample, bias=self.b[j], activation=1)
+        X.fused_gemm(passes, out=out, sample=sample, bias=self.b[j], activation=1, add=add)
         self.kernel_launches += 1
 
     def TrainOneBatch(self, step, data):
@@ -97,11 +98,19 @@ class FusedDBM(LossReadback):
         # ---- positive phase: data clamped, hidden layers start at zero, mean-field sweeps
         for j in range(1, L):
             X.assign_scalar(pos[j], 0)
-        for _ in range(self.hyp.mf_steps):
+        # W[0]' data is the same in every sweep: multiplied once where there is more than one
+        once = self.hyp.mf_steps > 1 and L > 2
+        if once:
+            X.fused_gemm(cm.split_passes(self.W[0].T, data, exact_b=True, a_aux=self.W_aux[0]), out=self.from_data)
+            self.kernel_launches += 1
+        for sweep in range(self.hyp.mf_steps):
             for j in range(1, L):
                 below = (data, True) if j == 1 else (pos[j - 1], False)
                 above = (pos[j + 1], False) if j < L - 1 else None
-                self._update_layer(X, j, below, above, pos[j], None)
+                if j == 1 and once and sweep > 0:
+                    self._update_layer(X, j, None, above, pos[j], None, add=self.from_data)
+                else:      # (in the first sweep the layer above is zero)
+                    self._update_layer(X, j, below, above if sweep > 0 or j > 1 else None, pos[j], None)
         # PCD reports the reconstruction of the input from the first hidden layer (deepnet/dbm.py:163-166)
         self._update_layer(X, 0, None, (pos[1], False), pos[0], None)
         X.sq_diff(pos[0], data, self.loss_acc)

@@ -234,6 +234,7 @@ typedef struct b200_fused_gemm {
   int aux_exp;           /*   ... with this exponent */
 } b200_fused_gemm;
 int fused_gemm(rnd_struct* rnd_state, b200_fused_gemm* f);
+int fused_gemm_add(rnd_struct* rnd_state, b200_fused_gemm* f, cudamat* add);   /* add (out's shape, or null) is added before the activation */
 
 /* lo = x - tf32(x); hi (may be NULL) = tf32(x): the split the kernels apply on the fly. */
 int split_tf32(cudamat* x, cudamat* hi, cudamat* lo);
@@ -412,7 +413,7 @@ int dp_wait(int timeout_ms);
  * 16 softmax_sample, 17 momentum_update_columns, 18 dp_allreduce_begin, 19 dp_allreduce_end,
  * 20 b200_set_sm_limit, 21 dp_peer_update, 22 rbm_bias_update,
  * 23 softmax_reconstruction, 24 document_lengths, 25 bias_updates, 26 update_all); m[], i0.., f0.. are its arguments in declaration order (matrices, then
- * integers, then floats; gemm for kind 0, and pointing to the b200_bias_layers of 25 and 26).  Stops at the first failure: returns its code, *failed_at its index. */
+ * integers, then floats; gemm for kind 0, whose m[0] is add or null, and pointing to the b200_bias_layers of 25 and 26).  Stops at the first failure: returns its code, *failed_at its index. */
 struct b200_fused_gemm;
 typedef struct b200_op {
   int kind;

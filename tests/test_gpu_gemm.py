@@ -970,3 +970,25 @@ def test_narrow_tiles_of_products_of_few_tiles(cm, M, N, K, two_pairs):
     unit.sample_bernoulli(target=again)                       # the same stream on the same probabilities
     np.testing.assert_array_equal(draws, np.array(again.asarray()))
     assert cm.read_status() == 0
+
+
+@pytest.mark.parametrize("path", [0, 1, 2, 3])
+@pytest.mark.parametrize("M,N,K", [(64, 4, 32), (500, 100, 1000), (129, 260, 96), (4, 1, 8), (1000, 2048, 40)])
+def test_added_matrix_joins_before_the_activation(cm, path, M, N, K):
+    """out = logistic(a.b + add + bias) and its draw in every kernel that ends a product: one launch, tcgen05 whole and cut
+    along K, CUDA cores; 1e-5 as for the product alone."""
+    rng = np.random.default_rng(M * N)
+    a, b = (rng.standard_normal((K, M)) * 0.1).astype(np.float32), rng.random((K, N)).astype(np.float32)
+    add, bias = rng.standard_normal((M, N)).astype(np.float32), rng.standard_normal((M, 1)).astype(np.float32)
+    out, plain, draw = cm.empty((M, N)), cm.empty((M, N)), cm.empty((M, N))
+    passes = cm.split_passes(cm.CUDAMatrix(a).T, cm.CUDAMatrix(b))
+    cm.CUDAMatrix.init_random(1)
+    cm.set_gemm_path(path)
+    cm.fused_gemm(passes, out=out, sample=draw, bias=cm.CUDAMatrix(bias), activation=1, add=cm.CUDAMatrix(add))
+    cm.fused_gemm(passes, out=plain, add=cm.CUDAMatrix(add))
+    pre = a.T.astype(np.float64) @ b + add
+    assert np.abs(get(out) - 1 / (1 + np.exp(-(pre + bias)))).max() < TOL
+    assert np.abs(get(plain) - pre).max() < TOL * np.abs(pre).max()
+    assert 0 < get(draw).mean() < 1 or M * N < 32
+    with pytest.raises(cm.CUDAMatException):
+        cm.fused_gemm(passes, out=out, add=cm.empty((M, N + 1)))
