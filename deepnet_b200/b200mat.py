@@ -763,8 +763,8 @@ def fused_gemm(passes, out=None, sample=None, bias=None, col_scale=None, activat
     (bfloat16 parts) of result and draw.  With operands in scaled half-precision form
     (`f16_passes`) the terms carry 2^(scale_exp + scale_exp_const) (scale_exp: 1 x 1 device matrix
     or None), which the kernel divides out; aux_f16: the aux outputs are written in that form
-    with exponent aux_exp.  Replaces the dot / add_dot / add_col_vec / sigmoid /
-    sample_bernoulli group of deepnet/dbm.py:88-105.
+    with exponent aux_exp.  `add` (a matrix of out's shape) needs an `out` and beta = 0.  Replaces the dot / add_dot /
+    add_col_vec / sigmoid / sample_bernoulli group of deepnet/dbm.py:88-105.
     """
     f = _build_fused_gemm(passes, out, sample, bias, col_scale, activation, alpha, beta, out_aux, sample_aux, scale_exp,
                           scale_exp_const, aux_f16, aux_exp)

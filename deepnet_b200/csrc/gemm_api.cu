@@ -80,23 +80,41 @@ int short_tf32(const GemmProblem& g) {
   return k < 128 || (pairs == 1 && low == 1) ? kOneLaunch : kAnyLength;
 }
 
-int run(const GemmProblem& g) {
-  if (g.prior) {
-    // the one-launch kernel reads another matrix there; for the others, whose products are long, it is copied to the output
-    if (g_path == 3 || (g_path == 0 && (gemm_tc_supported(g) ? small_beats_tc(g) : small_depth(g) <= kSmallDepth))) {
-      const int r = gemm_small(g, kSmallSplit);
-      if (r != ERROR_UNSUPPORTED) return r;
-    }
-    if (cudaMemcpyAsync(g.epi.out, g.prior, (size_t)g.M * g.N * sizeof(float), cudaMemcpyDeviceToDevice, stream()) != cudaSuccess)
-      return set_error(cudaGetErrorString(cudaGetLastError()));
-    GemmProblem copied = g;
-    copied.prior = nullptr;
-    return run(copied);
+__global__ void __launch_bounds__(256) k_copy(const float* x, float* y, long n, bool vec) {
+  grid_dependents_launch();
+  grid_dependency_wait();
+  const long tid = (long)blockIdx.x * blockDim.x + threadIdx.x, nth = (long)gridDim.x * blockDim.x;
+  if (vec) {
+    for (long i = tid; i < n / 4; i += nth) reinterpret_cast<float4*>(y)[i] = reinterpret_cast<const float4*>(x)[i];
+  } else {
+    for (long i = tid; i < n; i += nth) y[i] = x[i];
   }
-  if (product_is_scattered(g.epi.out)) return gemm_tc(g);   // (fails loudly when the tensor-core kernel cannot take it)
-  if (g_path == 2) return gemm_simt(g);
+}
+
+// The one-launch kernel reads the matrix that is added where it lies; the others, whose products are long, find it in the
+// output.  (A kernel, not cudaMemcpyAsync: the launches around it stay dependent.)
+int prior_to_output(GemmProblem& g) {
+  const long n = (long)g.M * g.N;
+  if (!g.prior || n == 0) return 0;
+  const bool vec = n % 4 == 0 && (((uintptr_t)g.prior | (uintptr_t)g.epi.out) & 15) == 0;
+  long blocks = ((vec ? n / 4 : n) + 255) / 256;
+  if (blocks > (long)sm_count() * 8) blocks = (long)sm_count() * 8;
+  if (launch_dependent(k_copy, dim3((unsigned)blocks), dim3(256), 0, stream(), g.prior, g.epi.out, n, vec) != cudaSuccess)
+    return set_error(cudaGetErrorString(cudaGetLastError()));
+  g.prior = nullptr;
+  return check_launch();
+}
+
+// A product takes the same way with a matrix to add as without.
+int run(GemmProblem& g) {
+  auto after_copy = [&](int (*kernel)(const GemmProblem&)) {
+    const int err = prior_to_output(g);
+    return err ? err : kernel(g);
+  };
+  if (product_is_scattered(g.epi.out)) return after_copy(gemm_tc);   // (fails loudly when the tensor-core kernel cannot take it)
+  if (g_path == 2) return after_copy(gemm_simt);
   if (g_path == 3) return gemm_small(g, kSmallSplit);
-  if (g_path == 4) return gemm_tc_packed(g);
+  if (g_path == 4) return after_copy(gemm_tc_packed);
   const bool tc = gemm_tc_supported(g);
   int r = ERROR_UNSUPPORTED;
   if (g_path == 0 && tc) {
@@ -108,11 +126,11 @@ int run(const GemmProblem& g) {
   }
   if (r != ERROR_UNSUPPORTED) return r;
   // (unsupported: more operand pairs or tiles than one tensor-core launch carries)
-  if (tc) r = gemm_tc(g);
-  else if (g_path == 0) r = gemm_tc_packed(g);
+  if (tc) r = after_copy(gemm_tc);
+  else if (g_path == 0) r = after_copy(gemm_tc_packed);
   if (r != ERROR_UNSUPPORTED || g_path == 1) return r;
   r = gemm_small(g, kSmallSplit);
-  return r != ERROR_UNSUPPORTED ? r : gemm_simt(g);
+  return r != ERROR_UNSUPPORTED ? r : after_copy(gemm_simt);
 }
 
 // hi may be null: the tensor core itself drops the low 13 mantissa bits of an fp32

@@ -234,7 +234,7 @@ typedef struct b200_fused_gemm {
   int aux_exp;           /*   ... with this exponent */
 } b200_fused_gemm;
 int fused_gemm(rnd_struct* rnd_state, b200_fused_gemm* f);
-int fused_gemm_add(rnd_struct* rnd_state, b200_fused_gemm* f, cudamat* add);   /* add (out's shape, or null) is added before the activation */
+int fused_gemm_add(rnd_struct* rnd_state, b200_fused_gemm* f, cudamat* add);   /* add (out's shape, or null; needs out and beta 0) is added before the activation */
 
 /* lo = x - tf32(x); hi (may be NULL) = tf32(x): the split the kernels apply on the fly. */
 int split_tf32(cudamat* x, cudamat* hi, cudamat* lo);

@@ -992,3 +992,19 @@ def test_added_matrix_joins_before_the_activation(cm, path, M, N, K):
     assert 0 < get(draw).mean() < 1 or M * N < 32
     with pytest.raises(cm.CUDAMatException):
         cm.fused_gemm(passes, out=out, add=cm.empty((M, N + 1)))
+
+
+@pytest.mark.parametrize("M,N,K,terms,exact", [(201, 101, 65, "tf32", False), (201, 101, 399, "tf32", True), (201, 101, 801, "tf32", True),
+                                               (601, 203, 1357, "tf32", False), (1021, 255, 1021, "bf16", False),
+                                               (2047, 511, 700, "tf32", False), (500, 100, 784, "bf16", True)])
+def test_a_matrix_to_add_leaves_the_product_where_it_was(cm, M, N, K, terms, exact):
+    """The product takes the same kernel and the same terms with a matrix to add as without: with zeros to add, bit for bit the
+    same result (odd matrices whose TF32 terms are short, long or have an exact operand, behind copies, and in one launch)."""
+    rng = np.random.default_rng(M + K)
+    a = rng.standard_normal((K, M)).astype(np.float32)
+    b = (rng.random((K, N)) < 0.5).astype(np.float32) if exact else rng.standard_normal((K, N)).astype(np.float32)
+    passes = cm.split_passes(cm.CUDAMatrix(a).T, cm.CUDAMatrix(b), exact_b=exact, terms=terms)
+    plain, added = cm.empty((M, N)), cm.empty((M, N))
+    cm.fused_gemm(passes, out=plain)
+    cm.fused_gemm(passes, out=added, add=cm.empty((M, N)))
+    np.testing.assert_array_equal(get(added), get(plain))
