@@ -1536,45 +1536,66 @@ static int splits_of(int ctas, int min_ki) {
   return want > 32 ? 32 : (want < 1 ? 1 : want);
 }
 
+static int g_tile_columns = 0, g_last_columns = 0;   // b200_test_tile_columns
+
+// What the converters make of a pair's fp32 tiles decides how long a k-block takes: nothing or one 16-bit plane (parts of the
+// other operand from an aux matrix), two (or one fp32 low part), and both parts of both operands, of bfloat16 or of TF32.
+enum { kLightPair, kHalfPair, kDerivedBf16, kDerivedTf32, kPairKinds };
+
 // Columns of a tile.  One CTA per 128 rows up to N = 128.  Wider products share 256 x 256 tiles between two CTAs, which runs
 // the tensor pipe at its rate, where the tiles fill the device; a product of few tiles is bound by what surrounds them, and
-// narrower tiles of a single CTA come off better: the epilogue of 128 accumulator columns per thread takes 19 000 clocks
-// for a partial tile and as many for an activation, that of 64 takes 3900 and 18 600, of 32 1900 and 8600.  Clocks of a
-// k-block: 1060, 960, 840.  Measured, 256 / 128 / 64 columns, us with the finishing launch:
-//   4096 x 256, K = 1024      30.3 / 25.4 / 25.8       2048 x 512, K = 2048    36.4 / 34.8 / 42.1
-//   1024 x 256, K = 4096      29.8 / 21.8 / 27.0       500 x 2048, K = 784     27.8 / 21.5 / 19.7
-//   1000 x 2048, K = 500      34.5 / 28.0 / 30.7       1024 x 4096, two pairs of K = 256, plain   28.9 / 39.9 / 67.3
+// narrower tiles of a single CTA come off better, unless they are bound by the converters, which derive the parts of a tile's
+// rows and columns once a tile.  The estimate, in us, is fitted to 1088 products of 19 shapes (256 to 4096 rows and columns), K
+// from 64 to 4096 and eight term lists (rms error 7 %); its choice is within 0.5 % of the best width on average, never behind
+// 256.  Measured, 256 / 128 / 64 columns:
+//   500 x 500, K = 784, activation, W's parts from memory          21.6 / 15.4 / 14.7
+//   1000 x 2048, K = 500, the same                                 31.2 / 22.9 / 24.3
+//   1024 x 256, K = 4096, the same                                 30.1 / 21.4 / 24.4
+//   784 x 1000, difference of two of K = 1024, all parts derived   37.4 / 43.9 / 64.1   (128 columns by an estimate without
+//   2048 x 512, K = 2048, TF32 parts derived                          38.7 / 44.7 / 63.4    the converters)
 // Products on 16-bit planes alone (the big models' own) and odd matrices keep the wide tiles.
 static int tile_columns(const GemmProblem& g) {
   if (g.N <= 64) return 64;
   if (g.N <= 128) return 128;
   if (g_split_mode != 0 || g.odd || g.M <= BM || product_is_scattered(g.epi.out)) return 256;
-  int slabs = 0, min_ki = 1 << 30;
-  for (int q = 0; q < g.npass; q++) {
-    const GemmPass& t = g.pass[q];
-    if (part_is_f16(t.a.part)) return 256;
-    if (q > 0 && same_operand(t.a, g.pass[q - 1].a) && same_operand(t.b, g.pass[q - 1].b) && t.k == g.pass[q - 1].k) continue;
-    const int ki = (t.k + 31) / 32;
-    slabs += ki;
+  int blocks[kPairKinds] = {0}, min_ki = 1 << 30;
+  for (int q = 0; q < g.npass;) {
+    const GemmPass& first = g.pass[q];
+    const int ki = (first.k + 31) / 32;
+    int planes = 0;
+    bool tf32 = false;
+    for (; q < g.npass; q++) {      // the terms of a pair
+      const GemmPass& t = g.pass[q];
+      if (part_is_f16(t.a.part)) return 256;
+      if (!same_operand(t.a, first.a) || !same_operand(t.b, first.b) || t.k != first.k) break;
+      planes += (part_is_16bit(t.a.part) && !t.a.aux) + (part_is_16bit(t.b.part) && !t.b.aux);
+      if (t.a.part == kPartLo32 || t.b.part == kPartLo32) {
+        planes += 2;
+        tf32 = true;
+      }
+    }
+    blocks[planes < 2 ? kLightPair : planes == 2 ? kHalfPair : tf32 ? kDerivedTf32 : kDerivedBf16] += ki;
     min_ki = ki < min_ki ? ki : min_ki;
   }
-  const bool plain = plain_result(g.epi);
+  if (g_tile_columns) return g_tile_columns;
+  // by width: 256, 128, 64
+  static const float block_us[kPairKinds][3] = {{0.53f, 0.49f, 0.40f}, {0.72f, 0.60f, 0.55f}, {0.76f, 0.81f, 0.82f}, {1.01f, 1.00f, 0.92f}};
+  static const float plain_us[3] = {7.7f, 1.6f, 0.5f}, activation_us[3] = {23.1f, 6.2f, 3.3f}, partial_us[3] = {7.8f, 0.5f, 0.0f};
+  const float* const whole_us = plain_result(g.epi) ? plain_us : activation_us;
   const int sms = sm_count();
   int best = 256;
-  float best_clocks = 0.0f;
-  for (int bn = 256; bn >= 64; bn /= 2) {
+  float best_us = 0.0f;
+  for (int i = 0, bn = 256; bn >= 64; i++, bn /= 2) {
     const long ctas = bn == 256 ? 2L * ((g.M + 255) / 256) * ((g.N + 255) / 256) : (long)((g.M + BM - 1) / BM) * ((g.N + bn - 1) / bn);
     const int splits = ctas < sms && min_ki >= 8 ? splits_of((int)ctas, min_ki) : 1;
-    const float waves = (float)((ctas * splits + sms - 1) / sms), depth = (float)slabs / splits;
-    const float block = bn == 256 ? 1060.0f : (bn == 128 ? 960.0f : 840.0f);
-    const float tile = splits > 1 ? (bn == 256 ? 18900.0f : (bn == 128 ? 3900.0f : 1900.0f)) + 10000.0f + 1200.0f * splits
-                       : plain    ? (bn == 256 ? 14200.0f : (bn == 128 ? 10000.0f : 7800.0f))
-                                  : (bn == 256 ? 20000.0f : (bn == 128 ? 18600.0f : 8600.0f));
-    const float clocks = 5000.0f + waves * (depth * block + tile);
-    // (a narrower tile has to come out ahead by what the estimate is good for)
-    if (bn == 256 || clocks < 0.95f * best_clocks) {
+    float us = 0.0f;
+    for (int t = 0; t < kPairKinds; t++) us += blocks[t] * block_us[t][i];
+    us = 4.3f + (float)((ctas * splits + sms - 1) / sms) * (us / splits + (splits > 1 ? partial_us[i] : whole_us[i]));
+    if (splits > 1) us += 3.3f + 0.27f * splits + 1.4e-6f * g.M * g.N * (splits + 1);   // the finishing launch
+    // (a narrower tile has to come out ahead)
+    if (bn == 256 || us < 0.97f * best_us) {
       best = bn;
-      best_clocks = clocks;
+      best_us = us;
     }
   }
   return best;
@@ -1588,6 +1609,7 @@ int gemm_tc(const GemmProblem& g) {
   if (!gemm_tc_supported(g))
     return scatter ? set_error("a product whose result is scattered to peers must run on the tensor cores") : ERROR_UNSUPPORTED;
   const int BN = tile_columns(g);
+  g_last_columns = BN;
   static int pair_mode = -1;   // B200_GEMM_2CTA=0 keeps one CTA per tile
   static int chunk_k = 0;
   if (pair_mode < 0) {
@@ -1905,6 +1927,13 @@ int gemm_tc(const GemmProblem& g) {
 extern "C" int b200_test_inject_stage_bytes(int extra_bytes) {
   b200::g_inject_stage_bytes = extra_bytes > 0 ? extra_bytes : 0;
   return 0;
+}
+
+// Test hook: the tiles' columns (64, 128, 256; 0 by the estimate) where the estimate has the choice.  Returns those of the last
+// tensor-core product.
+extern "C" int b200_test_tile_columns(int columns) {
+  if (columns == 0 || columns == 64 || columns == 128 || columns == 256) b200::g_tile_columns = columns;
+  return b200::g_last_columns;
 }
 
 #ifdef B200_GEMM_TIMING

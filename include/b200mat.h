@@ -319,6 +319,9 @@ int b200_sm_count(void);                  /* SMs in force (the device's, or the 
 int b200_test_inject_stage_bytes(int extra_bytes);
 /* Test hook: scratch beyond `bytes` is refused, as by a device without memory (0: no limit). */
 int b200_test_limit_scratch(size_t bytes);
+/* Test hook: columns of the tensor-core tiles (64, 128 or 256; 0 by the estimate) of products where the estimate has the choice.
+ * Returns those of the last product. */
+int b200_test_tile_columns(int columns);
 /* All steps of an annealing schedule (n inverse temperatures) of a binary RBM's partition function estimate
  * (deepnet/ais.py:152-170): w V x H and its aux, biases a (H) and b (V), chain states, sb (V) scratch, weights 1 x B added to. */
 int ais_binary_steps(rnd_struct* rnd_state, cudamat* w, cudamat* w_aux, cudamat* a, cudamat* b, cudamat* v_state,

@@ -938,13 +938,14 @@ def test_deep_unaligned_dot_keeps_infinities_in_all_layouts(cm, ta, tb, alpha):
     assert relerr(got[np.ix_(rest, cols)], want[np.ix_(rest, cols)]) < TOL
 
 
+@pytest.mark.parametrize("columns", [0, 64, 128])
 @pytest.mark.parametrize("M,N,K,two_pairs", [(4096, 256, 1024, False), (1024, 256, 4096, False), (500, 2048, 784, False),
                                              (1000, 2044, 500, False), (1000, 132, 260, False), (132, 1000, 300, True),
                                              (260, 516, 256, True)])
-def test_narrow_tiles_of_products_of_few_tiles(cm, M, N, K, two_pairs):
+def test_narrow_tiles_of_products_of_few_tiles(cm, M, N, K, two_pairs, columns):
     """Products whose 256-column tiles leave the device idle take tiles of 128 or 64 columns of a single CTA: ragged rows and
-    columns of either width, cut along K and not, against float64.  Bound: sums of K products in chunks of 128 (2048 behind
-    the logistic) at 2^-18 a term, 1e-5 of the largest result."""
+    columns of either width, cut along K and not, against float64.  Bound: sums of K products in chunks of 128 (2048 in a wide
+    tile behind the logistic) at 2^-18 a term, 1e-5 of the largest result."""
     rng = np.random.default_rng(M + N)
     w = [(rng.standard_normal((K, M)) * 0.05).astype(np.float32) for _ in range(1 + two_pairs)]
     x = [rng.random((K, N)).astype(np.float32) for _ in range(1 + two_pairs)]
@@ -955,11 +956,13 @@ def test_narrow_tiles_of_products_of_few_tiles(cm, M, N, K, two_pairs):
     out, sample, plain = cm.empty((M, N)), cm.empty((M, N)), cm.empty((M, N))
     cm.CUDAMatrix.init_random(3)
     cm.set_gemm_path(1)
+    cm._lib.b200_test_tile_columns(columns)
     try:
         cm.fused_gemm(passes, out=out, sample=sample, bias=cm.CUDAMatrix(b), activation=1)
         cm.fused_gemm(passes, out=plain)
     finally:
         cm.set_gemm_path(0)
+        assert cm._lib.b200_test_tile_columns(0) in (columns or 64, columns or 128, columns or 256)
     pre = sum(wi.T.astype(np.float64) @ xi for wi, xi in zip(w, x))
     want = 1 / (1 + np.exp(-(pre + b)))
     got, draws = np.array(out.asarray()), np.array(sample.asarray())
@@ -970,6 +973,20 @@ def test_narrow_tiles_of_products_of_few_tiles(cm, M, N, K, two_pairs):
     unit.sample_bernoulli(target=again)                       # the same stream on the same probabilities
     np.testing.assert_array_equal(draws, np.array(again.asarray()))
     assert cm.read_status() == 0
+
+
+@pytest.mark.parametrize("M,N,K,columns", [(784, 1000, 1024, 256), (4096, 132, 1024, 256), (512, 1024, 2048, 256), (500, 500, 500, 64)])
+def test_products_bound_by_the_converters_keep_wide_tiles(cm, M, N, K, columns):
+    """A difference of two products whose parts the kernel derives: 784 x 1000, K = 1024 takes 37 us on tiles of 256 columns and 44
+    on tiles of 128; 500 x 500, K = 500 takes 18 on 64 and 27 on 256."""
+    m = lambda r, c: cm.CUDAMatrix(np.ones((r, c), np.float32))
+    passes = cm.split_passes(m(M, K), m(N, K).T, terms="tf32") + cm.split_passes(m(M, K), m(N, K).T, negate=1, terms="tf32")
+    out = cm.empty((M, N))
+    cm.set_gemm_path(1)
+    cm.fused_gemm(passes, out=out)
+    cm.set_gemm_path(0)
+    assert cm._lib.b200_test_tile_columns(0) == columns
+    assert not get(out).any()
 
 
 @pytest.mark.parametrize("path", [0, 1, 2, 3])
