@@ -13,7 +13,8 @@
 // the fp32 value, by truncation); the states are 0 or 1, so that h.s + m.s + l.s are exact products.  The tensor core's
 // accumulator, which truncates, is added to an fp32 register after 32 of K.  tcgen05 has no use here: 8 or 16 chains a
 // cluster are the short side of every product.  mma.sync bfloat16 multiplies 1024 pairs a clock and SM (TF32 512, fp32
-// multiply-adds 128).
+// multiply-adds 128).  States a caller starts from may be anything: where bfloat16 does not hold them the first product is
+// taken in doubles.
 // Bound by instruction issue (the split of W) and the latency of the exchange.  784 x 500, 100 chains, clocks of a step:
 // up 4850, hidden units 3200, down 6140, visible units 3900, barriers 2000: 10.5 us, against 36 as two products and a
 // kernel between them (three launches); 100 steps with their set-up 2881 -> 1479 us.
@@ -115,9 +116,11 @@ struct ChainStates {
     uint32_t* w = reinterpret_cast<uint32_t*>(p);
     for (int i = threadIdx.x; i < N * row / 2; i += kChainThreads) w[i] = 0u;
   }
-  // the states of chains [0, n) from columns of K units, eight loads in flight per thread
-  __device__ __forceinline__ void load(const float* x, int n, int K) const {
+  // the states of chains [0, n) from columns of K units, eight loads in flight per thread; true where a thread met one that
+  // bfloat16 does not hold
+  __device__ __forceinline__ bool load(const float* x, int n, int K) const {
     const int items = n * K;
+    bool rounded = false;
     for (int i0 = threadIdx.x; i0 < items; i0 += 8 * kChainThreads) {
       float y[8];
 #pragma unroll
@@ -125,9 +128,14 @@ struct ChainStates {
 #pragma unroll
       for (int u = 0; u < 8; u++) {
         const int i = i0 + u * kChainThreads, c = i / K;
-        if (i < items) *at(c, i - c * K) = float_to_bf16(y[u]);
+        if (i < items) {
+          const uint16_t b = float_to_bf16(y[u]);
+          *at(c, i - c * K) = b;
+          rounded |= !(bf16_to_float(b) == y[u]);
+        }
       }
     }
+    return rounded;
   }
   // units [4 q0, 4 (q0 + nq)) of n chains from this block's copy into the others'
   __device__ __forceinline__ void share(const ChainCluster& k, int n, int q0, int nq) const {
@@ -292,6 +300,21 @@ struct ChainShare {
     float x = 0.0f;
     for (int s = 0; s < split; s++) x += sum[(s * tiles * 16 + j) * NS + c];
     return x;
+  }
+
+  // The same sums from states v (chains V apart) that bfloat16 does not hold, whole and in doubles: what a caller may start
+  // from, once a launch.
+  __device__ __forceinline__ void up_exact(const float* v, int n, float* sum) const {
+    sums_in_doubles(gw, v, sum, V, nj, n, split, tiles * 16 * NS);
+  }
+  static __device__ __noinline__ void sums_in_doubles(const float* w, const float* v, float* sum, int V, int nj, int n, int split,
+                                                      int part) {
+    for (int it = threadIdx.x; it < nj * n; it += kChainThreads) {
+      const int c = it / nj, j = it - c * nj;
+      double x = 0.0;
+      for (int i = 0; i < V; i++) x += (double)w[(long)j * V + i] * v[(long)c * V + i];
+      for (int s = 0; s < split; s++) sum[s * part + j * NS + c] = s ? 0.0f : (float)x;
+    }
   }
 
   template <bool kVec, bool kShared>
@@ -464,7 +487,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) k_ais_chains(const __grid_co
   w.template load<kVec>();
   for (int j = threadIdx.x; j < nj; j += kChainThreads) bh[j] = p.a[j0 + j];
   __syncthreads();
-  vs.load(p.v_sample + (long)c0 * V, n, V);
+  const bool rounded = __syncthreads_or(vs.load(p.v_sample + (long)c0 * V, n, V));
   for (int it = threadIdx.x; it < nj * n; it += kChainThreads) hgain[it] = 0.0;
   for (int it = threadIdx.x; it < 2 * visible.nq * n; it += kChainThreads) vgain[it] = 0.0;
   // b'v of the states the chains start from
@@ -477,7 +500,8 @@ __global__ void __launch_bounds__(kChainThreads, 1) k_ais_chains(const __grid_co
   for (int step = 0; step < args.steps; step++) {
     const bool last = step == args.steps - 1;
     const float s0 = args.beta[step], s = args.beta[step + 1];
-    w.template up<kVec>(vs, sum);
+    if (step == 0 && rounded) w.up_exact(p.v_sample + (long)c0 * V, n, sum);
+    else w.template up<kVec>(vs, sum);
     __syncthreads();
     {
       const PhiloxKey key = make_philox_key(p.seed, args.call0 + 2ull * step);
@@ -662,12 +686,19 @@ float products_us(int V, int H, int B) {
 
 }  // namespace
 
-// (the estimates of both sides are good for a fifth)
+static int g_ais_form = 0;    // 0: by the estimates; 1: one launch or none; 2: the products (tests)
+
+// Whether all steps go in one launch.  (The estimates of both sides are good for a fifth.)
+static bool in_one_launch(int V, int H, int B, int steps, ChainPlan& plan) {
+  if (V <= 0 || H <= 0 || B <= 0 || steps < 1 || g_ais_form == 2) return false;
+  const int typical = steps < kAisBatch ? steps : kAisBatch;
+  return plan_chains(V, H, B, typical, plan) && (g_ais_form == 1 || 1.2f * plan.us <= typical * products_us(V, H, B));
+}
+
 int ais_chains(const AisChains& a) {
-  if (a.V <= 0 || a.H <= 0 || a.B <= 0 || a.n < 2) return ERROR_UNSUPPORTED;
-  const int steps = a.n - 1, typical = steps < kAisBatch ? steps : kAisBatch;
+  const int steps = a.n - 1;
   ChainPlan plan;
-  if (!plan_chains(a.V, a.H, a.B, typical, plan) || 1.2f * plan.us > typical * products_us(a.V, a.H, a.B)) return ERROR_UNSUPPORTED;
+  if (!in_one_launch(a.V, a.H, a.B, steps, plan)) return g_ais_form == 1 ? set_error("the steps do not go in one launch") : ERROR_UNSUPPORTED;
   const bool vec = a.V % 4 == 0 && ((uintptr_t)a.w & 15) == 0;
   AisArgs p = {plan.s, a, 0, 0, {}, {}};
   p.s.col0 = rng_col0();
@@ -686,3 +717,16 @@ int ais_chains(const AisChains& a) {
 }
 
 }  // namespace b200
+
+// Test hook: 0 the faster form of ais_binary_steps, 1 all steps in one launch (an error where they do not go), 2 three launches a
+// step.
+extern "C" int b200_test_ais_form(int form) {
+  if (form < 0 || form > 2) return ERROR_UNSUPPORTED;
+  b200::g_ais_form = form;
+  return 0;
+}
+// 1: ais_binary_steps takes one launch for n inverse temperatures of B chains.
+extern "C" int b200_test_ais_in_one_launch(int V, int H, int B, int n) {
+  b200::ChainPlan plan;
+  return b200::in_one_launch(V, H, B, n - 1, plan) ? 1 : 0;
+}

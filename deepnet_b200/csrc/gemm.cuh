@@ -111,7 +111,7 @@ bool gemm_tc_supported(const GemmProblem& g);
 int gemm_tc_packed(const GemmProblem& g);   // the same behind a copy of the operands TMA cannot address
 
 // The annealing steps 1 .. n - 1 of a binary RBM in one launch (chains.cu); ERROR_UNSUPPORTED where single products are the
-// faster way.  The chains start from 0/1 states.
+// faster way.
 struct AisChains {
   const float *w, *a, *b;
   float *v_state, *v_sample, *h_pre, *h_sample, *sb, *weights;

@@ -322,6 +322,10 @@ int b200_test_limit_scratch(size_t bytes);
 /* Test hook: columns of the tensor-core tiles (64, 128 or 256; 0 by the estimate) of products where the estimate has the choice.
  * Returns those of the last product. */
 int b200_test_tile_columns(int columns);
+/* Test hooks: the form of ais_binary_steps (0 the faster one, 1 all steps in one launch or an error, 2 three launches a step); whether
+ * n inverse temperatures of B chains take one launch. */
+int b200_test_ais_form(int form);
+int b200_test_ais_in_one_launch(int V, int H, int B, int n);
 /* All steps of an annealing schedule (n inverse temperatures) of a binary RBM's partition function estimate
  * (deepnet/ais.py:152-170): w V x H and its aux, biases a (H) and b (V), chain states, sb (V) scratch, weights 1 x B added to. */
 int ais_binary_steps(rnd_struct* rnd_state, cudamat* w, cudamat* w_aux, cudamat* a, cudamat* b, cudamat* v_state,

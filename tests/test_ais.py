@@ -72,15 +72,27 @@ def test_ais_at_layer_sizes_of_the_reference_models(cm):
     assert abs(log_z - want) < 0.5
 
 
+ONE_LAUNCH, PRODUCTS = 1, 2
+
+
+@pytest.fixture
+def ais_form(cm):
+    yield cm._lib.b200_test_ais_form
+    cm._lib.b200_test_ais_form(0)
+
+
 @pytest.mark.gpu
+@pytest.mark.parametrize("form", [ONE_LAUNCH, PRODUCTS])
 @pytest.mark.parametrize("col0", [0, 3])
-@pytest.mark.parametrize("V,H,B", [(301, 517, 5), (17, 33, 203), (260, 255, 1)])
-def test_annealing_steps_match_the_call_by_call_form(cm, col0, V, H, B):
-    """The steps issued from C against the reference's calls on the device, chain by chain: layers of more than one pass of a
-    block and odd ones, nonzero biases, a shard whose first column is not a multiple of four.  Both consume one random
-    stream; a draw may differ where two correct probabilities straddle its uniform, about one in 10^7."""
+@pytest.mark.parametrize("V,H,B", [(301, 517, 5), (17, 33, 203), (260, 255, 1), (260, 132, 137)])
+def test_annealing_steps_match_the_call_by_call_form(cm, ais_form, form, col0, V, H, B):
+    """The steps issued from C, in either form, against the reference's calls on the device, chain by chain: layers of more than
+    one pass of a block and odd ones, products of both kernels, nonzero biases, a shard whose first column is not a multiple of
+    four.  Both consume one random stream; a draw may differ where two correct probabilities straddle its uniform, about one
+    in 10^7."""
     w, a, b = small_rbm(V=V, H=H, scale=0.1, seed=V)
     schedule = np.linspace(0.0, 1.0, 8)
+    assert ais_form(form) == 0
     cm.set_rng_column_offset(col0)
     try:
         got, want = (ais.ais_binary_rbm(cm, w, a, b, B, schedule, seed=9, fused=fused) for fused in (True, False))
@@ -92,24 +104,59 @@ def test_annealing_steps_match_the_call_by_call_form(cm, col0, V, H, B):
 
 
 @pytest.mark.gpu
-@pytest.mark.parametrize("V,H,B,steps", [(784, 500, 100, 20), (64, 9, 1, 4), (97, 128, 33, 300), (1024, 129, 37, 5), (5, 3, 2, 3)])
-def test_annealing_in_one_launch_matches_the_products(cm, V, H, B, steps):
-    """All steps in one launch against three launches a step (the products on CUDA cores), chain by chain: columns left in
-    global memory, whole and ragged quads of rows, fewer hidden units than blocks, more temperatures than travel with a launch.
-    One chain may go elsewhere, where a draw's uniform falls between two correct probabilities."""
+@pytest.mark.parametrize("V,H,B,steps", [(784, 500, 100, 20), (64, 9, 1, 4), (97, 128, 33, 300), (1024, 129, 37, 5), (5, 3, 2, 3),
+                                         (1023, 600, 20, 4), (1999, 70, 17, 3), (2001, 9, 3, 2), (1024, 1024, 120, 3)])
+def test_annealing_in_one_launch_matches_the_products(cm, ais_form, V, H, B, steps):
+    """All steps in one launch against three launches a step (the products on CUDA cores), chain by chain, with the states both
+    leave: columns left in global memory (some of them, all, of whole and of ragged quads of rows), fewer hidden units than
+    blocks, more temperatures than travel with a launch, 1 to 16 chains a cluster.  The draws are the same ones: a chain may go
+    elsewhere where two correct probabilities straddle a uniform (one draw in 10^7; only the longest run has that many)."""
     w, a, b = small_rbm(V=V, H=H, scale=0.05, seed=V)
     schedule = np.linspace(0.0, 1.0, steps + 1)
-    got = ais.ais_binary_rbm(cm, w, a, b, B, schedule, seed=9)
-    calls = cm.CUDAMatrix.rnd_state.calls
-    cm.set_gemm_path(2)
-    try:
-        want = ais.ais_binary_rbm(cm, w, a, b, B, schedule, seed=9)
-    finally:
-        cm.set_gemm_path(0)
+    rng = np.random.default_rng(V)
+    start, host = (rng.random((V, B)) < 0.5).astype(np.float32), {}
+    for form, path in ((ONE_LAUNCH, 0), (PRODUCTS, 2)):
+        m = dict(v_state=cm.CUDAMatrix(np.full((V, B), 0.5, np.float32)), v_sample=cm.CUDAMatrix(start), h_pre=cm.empty((H, B)),
+                 h_sample=cm.empty((H, B)), weights=cm.empty((1, B)))
+        W = cm.CUDAMatrix(w)
+        cm.CUDAMatrix.init_random(9)
+        assert ais_form(form) == 0
+        cm.set_gemm_path(path)
+        try:
+            cm.ais_binary_steps(W, W.split_bf16(cm.empty_aux((V, H))), cm.CUDAMatrix(a.reshape(H, 1)), cm.CUDAMatrix(b.reshape(V, 1)),
+                                schedule=schedule, **m)
+        finally:
+            cm.set_gemm_path(0)
+        assert cm.CUDAMatrix.rnd_state.calls == 2 * steps
+        host[form] = {k: np.array(x.asarray()) for k, x in m.items()}
+    got, want = host[ONE_LAUNCH], host[PRODUCTS]
+    assert all(np.isfinite(x).all() for x in got.values())
     # bound: the log weights of the other form are fp32 sums over `steps` of fp32 sums of V + H terms
-    assert (np.abs(got[1] - want[1]) > 1e-4 * np.abs(want[1]).max() + 1e-3).sum() <= 1
-    assert calls == cm.CUDAMatrix.rnd_state.calls == 1 + 2 * steps
+    same = np.abs(got["weights"] - want["weights"])[0] <= 1e-4 * np.abs(want["weights"]).max() + 1e-3
+    assert (~same).sum() <= (1 if steps * (V + H) * B > 10 ** 6 else 0)
+    for k in ("v_sample", "h_sample"):
+        np.testing.assert_array_equal(got[k][:, same], want[k][:, same])
+    np.testing.assert_allclose(got["v_state"][:, same], want["v_state"][:, same], rtol=0, atol=1e-5)
+    np.testing.assert_allclose(got["h_pre"][:, same], want["h_pre"][:, same], rtol=0, atol=1e-5 * np.abs(want["h_pre"]).max())
     assert cm.read_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("V,H,B", [(300, 200, 40), (97, 33, 5), (1023, 301, 9)])
+def test_annealing_starts_from_states_of_any_value(cm, ais_form, V, H, B):
+    """Means and counts, not only 0 and 1: the first pre-activations of the form in one launch, against float64.  Bound: 2^-24 a
+    sum of doubles rounded once, and the bias added."""
+    w, a, b = small_rbm(V=V, H=H, scale=0.1, seed=V)
+    rng = np.random.default_rng(B)
+    v = rng.random((V, B)).astype(np.float32)
+    v[:, 0] = rng.integers(0, 1000, V)
+    h_pre, W = cm.empty((H, B)), cm.CUDAMatrix(w)
+    cm.CUDAMatrix.init_random(2)
+    assert ais_form(ONE_LAUNCH) == 0
+    cm.ais_binary_steps(W, W.split_bf16(cm.empty_aux((V, H))), cm.CUDAMatrix(a.reshape(H, 1)), cm.CUDAMatrix(b.reshape(V, 1)),
+                        cm.CUDAMatrix(v), cm.CUDAMatrix(v), h_pre, cm.empty((H, B)), cm.empty((1, B)), [0.0, 0.5])
+    want = w.T.astype(np.float64) @ v + a[:, None]
+    assert (np.abs(np.array(h_pre.asarray()) - want).max(axis=0) <= 2e-7 * np.abs(want).max(axis=0)).all()
 
 
 @pytest.mark.gpu
