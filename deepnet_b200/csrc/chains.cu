@@ -571,6 +571,7 @@ __global__ void __launch_bounds__(kChainThreads, 1) k_ais_chains(const __grid_co
 // f(std::integral_constant<int, NT>) of the instance that takes n chains a cluster.
 constexpr int kMaxChains = 16;
 template <typename F>
+constexpr int kMaxUnits = 1 << 16;   // of a layer: far more than shared memory takes, and sizes that stay within an int
 int with_chains(int n, F f) {
   return n <= 8 ? f(std::integral_constant<int, 1>{}) : f(std::integral_constant<int, 2>{});
 }
@@ -634,6 +635,7 @@ struct ChainPlan {
 // 2100, 7600, 2550 and 1620, 1640, 1490, 4560, 1900 with 16 of either.
 bool plan_chains(int V, int H, int B, int steps, ChainPlan& best) {
   best.us = 1e30f;
+  if (V > kMaxUnits || H > kMaxUnits) return false;
   for (int blocks : {8, 16}) {
     const int room = clusters_at_once(blocks);
     if (!room) continue;

@@ -160,6 +160,14 @@ def test_annealing_starts_from_states_of_any_value(cm, ais_form, V, H, B):
 
 
 @pytest.mark.gpu
+def test_annealing_of_layers_far_beyond_shared_memory_takes_the_products(cm):
+    """Sizes that wrap around 2^31 when a block's shared memory is added up."""
+    for units in (460174946, 460175205, 2 ** 31 - 100):
+        assert not cm._lib.b200_test_ais_in_one_launch(units, 1, 1, 101)
+        assert not cm._lib.b200_test_ais_in_one_launch(1, units, 1, 101)
+
+
+@pytest.mark.gpu
 def test_annealing_steps_refuse_shapes_that_do_not_fit(cm):
     cm.CUDAMatrix.init_random(1)
     V, H, B = 12, 8, 5
