@@ -160,6 +160,16 @@ def test_annealing_starts_from_states_of_any_value(cm, ais_form, V, H, B):
 
 
 @pytest.mark.gpu
+def test_annealing_takes_one_launch_only_where_that_is_faster(cm):
+    """Measured, us a step, one launch / products: 784 x 500 with 100 chains 10.5 / 25, with 500 43 / 39, with 2048 137 / 60; 2000 x
+    500 with 250 chains 72 / 42."""
+    takes = lambda V, H, B, steps: cm._lib.b200_test_ais_in_one_launch(V, H, B, steps + 1)
+    assert takes(784, 500, 100, 100) and takes(784, 500, 250, 100) and takes(64, 64, 250, 10)
+    assert not takes(784, 500, 500, 100) and not takes(784, 500, 1000, 100) and not takes(784, 500, 2048, 100)
+    assert not takes(2000, 500, 250, 100) and not takes(784, 500, 100, 1)
+
+
+@pytest.mark.gpu
 def test_annealing_of_layers_far_beyond_shared_memory_takes_the_products(cm):
     """Sizes that wrap around 2^31 when a block's shared memory is added up."""
     for units in (460174946, 460175205, 2 ** 31 - 100):
