@@ -237,7 +237,7 @@ __global__ void __launch_bounds__(256) k_sample_multinomial(const float* __restr
       }
     }
     float inv[4];                                 // (1 + 2e-6) / bound, or 0: no usable bound for this draw
-    // Most words are out for all four draws at once, and one integer comparison says so: with c = pr times the
+    // Most words are out for all four draws at once, and one integer comparison says so: with c = |pr| times the
     // largest inv, every word x of the block below (1 - c - 2^-20) 2^32 has 1 - u >= pr * inv in the comparison
     // below, whose roundings come to less than 2^-21.  What is left goes through that comparison as before.  The
     // bound is shared again after 2048 words: from the first 512 alone a tenth of the words pass somewhere in a warp.
@@ -271,7 +271,7 @@ __global__ void __launch_bounds__(256) k_sample_multinomial(const float* __restr
       for (; r < end; r += blockDim.x) {
         const uint4 wd = philox4x32_10((uint32_t)r, (uint32_t)blk, key);
         const float pr = p[r];
-        const uint32_t out_below = __float2uint_rd(((1.0f - 9.5367432e-7f) - pr * most) * 4294967296.0f);   // (NaN: 0)
+        const uint32_t out_below = __float2uint_rd(((1.0f - 9.5367432e-7f) - fabsf(pr) * most) * 4294967296.0f);   // (NaN: 0)
         if (max(max(wd.x, wd.y), max(wd.z, wd.w)) < out_below) continue;
         const float u[4] = {word_to_uniform(wd.x), word_to_uniform(wd.y), word_to_uniform(wd.z), word_to_uniform(wd.w)};
 #pragma unroll

@@ -319,6 +319,25 @@ def test_multinomial_draws_equal_the_call_sequence_at_any_vocabulary(cm, V):
     np.testing.assert_array_equal(fused.sum(axis=0), lens.ravel())
 
 
+@pytest.mark.parametrize("V", [10, 600, 5000])
+def test_multinomial_draws_without_a_positive_word_equal_the_call_sequence(cm, V):
+    """Values of either sign: where no word of the first is positive nothing bounds the race, and every word stays in it."""
+    rng = np.random.default_rng(V)
+    p = -rng.random((V, 2)).astype(np.float32) - 0.01
+    p[V - 1, 1] = 0.5
+    lens = np.array([[30, 9]], np.float32)
+    lay = dbm.ReplicatedSoftmaxLayer(cm, "v", V, dbm.Hyperparams(sample_input=True), is_input=True)
+    lay.AllocateMemory(2)
+    lay.state.assign(cm.CUDAMatrix(p))
+    lay.NN.assign(cm.CUDAMatrix(lens))
+    cm.CUDAMatrix.init_random(8)
+    lay.Sample()
+    cm.CUDAMatrix.init_random(8)
+    fused = get(cm.CUDAMatrix(p).sample_multinomial(cm.CUDAMatrix(lens), cm.empty((V, 2))))
+    np.testing.assert_array_equal(fused, get(lay.sample))
+    np.testing.assert_array_equal(fused[:, 1], 9.0 * (np.arange(V) == V - 1))
+
+
 @pytest.mark.parametrize("scale", [0.02, 1.0])
 def test_fused_engine_replicated_softmax_matches_oracle(cm, oracle, scale):
     # config 2 at 1/50 size and at its full size (10 000 words, 512 hidden units, documents of about
