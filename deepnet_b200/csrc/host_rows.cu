@@ -5,8 +5,16 @@
 // (deepnet/extract_rbm_representation.py).  Here the copy lands in pinned pieces on a stream of its own and a few threads
 // carry the pieces to where they belong, while the caller goes on to the next minibatch: eight of 250 x 1000 with their
 // reconstruction error 1154 -> 540 us.
-// One staging area per process (4 MB and four threads, made on first use, given back by cublas_shutdown): whoever
+// One staging area per process (4 MB and six threads, made on first use, given back by cublas_shutdown): whoever
 // begins while another thread holds it is told so and copies the plain way.
+//
+// The carriers are bound by the page faults of the fresh result, which more than two or three threads only make dearer, unless its
+// pages are large ones.  At most two wait for their piece (busily: with blocking waits the call took twice as long); the others
+// sleep until pieces have landed.  us a call and cores busy, by carriers / of them waiting:
+//                                        2 / 2        3 / 2        4 / 4        6 / 2
+//   eight minibatches of 250 x 1000      504, 2.5     552, 3.1     556, 4.0     602, 3.4
+//   eight of 500 x 2048                  1259, 2.4    1217, 3.5    1316, 4.4    1517, 4.0
+//   two of 1024 x 8192                   9588, 2.0    7849, 2.9    7231, 4.0    6013, 4.8
 #include <condition_variable>
 #include <cstring>
 #include <deque>
@@ -20,12 +28,14 @@ using namespace b200;
 
 namespace {
 
-constexpr int kPieces = 16, kCarriers = 4;
+constexpr int kPieces = 16, kCarriers = 6, kWaiting = 2;
+constexpr int kFewCarriers = 3;                     // ... of matrices below
+constexpr size_t kManyCarriersBytes = 16 << 20;
 constexpr size_t kPieceBytes = 256 * 1024;
 
 struct RowsStaging {
   std::mutex mu;
-  std::condition_variable work, freed;
+  std::condition_variable work, more_work, freed;     // of the first carriers, of the others, of the caller
   struct Job {
     int piece;
     float* dst;
@@ -37,19 +47,30 @@ struct RowsStaging {
   cudaEvent_t landed[kPieces] = {nullptr}, ready = nullptr, done[2] = {nullptr, nullptr};
   cudaStream_t copies = nullptr;
   bool free_piece[kPieces];
-  int device = 0, in_flight = 0, adds = 0;
+  int device = 0, in_flight = 0, adds = 0, waiting = 0, carrying = kFewCarriers;   // (threads that may carry)
   bool held = false, stop = false, made = false, failed = false;
 
-  void carry() {
+  void wake_one() {
+    work.notify_one();
+    if (carrying > kFewCarriers) more_work.notify_one();
+  }
+  void carry(int self) {
     cudaSetDevice(device);
     std::unique_lock<std::mutex> lock(mu);
     for (;;) {
-      work.wait(lock, [&] { return stop || !jobs.empty(); });
+      (self < kFewCarriers ? work : more_work).wait(lock, [&] {
+        return stop || (!jobs.empty() && waiting < kWaiting && self < carrying);
+      });
       if (jobs.empty()) return;
       const Job j = jobs.front();
       jobs.pop_front();
+      waiting++;
       lock.unlock();
       const bool ok = cudaEventSynchronize(landed[j.piece]) == cudaSuccess;
+      lock.lock();
+      waiting--;
+      if (!jobs.empty()) wake_one();
+      lock.unlock();
       if (ok) memcpy(j.dst, pinned + j.piece * kPieceBytes, j.bytes);
       lock.lock();
       failed |= !ok;
@@ -64,6 +85,7 @@ struct RowsStaging {
       stop = true;
     }
     work.notify_all();
+    more_work.notify_all();
     for (std::thread& t : carriers) t.join();
     carriers.clear();
     if (pinned) cudaFreeHost(pinned);
@@ -87,7 +109,7 @@ struct RowsStaging {
     for (cudaEvent_t& e : landed) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
     for (bool& f : free_piece) f = true;
     try {
-      for (int i = 0; ok && i < kCarriers; i++) carriers.emplace_back([this] { carry(); });
+      for (int i = 0; ok && i < kCarriers; i++) carriers.emplace_back([this, i] { carry(i); });
     } catch (...) {
       ok = false;
     }
@@ -141,6 +163,10 @@ int b200_rows_add(cudamat* src, float* dst) {
   if (cudaEventRecord(s.ready, stream()) != cudaSuccess || cudaStreamWaitEvent(s.copies, s.ready, 0) != cudaSuccess)
     return set_error(cudaGetErrorString(cudaGetLastError()));
   const size_t bytes = (size_t)numel(src) * sizeof(float);
+  {
+    std::lock_guard<std::mutex> lock(s.mu);
+    s.carrying = bytes < kManyCarriersBytes ? kFewCarriers : kCarriers;
+  }
   for (size_t at = 0; at < bytes; at += kPieceBytes) {
     const size_t n = bytes - at < kPieceBytes ? bytes - at : kPieceBytes;
     int piece = -1;
@@ -164,7 +190,7 @@ int b200_rows_add(cudamat* src, float* dst) {
     }
     s.jobs.push_back({piece, (float*)((char*)dst + at), n});
     s.in_flight++;
-    s.work.notify_one();
+    s.wake_one();
   }
   // the matrix of the call before has been read once this stream is past its copies
   if (s.adds > 0 && cudaStreamWaitEvent(stream(), s.done[(s.adds - 1) & 1], 0) != cudaSuccess)
