@@ -1246,10 +1246,14 @@ def copy_to_rows(mat, rows):
 
 class RowsOut(object):
     """`copy_to_rows` behind the work that produces the matrices: `with RowsOut() as out: out.add(mat, rows)`.  Work enqueued
-    after an `add` may rewrite the matrix of the `add` before it; the rows are there when the block ends."""
+    after an `add` may rewrite the matrix of the `add` before it; the rows are there when the block ends.  behind=False: plain
+    copies, as where the staging area cannot be had."""
+
+    def __init__(self, behind=True):
+        self.behind = behind
 
     def __enter__(self):
-        self.held = bool(_lib.b200_rows_begin())
+        self.held = self.behind and bool(_lib.b200_rows_begin())
         return self
 
     def add(self, mat, rows):

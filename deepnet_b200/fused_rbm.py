@@ -478,7 +478,9 @@ class FusedRBM(LossReadback):
         soft = self.visible == REPLICATED_SOFTMAX
         if n > 1 and self._h_out is None:
             self._h_out = cm.empty((self.H, B))
-        with cm.RowsOut() as out:
+        # one small minibatch has nothing to hide its copy behind: 784 x 500 with 100 cases 53 us copied the plain way, 62 by
+        # the threads; with 400 cases of 500 100 and 94
+        with cm.RowsOut(n > 1 or rep.nbytes >= 1 << 19) as out:
             for b in range(n):
                 v0 = data.slice(b * B, (b + 1) * B)
                 h = self.h_pos if (n - 1 - b) % 2 == 0 else self._h_out    # one is on its way to the host, the last stays
