@@ -822,7 +822,7 @@ def _build_fused_gemm(passes, out=None, sample=None, bias=None, col_scale=None, 
  OP_SPLIT_BF16, OP_ALLREDUCE, OP_SOFTMAX_SCALED, OP_SAMPLE_MULTINOMIAL, OP_DIV_BY_ROW, OP_ADD_SCALAR, OP_ASSIGN_SCALAR,
  OP_COPY, OP_SAMPLE_BERNOULLI, OP_SOFTMAX_SAMPLE, OP_MOMENTUM_UPDATE_COLUMNS, OP_ALLREDUCE_BEGIN, OP_ALLREDUCE_END,
  OP_SM_LIMIT, OP_DP_PEER_UPDATE, OP_RBM_BIAS_UPDATE, OP_SOFTMAX_RECONSTRUCTION,
- OP_DOCUMENT_LENGTHS, OP_BIAS_UPDATES, OP_UPDATE_ALL) = range(27)
+ OP_DOCUMENT_LENGTHS, OP_BIAS_UPDATES, OP_UPDATE_ALL, OP_SIGMOID) = range(28)
 
 
 class _Op(ct.Structure):
@@ -930,6 +930,9 @@ class Immediate(object):
 
     def copy(self, src, dst):
         dst.assign(src)
+
+    def sigmoid(self, mat, target):
+        sigmoid(mat, target)
 
     def sample_bernoulli(self, mat, target):
         mat.sample_bernoulli(target)
@@ -1053,6 +1056,9 @@ class Program(object):
     def copy(self, src, dst):
         return self._add(OP_COPY, (src, dst))
 
+    def sigmoid(self, mat, target):
+        return self._add(OP_SIGMOID, (mat, target))
+
     def sample_bernoulli(self, mat, target):
         return self._add(OP_SAMPLE_BERNOULLI, (mat, target))
 
@@ -1165,6 +1171,11 @@ def set_sm_limit(sms):
 
 def sm_count():
     return _lib.b200_sm_count()
+
+
+def product_depth(m, n, slabs):
+    """Slabs of 32 of K that a CTA of the one-launch kernel walks for an m x n product of `slabs` slabs."""
+    return _lib.b200_product_depth(ct.c_int(m), ct.c_int(n), ct.c_int(slabs))
 
 
 def set_split_k(mode):

@@ -581,6 +581,13 @@ long cut_up(const GemmProblem& g, SmallParams& p) {
   return tiles * p.splits;
 }
 
+// Slabs of K that one SM walks.
+int walked_slabs(const GemmProblem& g, SmallParams& p) {
+  const long ctas = cut_up(g, p), room = 2L * sm_count();
+  const long depth = (p.slabs + p.splits - 1) / p.splits * ((ctas + room - 1) / room);
+  return depth < (1 << 30) ? (int)depth : 1 << 30;
+}
+
 int allow_shared_memory() {
   static bool attr_set[64] = {false};
   int dev = 0;
@@ -653,9 +660,7 @@ int recompute_nonfinite(const GemmProblem& g) {
 int small_depth(const GemmProblem& g) {
   SmallParams p;
   if (g.M <= 0 || g.N <= 0 || !gather_pairs(g, p)) return 0;
-  const long ctas = cut_up(g, p), room = 2L * sm_count();
-  const long depth = (p.slabs + p.splits - 1) / p.splits * ((ctas + room - 1) / room);
-  return depth < (1 << 30) ? (int)depth : 1 << 30;
+  return walked_slabs(g, p);
 }
 
 // Whether one launch is faster than the tcgen05 kernel on operands that both take: both sides estimated in us, from
@@ -734,3 +739,14 @@ int gemm_small(const GemmProblem& g, SmallForm form) {
 }
 
 }  // namespace b200
+
+// Slabs of 32 of K that an SM walks in the one-launch kernel for an m x n product of so many slabs.
+extern "C" int b200_product_depth(int m, int n, int slabs) {
+  if (m <= 0 || n <= 0 || slabs <= 0) return 0;
+  b200::GemmProblem g;
+  g.M = m;
+  g.N = n;
+  b200::SmallParams p;
+  p.slabs = slabs;
+  return b200::walked_slabs(g, p);
+}

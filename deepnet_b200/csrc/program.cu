@@ -43,6 +43,7 @@ int div_by_row_vec(cudamat* mat, cudamat* vec, cudamat* target);
 int add_scalar(cudamat* mat, float alpha, cudamat* target);
 int assign_scalar(cudamat* mat, float alpha);
 int copy_on_device(cudamat* mat1, cudamat* mat2);
+int apply_sigmoid(cudamat* mat, cudamat* target);
 int sample_bernoulli(rnd_struct* rnd_state, cudamat* mat, cudamat* target);
 int softmax_sample(rnd_struct* rnd_state, cudamat* pre, cudamat* bias, cudamat* state, cudamat* sample);
 }
@@ -75,6 +76,7 @@ enum {
   B200_OP_DOCUMENT_LENGTHS = 24,  // m0 counts, m1 nn, m2 norm, f0 tiny
   B200_OP_BIAS_UPDATES = 25,      // gemm points to a b200_bias_layers; f0 inv_batch, f1 momentum, f2 eps
   B200_OP_UPDATE_ALL = 26,        // the same, m0 w, m1 delta, m2 suff, m3 w_aux; f0 inv_batch, f1 mom_b, f2 eps_b, f3 mom_w, f4 eps_w, f5 l2, f6 l1
+  B200_OP_SIGMOID = 27,           // m0 mat, m1 target
   B200_OP_COUNT
 };
 
@@ -127,6 +129,7 @@ extern "C" int b200_run_program(rnd_struct* rnd_state, b200_op* ops, int n, int*
       case B200_OP_SOFTMAX_RECONSTRUCTION: err = softmax_reconstruction(o.m[0], o.m[1], o.m[2], o.m[3], o.m[4], o.m[5]); break;
       case B200_OP_DOCUMENT_LENGTHS: err = document_lengths(o.m[0], o.m[1], o.m[2], o.f0); break;
       case B200_OP_BIAS_UPDATES: err = bias_updates(reinterpret_cast<b200_bias_layers*>(o.gemm), o.f0, o.f1, o.f2); break;
+      case B200_OP_SIGMOID: err = apply_sigmoid(o.m[0], o.m[1]); break;
       case B200_OP_UPDATE_ALL:
         err = update_all(reinterpret_cast<b200_bias_layers*>(o.gemm), o.m[0], o.m[1], o.m[2], o.m[3], o.f0, o.f1, o.f2, o.f3, o.f4, o.f5, o.f6);
         break;

@@ -40,7 +40,7 @@ class FusedDBM(LossReadback):
         self.pos = [z(n, B) for n in sizes]
         self.neg = [z(n, B) for n in sizes]
         self.neg_sample = [z(n, B) for n in sizes]
-        self.from_data = z(sizes[1], B)           # W[0]' data of the positive phase
+        self.from_data = z(sizes[1], B)           # W[0]' data and bias of the positive phase
         self.loss_acc = z(1, 1)
         self._sched = Parameter(cm, hyperparams)
         self.kernel_launches = 0
@@ -50,16 +50,31 @@ class FusedDBM(LossReadback):
         self._programs = {}
         self._batch = cm.CUDAMatrix._from_mat(cm.cudamat())
 
+    def _data_once(self):
+        """Whether W[0]' data is multiplied once a positive phase, not in every sweep together with W[1]'s product.  It costs a launch
+        (3 us) and, each sweep, the reading of the result; a sweep saves about a microsecond for every slab of K its product is
+        shallower.  Measured, us an update with one Gibbs sweep, in every sweep / once: 784-500-1000, 100 cases, 10 mean-field
+        sweeps 328 / 298, 3 sweeps 152 / 151; 64-64-64 193 / 211; 256-256-1500, 16 cases 262 / 292; 500-2048-500, 1030 cases 772 /
+        896 (wide layers: tcgen05 products, the result is copied to the output first)."""
+        if self.L < 3 or self.hyp.mf_steps < 2:
+            return False
+        V, H, above = self.sizes[:3]
+        slabs = lambda k: (k + 31) // 32
+        depth = lambda s: self.cm.product_depth(H, self.B, s)
+        saved = depth(slabs(V) + slabs(above)) - depth(slabs(above))
+        return (saved >= 2 and (self.hyp.mf_steps - 1) * saved >= 6
+                and (H * self.B <= 1 << 20 or (V >= 1024 and V >= 2 * above)))
+
     def _update_layer(self, X, j, below, above, out, sample, add=None):
-        """state_j = sigmoid(W[j-1]' below + W[j] above + add + b_j) (deepnet/dbm.py:82-105), optional draw.
-        below / above = (state, exact): exact states (0/1) have no low part."""
+        """state_j = sigmoid(W[j-1]' below + W[j] above + b_j) (deepnet/dbm.py:82-105), optional draw; `add` stands for what the
+        layer gets from below and its bias.  below / above = (state, exact): exact states (0/1) have no low part."""
         P = self.cm.split_passes
         passes = []
         if below is not None:
             passes += P(self.W[j - 1].T, below[0], exact_b=below[1], a_aux=self.W_aux[j - 1])
         if above is not None:
             passes += P(self.W[j], above[0], exact_b=above[1], a_aux=self.W_aux[j])
-        X.fused_gemm(passes, out=out, sample=sample, bias=self.b[j], activation=1, add=add)
+        X.fused_gemm(passes, out=out, sample=sample, bias=self.b[j] if add is None else None, activation=1, add=add)
         self.kernel_launches += 1
 
     def TrainOneBatch(self, step, data):
@@ -98,19 +113,24 @@ class FusedDBM(LossReadback):
         # ---- positive phase: data clamped, hidden layers start at zero, mean-field sweeps
         for j in range(1, L):
             X.assign_scalar(pos[j], 0)
-        # W[0]' data is the same in every sweep: multiplied once where there is more than one
-        once = self.hyp.mf_steps > 1 and L > 2
+        # W[0]' data (and the bias) is the same in every sweep
+        once = self._data_once()
         if once:
-            X.fused_gemm(cm.split_passes(self.W[0].T, data, exact_b=True, a_aux=self.W_aux[0]), out=self.from_data)
+            X.fused_gemm(cm.split_passes(self.W[0].T, data, exact_b=True, a_aux=self.W_aux[0]), out=self.from_data, bias=self.b[1])
             self.kernel_launches += 1
         for sweep in range(self.hyp.mf_steps):
             for j in range(1, L):
                 below = (data, True) if j == 1 else (pos[j - 1], False)
                 above = (pos[j + 1], False) if j < L - 1 else None
-                if j == 1 and once and sweep > 0:
+                if sweep == 0 and j == 1:      # (the layer above is zero)
+                    above = None
+                if j > 1 or not once:
+                    self._update_layer(X, j, below, above, pos[j], None)
+                elif sweep == 0:
+                    X.sigmoid(self.from_data, pos[1])
+                    self.kernel_launches += 1
+                else:
                     self._update_layer(X, j, None, above, pos[j], None, add=self.from_data)
-                else:      # (in the first sweep the layer above is zero)
-                    self._update_layer(X, j, below, above if sweep > 0 or j > 1 else None, pos[j], None)
         # PCD reports the reconstruction of the input from the first hidden layer (deepnet/dbm.py:163-166)
         self._update_layer(X, 0, None, (pos[1], False), pos[0], None)
         X.sq_diff(pos[0], data, self.loss_acc)

@@ -313,6 +313,7 @@ int b200_set_dependent_launch(int on);
  * beside the persistent tensor-core kernel.  No counterpart in the reference. */
 int b200_set_sm_limit(int sms);
 int b200_sm_count(void);                  /* SMs in force (the device's, or the limit) */
+int b200_product_depth(int m, int n, int slabs);   /* slabs of 32 of K an SM walks for an m x n product of so many, in one launch */
 /* Test hook, host side only: the next tensor-core product expects extra_bytes more per stage than
  * its copies deliver, so one of its bounded waits must run out (status word set, kernel returns).
  * No counterpart in the reference. */
@@ -419,7 +420,7 @@ int dp_wait(int timeout_ms);
  * 11 div_by_row_vec, 12 add_scalar, 13 assign_scalar, 14 copy_on_device, 15 sample_bernoulli,
  * 16 softmax_sample, 17 momentum_update_columns, 18 dp_allreduce_begin, 19 dp_allreduce_end,
  * 20 b200_set_sm_limit, 21 dp_peer_update, 22 rbm_bias_update,
- * 23 softmax_reconstruction, 24 document_lengths, 25 bias_updates, 26 update_all); m[], i0.., f0.. are its arguments in declaration order (matrices, then
+ * 23 softmax_reconstruction, 24 document_lengths, 25 bias_updates, 26 update_all, 27 apply_sigmoid); m[], i0.., f0.. are its arguments in declaration order (matrices, then
  * integers, then floats; gemm for kind 0, whose m[0] is add or null, and pointing to the b200_bias_layers of 25 and 26).  Stops at the first failure: returns its code, *failed_at its index. */
 struct b200_fused_gemm;
 typedef struct b200_op {

@@ -696,3 +696,54 @@ def test_representations_leave_while_the_next_minibatch_is_computed(cm):
         np.testing.assert_array_equal(get(eng.h_pos).T, got[(n - 1) * B:])
         assert np.abs(got - 1 / (1 + np.exp(-(x.T.astype(np.float64) @ w)))).max() < 1e-5
     assert cm.read_status() == 0
+
+
+@pytest.mark.parametrize("once", [False, True])
+@pytest.mark.parametrize("sizes,B,mf,gibbs", [((60, 40), 20, 3, 1), ((61, 40, 33), 7, 1, 2), ((60, 44, 32), 20, 2, 1), ((64, 40, 100), 33, 3, 2),
+                                              ((50, 41, 33, 20), 12, 3, 1), ((40, 36, 30, 26, 20, 17), 9, 2, 1),
+                                              ((48, 20, 24), 1025, 2, 1), ((64, 1040, 20), 1028, 2, 1)])
+def test_dbm_of_any_depth_matches_oracle(cm, oracle, sizes, B, mf, gibbs, once, monkeypatch):
+    """Two to six layers (biases beyond the fourth in a launch of their own), one to three mean-field sweeps with W1'data in every
+    sweep and multiplied once, odd sizes, cases past what the bias launch takes and products that find what is added in their
+    output."""
+    from deepnet_b200.fused_dbm import FusedDBM
+    monkeypatch.setattr(FusedDBM, "_data_once", lambda self: once and self.L > 2 and self.hyp.mf_steps > 1)
+    rng = np.random.default_rng(sum(sizes) + B)
+    hyp = dbm.Hyperparams(base_epsilon=0.05, initial_momentum=0.5, final_momentum=0.9, momentum_change_steps=10, mf_steps=mf,
+                          gibbs_steps=gibbs)
+    names = ["l%d" % i for i in range(len(sizes))]
+    w = [(rng.standard_normal((sizes[i], sizes[i + 1])) * 0.1).astype(np.float32) for i in range(len(sizes) - 1)]
+    layers = [dict(name=n, activation=dbm.LOGISTIC, numdims=d, is_input=i == 0) for i, (n, d) in enumerate(zip(names, sizes))]
+    edges = [dict(node1=names[i], node2=names[i + 1], weight=w[i]) for i in range(len(w))]
+    data = (rng.random((sizes[0], 2 * B)) < 0.3).astype(np.float32)
+    cfg = dict(layers=layers, edges=edges, hyperparams=hyp, batchsize=B, optimizer=dbm.PCD, seed=4, data=data)
+    mo, lo = run_driver(oracle, cfg, 2 * B, 2)
+    eng = FusedDBM(cm, list(sizes), B, w, hyp, seed=4)
+    dev, lg = cm.CUDAMatrix(data), []
+    for step in range(2):
+        eng.TrainOneBatch(step, dev.slice(step * B, (step + 1) * B))
+        lg.append(eng.read_loss())
+    np.testing.assert_allclose(lg, lo, rtol=1e-5)
+    for i, e in enumerate(mo.edge):
+        assert relerr(get(eng.W[i]), get(e.params["weight"])) < TOL
+    for j, l in enumerate(mo.layer):
+        assert relerr(get(eng.pos[j]), get(l.pos_state)) < TOL, l.name
+        if j > 0:
+            np.testing.assert_array_equal(get(eng.neg_sample[j]), get(l.neg_sample))
+        assert np.abs(get(eng.b[j]) - get(l.params["bias"])).max() < 1e-6
+    assert cm.read_status() == 0
+
+
+def test_dbm_multiplies_the_data_once_only_where_that_pays(cm):
+    """us an update, in every sweep / once: 784-500-1000, 100 cases, 10 sweeps 328 / 298; 64-64-64 193 / 211; 256-256-1500, 16 cases
+    262 / 292; 500-2048-500, 1030 cases 772 / 896."""
+    from deepnet_b200.fused_dbm import FusedDBM
+
+    def once(sizes, B, mf):
+        w = [np.zeros((sizes[i], sizes[i + 1]), np.float32) for i in range(len(sizes) - 1)]
+        eng = FusedDBM(cm, sizes, B, w, dbm.Hyperparams(mf_steps=mf, gibbs_steps=1))
+        return eng._data_once()
+
+    assert once([784, 500, 1000], 100, 10) and once([784, 500, 1000], 100, 3) and once([1500, 256, 256], 16, 3)
+    assert not once([784, 500, 1000], 100, 2) and not once([784, 500], 100, 10) and not once([64, 64, 64], 100, 10)
+    assert not once([256, 256, 1500], 16, 10) and not once([500, 2048, 500], 1030, 10)
