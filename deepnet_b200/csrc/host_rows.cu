@@ -5,16 +5,17 @@
 // (deepnet/extract_rbm_representation.py).  Here the copy lands in pinned pieces on a stream of its own and a few threads
 // carry the pieces to where they belong, while the caller goes on to the next minibatch: eight of 250 x 1000 with their
 // reconstruction error 1154 -> 540 us.
-// One staging area per process (4 MB and six threads, made on first use, given back by cublas_shutdown): whoever
+// One staging area per process (4 MB and four threads, made on first use, given back by cublas_shutdown): whoever
 // begins while another thread holds it is told so and copies the plain way.
 //
 // The carriers are bound by the page faults of the fresh result, which more than two or three threads only make dearer, unless its
-// pages are large ones.  At most two wait for their piece (busily: with blocking waits the call took twice as long); the others
+// matrices are large.  At most two wait for their piece (busily: with blocking waits the call took twice as long); the others
 // sleep until pieces have landed.  us a call and cores busy, by carriers / of them waiting:
-//                                        2 / 2        3 / 2        4 / 4        6 / 2
-//   eight minibatches of 250 x 1000      504, 2.5     552, 3.1     556, 4.0     602, 3.4
-//   eight of 500 x 2048                  1259, 2.4    1217, 3.5    1316, 4.4    1517, 4.0
-//   two of 1024 x 8192                   9588, 2.0    7849, 2.9    7231, 4.0    6013, 4.8
+//                                        2 / 2        3 / 2        4 / 2        4 / 4        6 / 2
+//   eight minibatches of 250 x 1000      504, 2.5     552, 3.1     579, 3.3     556, 4.0     602, 3.4
+//   eight of 500 x 2048                  1259, 2.4    1217, 3.5    1381, 3.9    1316, 4.4    1517, 4.0
+//   two of 1024 x 8192                   9588, 2.0    7849, 2.9    7075, 3.6    7231, 4.0    6013, 4.8
+//   two of 4096 x 2048, large pages                                             2627, 4.4    3062, 4.3
 #include <condition_variable>
 #include <cstring>
 #include <deque>
@@ -28,7 +29,7 @@ using namespace b200;
 
 namespace {
 
-constexpr int kPieces = 16, kCarriers = 6, kWaiting = 2;
+constexpr int kPieces = 16, kCarriers = 4, kWaiting = 2;
 constexpr int kFewCarriers = 3;                     // ... of matrices below
 constexpr size_t kManyCarriersBytes = 16 << 20;
 constexpr size_t kPieceBytes = 256 * 1024;
