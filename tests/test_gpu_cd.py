@@ -747,3 +747,37 @@ def test_dbm_multiplies_the_data_once_only_where_that_pays(cm):
     assert once([784, 500, 1000], 100, 10) and once([784, 500, 1000], 100, 3) and once([1500, 256, 256], 16, 3)
     assert not once([784, 500, 1000], 100, 2) and not once([784, 500], 100, 10) and not once([64, 64, 64], 100, 10)
     assert not once([256, 256, 1500], 16, 10) and not once([500, 2048, 500], 1030, 10)
+
+
+def test_recorded_operations_equal_the_calls(cm):
+    """Every operation of the vocabulary that no engine records today, recorded and replayed, against its call: same bits."""
+    rng = np.random.default_rng(12)
+    f = lambda *shape: rng.random(shape).astype(np.float32) + 0.1
+    V, H, B = 33, 20, 9
+    host = dict(m=f(V, B), n=f(V, B), h=f(H, B), g=f(H, B), nn=np.floor(9 * f(1, B)), b=f(V + H, 1), db=f(V + H, 1), w=f(V, H), d=f(V, H),
+                s=f(V, H))
+    results = []
+    for recorded in (False, True):
+        d = {k: cm.CUDAMatrix(v) for k, v in host.items()}
+        t = [cm.empty(shape) for shape in ((V, B), (1, B), (V, B), (V, B), (V + H, 1), (1, 1), (V, B), (V, B))]
+        cm.CUDAMatrix.init_random(5)
+        X = cm.Program() if recorded else cm.Immediate()
+        X.softmax_scaled(d["m"], d["nn"], t[0])
+        X.sum(d["m"], 0, t[1])
+        X.add_sums(t[1], d["n"], 0, 0.5)
+        X.add_scalar(t[1], 1e-3)
+        X.div_by_row(d["n"], t[1], t[2])
+        X.sigmoid(d["m"], t[3])
+        X.rbm_bias_update(d["m"], d["n"], d["h"], d["g"], t[4], d["b"], d["db"], t[5], 1.0 / B, 0.5, 0.1)
+        X.momentum_update(d["w"], d["d"], None, d["s"], 1.0 / B, 0.9, 0.2, l2=1e-3, l1=1e-4)
+        X.sample_bernoulli(d["m"], t[6])
+        X.copy(t[6], t[7])
+        X.assign_scalar(t[6], 2.0)
+        if recorded:
+            assert len(X) == 11
+            X.run()
+        results.append([get(x) for x in t + [d["b"], d["db"], d["w"], d["d"]]] + [cm.CUDAMatrix.rnd_state.calls])
+    for a, b in zip(*results):
+        np.testing.assert_array_equal(a, b)
+    np.testing.assert_allclose(results[0][0].sum(axis=0), host["nn"][0], rtol=1e-5)
+    assert results[0][-1] == 1 and results[0][5][0, 0] > 0

@@ -993,7 +993,7 @@ def test_products_bound_by_the_converters_keep_wide_tiles(cm, M, N, K, columns):
 @pytest.mark.parametrize("M,N,K", [(64, 4, 32), (500, 100, 1000), (129, 260, 96), (4, 1, 8), (1000, 2048, 40)])
 def test_added_matrix_joins_before_the_activation(cm, path, M, N, K):
     """out = logistic(a.b + add + bias) and its draw in every kernel that ends a product: one launch, tcgen05 whole and cut
-    along K, CUDA cores; 1e-5 as for the product alone."""
+    along K, CUDA cores; 1e-5 as for the product alone.  The draw is that of the result on the same stream."""
     rng = np.random.default_rng(M * N)
     a, b = (rng.standard_normal((K, M)) * 0.1).astype(np.float32), rng.random((K, N)).astype(np.float32)
     add, bias = rng.standard_normal((M, N)).astype(np.float32), rng.standard_normal((M, 1)).astype(np.float32)
@@ -1006,7 +1006,11 @@ def test_added_matrix_joins_before_the_activation(cm, path, M, N, K):
     pre = a.T.astype(np.float64) @ b + add
     assert np.abs(get(out) - 1 / (1 + np.exp(-(pre + bias)))).max() < TOL
     assert np.abs(get(plain) - pre).max() < TOL * np.abs(pre).max()
-    assert 0 < get(draw).mean() < 1 or M * N < 32
+    cm.set_gemm_path(0)
+    again = cm.empty((M, N))
+    cm.CUDAMatrix.init_random(1)
+    cm.CUDAMatrix(get(out)).sample_bernoulli(target=again)
+    np.testing.assert_array_equal(get(draw), get(again))
     with pytest.raises(cm.CUDAMatException):
         cm.fused_gemm(passes, out=out, add=cm.empty((M, N + 1)))
 
