@@ -12,9 +12,11 @@ probabilities, deepnet/ais.py:158), not the sample.  `exact_log_z` is deepnet/ai
 (`ExactZ_binary_binary`): the sum over all 2^V visible configurations with the hidden units
 summed out analytically.
 
-On b200mat a step of the binary RBM is two fused products (bias, schedule factor, logistic and draw in the
-epilogue) around one kernel for the importance weights and the hidden draw; `fused=False` keeps the reference's call-by-call form, which the CPU restatement
-runs too.  Both forms consume the random stream identically (two sampling calls per step).
+On b200mat all steps of the binary RBM are one launch where that is the faster way (each group of chains goes through
+all of them in a cluster of thread blocks that shares W), else two fused products a step (bias, schedule factor, logistic and
+draw in the epilogue) around one kernel for the importance weights and the hidden draw; `fused=False` keeps the
+reference's call-by-call form, which the CPU restatement runs too.  All forms consume the random stream identically (two
+sampling calls per step).
 """
 import numpy as np
 
@@ -48,7 +50,7 @@ def ais_binary_rbm(cm, weight, hidden_bias, visible_bias, num_chains, schedule, 
     v_state.sample_bernoulli(target=v_sample)
     w_ais = cm.CUDAMatrix(np.zeros((1, B), np.float32))
     w_aux = w.split_bf16(cm.empty_aux((V, H))) if fused else None
-    if fused:   # all steps from C: two products and one kernel each
+    if fused:   # all steps from C
         cm.ais_binary_steps(w, w_aux, a, b, v_state, v_sample, h_state, h_sample, w_ais, schedule)
     for i in range(1, 0 if fused else len(schedule)):
         s_prev, s = float(schedule[i - 1]), float(schedule[i])

@@ -16,8 +16,9 @@
 // multiply-adds 128).  States a caller starts from may be anything: where bfloat16 does not hold them the first product is
 // taken in doubles.
 // Bound by instruction issue (the split of W) and the latency of the exchange.  784 x 500, 100 chains, clocks of a step:
-// up 4850, hidden units 3200, down 6140, visible units 3900, barriers 2000: 10.5 us, against 36 as two products and a
-// kernel between them (three launches); 100 steps with their set-up 2881 -> 1479 us.
+// up 4850, hidden units 3200, down 6140, visible units 3900, barriers 2000: 10.5 us, against 25 as two products and a
+// kernel between them (three launches; 36 with the products as they were).  The steps are a millisecond of a call of
+// `ais_binary_rbm` with a hundred of them; the rest is the caller's set-up.
 #include <cmath>
 #include <initializer_list>
 #include <type_traits>

@@ -663,11 +663,15 @@ int small_depth(const GemmProblem& g) {
   return walked_slabs(g, p);
 }
 
-// Whether one launch is faster than the tcgen05 kernel on operands that both take: both sides estimated in us, from
-// about 150 products of 64 x 32 to 4096 x 1024 outputs and K from 16 to 4096.  The line is not one depth: the tcgen05
-// kernel spends 13 us on a plain product of many tiles where this one goes through several waves (2048 x 2048, two pairs of
-// K = 32: 14.9 against 27.1 us at 8 slabs an SM), 39 us on an activation of short K (1024 x 1024, K = 128: 39.5 against
-// 12.2), and cuts a long K over more CTAs (500 x 100, K = 2800: 16.9 against 18.1).
+// Whether a product that both kernels take goes in one launch here.  The other side is estimated as the tcgen05 kernel with tiles
+// of 256 columns wherever N > 128, fitted (as this one) to about 150 products of 64 x 32 to 4096 x 1024 outputs and K from 16 to
+// 4096.  Narrower tiles since made it faster than that by up to a third, yet the line stays: what lies between is three to five
+// times as exact here, where additions round and the terms are split TF32.  Logistic layer on 0/1 input, us and relative
+// error against float64, here / there:
+//   1024 x 256, K = 2048    23.7, 6.3e-8 / 17.2, 2.5e-7       500 x 1000, K = 784    20.8, 5.4e-8 / 16.0, 1.8e-7
+//   1024 x 1024, K = 384    19.3, 5.0e-8 / 11.9, 1.3e-7       1024 x 1024, K = 128   10.3, 4.7e-8 /  8.8, 8.8e-8
+// On the line's other sides: 2048 x 2048, two pairs of K = 32: 27.1 us here (several waves), 14.9 there; 500 x 100, K = 2800: 18.1
+// here, 16.9 there.
 bool small_beats_tc(const GemmProblem& g) {
   SmallParams p;
   if (g.M <= 0 || g.N <= 0 || !gather_pairs(g, p)) return false;

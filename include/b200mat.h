@@ -328,7 +328,7 @@ int b200_test_tile_columns(int columns);
 int b200_test_ais_form(int form);
 int b200_test_ais_in_one_launch(int V, int H, int B, int n);
 /* All steps of an annealing schedule (n inverse temperatures) of a binary RBM's partition function estimate
- * (deepnet/ais.py:152-170): w V x H and its aux, biases a (H) and b (V), chain states, sb (V) scratch, weights 1 x B added to. */
+ * (deepnet/ais.py:152-170): w V x H and its aux, biases a (H) and b (V), chain states (of any value to start from), sb (V) scratch, weights 1 x B added to. */
 int ais_binary_steps(rnd_struct* rnd_state, cudamat* w, cudamat* w_aux, cudamat* a, cudamat* b, cudamat* v_state,
                      cudamat* v_sample, cudamat* h_pre, cudamat* h_sample, cudamat* sb, cudamat* weights,
                      const double* schedule, int n);
