@@ -8,14 +8,15 @@
 // One staging area per process (4 MB and four threads, made on first use, given back by cublas_shutdown): whoever
 // begins while another thread holds it is told so and copies the plain way.
 //
-// The carriers are bound by the page faults of the fresh result, which more than two or three threads only make dearer, unless its
-// matrices are large.  At most two wait for their piece (busily: with blocking waits the call took twice as long); the others
-// sleep until pieces have landed.  us a call and cores busy, by carriers / of them waiting:
-//                                        2 / 2        3 / 2        4 / 2        4 / 4        6 / 2
-//   eight minibatches of 250 x 1000      504, 2.5     552, 3.1     579, 3.3     556, 4.0     602, 3.4
-//   eight of 500 x 2048                  1259, 2.4    1217, 3.5    1381, 3.9    1316, 4.4    1517, 4.0
-//   two of 1024 x 8192                   9588, 2.0    7849, 2.9    7075, 3.6    7231, 4.0    6013, 4.8
-//   two of 4096 x 2048, large pages                                             2627, 4.4    3062, 4.3
+// Every carrier takes a piece before it has landed, so that it is awake in time.  The two whose pieces land next wait busily
+// (with blocking waits the call above took 603 us and more, against 556), the others look every ten microseconds.  Cores
+// occupied with all four waiting busily / so: 4.1 / 3.3 in the call above, 4.4 / 3.6 in eight minibatches of 500 x 2048
+// (1418 / 1297 us).  Fewer carriers, asleep until a piece has landed, gained as much on large results and lost up to 8 % on
+// small ones; six lost 16 % where the result's pages are large.
+#include <sys/prctl.h>
+#include <time.h>
+
+#include <atomic>
 #include <condition_variable>
 #include <cstring>
 #include <deque>
@@ -29,14 +30,12 @@ using namespace b200;
 
 namespace {
 
-constexpr int kPieces = 16, kCarriers = 4, kWaiting = 2;
-constexpr int kFewCarriers = 3;                     // ... of matrices below
-constexpr size_t kManyCarriersBytes = 16 << 20;
+constexpr int kPieces = 16, kCarriers = 4, kBusy = 2;
 constexpr size_t kPieceBytes = 256 * 1024;
 
 struct RowsStaging {
   std::mutex mu;
-  std::condition_variable work, more_work, freed;     // of the first carriers, of the others, of the caller
+  std::condition_variable work, freed;
   struct Job {
     int piece;
     float* dst;
@@ -48,30 +47,33 @@ struct RowsStaging {
   cudaEvent_t landed[kPieces] = {nullptr}, ready = nullptr, done[2] = {nullptr, nullptr};
   cudaStream_t copies = nullptr;
   bool free_piece[kPieces];
-  int device = 0, in_flight = 0, adds = 0, waiting = 0, carrying = kFewCarriers;   // (threads that may carry)
+  int device = 0, in_flight = 0, adds = 0;
+  std::atomic<long> taken{0}, seen{0};     // pieces carriers have taken, and seen land
   bool held = false, stop = false, made = false, failed = false;
 
-  void wake_one() {
-    work.notify_one();
-    if (carrying > kFewCarriers) more_work.notify_one();
+  // The order-th piece (of all ever taken) has landed.
+  bool wait_for(cudaEvent_t event, long order) {
+    for (;;) {
+      const cudaError_t e = cudaEventQuery(event);
+      if (e != cudaErrorNotReady) return e == cudaSuccess;
+      if (order - seen < kBusy) return cudaEventSynchronize(event) == cudaSuccess;
+      const timespec ten_us = {0, 10000};
+      nanosleep(&ten_us, nullptr);
+    }
   }
-  void carry(int self) {
+  void carry() {
     cudaSetDevice(device);
+    prctl(PR_SET_TIMERSLACK, 1000ul);     // (of this thread: a nap of 10 us takes 60 by default)
     std::unique_lock<std::mutex> lock(mu);
     for (;;) {
-      (self < kFewCarriers ? work : more_work).wait(lock, [&] {
-        return stop || (!jobs.empty() && waiting < kWaiting && self < carrying);
-      });
+      work.wait(lock, [&] { return stop || !jobs.empty(); });
       if (jobs.empty()) return;
       const Job j = jobs.front();
       jobs.pop_front();
-      waiting++;
+      const long order = taken++;
       lock.unlock();
-      const bool ok = cudaEventSynchronize(landed[j.piece]) == cudaSuccess;
-      lock.lock();
-      waiting--;
-      if (!jobs.empty()) wake_one();
-      lock.unlock();
+      const bool ok = wait_for(landed[j.piece], order);
+      seen++;
       if (ok) memcpy(j.dst, pinned + j.piece * kPieceBytes, j.bytes);
       lock.lock();
       failed |= !ok;
@@ -86,7 +88,6 @@ struct RowsStaging {
       stop = true;
     }
     work.notify_all();
-    more_work.notify_all();
     for (std::thread& t : carriers) t.join();
     carriers.clear();
     if (pinned) cudaFreeHost(pinned);
@@ -110,7 +111,7 @@ struct RowsStaging {
     for (cudaEvent_t& e : landed) ok = ok && cudaEventCreateWithFlags(&e, cudaEventDisableTiming) == cudaSuccess;
     for (bool& f : free_piece) f = true;
     try {
-      for (int i = 0; ok && i < kCarriers; i++) carriers.emplace_back([this, i] { carry(i); });
+      for (int i = 0; ok && i < kCarriers; i++) carriers.emplace_back([this] { carry(); });
     } catch (...) {
       ok = false;
     }
@@ -164,10 +165,6 @@ int b200_rows_add(cudamat* src, float* dst) {
   if (cudaEventRecord(s.ready, stream()) != cudaSuccess || cudaStreamWaitEvent(s.copies, s.ready, 0) != cudaSuccess)
     return set_error(cudaGetErrorString(cudaGetLastError()));
   const size_t bytes = (size_t)numel(src) * sizeof(float);
-  {
-    std::lock_guard<std::mutex> lock(s.mu);
-    s.carrying = bytes < kManyCarriersBytes ? kFewCarriers : kCarriers;
-  }
   for (size_t at = 0; at < bytes; at += kPieceBytes) {
     const size_t n = bytes - at < kPieceBytes ? bytes - at : kPieceBytes;
     int piece = -1;
@@ -191,7 +188,7 @@ int b200_rows_add(cudamat* src, float* dst) {
     }
     s.jobs.push_back({piece, (float*)((char*)dst + at), n});
     s.in_flight++;
-    s.wake_one();
+    s.work.notify_one();
   }
   // the matrix of the call before has been read once this stream is past its copies
   if (s.adds > 0 && cudaStreamWaitEvent(stream(), s.done[(s.adds - 1) & 1], 0) != cudaSuccess)
