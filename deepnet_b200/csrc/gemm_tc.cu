@@ -1546,8 +1546,8 @@ enum { kLightPair, kHalfPair, kDerivedBf16, kDerivedTf32, kPairKinds };
 // the tensor pipe at its rate, where the tiles fill the device; a product of few tiles is bound by what surrounds them, and
 // narrower tiles of a single CTA come off better, unless they are bound by the converters, which derive the parts of a tile's
 // rows and columns once a tile.  The estimate, in us, is fitted to 1088 products of 19 shapes (256 to 4096 rows and columns), K
-// from 64 to 4096 and eight term lists (rms error 7 %); its choice is within 0.5 % of the best width on average, never behind
-// 256.  Measured, 256 / 128 / 64 columns:
+// from 64 to 4096 and eight term lists (rms error 7 %); its choice is within 0.5 % of the best width on average (0.7 % on 1736 products of
+// 20 other shapes), in neither set behind 256.  Measured, 256 / 128 / 64 columns:
 //   500 x 500, K = 784, activation, W's parts from memory          21.6 / 15.4 / 14.7
 //   1000 x 2048, K = 500, the same                                 31.2 / 22.9 / 24.3
 //   1024 x 256, K = 4096, the same                                 30.1 / 21.4 / 24.4
