@@ -42,7 +42,8 @@ namespace b200 {
 
 cudaStream_t stream();                 // the stream every operation of the library runs on
 cudaStream_t stream_if_initialised();  // the same, or the default stream when the library was never initialised
-int sm_count();                        // SMs of the current device
+int sm_count();                        // SMs of the current device a kernel may size its grid for (b200_set_sm_limit)
+int device_sms();                      // all of them
 int check_launch();                    // cudaGetLastError -> 0 or CUDA_ERROR (message kept); CUDA_ERROR when the library failed to initialise
 int check_launch_any_stream();         // the same for entry points that also run without the library stream
 int set_error(const char* msg);        // records msg, returns CUDA_ERROR

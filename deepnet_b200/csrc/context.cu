@@ -92,6 +92,10 @@ int sm_count() {
   const int n = g_sm_count > 0 ? g_sm_count : 148;
   return (g_sm_limit > 0 && g_sm_limit < n) ? g_sm_limit : n;
 }
+int device_sms() {
+  ensure_init();
+  return g_sm_count > 0 ? g_sm_count : 148;
+}
 int rng_col0() { return g_col0; }
 int* status_word() {
   ensure_init();

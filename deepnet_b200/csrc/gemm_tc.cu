@@ -24,6 +24,8 @@
 //                 They fold every finished chunk of the product into fp32 registers (two TMEM
 //                 accumulators ping-pong with the MMA issuer) and run the fused epilogue from
 //                 those registers at the end of the tile.
+// Products that fill the device at most a few times take the same mainloop with one work item per CTA: the tile ends in
+// shared memory, K is cut over the CTAs of a cluster, and all warps share the epilogue (TileEpilogue, choose_plan).
 // Every mbarrier wait is bounded; on expiry the kernel records a status word, drains
 // and frees its tensor memory and returns.
 #include <cuda.h>
@@ -101,7 +103,7 @@ constexpr int kMaxMaps = 16;    // tensor maps: operand tiles as loaded, then th
 struct TcParams {
   CUtensorMap maps[kMaxMaps];
   TcGroup group[kMaxGroups];
-  int ngroups;
+  int ngroups, nloads;     // nloads: tensor maps of operands
   int M, N, tiles_m, tiles_n;
   int bk;                  // floats of K per k-block: 32 or 16
   int num_stages;          // ring depth
@@ -299,8 +301,9 @@ __device__ __forceinline__ void mma_commit_pair(uint32_t bar, uint16_t cta_mask)
 __device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
   asm volatile(
       "{\n\t.reg .b32 ra;\n\t"
-      "mapa.shared::cluster.u32 ra, %0, 0;\n\t"
-      "mbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}" ::"r"(bar)
+      "mapa.shared::cluster.u32 ra, %0, %1;\n\t"
+      "mbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}" ::"r"(bar),
+      "r"(cluster_ctarank() & ~1u)
       : "memory");
 }
 
@@ -366,7 +369,8 @@ struct TcConfig {
 //   kEpiGeneric    every option tested at run time
 //   kEpiPartial    kEpiPlain for one split of a split-K product: raw partial sums to the workspace
 //                  (the only variant that carries the work-item bookkeeping of split-K)
-enum { kEpiPlain = 0, kEpiGeneric = 1, kEpiSig = 2, kEpiSigSample = 3, kEpiLin = 4, kEpiPartial = 5 };
+//   kEpiTile       every option, for products whose CTAs have one work item each: see TileEpilogue
+enum { kEpiPlain = 0, kEpiGeneric = 1, kEpiSig = 2, kEpiSigSample = 3, kEpiLin = 4, kEpiPartial = 5, kEpiTile = 6 };
 __host__ __device__ constexpr bool epi_is_plain(int e) { return e == kEpiPlain || e == kEpiPartial; }
 
 // Two packed bfloat16 (round to nearest even): `lo` goes to the lower address.
@@ -423,11 +427,199 @@ __device__ __forceinline__ void convert16(const uint32_t (&s)[4], bool lo32, uin
   }
 }
 
+// A 16-byte read of shared memory of the cluster, and the address of this CTA's location in CTA `rank` of it.
+__device__ __forceinline__ float4 ld_cluster128(uint32_t addr) {
+  float4 v;
+  asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "r"(addr)
+               : "memory");
+  return v;
+}
+__device__ __forceinline__ uint32_t in_cta(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+
+__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+
+// The end of a product whose CTAs have one work item each.  Nothing follows that an epilogue on the warps that drained
+// the accumulators could overlap, so the tile goes through shared memory (the ring is free by then) and all the block's
+// warps share the work; the splits of a tile are one thread-block cluster, whose CTAs each sum one share of the columns
+// over all of them through distributed shared memory, in split order (the same bits every run, and the ones a finishing
+// launch would give).  Partial tiles are [column][128 rows]; a thread takes four rows of four columns, one Philox block a
+// row, and stores 16 bytes a column where the columns start on them.  Bound by instruction fetch (the code runs a few
+// times a CTA): every option is one branch per sixteen elements, not one per element.
+template <int BN, int kWarps>
+struct TileEpilogue {
+  // what the loop needs from global memory, fetched before the barrier that the partial tiles wait for
+  float bias[4], alpha;
+  int m, rows;
+
+  __device__ __forceinline__ void fetch(const TcParams& p, int m_tile) {
+    m = m_tile + 4 * (threadIdx.x & 31);
+    rows = min(4, p.M - m);
+    const GemmEpilogue& e = p.epi;
+    alpha = e.alpha * exp2f(-((e.scale_exp ? *e.scale_exp : 0.0f) + (float)e.scale_exp_const));
+#pragma unroll
+    for (int r = 0; r < 4; r++) bias[r] = e.bias && r < rows ? e.bias[m + r] : 0.0f;
+  }
+
+  // 32-bit stores of rows m .. m + 3 of four columns
+  static __device__ __forceinline__ void store(float* out, long ld, int cols, int rows, bool wide, const float (&x)[4][4]) {
+    if (wide) {
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (j < cols) *reinterpret_cast<float4*>(out + j * ld) = make_float4(x[j][0], x[j][1], x[j][2], x[j][3]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+          if (j < cols && r < rows) out[j * ld + r] = x[j][r];
+    }
+  }
+  // the same of one 16-bit plane, two rows a register
+  static __device__ __forceinline__ void store16(uint16_t* out, long ld, int cols, int rows, bool wide, const uint32_t (&x)[4][2]) {
+    if (wide) {
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+        if (j < cols) *reinterpret_cast<uint2*>(out + j * ld) = make_uint2(x[j][0], x[j][1]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 4; j++)
+#pragma unroll
+        for (int r = 0; r < 4; r++)
+          if (j < cols && r < rows) out[j * ld + r] = (uint16_t)(x[j][r >> 1] >> (16 * (r & 1)));
+    }
+  }
+
+  __device__ __forceinline__ void run(const TcParams& p, uint32_t tile, int split, uint32_t first_rank, uint32_t rank_step,
+                                      int n_tile) {
+    const GemmEpilogue e = p.epi;
+    const int S = p.splits, last = (BN / 4) * (split + 1) / S;
+    if (rows <= 0) return;
+#pragma unroll 1
+    for (int q = (BN / 4) * split / S + ((threadIdx.x >> 5) % kWarps); q < last; q += kWarps) {
+      const int n = n_tile + 4 * q, cols = min(4, p.N - n);
+      if (cols <= 0) break;
+      float x[4][4];           // [column][row]
+      const uint32_t at = tile + (uint32_t)(4 * q * BM + 4 * (threadIdx.x & 31)) * 4u;
+      if (S == 1) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const float4 v = lds128(at + j * (BM * 4));
+          x[j][0] = v.x; x[j][1] = v.y; x[j][2] = v.z; x[j][3] = v.w;
+        }
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++) x[j][0] = x[j][1] = x[j][2] = x[j][3] = 0.0f;
+#pragma unroll 2
+        for (int s = 0; s < S; s++) {
+          const uint32_t from = in_cta(at, first_rank + s * rank_step);
+          float4 v[4];
+#pragma unroll
+          for (int j = 0; j < 4; j++) v[j] = ld_cluster128(from + j * (BM * 4));
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            x[j][0] += v[j].x; x[j][1] += v[j].y; x[j][2] += v[j].z; x[j][3] += v[j].w;
+          }
+        }
+      }
+      const long off = (long)n * e.ldo + m, word = 2L * n * e.ld_aux + m;   // (16-bit words of plane 0)
+      float scale[4] = {1.0f, 1.0f, 1.0f, 1.0f};
+      if (e.col_scale) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) scale[j] = j < cols ? e.col_scale[n + j] : 0.0f;
+      }
+      if (e.beta != 0.0f) {
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+          for (int r = 0; r < 4; r++)
+            x[j][r] = alpha * x[j][r] + (j < cols && r < rows ? e.beta * e.out[off + j * (long)e.ldo + r] : 0.0f);
+      } else {
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+          for (int r = 0; r < 4; r++) x[j][r] *= alpha;
+      }
+      if (e.bias) {
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+          for (int r = 0; r < 4; r++) x[j][r] = fmaf(bias[r], scale[j], x[j][r]);
+      }
+      if (e.activation == 1) {
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+          for (int r = 0; r < 4; r++) x[j][r] = sigmoid_accurate(x[j][r]);
+      }
+      const bool wide = rows == 4 && e.ldo % 4 == 0 && (((uintptr_t)e.out | (uintptr_t)e.sample) & 15) == 0;
+      const bool wide16 = rows == 4 && (((uintptr_t)e.out_aux | (uintptr_t)e.sample_aux) & 7) == 0;
+      if (e.out) store(e.out + off, e.ldo, cols, rows, wide, x);
+      if (e.out_aux) {
+        uint16_t* const o = reinterpret_cast<uint16_t*>(e.out_aux) + word;
+        uint32_t lo[4][2], hi[4][2];
+        if (e.aux_f16) {
+          const float aux_scale = exp2f((float)e.aux_exp);
+#pragma unroll
+          for (int j = 0; j < 4; j++)
+#pragma unroll
+            for (int r = 0; r < 4; r += 2) {
+              uint16_t l[2], h[2];
+              split_f16(x[j][r], aux_scale, l[0], h[0]);
+              split_f16(x[j][r + 1], aux_scale, l[1], h[1]);
+              lo[j][r >> 1] = l[0] | (uint32_t)l[1] << 16;
+              hi[j][r >> 1] = h[0] | (uint32_t)h[1] << 16;
+            }
+        } else {
+#pragma unroll
+          for (int j = 0; j < 4; j++)
+#pragma unroll
+            for (int r = 0; r < 4; r += 2) {
+              lo[j][r >> 1] = pack_bf16(tf32_rest(x[j][r]), tf32_rest(x[j][r + 1]));
+              hi[j][r >> 1] = pack_bf16(x[j][r], x[j][r + 1]);
+            }
+        }
+        store16(o, 2L * e.ld_aux, cols, rows, wide16, lo);
+        store16(o + e.ld_aux, 2L * e.ld_aux, cols, rows, wide16, hi);
+      }
+      if (e.sample || e.sample_aux) {
+        uint32_t w[4][4];        // [row][column]
+#pragma unroll
+        for (int r = 0; r < 4; r++) {
+          const uint4 b = philox4x32_10((uint32_t)(m + r), (uint32_t)((n + e.col0) >> 2), e.key);
+          w[r][0] = b.x; w[r][1] = b.y; w[r][2] = b.z; w[r][3] = b.w;
+        }
+#pragma unroll
+        for (int j = 0; j < 4; j++)
+#pragma unroll
+          for (int r = 0; r < 4; r++) x[j][r] = word_to_uniform(w[r][j]) < x[j][r] ? 1.0f : 0.0f;
+        if (e.sample) store(e.sample + off, e.ldo, cols, rows, wide, x);
+        if (e.sample_aux) {
+          const uint32_t one = e.aux_f16 ? __half_as_ushort(__float2half_rn(exp2f((float)e.aux_exp))) : 0x3f80u;
+          uint32_t on[4][2];
+#pragma unroll
+          for (int j = 0; j < 4; j++)
+#pragma unroll
+            for (int r = 0; r < 4; r += 2) on[j][r >> 1] = (x[j][r] != 0.0f ? one : 0u) | (x[j][r + 1] != 0.0f ? one << 16 : 0u);
+          store16(reinterpret_cast<uint16_t*>(e.sample_aux) + word + e.ld_aux, 2L * e.ld_aux, cols, rows, wide16, on);
+        }
+      }
+    }
+  }
+};
+
 // kTwo: two CTAs of a cluster share one 256 x BN tile (cta_group::2): each stages its own 128
 // rows of A and half of B's rows, the leader issues the MMAs for both.
 template <int BN, int kEpi, bool kTwo>
 __global__ void __launch_bounds__(kThreadsTc, 1) k_gemm_tc(const __grid_constant__ TcParams p) {
   using Cfg = TcConfig<BN>;
+  // (up to 64 accumulator columns a thread, the kernel's 128 registers do for every role)
+  constexpr bool kSplitRegs = kEpi != kEpiTile || BN > 128;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t out_stage_base = smem_base + kStageBudget;
@@ -452,9 +644,12 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_gemm_tc(const __grid_constant
 
   grid_dependents_launch();   // the next kernel of the stream may be scheduled as SMs free up
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int splits = (kEpi == kEpiPartial) ? p.splits : 1;
+  // the first copy through a tensor map waits for the map: fetched while the barriers are set up and the previous kernel ends
+  if (warp == 2 && lane < p.nloads) asm volatile("prefetch.tensormap [%0];" ::"l"(&p.maps[lane]) : "memory");
+  const int splits = (kEpi == kEpiPartial || kEpi == kEpiTile) ? p.splits : 1;
   const int num_tiles = p.tiles_m * p.tiles_n * splits;     // work items: every role walks the same list
-  const uint32_t rank = kTwo ? cluster_ctarank() : 0u;        // 0 = leader of the pair
+  const uint32_t rank = kTwo ? cluster_ctarank() & 1u : 0u;   // 0 = leader of the pair
+  // (kEpiTile: as many CTAs or pairs as work items, the splits of a tile next to each other in one cluster)
   const int first_tile = kTwo ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
   const int tile_step = kTwo ? (int)(gridDim.x >> 1) : (int)gridDim.x;
   constexpr int TILE_M = kTwo ? 2 * BM : BM;                  // rows of the tile a CTA (pair) owns
@@ -509,9 +704,9 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_gemm_tc(const __grid_constant
     return n;
   };
 
-  // Every warpgroup (four warps) passes ONE setmaxnreg instruction, at the top of its branch.
+  // Every warpgroup (four warps) passes ONE setmaxnreg instruction, at the top of its branch, or none.
   if (warp < kFirstConvWarp) {
-  asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
+  if (kSplitRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     // The whole warp runs the loop; copy u = 8 * load + box (up to six loads of up to 8 boxes: an
@@ -614,6 +809,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_gemm_tc(const __grid_constant
     // issuing thread, not the tensor pipe, bounds the kernel.
     if (rank == 0) {
       const bool elected = elect_one();
+      const uint16_t pair_mask = kTwo ? (uint16_t)(3u << cluster_ctarank()) : (uint16_t)1;   // (the leader's rank is even)
       uint32_t chunk = 0;
       int stage = 0;
       uint32_t phase = 0;
@@ -683,7 +879,8 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_gemm_tc(const __grid_constant
               // flight.  The tiles were written through the async proxy (TMA) or made visible to it by
               // the converters' proxy fence, ordered by the mbarriers.
               const uint32_t d_tmem = tmem_base + acc * BN;
-              const uint32_t sb = (smem_base + stage * stage_bytes) >> 4;   // stage address, 16-byte units
+              // stage address, 16-byte units (the bits above name the CTA of the cluster: no part of a descriptor's address)
+              const uint32_t sb = ((smem_base + stage * stage_bytes) >> 4) & 0x3fffu;
 #pragma unroll
               for (int i = 0; i < kMaxMma; i++) {
                 if (i < nm) {
@@ -717,7 +914,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_gemm_tc(const __grid_constant
               fresh = 0;
               // the stage is free (in both CTAs of a pair) once these MMAs have read it
               if (elected) {
-                if (kTwo) mma_commit_pair(empty_bar(stage), 3);
+                if (kTwo) mma_commit_pair(empty_bar(stage), pair_mask);
                 else mma_commit(empty_bar(stage));
               }
               if (++stage == num_stages) {
@@ -728,7 +925,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_gemm_tc(const __grid_constant
               if (++in_chunk == kChunkIters || in_tile == total_k_iters) {
                 // chunk complete: hand it to the epilogue warps (of both CTAs)
                 if (elected) {
-                  if (kTwo) mma_commit_pair(tfull_bar(acc), 3);
+                  if (kTwo) mma_commit_pair(tfull_bar(acc), pair_mask);
                   else mma_commit(tfull_bar(acc));
                 }
                 chunk++;
@@ -770,7 +967,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_gemm_tc(const __grid_constant
     }
   }   // warps 2, 3: nothing to do
   } else if (warp < kFirstEpiWarp) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
+    if (kSplitRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegs));
     // ------------------------------------------------------------ converters
     // For every k-block: wait for this CTA's fp32 tiles, write the derived tiles next to them in
     // the layout TMA would have produced for a tensor of that element type, make them visible to
@@ -869,7 +1066,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_gemm_tc(const __grid_constant
     (void)t_cfull; (void)t_conv;
 #endif
   } else {
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kEpiRegs));
+    if (kSplitRegs) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kEpiRegs));
     // ------------------------------------------------------------ epilogue warps
     constexpr int COLS = Cfg::kColsPerWarp;
     const int ew = warp - kFirstEpiWarp;
@@ -923,6 +1120,13 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_gemm_tc(const __grid_constant
 #ifdef B200_GEMM_TIMING
       const long long t_e0 = clock64();
 #endif
+      if constexpr (kEpi == kEpiTile) {
+        // every product of the tile is done, so nothing reads or writes the ring any more
+        const uint32_t at = smem_base + (uint32_t)(col_base * BM + wq * 32 + lane) * 4u;
+#pragma unroll
+        for (int j = 0; j < COLS; j++) asm volatile("st.shared.f32 [%0], %1;" ::"r"(at + j * (BM * 4)), "f"(accum[j]) : "memory");
+        continue;
+      }
       const int m = tm * TILE_M + (int)rank * BM + wq * 32 + lane;
       const int nc = tn * BN + col_base;
       if (m < pM && nc < pN) {
@@ -955,7 +1159,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_gemm_tc(const __grid_constant
           }
         }
       }
-      if (!epi_is_plain(kEpi)) {
+      if (!epi_is_plain(kEpi) && kEpi != kEpiTile) {
         // Activation epilogues leave through shared memory and TMA stores.  Per-thread global
         // stores (three arrays, 128 columns, 32 KB apart) cost 55 us per tile here against 7 us
         // for the arithmetic; a batch of four columns (one Philox block) is staged as
@@ -1090,6 +1294,18 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_gemm_tc(const __grid_constant
     // tiles delivered to other GPUs: this thread's stores are performed system-wide before it leaves (once
     // per launch; a fence per tile held the epilogue, and with it the issuer, for 0.24 ms per product)
     if (kEpi == kEpiPlain && p.scatter_cols > 0) __threadfence_system();
+    if constexpr (kEpi == kEpiTile && kSplitRegs) {
+      // (tiles of 256 columns: the warps that hold the registers do this alone)
+      const int t = first_tile / splits, sp = first_tile - t * splits;
+      int tm, tn;
+      tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
+      const int m_tile = tm * TILE_M + (int)rank * BM;
+      TileEpilogue<BN, kEpiWarps> te;
+      te.fetch(p, m_tile);
+      if (splits > 1) cluster_sync();
+      else named_bar_sync(1, 32 * kEpiWarps);
+      te.run(p, smem_base, sp, rank, kTwo ? 2u : 1u, tn * BN);
+    }
 #ifdef B200_GEMM_TIMING
     if (p.dbg && threadIdx.x == 32 * kFirstEpiWarp) {
       p.dbg[blockIdx.x * 8 + 4] = (unsigned long long)t_tfull;
@@ -1100,10 +1316,32 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_gemm_tc(const __grid_constant
 #endif
   }
 
+  if constexpr (kEpi == kEpiTile && kSplitRegs) {
+    __syncwarp();
+    if (splits > 1 && warp < kFirstEpiWarp) cluster_sync();   // the other warps' part of the barrier above
+  }
+  if constexpr (kEpi == kEpiTile && !kSplitRegs) {
+    const int t = first_tile / splits, sp = first_tile - t * splits;
+    int tm, tn;
+    tile_coords(t, p.tiles_m, p.tiles_n, tm, tn);
+    const int m_tile = tm * TILE_M + (int)rank * BM;
+    TileEpilogue<BN, kThreadsTc / 32> te;
+    te.fetch(p, m_tile);
+    // all partial tiles of the cluster are in shared memory (after a wait that gave up, of no meaning: the status word says so)
+    if (splits > 1) cluster_sync();
+    else __syncthreads();
+    te.run(p, smem_base, sp, rank, kTwo ? 2u : 1u, tn * BN);
+    // nobody leaves while its partial tile may still be read (what was read has arrived: nothing to order)
+    if (splits > 1 || kTwo) {
+      __syncwarp();
+      asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");
+      cluster_wait();
+    }
+  }
   // ---------------------------------------------------------------- teardown
   tc_fence_before();
   __syncthreads();
-  if (kTwo) cluster_sync();   // neither CTA leaves (or frees tensor memory) while its peer may still use it
+  if (kTwo && (kEpi != kEpiTile || kSplitRegs)) cluster_sync();   // neither CTA leaves (or frees tensor memory) while its peer may still use it
   if (warp == 1) {
     tc_fence_after();
     if (kTwo) tmem_dealloc2(tmem_base, Cfg::kTmemCols);
@@ -1252,68 +1490,83 @@ static_assert(sizeof(TcParams) <= 4096, "kernel parameter block");
 // kernel drains and returns.  Nothing traps, faults or spins without bound.
 int g_inject_stage_bytes = 0;
 
+// What a kernel needs before its first launch on a device, and how many of its clusters of `ctas` CTAs the device keeps
+// resident at once (a CTA takes an SM; the clusters leave some over in every group of SMs that can share one).  Both
+// belong to a device, not to the process: kept per device ordinal for a host that drives several GPUs.
+constexpr int kLargestCluster = 8;
 template <int BN, int kEpi, bool kTwo>
-int launch_tc(TcParams& p) {
+int resident_clusters(int ctas, int& clusters) {
   using Cfg = TcConfig<BN>;
-  // The shared-memory attribute of a kernel and the number of resident CTA pairs belong to a
-  // device, not to the process: kept per device ordinal for a host that drives several GPUs.
   constexpr int kMaxDev = 64;
   static bool attr_set[kMaxDev] = {false};
-  static int pairs_of[kMaxDev] = {0};
+  static int resident[kMaxDev][kLargestCluster + 1] = {{0}};
   static std::mutex mu;
   auto kernel = k_gemm_tc<BN, kEpi, kTwo>;
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) return set_error("cudaGetDevice failed");
-  int max_pairs = 0;
-  {
-    std::lock_guard<std::mutex> lock(mu);
-    if (!attr_set[dev]) {
-      if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess)
-        return set_error("cudaFuncSetAttribute(max dynamic shared memory) failed");
-      if (kTwo) {
-        // how many CTA pairs the device can keep resident at once (a pair needs two SMs of one TPC)
-        cudaLaunchConfig_t q = {};
-        q.gridDim = dim3(2 * (sm_count() / 2));
-        q.blockDim = dim3(kThreadsTc);
-        q.dynamicSmemBytes = Cfg::kSmemBytes;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = 2;
-        at[0].val.clusterDim.y = 1;
-        at[0].val.clusterDim.z = 1;
-        q.attrs = at;
-        q.numAttrs = 1;
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, kernel, &q) != cudaSuccess || n < 1) {
-          cudaGetLastError();
-          return set_error("cudaOccupancyMaxActiveClusters failed for the paired-CTA product");
-        }
-        pairs_of[dev] = n;
-      }
-      attr_set[dev] = true;
-    }
-    max_pairs = pairs_of[dev];
+  std::lock_guard<std::mutex> lock(mu);
+  if (!attr_set[dev]) {
+    if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess)
+      return set_error("cudaFuncSetAttribute(max dynamic shared memory) failed");
+    attr_set[dev] = true;
   }
+  if (ctas == 1) {
+    clusters = sm_count();
+    return 0;
+  }
+  if (!resident[dev][ctas]) {
+    cudaLaunchConfig_t q = {};
+    q.gridDim = dim3((unsigned)(ctas * (sm_count() / ctas)));
+    q.blockDim = dim3(kThreadsTc);
+    q.dynamicSmemBytes = Cfg::kSmemBytes;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = (unsigned)ctas;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = 1;
+    q.attrs = at;
+    q.numAttrs = 1;
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &q) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      return set_error("cudaOccupancyMaxActiveClusters failed for a tensor-core product");
+    }
+    resident[dev][ctas] = n;
+  }
+  clusters = resident[dev][ctas];
+  return 0;
+}
+
+template <int BN, int kEpi, bool kTwo>
+int launch_tc(TcParams& p) {
+  using Cfg = TcConfig<BN>;
+  auto kernel = k_gemm_tc<BN, kEpi, kTwo>;
   constexpr int TILE_M = kTwo ? 2 * BM : BM;
   p.tiles_m = (p.M + TILE_M - 1) / TILE_M;
   p.tiles_n = (p.N + BN - 1) / BN;
   const int tiles = p.tiles_m * p.tiles_n * p.splits;   // work items
-  if (!kTwo) {
-    const int grid = tiles < sm_count() ? tiles : sm_count();
-    if (launch_dependent(kernel, dim3(grid), dim3(kThreadsTc), Cfg::kSmemBytes, stream(), p) != cudaSuccess)
-      return set_error(cudaGetErrorString(cudaGetLastError()));
-    return check_launch();
+  const int cluster = (kTwo ? 2 : 1) * (kEpi == kEpiTile ? p.splits : 1);
+  int resident = 0;
+  const int err = resident_clusters<BN, kEpi, kTwo>(cluster, resident);
+  if (err) return err;
+  int ctas;
+  if (kEpi == kEpiTile) {
+    ctas = (kTwo ? 2 : 1) * tiles;
+  } else if (kTwo) {
+    int pairs = tiles < resident ? tiles : resident;
+    if (pairs > sm_count() / 2) pairs = sm_count() / 2;   // an SM limit in force (b200_set_sm_limit) leaves the rest free
+    ctas = 2 * pairs;
+  } else {
+    ctas = tiles < sm_count() ? tiles : sm_count();
   }
-  int pairs = tiles < max_pairs ? tiles : max_pairs;
-  if (pairs > sm_count() / 2) pairs = sm_count() / 2;   // an SM limit in force (b200_set_sm_limit) leaves the rest free
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(2 * pairs);
+  cfg.gridDim = dim3((unsigned)ctas);
   cfg.blockDim = dim3(kThreadsTc);
   cfg.dynamicSmemBytes = Cfg::kSmemBytes;
   cfg.stream = stream();
   cudaLaunchAttribute at[2];
   at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = 2;
+  at[0].val.clusterDim.x = (unsigned)cluster;
   at[0].val.clusterDim.y = 1;
   at[0].val.clusterDim.z = 1;
   at[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
@@ -1538,35 +1791,57 @@ static int splits_of(int ctas, int min_ki) {
 
 static int g_tile_columns = 0, g_last_columns = 0;   // b200_test_tile_columns
 
-// What the converters make of a pair's fp32 tiles decides how long a k-block takes: nothing or one 16-bit plane (parts of the
-// other operand from an aux matrix), two (or one fp32 low part), and both parts of both operands, of bfloat16 or of TF32.
-enum { kLightPair, kHalfPair, kDerivedBf16, kDerivedTf32, kPairKinds };
+// How a product is laid out.  tile: one work item per CTA (pair), the splits of a tile in one cluster (TileEpilogue); else
+// persistent CTAs, and a finishing launch behind the splits.
+struct TcPlan {
+  int columns;       // of a tile
+  bool two;          // 256 rows shared by two CTAs
+  bool tile;
+  int splits;
+};
+// What a k-block of a pair costs depends on what is staged and derived for it: nothing or one 16-bit plane derived (parts of the
+// other operand from an aux matrix), two (or one fp32 low part), both parts of both operands, of bfloat16 or of TF32; or 16-bit
+// planes alone, 64 elements of K a block, in two terms or three.
+enum { kLightPair, kHalfPair, kDerivedBf16, kDerivedTf32, kTwoPlanes, kThreePlanes, kPairKinds };
+enum { kForms = 4 };
+static const int kFormColumns[kForms] = {256, 128, 128, 64};
+static const bool kFormTwo[kForms] = {true, true, false, false};
 
-// Columns of a tile.  One CTA per 128 rows up to N = 128.  Wider products share 256 x 256 tiles between two CTAs, which runs
-// the tensor pipe at its rate, where the tiles fill the device; a product of few tiles is bound by what surrounds them, and
-// narrower tiles of a single CTA come off better, unless they are bound by the converters, which derive the parts of a tile's
-// rows and columns once a tile.  The estimate, in us, is fitted to 1088 products of 19 shapes (256 to 4096 rows and columns), K
-// from 64 to 4096 and eight term lists (rms error 7 %); its choice is within 0.5 % of the best width on average (0.7 % on 1736 products of
-// 20 other shapes), in neither set behind 256.  Measured, 256 / 128 / 64 columns:
-//   500 x 500, K = 784, activation, W's parts from memory          21.6 / 15.4 / 14.7
-//   1000 x 2048, K = 500, the same                                 31.2 / 22.9 / 24.3
-//   1024 x 256, K = 4096, the same                                 30.1 / 21.4 / 24.4
-//   784 x 1000, difference of two of K = 1024, all parts derived   37.4 / 43.9 / 64.1   (128 columns by an estimate without
-//   2048 x 512, K = 2048, TF32 parts derived                          38.7 / 44.7 / 63.4    the converters)
-// Products on 16-bit planes alone (the big models' own) and odd matrices keep the wide tiles.
-static int tile_columns(const GemmProblem& g) {
-  if (g.N <= 64) return 64;
-  if (g.N <= 128) return 128;
-  if (g_split_mode != 0 || g.odd || g.M <= BM || product_is_scattered(g.epi.out)) return 256;
-  int blocks[kPairKinds] = {0}, min_ki = 1 << 30;
+static int resident_tiles(int form, int splits, int& clusters) {
+  switch (form) {
+    case 0: return resident_clusters<256, kEpiTile, true>(2 * splits, clusters);
+    case 1: return resident_clusters<128, kEpiTile, true>(2 * splits, clusters);
+    case 2: return resident_clusters<128, kEpiTile, false>(splits, clusters);
+    default: return resident_clusters<64, kEpiTile, false>(splits, clusters);
+  }
+}
+
+// The layout of a product, by an estimate of all of them in us.  With one work item per CTA, tiles of 256 x 256 and 256 x 128 of
+// two CTAs and of 128 x 128 and 128 x 64 of one, each with K cut over up to 8 CTAs of a cluster: fitted to 3300 products of 35
+// shapes and eleven term lists (64 to 10000 rows and columns, K from 64 to 10000; rms error 5 %).  With persistent CTAs: fitted
+// to 1500 of them and 1088 others.  Measured, the best persistent layout with its finishing launch / the best of one work item:
+//   500 x 2048, K = 784, draw, W's parts from memory           18.8 / 15.0
+//   4096 x 256, K = 1024, the same, three / two planes          21.3 / 16.5, 26.9 / 12.0, 27.5 / 12.9
+//   1024 x 256, K = 4096, two planes                            29.2 / 15.0
+//   1024 x 4096, K = 1024, draw, W's parts from memory          51.6 / 30.8
+//   784 x 1000, K = 256, difference of two, all parts derived   17.2 / 14.7
+//   512 x 100, K = 10000, W's parts from memory                 21.7 / 23.8   (few tiles: K over 32 CTAs, past what a cluster holds)
+//   784 x 500, K = 100, plain                                    8.1 /  8.8   (nothing to do but store: straight from the registers)
+//   4096 x 4096, K = 128, plain                                 33.9 / 51.5   (several waves, whose stores overlap the next)
+// What is cut along K by the classic layout only, and odd matrices' long plain sums, stay there.
+static int choose_plan(const GemmProblem& g, bool all16, bool pairs_allowed, TcPlan& plan) {
+  const bool scatter = product_is_scattered(g.epi.out);
+  const GemmEpilogue& e = g.epi;
+  const bool plain = plain_result(e), wide_only = scatter || g.M <= BM;
+  const int sms = sm_count(), bk = all16 ? 64 : 32;
+  int blocks[kMaxPass], kind[kMaxPass], pairs = 0, min_ki = 1 << 30;
   for (int q = 0; q < g.npass;) {
     const GemmPass& first = g.pass[q];
-    const int ki = (first.k + 31) / 32;
-    int planes = 0;
+    const int ki = (first.k + bk - 1) / bk;
+    int planes = 0, terms = 0;
     bool tf32 = false;
-    for (; q < g.npass; q++) {      // the terms of a pair
+    for (; q < g.npass; q++, terms++) {      // the terms of a pair
       const GemmPass& t = g.pass[q];
-      if (part_is_f16(t.a.part)) return 256;
       if (!same_operand(t.a, first.a) || !same_operand(t.b, first.b) || t.k != first.k) break;
       planes += (part_is_16bit(t.a.part) && !t.a.aux) + (part_is_16bit(t.b.part) && !t.b.aux);
       if (t.a.part == kPartLo32 || t.b.part == kPartLo32) {
@@ -1574,31 +1849,97 @@ static int tile_columns(const GemmProblem& g) {
         tf32 = true;
       }
     }
-    blocks[planes < 2 ? kLightPair : planes == 2 ? kHalfPair : tf32 ? kDerivedTf32 : kDerivedBf16] += ki;
+    kind[pairs] = all16 ? (terms < 3 ? kTwoPlanes : kThreePlanes) : planes < 2 ? kLightPair : planes == 2 ? kHalfPair : tf32 ? kDerivedTf32 : kDerivedBf16;
+    blocks[pairs++] = ki;
     min_ki = ki < min_ki ? ki : min_ki;
   }
-  if (g_tile_columns) return g_tile_columns;
-  // by width: 256, 128, 64
-  static const float block_us[kPairKinds][3] = {{0.53f, 0.49f, 0.40f}, {0.72f, 0.60f, 0.55f}, {0.76f, 0.81f, 0.82f}, {1.01f, 1.00f, 0.92f}};
-  static const float plain_us[3] = {7.7f, 1.6f, 0.5f}, activation_us[3] = {23.1f, 6.2f, 3.3f}, partial_us[3] = {7.8f, 0.5f, 0.0f};
-  const float* const whole_us = plain_result(g.epi) ? plain_us : activation_us;
-  const int sms = sm_count();
-  int best = 256;
-  float best_us = 0.0f;
-  for (int i = 0, bn = 256; bn >= 64; i++, bn /= 2) {
-    const long ctas = bn == 256 ? 2L * ((g.M + 255) / 256) * ((g.N + 255) / 256) : (long)((g.M + BM - 1) / BM) * ((g.N + bn - 1) / bn);
-    const int splits = ctas < sms && min_ki >= 8 ? splits_of((int)ctas, min_ki) : 1;
-    float us = 0.0f;
-    for (int t = 0; t < kPairKinds; t++) us += blocks[t] * block_us[t][i];
-    us = 4.3f + (float)((ctas * splits + sms - 1) / sms) * (us / splits + (splits > 1 ? partial_us[i] : whole_us[i]));
-    if (splits > 1) us += 3.3f + 0.27f * splits + 1.4e-6f * g.M * g.N * (splits + 1);   // the finishing launch
-    // (a narrower tile has to come out ahead)
-    if (bn == 256 || us < 0.97f * best_us) {
-      best = bn;
-      best_us = us;
+  auto walk = [&](const float (*us)[kForms], int form, int splits) {   // the k-blocks of one split
+    float t = 0.0f;
+    for (int i = 0; i < pairs; i++) t += (float)((blocks[i] + splits - 1) / splits) * us[kind[i]][form];
+    return t;
+  };
+  auto tiles_of = [&](int form) {
+    const int rows = kFormTwo[form] ? 2 * BM : BM;
+    return (long)((g.M + rows - 1) / rows) * ((g.N + kFormColumns[form] - 1) / kFormColumns[form]);
+  };
+  // columns by form: 256 and 128 shared by two CTAs, 128, 64
+  static const float block_us[kPairKinds][kForms] = {{0.42f, 0.43f, 0.44f, 0.41f}, {0.63f, 0.59f, 0.61f, 0.58f}, {0.73f, 0.85f, 0.79f, 0.84f},
+                                                     {0.92f, 0.88f, 0.89f, 0.89f}, {0.56f, 0.35f, 0.45f, 0.39f}, {0.84f, 0.45f, 0.58f, 0.48f}};
+  static const float start_us[kForms] = {9.6f, 5.5f, 6.8f, 6.2f}, share_us[kForms] = {0.0f, 0.8f, 0.04f, 0.0f}, split_us[kForms] = {0.41f, 0.66f, 0.37f, 0.24f};
+  const bool draw = e.sample || e.sample_aux, aux = e.out_aux || e.sample_aux;
+  const float outputs_us = (plain ? 0.0f : 0.4f) + (draw ? 0.9f : 0.0f) + (aux ? 0.95f : 0.0f);   // per 64 columns of a CTA's share
+  plan.tile = false;
+  float best = 0.0f;
+  int best_form = 0;
+  if (!scatter && g.M > 0 && (g_split_mode == 0 || g_split_mode > 1)) {
+    for (int form = 0; form < kForms; form++) {
+      const int per = kFormTwo[form] ? 2 : 1, columns = kFormColumns[form];
+      if ((kFormTwo[form] && (g.M <= BM || !pairs_allowed)) || (columns > 64 && g.N <= columns / 2)) continue;
+      if (g_tile_columns && g.N > 128 && columns != g_tile_columns) continue;
+      const long tiles = tiles_of(form);
+      for (int s = 1; s * per <= kLargestCluster; s++) {
+        if (s > 1 && (tiles * s * per > sms || s * 4 > min_ki)) break;
+        if (g_split_mode > 1 && s != (g_split_mode < min_ki ? g_split_mode : min_ki)) continue;
+        int room = 0;
+        const int err = resident_tiles(form, s, room);
+        if (err) return err;
+        if (room * per * s > sms) room = sms / (per * s);     // (an SM limit in force)
+        if (room < 1) continue;
+        const long waves = (tiles + room - 1) / room;
+        if (waves > 1 && (s > 1 || plain || waves > 4 || sms < device_sms())) continue;
+        const float share = (float)columns / (64.0f * s);
+        float us = (float)waves * (start_us[form] + walk(block_us, form, s) + share * (share_us[form] + outputs_us)) + (s > 1 ? split_us[form] * s : 0.0f);
+        // what the converters bound gains little from narrow tiles, which derive every part more often
+        if (columns < 256 && (kind[0] == kDerivedTf32 || kind[pairs - 1] == kDerivedTf32) && min_ki > 16) us *= 1.12f;
+        if (!plan.tile || us < best) {
+          plan.tile = true;
+          plan.columns = columns;
+          plan.two = kFormTwo[form];
+          plan.splits = s;
+          best = us;
+          best_form = form;
+        }
+      }
     }
   }
-  return best;
+  // the persistent layouts: 256 columns shared by two CTAs, 128, 64
+  if (plan.tile && !plain && (tiles_of(best_form) <= sms / (plan.two ? 2 : 1)) && (min_ki < 64 || plan.splits * (plan.two ? 2 : 1) * tiles_of(best_form) * 2 > sms)) return 0;
+  static const float persistent_us[kPairKinds][kForms] = {{0.53f, 0.0f, 0.49f, 0.40f}, {0.72f, 0.0f, 0.60f, 0.55f}, {0.76f, 0.0f, 0.81f, 0.82f},
+                                                          {1.01f, 0.0f, 1.00f, 0.92f}, {0.62f, 0.0f, 0.53f, 0.45f}, {0.88f, 0.0f, 0.67f, 0.55f}};
+  static const float plain_us[kForms] = {7.7f, 0.0f, 1.6f, 0.5f}, activation_us[kForms] = {23.1f, 0.0f, 6.2f, 3.3f}, partial_us[kForms] = {7.8f, 0.0f, 0.5f, 0.0f};
+  const float* const whole_us = plain ? plain_us : activation_us;
+  int columns = g.N <= 64 ? 64 : g.N <= 128 ? 128 : 256;
+  float classic = 0.0f;
+  for (int form = 0; form < kForms; form++) {
+    if (form == 1) continue;
+    const int bn = kFormColumns[form];
+    if (g.N <= 128 ? bn != columns : bn < 256 && (wide_only || g.odd || g_split_mode != 0 || (all16 && !plain))) continue;
+    if (g_tile_columns && g.N > 128 && !wide_only && bn != g_tile_columns) continue;
+    const long ctas = (long)((kFormTwo[form] && g.M > BM) ? 2 : 1) * tiles_of(form);
+    const int splits = ctas < sms && min_ki >= 8 ? splits_of((int)ctas, min_ki) : 1;
+    float us = 0.0f;
+    for (int i = 0; i < pairs; i++) us += blocks[i] * persistent_us[kind[i]][form];
+    const float waves = (float)((ctas * splits + sms - 1) / sms), end = splits > 1 ? partial_us[form] : whole_us[form];
+    if (waves > 1.0f && !plain && form == 0) {   // an activation runs beside the next tile's k-blocks
+      const bool planes_only = !e.out && !e.sample;
+      const float act = planes_only ? 10.0f : 20.8f + (draw ? 13.0f : 0.0f) + (aux ? 12.7f : 0.0f);
+      us = 4.3f + waves * (us > act ? us : act) + act;
+    } else {
+      us = 4.3f + waves * (us / splits + end);
+    }
+    if (splits > 1) us += 3.3f + 0.27f * splits + 1.4e-6f * g.M * g.N * (splits + 1);   // the finishing launch
+    // (a narrower tile has to come out ahead)
+    if (classic == 0.0f || us < 0.97f * classic) {
+      columns = bn;
+      classic = us;
+    }
+  }
+  // (a draw between the two goes to the persistent layout: it keeps the routes it had)
+  if (plan.tile && (best < 0.95f * classic || g_split_mode > 1)) return 0;
+  plan.tile = false;
+  plan.columns = columns;
+  plan.two = columns == 256 && g.M > BM && pairs_allowed;
+  return 0;
 }
 
 int gemm_tc(const GemmProblem& g) {
@@ -1608,8 +1949,7 @@ int gemm_tc(const GemmProblem& g) {
   const bool scatter = g_scatter_n > 0 && g.epi.out != nullptr && g.epi.out == g_scatter_match;
   if (!gemm_tc_supported(g))
     return scatter ? set_error("a product whose result is scattered to peers must run on the tensor cores") : ERROR_UNSUPPORTED;
-  const int BN = tile_columns(g);
-  g_last_columns = BN;
+
   static int pair_mode = -1;   // B200_GEMM_2CTA=0 keeps one CTA per tile
   static int chunk_k = 0;
   if (pair_mode < 0) {
@@ -1618,9 +1958,6 @@ int gemm_tc(const GemmProblem& g) {
     const char* c = getenv("B200_CHUNK_K");
     chunk_k = c ? atoi(c) : 0;
   }
-  // pairs of CTAs (cta_group::2) on 256-row tiles when the product has at least two row tiles
-  const bool two = pair_mode != 0 && BN == 256 && g.M > BM;
-  const int BN_LOCAL = two ? BN / 2 : BN;      // rows of B staged per CTA
   // Elements of K per k-block: 32 (one 128-byte swizzle row of floats; 16 doubles the stage count but
   // measured slower: 64-byte rows, twice the MMA and TMA issues).  When every term reads 16-bit planes
   // from aux matrices (no fp32 tile, nothing derived) a k-block is 64 elements: again 128-byte rows,
@@ -1636,6 +1973,13 @@ int gemm_tc(const GemmProblem& g) {
     all16 = part_is_16bit(ps.a.part) && part_is_16bit(ps.b.part) && ps.a.aux && ps.b.aux;
   }
   const int bk = all16 ? 64 : 32;
+  TcPlan plan = {256, false, false, 1};
+  const int plan_err = choose_plan(g, all16, pair_mode != 0, plan);
+  if (plan_err) return plan_err;
+  const int BN = plan.columns;
+  const bool two = plan.two;
+  const int BN_LOCAL = two ? BN / 2 : BN;      // rows of B staged per CTA
+  g_last_columns = BN;
   TcParams p;
   p.M = g.M;
   p.N = g.N;
@@ -1769,6 +2113,7 @@ int gemm_tc(const GemmProblem& g) {
     g_inject_stage_bytes = 0;
   }
   p.ngroups = ngroups;
+  p.nloads = nmaps;
   p.direct = 1;
   for (int gi = 0; gi < ngroups; gi++)
     if (p.group[gi].nconv > 0) p.direct = 0;
@@ -1791,7 +2136,7 @@ int gemm_tc(const GemmProblem& g) {
   // Tiles narrower than the widest are the ones that were cut along K more often, into shorter sums: 128 products keep their
   // error where it was or below (500 x 2048, K = 784 behind a logistic: 4.2e-7 as cut wide tiles, 6.3e-7 with 2048), and the
   // drain of 32 or 64 columns fits between two chunks.
-  const bool narrow = BN < 256 && g.N > 128;
+  const bool narrow = plan.tile || (BN < 256 && g.N > 128);
   const int ck = chunk_k >= 16 ? chunk_k : narrow && !odd ? 128 : odd ? (g.epi.activation == 1 ? 128 : 32) : (g.epi.activation == 1 ? 2048 : 128);
   p.chunk_iters = ck / bk < 1 ? 1 : ck / bk;
 
@@ -1819,6 +2164,10 @@ int gemm_tc(const GemmProblem& g) {
       want = g_split_mode < min_ki ? g_split_mode : min_ki;
     }
     if (scatter) want = 1;   // a partial is not a result: the panels go out whole
+    if (plan.tile) {
+      p.splits = plan.splits;
+      want = 1;
+    }
     float* ws = nullptr;
     if (want > 1) {
       if (!odd || !stream_capturing()) ws = (float*)workspace(2, (size_t)want * g.M * g.N * sizeof(float));
@@ -1845,7 +2194,9 @@ int gemm_tc(const GemmProblem& g) {
   }
   const GemmEpilogue& e = p.epi;
   int epi = kEpiGeneric;
-  if (!e.bias && e.activation == 0 && !e.sample && !e.out_aux && !e.sample_aux && e.out) {
+  if (plan.tile) {
+    epi = kEpiTile;
+  } else if (!e.bias && e.activation == 0 && !e.sample && !e.out_aux && !e.sample_aux && e.out) {
     epi = p.splits > 1 ? kEpiPartial : kEpiPlain;
   } else if (e.bias && !e.col_scale && e.beta == 0.0f && (e.out || e.sample || e.out_aux || e.sample_aux)) {
     if (e.activation == 1 && (e.sample || e.sample_aux)) epi = kEpiSigSample;
@@ -1865,12 +2216,12 @@ int gemm_tc(const GemmProblem& g) {
     const char* sv = getenv("B200_EPI_STORE16");
     store16_mode = sv ? atoi(sv) : 1;
   }
-  p.direct_store = !epi_is_plain(epi) &&
+  p.direct_store = !epi_is_plain(epi) && epi != kEpiTile &&
                    (!tma_outputs_ok(e) || (store16_mode != 0 && !e.out && !e.sample && (e.out_aux || e.sample_aux)) ||
                     // a CTA with one tile has no next one whose first chunk waits: 18 600 clocks against 26 500 staged
                     (BN == 128 && g.N > 128 && (long)((g.M + BM - 1) / BM) * ((g.N + BN - 1) / BN) <= sm_count()));
   for (int i = 0; i < kOutArrays; i++) p.out_map[i] = -1;
-  if (!epi_is_plain(epi) && !p.direct_store) {
+  if (!epi_is_plain(epi) && epi != kEpiTile && !p.direct_store) {
     // outputs of the activation epilogues, stored as boxes of 128 rows x 4 columns: M x N floats
     // with columns ldo apart, or one bfloat16 plane of an aux matrix (columns 2 ld_aux bfloat16
     // apart, plane 1 starting ld_aux bfloat16 into the column)
@@ -1896,6 +2247,8 @@ int gemm_tc(const GemmProblem& g) {
     default: return launch_tc<BNV, kEpiGeneric, TWO>(p);              \
   }
   auto launch = [&]() -> int {
+    if (epi == kEpiTile)
+      return two && BN == 128 ? launch_tc<128, kEpiTile, true>(p) : two ? launch_tc<256, kEpiTile, true>(p) : BN == 128 ? launch_tc<128, kEpiTile, false>(p) : launch_tc<64, kEpiTile, false>(p);
     if (BN == 256 && two) { B200_TC_CASE(256, true) }
     if (BN == 256) { B200_TC_CASE(256, false) }
     if (BN == 128) { B200_TC_CASE(128, false) }
@@ -1911,7 +2264,7 @@ int gemm_tc(const GemmProblem& g) {
 #else
   const int err = launch();
 #endif
-  if (err || p.splits == 1) return err;
+  if (err || p.splits == 1 || epi == kEpiTile) return err;
   const long items = (long)g.M * ((g.N + 3) / 4);
   long blocks = (items + 255) / 256;
   if (blocks > (long)sm_count() * 8) blocks = (long)sm_count() * 8;

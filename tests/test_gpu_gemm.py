@@ -975,6 +975,56 @@ def test_narrow_tiles_of_products_of_few_tiles(cm, M, N, K, two_pairs, columns):
     assert cm.read_status() == 0
 
 
+@pytest.mark.parametrize("columns", [64, 128, 256])
+@pytest.mark.parametrize("splits", [0, 2, 3, 7])
+@pytest.mark.parametrize("M,N,K", [(130, 129, 900), (257, 260, 1024), (1001, 515, 904), (516, 1029, 900)])
+def test_one_work_item_per_cta(cm, M, N, K, splits, columns):
+    """Tiles that end in shared memory, K cut over a cluster or not: ragged rows (columns of the result that start on no
+    16 bytes) and ragged columns, every output and option of the epilogue, both forms of the 16-bit planes.  Bound: sums of K
+    products in chunks of 128 at 2^-18 a term, 1e-5 of the largest result; draws and planes follow from the result exactly."""
+    rng = np.random.default_rng(M + K + splits)
+    w = (rng.standard_normal((K, M)) * 0.05).astype(np.float32)
+    x = rng.random((K, N)).astype(np.float32)
+    b, c = rng.standard_normal((M, 1)).astype(np.float32), rng.random((1, N)).astype(np.float32)
+    add = rng.standard_normal((M, N)).astype(np.float32)
+    W, X = cm.CUDAMatrix(w), cm.CUDAMatrix(x)
+    scale = cm.f16_scale_state(np.abs(w).max())
+    wf, xf = W.split_f16(cm.empty_aux(w.shape), exp_dev=scale.slice(0, 1)), X.split_f16(cm.empty_aux(x.shape), exp_const=14)
+    out, aux, smp, smp_aux, plain, scaled, draw = (cm.empty((M, N)), cm.empty_aux((M, N)), cm.empty((M, N)), cm.empty_aux((M, N)),
+                                                   cm.empty((M, N)), cm.empty((M, N)), cm.empty((M, N)))
+    bias = cm.CUDAMatrix(b)
+    cm.CUDAMatrix.init_random(5)
+    cm.set_gemm_path(1)
+    cm._lib.b200_test_tile_columns(columns)
+    cm.set_split_k(splits)
+    try:
+        cm.fused_gemm(cm.f16_passes(W.T, wf, X, xf), out=out, out_aux=aux, sample=smp, sample_aux=smp_aux, bias=bias, activation=1,
+                      scale_exp=scale.slice(0, 1), scale_exp_const=14, aux_f16=True, aux_exp=14)
+        cm.fused_gemm(cm.split_passes(W.T, X, terms="tf32"), out=plain, add=cm.CUDAMatrix(add))
+        cm.fused_gemm(cm.split_passes(W.T, X), out=scaled, sample=draw, bias=bias, col_scale=cm.CUDAMatrix(c), activation=1)
+    finally:
+        cm.set_gemm_path(0)
+        cm.set_split_k(0)
+        cm._lib.b200_test_tile_columns(0)
+    pre = w.T.astype(np.float64) @ x
+    sig = lambda z: 1 / (1 + np.exp(-z))
+    got = get(out)
+    assert np.abs(got - sig(pre + b)).max() < 1e-5
+    assert np.abs(get(plain) - pre - add).max() < 1e-5 * np.abs(pre).max()
+    assert np.abs(get(scaled) - sig(pre + b * c)).max() < 1e-5
+    cm.CUDAMatrix.init_random(5)
+    for probs, draws in ((got, get(smp)), (get(scaled), get(draw))):
+        again = cm.empty((M, N))
+        cm.CUDAMatrix(probs).sample_bernoulli(target=again)
+        np.testing.assert_array_equal(draws, get(again))
+    lo, hi = f16_planes(aux)
+    want_hi = (got * np.float32(2.0 ** 14)).astype(np.float16).astype(np.float32)
+    np.testing.assert_array_equal(hi, want_hi)
+    np.testing.assert_array_equal(lo, (got * np.float32(2.0 ** 14) - want_hi).astype(np.float16).astype(np.float32))
+    np.testing.assert_array_equal(f16_planes(smp_aux)[1], get(smp) * 2.0 ** 14)
+    assert cm.read_status() == 0
+
+
 @pytest.mark.parametrize("M,N,K,columns", [(784, 1000, 1024, 256), (4096, 132, 1024, 256), (512, 1024, 2048, 256), (500, 500, 500, 64)])
 def test_products_bound_by_the_converters_keep_wide_tiles(cm, M, N, K, columns):
     """A difference of two products whose parts the kernel derives: 784 x 1000, K = 1024 takes 37 us on tiles of 256 columns and 44
