@@ -863,10 +863,13 @@ class Immediate(object):
         _check(_lib.bias_updates(ct.byref(_build_bias_layers(layers, sq_acc)), ct.c_float(inv_batch), ct.c_float(momentum),
                                  ct.c_float(eps)))
 
-    def update_all(self, layers, w, delta, suff, w_aux, inv_batch, mom_b, eps_b, mom_w, eps_w, l2=0.0, l1=0.0, sq_acc=None):
-        """`bias_updates` of the layers and `momentum_update` of w with its bfloat16 parts, in one launch."""
-        _check(_lib.update_all(ct.byref(_build_bias_layers(layers, sq_acc)), w.p_mat, delta.p_mat, suff.p_mat, w_aux.p_mat,
-                               *(ct.c_float(x) for x in (inv_batch, mom_b, eps_b, mom_w, eps_w, l2, l1))))
+    def update_all(self, layers, w, delta, suff, w_aux, inv_batch, mom_b, eps_b, mom_w, eps_w, l2=0.0, l1=0.0, sq_acc=None,
+                   w_scale=None):
+        """`bias_updates` of the layers and `momentum_update` of w with its bfloat16 parts (with w_scale: its scaled
+        half-precision form), in one launch."""
+        _check(_lib.update_all_scaled(ct.byref(_build_bias_layers(layers, sq_acc)), w.p_mat, delta.p_mat, suff.p_mat, w_aux.p_mat,
+                                      w_scale.p_mat if w_scale is not None else None,
+                                      *(ct.c_float(x) for x in (inv_batch, mom_b, eps_b, mom_w, eps_w, l2, l1))))
 
     def rbm_bias_update(self, v_pos, v_neg, h_pos, h_neg, suff, b, db, sq_acc, inv_batch, momentum, eps):
         _check(_lib.rbm_bias_update(v_pos.p_mat, v_neg.p_mat, h_pos.p_mat, h_neg.p_mat, suff.p_mat, b.p_mat, db.p_mat,
@@ -995,11 +998,12 @@ class Program(object):
         self._keep.append(sq_acc)
         return self._add(OP_BIAS_UPDATES, (), (), (inv_batch, momentum, eps), gemm=_build_bias_layers(layers, sq_acc))
 
-    def update_all(self, layers, w, delta, suff, w_aux, inv_batch, mom_b, eps_b, mom_w, eps_w, l2=0.0, l1=0.0, sq_acc=None):
+    def update_all(self, layers, w, delta, suff, w_aux, inv_batch, mom_b, eps_b, mom_w, eps_w, l2=0.0, l1=0.0, sq_acc=None,
+                   w_scale=None):
         for mats in layers:
             self._keep.extend(mats)
         self._keep.append(sq_acc)
-        return self._add(OP_UPDATE_ALL, (w, delta, suff, w_aux), (), (inv_batch, mom_b, eps_b, mom_w, eps_w, l2, l1),
+        return self._add(OP_UPDATE_ALL, (w, delta, suff, w_aux, w_scale), (), (inv_batch, mom_b, eps_b, mom_w, eps_w, l2, l1),
                          gemm=_build_bias_layers(layers, sq_acc))
 
     def rbm_bias_update(self, v_pos, v_neg, h_pos, h_neg, suff, b, db, sq_acc, inv_batch, momentum, eps):

@@ -30,8 +30,8 @@ int dp_peer_update(cudamat* w, cudamat* delta, cudamat* w_aux, cudamat* w_scale,
 int rbm_bias_update(cudamat* v_pos, cudamat* v_neg, cudamat* h_pos, cudamat* h_neg, cudamat* suff, cudamat* b, cudamat* db,
                     cudamat* sq_acc, float inv_batch, float momentum, float eps);
 int bias_updates(b200_bias_layers* t, float inv_batch, float momentum, float eps);
-int update_all(b200_bias_layers* t, cudamat* w, cudamat* delta, cudamat* suff, cudamat* w_aux, float inv_batch, float mom_b,
-               float eps_b, float mom_w, float eps_w, float l2, float l1);
+int update_all_scaled(b200_bias_layers* t, cudamat* w, cudamat* delta, cudamat* suff, cudamat* w_aux, cudamat* w_scale,
+                      float inv_batch, float mom_b, float eps_b, float mom_w, float eps_w, float l2, float l1);
 int split_f16(cudamat* x, cudamat* aux, cudamat* exp_dev, int exp_const);
 int split_bf16(cudamat* x, cudamat* aux);
 int dp_allreduce(cudamat* mat);
@@ -75,7 +75,7 @@ enum {
   B200_OP_SOFTMAX_RECONSTRUCTION = 23,   // m0 pre, m1 nn, m2 state, m3 norm, m4 data?, m5 acc?
   B200_OP_DOCUMENT_LENGTHS = 24,  // m0 counts, m1 nn, m2 norm, f0 tiny
   B200_OP_BIAS_UPDATES = 25,      // gemm points to a b200_bias_layers; f0 inv_batch, f1 momentum, f2 eps
-  B200_OP_UPDATE_ALL = 26,        // the same, m0 w, m1 delta, m2 suff, m3 w_aux; f0 inv_batch, f1 mom_b, f2 eps_b, f3 mom_w, f4 eps_w, f5 l2, f6 l1
+  B200_OP_UPDATE_ALL = 26,        // the same, m0 w, m1 delta, m2 suff, m3 w_aux, m4 w_scale?; f0 inv_batch, f1 mom_b, f2 eps_b, f3 mom_w, f4 eps_w, f5 l2, f6 l1
   B200_OP_SIGMOID = 27,           // m0 mat, m1 target
   B200_OP_COUNT
 };
@@ -131,7 +131,7 @@ extern "C" int b200_run_program(rnd_struct* rnd_state, b200_op* ops, int n, int*
       case B200_OP_BIAS_UPDATES: err = bias_updates(reinterpret_cast<b200_bias_layers*>(o.gemm), o.f0, o.f1, o.f2); break;
       case B200_OP_SIGMOID: err = apply_sigmoid(o.m[0], o.m[1]); break;
       case B200_OP_UPDATE_ALL:
-        err = update_all(reinterpret_cast<b200_bias_layers*>(o.gemm), o.m[0], o.m[1], o.m[2], o.m[3], o.f0, o.f1, o.f2, o.f3, o.f4, o.f5, o.f6);
+        err = update_all_scaled(reinterpret_cast<b200_bias_layers*>(o.gemm), o.m[0], o.m[1], o.m[2], o.m[3], o.m[4], o.f0, o.f1, o.f2, o.f3, o.f4, o.f5, o.f6);
         break;
       default: break;
     }

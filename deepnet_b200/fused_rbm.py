@@ -95,12 +95,14 @@ class FusedRBM(LossReadback):
         # ... and for the states only when the products are big: a small model is bound by launch
         # latency, where the extra split launch and the wider epilogue cost more than they save
         env = os.environ.get("B200_RBM_STATE_AUX")
-        self.state_aux = (V * H * batchsize >= 1 << 32) if env is None else env != "0"
+        big = V * H * batchsize >= 1 << 32
+        # the half-precision form below serves every model but the small ones (and, over several ranks, the big ones)
+        f16_ok = binary_data and visible == LOGISTIC and os.environ.get("B200_RBM_F16", "1") != "0"
+        self.state_aux = big or (f16_ok and world_size == 1 and self._planes_pay()) if env is None else env != "0"
         # With 0/1 data and logistic units every operand's range is known, and the big products run
         # on the scaled half-precision form of W and of the states (three fp16 terms, no TF32 term,
         # no fp32 operand read): W * 2^e with e kept by the update kernel, states * 2^14.
-        self.f16 = (self.state_aux and binary_data and visible == LOGISTIC
-                    and os.environ.get("B200_RBM_F16", "1") != "0")
+        self.f16 = self.state_aux and f16_ok
         if self.f16:
             self.W_scale = cm.f16_scale_state(float(np.abs(w).max()))
             self.W_exp = self.W_scale.slice(0, 1)
@@ -166,6 +168,15 @@ class FusedRBM(LossReadback):
         self._batch = cm.CUDAMatrix._from_mat(cm.cudamat())   # the recorded step's view of the current minibatch
         self._batch_aux = cm.CUDAMatrix._from_mat(cm.cudamat())   # ... and of its 16-bit parts, when the caller has them
         self._given_aux = None
+
+    def _planes_pay(self):
+        """Whether the products come off better on half-precision planes (tcgen05, no fp32 operand read) than in one launch or
+        with parts derived in the kernel, by what an update costs (us, CD-1 / CD-3, planes against the better of the others):
+        784 x 500, 100 cases 50.3 / 49.1, 87 / 91; 250 cases 57 / 64, 97 / 117; 1000 x 200, 100 cases 48 / 44, 85 / 91; 1357 x 601,
+        203 cases 62 / 114, 105 / 228; 2048 x 2048, 512 cases 123 / 135, 193 / 242; 784 x 500, 20 cases 47 / 41, 87 / 79.  The
+        split of the minibatch is what the smaller ones lose, once an update."""
+        work = self.V * self.H * self.B
+        return work >= 1 << 26 or (self.hyp.gibbs_steps > 1 and work >= 1 << 24)
 
     def _act(self, layer_activation):
         return 1 if layer_activation == LOGISTIC else 0
@@ -257,7 +268,7 @@ class FusedRBM(LossReadback):
             layers = [(bias[0], bias[1], self.suff_bv, self.bv, self.dbv), (self.h_pos, self.h_neg, self.suff_bh, self.bh, self.dbh)]
             u = self._op(X, "update", 0, 8.0 * (V + H) * self.B + 6 * wb, "update_all", layers, self.W, self.dW, self.suff_W,
                          self.W_aux, sc["inv_b"], sc["mom"], sc["eps"], sc["emom"], sc["eeps"], l2=sc["l2"], l1=sc["l1"],
-                         sq_acc=bias[2])
+                         sq_acc=bias[2], w_scale=w_scale)
             if self.B > 1024:      # past that the operation is made of its separate launches
                 self.kernel_launches += 5 if bias[2] is not None else 4
             return ("update", u), None
@@ -333,12 +344,13 @@ class FusedRBM(LossReadback):
         gf = 2.0 * V * H * B
         vb, hb, wb = 4.0 * V * B, 4.0 * H * B, 4.0 * V * H
         act = dict(scale_exp=We, scale_exp_const=E, aux_f16=True, aux_exp=E)
+        # statistics stay here: biases, weights and their planes in one operation (past 1024 cases it would be made of its parts)
+        tail = self.world_size == 1 and not self.dp_peer and B <= 1024
         if self._given_aux is None:
             self._op(X, "split", 0, 2 * vb, "split_f16", v0, v0a, None, E)
         # positive phase: h0 = sigmoid(W' v0 + b_h), its Bernoulli sample, and the parts of both
-        self._op(X, "gemm_up", gf, 3.5 * hb, "fused_gemm", F(W.T, Wa, v0, v0a, exact_b=True), out=self.h_pos,
-                 out_aux=self.h_pos_aux, sample=self.h_samp, sample_aux=self.h_samp_aux, bias=self.bh, activation=1,
-                 **act)
+        self._op(X, "gemm_up", gf, 2.5 * hb, "fused_gemm", F(W.T, Wa, v0, v0a, exact_b=True), out=self.h_pos,
+                 out_aux=self.h_pos_aux, sample_aux=self.h_samp_aux, bias=self.bh, activation=1, **act)
         for i in range(k):
             last = i == k - 1
             # the fp32 visible means are read by the error of the first reconstruction and by the
@@ -347,8 +359,9 @@ class FusedRBM(LossReadback):
             self._op(X, "gemm_down", gf, 2 * vb, "fused_gemm", F(W, Wa, self.h_samp, self.h_samp_aux, exact_b=True),
                      out=self.v_neg if (i == 0 or last) else None,
                      out_aux=self.v_neg_aux if (last or not draw_v) else None,
-                     sample_aux=self.v_samp_aux if draw_v else None, bias=self.bv, activation=1, **act)
-            if i == 0:
+                     sample=self.v_samp if draw_v and last and tail else None, sample_aux=self.v_samp_aux if draw_v else None,
+                     bias=self.bv, activation=1, **act)
+            if i == 0 and not (tail and k == 1):
                 self._op(X, "sq_err", 0, 2 * vb, "sq_diff", self.v_neg, v0, self.loss_acc)
             # the hidden means (and their parts) are only read after the last step, by the statistics
             # (the next product reads the draw's half-precision plane; the fp32 draw is kept for the caller)
@@ -372,6 +385,8 @@ class FusedRBM(LossReadback):
             pos = F(v0, v0a, self.h_pos.T, self.h_pos_aux, exact_a=True)
             neg = F(self.v_neg, self.v_neg_aux, self.h_neg.T, self.h_neg_aux, negate=1)
             self._op(X, "gemm_stats", 2 * gf, wb, "fused_gemm", pos + neg, out=self.suff_W, scale_exp_const=2 * E)
+            if tail:
+                return self._issue_updates(X, sc, wb, w_scale=self.W_scale, bias=(v0, self.v_neg, self.loss_acc if k == 1 else None))
             self._op(X, "row_sum", 0, 2 * vb, "row_sum_diff", v0, self.v_neg, self.suff_bv)
             self._op(X, "row_sum", 0, 2 * hb, "row_sum_diff", self.h_pos, self.h_neg, self.suff_bh)
             self.kernel_launches += 2                  # the exponent launch and the pass that writes W's aux

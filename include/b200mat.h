@@ -339,7 +339,7 @@ int b200_rows_add(cudamat* src, float* dst);
 int b200_rows_end(void);
 /* Bias statistics (suff = row sums of pos - neg) and bias update of up to four layers in one launch; sq_acc (optional) += squared
  * difference of the first layer's states.  update_all: the same and momentum_update of a weight matrix with its bfloat16
- * parts, in one launch. */
+ * parts, in one launch; update_all_scaled: with w_scale (see momentum_update) its scaled half-precision form instead. */
 typedef struct b200_bias_layers {
   cudamat *pos[4], *neg[4], *suff[4], *b[4], *db[4], *sq_acc;
   int layers;
@@ -347,6 +347,8 @@ typedef struct b200_bias_layers {
 int bias_updates(b200_bias_layers* t, float inv_batch, float momentum, float eps);
 int update_all(b200_bias_layers* t, cudamat* w, cudamat* delta, cudamat* suff, cudamat* w_aux, float inv_batch, float mom_b,
                float eps_b, float mom_w, float eps_w, float l2, float l1);
+int update_all_scaled(b200_bias_layers* t, cudamat* w, cudamat* delta, cudamat* suff, cudamat* w_aux, cudamat* w_scale,
+                      float inv_batch, float mom_b, float eps_b, float mom_w, float eps_w, float l2, float l1);
 /* Bias statistics, bias update and (sq_acc, optional) squared reconstruction error of an RBM with packed biases
  * [visible | hidden] in one launch (deepnet/layer.py:202-213, parameter.py:80-106, logistic_layer.py:48-52). */
 int rbm_bias_update(cudamat* v_pos, cudamat* v_neg, cudamat* h_pos, cudamat* h_neg, cudamat* suff, cudamat* b, cudamat* db,

@@ -678,6 +678,73 @@ def test_updates_in_one_launch_match_the_separate_calls(cm, sizes, B, rows):
     assert abs(results[0][2] - results[1][2]) <= 1e-6 * results[1][2]
 
 
+@pytest.mark.parametrize("rows", [64, 37])
+@pytest.mark.parametrize("growth", [0.0, 1.0, 1000.0, -1.0])
+def test_updates_in_one_launch_keep_the_exponent_of_the_planes(cm, rows, growth):
+    """The scaled half-precision planes written by the launch that updates everything: bit for bit those of momentum_update,
+    over two updates, where the exponent stays, where the weights outgrow it (every plane rewritten) and where they vanish."""
+    rng = np.random.default_rng(rows)
+    f = lambda *s: rng.standard_normal(s).astype(np.float32)
+    B, n = 20, 45
+    layers_h = [(f(rows, B), f(rows, B), f(rows, 1), f(rows, 1)), (f(n, B), f(n, B), f(n, 1), f(n, 1))]
+    w = f(rows, n)
+    d = -w if growth < 0 else growth * f(rows, n)          # -1: the update takes the weights away
+    g = np.zeros_like(w) if growth < 0 else f(rows, n)
+    X, results = cm.Immediate(), []
+    for fused in (True, False):
+        layers = [(cm.CUDAMatrix(p), cm.CUDAMatrix(q), cm.empty((p.shape[0], 1)), cm.CUDAMatrix(b), cm.CUDAMatrix(db))
+                  for p, q, b, db in layers_h]
+        W, D, S = cm.CUDAMatrix(w), cm.CUDAMatrix(d), cm.CUDAMatrix(g)
+        scale = cm.f16_scale_state(np.abs(w).max())
+        aux = W.split_f16(cm.empty_aux((rows, n)), exp_dev=scale.slice(0, 1))
+        for _ in range(2):
+            if fused:
+                X.update_all(layers, W, D, S, aux, 1.0 / B, 0.5, 0.1, 1.0, -1.0 if growth < 0 else 0.2, w_scale=scale)
+            else:
+                X.momentum_update(W, D, None, S, 1.0 / B, 1.0, -1.0 if growth < 0 else 0.2, w_aux=aux, w_scale=scale)
+        results.append([get(W), get(D)] + list(_f16_planes(aux)) + [get(scale)[:, :3]])
+    for a, b in zip(*results):
+        np.testing.assert_array_equal(a, b)
+    if growth > 1:
+        assert results[0][4][0, 0] < cm.f16_scale_state(np.abs(w).max()).asarray()[0, 0]
+    e = results[0][4][0, 0]
+    np.testing.assert_array_equal(results[0][3], (results[0][0] * np.float32(2.0) ** e).astype(np.float16).astype(np.float32))
+
+
+@pytest.mark.parametrize("V,H,B,gibbs,sample", [(301, 203, 78, 1, False), (130, 67, 1030, 2, False), (97, 515, 33, 3, True)])
+def test_half_precision_engine_on_odd_models_matches_oracle(cm, oracle, V, H, B, gibbs, sample, monkeypatch):
+    """Odd layers and batches on half-precision planes (the update in one launch, and past 1024 cases in its parts): draws bit
+    for bit, parameters and states to 1e-5 of the largest."""
+    monkeypatch.setenv("B200_RBM_STATE_AUX", "1")
+    rng = np.random.default_rng(V)
+    hyp = dbm.Hyperparams(base_epsilon=0.05, initial_momentum=0.5, final_momentum=0.9, momentum_change_steps=10, gibbs_steps=gibbs,
+                          sample_input=sample)
+    w = (0.05 * rng.standard_normal((V, H))).astype(np.float32)
+    x = (rng.random((V, 2 * B)) < 0.3).astype(np.float32)
+    edge = hyp.copy(apply_l2_decay=True, l2_decay=2e-4)
+    layers = [dict(name="v", activation=dbm.LOGISTIC, numdims=V, is_input=True), dict(name="h", activation=dbm.LOGISTIC, numdims=H)]
+    ref = dbm.DBM(oracle, layers, [dict(node1="v", node2="h", weight=w, hyperparams=edge)], hyp, B, dbm.CD, seed=9)
+    eng = FusedRBM(cm, V, H, B, w, hyp, edge_hyperparams=edge, binary_data=True, seed=9)
+    assert eng.f16
+    xo, xg = oracle.CUDAMatrix(x), cm.CUDAMatrix(x)
+    for step in range(3):
+        s = (step % 2) * B
+        ref.SetBatch([xo.slice(s, s + B)])
+        want = ref.TrainOneBatch(step)[0]
+        eng.TrainOneBatch(step, xg.slice(s, s + B))
+        np.testing.assert_allclose(eng.read_loss(), want, rtol=1e-5)
+    assert relerr(get(eng.W), get(ref.edge[0].params["weight"])) < TOL
+    assert relerr(get(eng.dW), get(ref.edge[0].gradient_history)) < 2 * TOL
+    assert relerr(get(eng.v_neg), get(ref.GetLayerByName("v").state)) < TOL
+    assert relerr(get(eng.h_neg), get(ref.GetLayerByName("h").state)) < TOL
+    np.testing.assert_array_equal(get(eng.h_samp), get(ref.GetLayerByName("h").sample))
+    if sample and B <= 1024:
+        np.testing.assert_array_equal(get(eng.v_samp), get(ref.GetLayerByName("v").sample))
+    for mine, theirs in ((eng.bv, "v"), (eng.bh, "h")):
+        assert relerr(get(mine), get(ref.GetLayerByName(theirs).params["bias"])) < TOL
+    assert cm.read_status() == 0
+
+
 def test_representations_leave_while_the_next_minibatch_is_computed(cm):
     """Several pieces a minibatch and a ragged last one, an even and an odd number of minibatches, and the staging area taken by
     someone else (plain copies): the rows are the products', bit for bit."""
