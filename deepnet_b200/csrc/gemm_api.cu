@@ -260,10 +260,11 @@ __device__ __forceinline__ void update_one(float& w, float& d, float g, float su
 // What ends an update beside the weights, in one launch: for every unit r of up to four layers
 //   suff[r] = sum_c pos[r, c] - neg[r, c]   (deepnet/layer.py:202-213), then the parameter update of the biases,
 // and, with `acc`, acc[0] += sum (pos - neg)^2 of the first, the reconstruction error of deepnet/logistic_layer.py:48-52
-// (the visible rows are being read anyway).  A block owns 32 rows whole (8 lanes of columns, folded in order), so the sums
-// need no second pass; the error's partial sums (doubles) are folded by the block that finishes last, in order.
-// Latency bound at the sizes it is used for.  Four launches before: 784 + 500 units, 100 cases: 10.6 -> 4 us.
-constexpr int kTailLanes = 8;
+// (the visible rows are being read anyway).  A block owns 32 rows whole (32 lanes of cases, four rows a thread, folded in
+// order), so the sums need no second pass; the error's partial sums (doubles) are folded by the block that finishes last, in
+// order.  Latency bound at the sizes it is used for.  Four launches before: 784 + 500 units, 100 cases: 10.6 -> 4 us; with 8
+// lanes of cases and one row a thread the walk over 512 cases stood behind the weights' blocks (2048 x 2048: 22.2 -> 13.9 us).
+constexpr int kTailLanes = 32, kTailThreads = 8 * kTailLanes;
 constexpr int kTailLayers = 4;
 struct TailLayer {
   const float *pos, *neg;
@@ -279,75 +280,93 @@ struct TailArgs {
 };
 __device__ __forceinline__ void bias_tail(const TailArgs& a) {
   __shared__ float sums[kTailLanes][33];
-  __shared__ double sq[kTailLanes];
+  __shared__ double sq[kTailThreads / 32];
   __shared__ bool is_last;
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5, cases = a.cases;
+  const int tx = threadIdx.x & 7, ty = threadIdx.x >> 3, cases = a.cases;
   int which = 0;
   while (which + 1 < a.layers && (int)blockIdx.x >= a.l[which + 1].block0) which++;
   const TailLayer l = a.l[which];
-  const int r = 32 * ((int)blockIdx.x - l.block0) + tx;
+  const int r0 = 32 * ((int)blockIdx.x - l.block0), r = r0 + 4 * tx;
   const bool err = which == 0 && a.acc != nullptr;
   const int err_blocks = (a.l[0].rows + 31) / 32;
-  float s = 0.0f;
+  float s[4] = {0.0f, 0.0f, 0.0f, 0.0f};
   double e = 0.0;
+  const bool vec = l.rows % 4 == 0 && (((uintptr_t)l.pos | (uintptr_t)l.neg) & 15) == 0;
+  auto difference = [&](int c) {
+    const long o = (long)c * l.rows + r;
+    if (vec) {
+      const float4 p = *reinterpret_cast<const float4*>(l.pos + o), n = *reinterpret_cast<const float4*>(l.neg + o);
+      return make_float4(p.x - n.x, p.y - n.y, p.z - n.z, p.w - n.w);
+    }
+    return make_float4(l.pos[o] - l.neg[o], r + 1 < l.rows ? l.pos[o + 1] - l.neg[o + 1] : 0.0f,
+                       r + 2 < l.rows ? l.pos[o + 2] - l.neg[o + 2] : 0.0f, r + 3 < l.rows ? l.pos[o + 3] - l.neg[o + 3] : 0.0f);
+  };
+  auto add = [&](const float4& d) {
+    s[0] += d.x;
+    s[1] += d.y;
+    s[2] += d.z;
+    s[3] += d.w;
+    if (err) e += ((double)d.x * d.x + (double)d.y * d.y) + ((double)d.z * d.z + (double)d.w * d.w);
+  };
   if (r < l.rows) {
     int c = ty;
     for (; c + 3 * kTailLanes < cases; c += 4 * kTailLanes) {   // eight loads in flight
-      float d[4];
+      float4 d[4];
 #pragma unroll
-      for (int i = 0; i < 4; i++) {
-        const long o = (long)(c + i * kTailLanes) * l.rows + r;
-        d[i] = l.pos[o] - l.neg[o];
-      }
+      for (int i = 0; i < 4; i++) d[i] = difference(c + i * kTailLanes);
 #pragma unroll
-      for (int i = 0; i < 4; i++) s += d[i];
-      e += ((double)d[0] * d[0] + (double)d[1] * d[1]) + ((double)d[2] * d[2] + (double)d[3] * d[3]);
+      for (int i = 0; i < 4; i++) add(d[i]);
     }
-    for (; c < cases; c += kTailLanes) {
-      const long o = (long)c * l.rows + r;
-      const float d = l.pos[o] - l.neg[o];
-      s += d;
-      e += (double)d * d;
-    }
+    for (; c < cases; c += kTailLanes) add(difference(c));
   }
-  sums[ty][tx] = s;
+#pragma unroll
+  for (int i = 0; i < 4; i++) sums[ty][4 * tx + i] = s[i];
   if (err) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
-    if (tx == 0) sq[ty] = e;
+    if ((threadIdx.x & 31) == 0) sq[threadIdx.x >> 5] = e;
   }
   __syncthreads();
-  if (ty == 0 && r < l.rows) {
+  {
+    const int row = threadIdx.x & 31, first = threadIdx.x >> 5;   // lanes first, first + 8, ...
     float t = 0.0f;
 #pragma unroll
-    for (int j = 0; j < kTailLanes; j++) t += sums[j][tx];
-    l.suff[r] = t;
-    float w = l.b[r], d = l.db[r];
+    for (int j = 0; j < kTailLanes; j += 8) t += sums[first + j][row];
+    sums[first][row] = t;    // (the only thread that reads it before the barrier)
+  }
+  __syncthreads();
+  if (threadIdx.x < 32 && r0 + (int)threadIdx.x < l.rows) {
+    const int row = r0 + (int)threadIdx.x;
+    float t = 0.0f;
+#pragma unroll
+    for (int j = 0; j < 8; j++) t += sums[j][threadIdx.x];
+    l.suff[row] = t;
+    float w = l.b[row], d = l.db[row];
     update_one(w, d, 0.0f, t, a.ninv_batch, a.momentum, a.neps, 0.0f, 0.0f);
-    l.b[r] = w;
-    l.db[r] = d;
+    l.b[row] = w;
+    l.db[row] = d;
   }
   if (!err) return;
   if (threadIdx.x == 0) {
     double t = 0.0;
-    for (int j = 0; j < kTailLanes; j++) t += sq[j];
+    for (int j = 0; j < kTailThreads / 32; j++) t += sq[j];
     a.part[blockIdx.x] = t;
     __threadfence();
     is_last = atomicAdd(a.counter, 1u) == (unsigned)(err_blocks - 1);
   }
   __syncthreads();
-  if (!is_last || ty != 0) return;
+  if (!is_last || threadIdx.x >= 32) return;
   __threadfence();
   double t = 0.0;
-  for (int i = tx; i < err_blocks; i += 32) t += __ldcg(a.part + i);
+  for (int i = threadIdx.x; i < err_blocks; i += 32) t += __ldcg(a.part + i);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-  if (tx == 0) {
+  if (threadIdx.x == 0) {
     *a.acc += (float)t;
     *a.counter = 0u;
   }
 }
-__global__ void __launch_bounds__(32 * kTailLanes) k_bias_tail(const __grid_constant__ TailArgs a) {
+__global__ void __launch_bounds__(kTailThreads) k_bias_tail(const __grid_constant__ TailArgs a) {
   grid_dependents_launch();
   grid_dependency_wait();
   bias_tail(a);
@@ -427,7 +446,7 @@ extern "C" int bias_updates(b200_bias_layers* t, float inv_batch, float momentum
       err = momentum_update(t->b[i], t->db[i], nullptr, t->suff[i], nullptr, nullptr, inv_batch, momentum, eps, 0.0f, 0.0f);
     return err;
   }
-  if (launch_dependent(k_bias_tail, dim3((unsigned)blocks), dim3(32 * kTailLanes), 0, stream(), a) != cudaSuccess)
+  if (launch_dependent(k_bias_tail, dim3((unsigned)blocks), dim3(kTailThreads), 0, stream(), a) != cudaSuccess)
     return set_error(cudaGetErrorString(cudaGetLastError()));
   return check_launch();
 }
@@ -526,9 +545,19 @@ __device__ __forceinline__ void update_weights(float* w, float* delta, float* gr
       }
     }
   }
-  if (kAux == 2) {   // non-negative floats order like their bit patterns
+  if (kAux == 2) {
+    // Non-negative floats order like their bit patterns.  One atomic a block, and only by blocks that raise the maximum: one a
+    // warp, all on one word, took 15 us of the 33 of a 2048 x 2048 update.
+    __shared__ unsigned warp_max[8];
     const unsigned m = __reduce_max_sync(0xffffffffu, __float_as_uint(wmax));
-    if ((threadIdx.x & 31) == 0) atomicMax(reinterpret_cast<unsigned*>(scale) + 2, m);
+    if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = m;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      unsigned b = warp_max[0];
+      for (int i = 1; i < 8; i++) b = max(b, warp_max[i]);
+      unsigned* const at = reinterpret_cast<unsigned*>(scale) + 2;
+      if (b > *(volatile unsigned*)at) atomicMax(at, b);
+    }
   }
 }
 
@@ -574,7 +603,7 @@ __device__ __forceinline__ bool update_scale(float* scale) {
 }
 
 // kAux 2: the block that finishes last decides on the exponent, and rewrites the planes alone in the rare update that has to
-// (weights grown eightfold or halved): two launches less, 2048 x 2048 with 512 cases 16.0 -> 12.7 us.
+// (weights grown eightfold or halved): two launches less.
 template <int kAux>
 __global__ void __launch_bounds__(256) k_update_all(const __grid_constant__ TailArgs a, const __grid_constant__ UpdateArgs u,
                                                     int tail_blocks) {
