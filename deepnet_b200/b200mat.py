@@ -822,7 +822,8 @@ def _build_fused_gemm(passes, out=None, sample=None, bias=None, col_scale=None, 
  OP_SPLIT_BF16, OP_ALLREDUCE, OP_SOFTMAX_SCALED, OP_SAMPLE_MULTINOMIAL, OP_DIV_BY_ROW, OP_ADD_SCALAR, OP_ASSIGN_SCALAR,
  OP_COPY, OP_SAMPLE_BERNOULLI, OP_SOFTMAX_SAMPLE, OP_MOMENTUM_UPDATE_COLUMNS, OP_ALLREDUCE_BEGIN, OP_ALLREDUCE_END,
  OP_SM_LIMIT, OP_DP_PEER_UPDATE, OP_RBM_BIAS_UPDATE, OP_SOFTMAX_RECONSTRUCTION,
- OP_DOCUMENT_LENGTHS, OP_BIAS_UPDATES, OP_UPDATE_ALL, OP_SIGMOID) = range(28)
+ OP_DOCUMENT_LENGTHS, OP_BIAS_UPDATES, OP_UPDATE_ALL, OP_SIGMOID,
+ OP_SPLIT_RANGED) = range(29)
 
 
 class _Op(ct.Structure):
@@ -885,6 +886,11 @@ class Immediate(object):
 
     def split_f16(self, x, aux, exp_dev=None, exp_const=0):
         x.split_f16(aux, exp_dev, exp_const)
+
+    def split_ranged(self, x, aux, data, data_aux, state, w_scale, step, last):
+        """The planes of real-valued states and their common exponent (`split_ranged` in b200mat.h)."""
+        _check(_lib.split_ranged(x.p_mat, aux.p_mat, data.p_mat, data_aux.p_mat, state.p_mat, w_scale.p_mat, ct.c_int(step),
+                                 ct.c_int(int(last))))
 
     def split_bf16(self, x, aux):
         x.split_bf16(aux)
@@ -1029,6 +1035,9 @@ class Program(object):
 
     def split_f16(self, x, aux, exp_dev=None, exp_const=0):
         return self._add(OP_SPLIT_F16, (x, aux, exp_dev), (exp_const,))
+
+    def split_ranged(self, x, aux, data, data_aux, state, w_scale, step, last):
+        return self._add(OP_SPLIT_RANGED, (x, aux, data, data_aux, state, w_scale), (step, int(last)))
 
     def split_bf16(self, x, aux):
         return self._add(OP_SPLIT_BF16, (x, aux))

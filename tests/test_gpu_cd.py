@@ -678,14 +678,15 @@ def test_updates_in_one_launch_match_the_separate_calls(cm, sizes, B, rows):
     assert abs(results[0][2] - results[1][2]) <= 1e-6 * results[1][2]
 
 
-@pytest.mark.parametrize("rows", [64, 37])
+@pytest.mark.parametrize("rows,n", [(64, 45), (37, 45), (1024, 516)])
 @pytest.mark.parametrize("growth", [0.0, 1.0, 1000.0, -1.0])
-def test_updates_in_one_launch_keep_the_exponent_of_the_planes(cm, rows, growth):
+def test_updates_in_one_launch_keep_the_exponent_of_the_planes(cm, rows, n, growth):
     """The scaled half-precision planes written by the launch that updates everything: bit for bit those of momentum_update,
-    over two updates, where the exponent stays, where the weights outgrow it (every plane rewritten) and where they vanish."""
+    over two updates, where the exponent stays, where the weights outgrow it (every plane rewritten, by one block and by a launch
+    of its own) and where they vanish."""
     rng = np.random.default_rng(rows)
     f = lambda *s: rng.standard_normal(s).astype(np.float32)
-    B, n = 20, 45
+    B = 20
     layers_h = [(f(rows, B), f(rows, B), f(rows, 1), f(rows, 1)), (f(n, B), f(n, B), f(n, 1), f(n, 1))]
     w = f(rows, n)
     d = -w if growth < 0 else growth * f(rows, n)          # -1: the update takes the weights away
@@ -742,6 +743,39 @@ def test_half_precision_engine_on_odd_models_matches_oracle(cm, oracle, V, H, B,
         np.testing.assert_array_equal(get(eng.v_samp), get(ref.GetLayerByName("v").sample))
     for mine, theirs in ((eng.bv, "v"), (eng.bh, "h")):
         assert relerr(get(mine), get(ref.GetLayerByName(theirs).params["bias"])) < TOL
+    assert cm.read_status() == 0
+
+
+@pytest.mark.parametrize("V,H,B,gibbs,scale", [(64, 128, 40, 1, 1.0), (301, 203, 78, 3, 1.0), (130, 67, 1030, 2, 1e-3), (97, 515, 33, 1, 300.0),
+                                               (60, 40, 16, 2, 0.0)])
+def test_half_precision_engine_on_real_data_matches_oracle(cm, oracle, V, H, B, gibbs, scale, monkeypatch):
+    """Linear visible units on half-precision planes, whose exponent follows the minibatch and what is reconstructed from it:
+    data of any magnitude, all zero among them (the reconstruction then sets the exponent), and one outlier of a thousand times
+    the rest; draws bit for bit, parameters and states to 1e-5 of the largest."""
+    monkeypatch.setenv("B200_RBM_STATE_AUX", "1")
+    rng = np.random.default_rng(V)
+    hyp = dbm.Hyperparams(base_epsilon=1e-3 / max(scale, 1.0) ** 2, initial_momentum=0.5, final_momentum=0.9, momentum_change_steps=10,
+                          gibbs_steps=gibbs)
+    w = (0.05 / max(scale, 1.0) * rng.standard_normal((V, H))).astype(np.float32)
+    x = (scale * rng.standard_normal((V, 2 * B))).astype(np.float32)
+    if scale == 1e-3:
+        x[5, 7] = 1.0
+    layers = [dict(name="v", activation=dbm.LINEAR, numdims=V, is_input=True), dict(name="h", activation=dbm.LOGISTIC, numdims=H)]
+    ref = dbm.DBM(oracle, layers, [dict(node1="v", node2="h", weight=w, hyperparams=hyp)], hyp, B, dbm.CD, seed=9)
+    eng = FusedRBM(cm, V, H, B, w, hyp, visible=dbm.LINEAR, seed=9)
+    assert eng.f16
+    xo, xg = oracle.CUDAMatrix(x), cm.CUDAMatrix(x)
+    for step in range(3):
+        s = (step % 2) * B
+        ref.SetBatch([xo.slice(s, s + B)])
+        want = ref.TrainOneBatch(step)[0]
+        eng.TrainOneBatch(step, xg.slice(s, s + B))
+        np.testing.assert_allclose(eng.read_loss(), want, rtol=1e-5)
+    assert relerr(get(eng.W), get(ref.edge[0].params["weight"])) < TOL
+    assert relerr(get(eng.dW), get(ref.edge[0].gradient_history)) < 2 * TOL
+    assert relerr(get(eng.v_neg), get(ref.GetLayerByName("v").state)) < TOL
+    assert relerr(get(eng.h_neg), get(ref.GetLayerByName("h").state)) < TOL
+    np.testing.assert_array_equal(get(eng.h_samp), get(ref.GetLayerByName("h").sample))
     assert cm.read_status() == 0
 
 
