@@ -4,7 +4,7 @@
 // issues nothing: 110 us a megabyte, most of a minibatch's time where representations are written out
 // (deepnet/extract_rbm_representation.py).  Here the copy lands in pinned pieces on a stream of its own and a few threads
 // carry the pieces to where they belong, while the caller goes on to the next minibatch: eight of 250 x 1000 with their
-// reconstruction error 1154 -> 540 us.
+// reconstruction error 1154 -> 540 us, and 365 with several minibatches a product and pieces copied several at a time.
 // One staging area per process (4 MB and four threads, made on first use, given back by cublas_shutdown): whoever
 // begins while another thread holds it is told so and copies the plain way.
 //
@@ -30,14 +30,18 @@ using namespace b200;
 
 namespace {
 
-constexpr int kPieces = 16, kCarriers = 4, kBusy = 2;
-constexpr size_t kPieceBytes = 256 * 1024;
+// A copy from the device fills up to kRun neighbouring pieces, as many as are free (256 KB take 13 us one by one, 1 MB 24).  A
+// thread carries a piece at a time, of a matrix of no more than one piece a part of it, so that all threads have one (100 x 500: 142 ->
+// 65 us; parts of 64 KB cost large results up to a third).
+constexpr int kPieces = 16, kRun = 4, kCarriers = 4, kBusy = 2;
+constexpr size_t kPieceBytes = 256 * 1024, kPartBytes = 64 * 1024;
 
 struct RowsStaging {
   std::mutex mu;
   std::condition_variable work, freed;
   struct Job {
-    int piece;
+    int piece, event;
+    size_t from;           // in the pinned area
     float* dst;
     size_t bytes;
   };
@@ -47,7 +51,8 @@ struct RowsStaging {
   cudaEvent_t landed[kPieces] = {nullptr}, ready = nullptr, done[2] = {nullptr, nullptr};
   cudaStream_t copies = nullptr;
   bool free_piece[kPieces];
-  int device = 0, in_flight = 0, adds = 0;
+  int parts[kPieces] = {0};      // of a piece, still to be carried
+  int device = 0, in_flight = 0, adds = 0, copied = 0;    // copied: copies so far; each has the next event in turn
   std::atomic<long> taken{0}, seen{0};     // pieces carriers have taken, and seen land
   bool held = false, stop = false, made = false, failed = false;
 
@@ -72,12 +77,12 @@ struct RowsStaging {
       jobs.pop_front();
       const long order = taken++;
       lock.unlock();
-      const bool ok = wait_for(landed[j.piece], order);
+      const bool ok = wait_for(landed[j.event], order);
       seen++;
-      if (ok) memcpy(j.dst, pinned + j.piece * kPieceBytes, j.bytes);
+      if (ok) memcpy(j.dst, pinned + j.from, j.bytes);
       lock.lock();
       failed |= !ok;
-      free_piece[j.piece] = true;
+      if (--parts[j.piece] == 0) free_piece[j.piece] = true;
       in_flight--;
       freed.notify_all();
     }
@@ -165,30 +170,37 @@ int b200_rows_add(cudamat* src, float* dst) {
   if (cudaEventRecord(s.ready, stream()) != cudaSuccess || cudaStreamWaitEvent(s.copies, s.ready, 0) != cudaSuccess)
     return set_error(cudaGetErrorString(cudaGetLastError()));
   const size_t bytes = (size_t)numel(src) * sizeof(float);
-  for (size_t at = 0; at < bytes; at += kPieceBytes) {
-    const size_t n = bytes - at < kPieceBytes ? bytes - at : kPieceBytes;
-    int piece = -1;
+  for (size_t at = 0; at < bytes;) {
+    int first = 0, pieces = 0;
     {
       std::unique_lock<std::mutex> lock(s.mu);
       s.freed.wait(lock, [&] {
-        for (piece = 0; piece < kPieces; piece++)
-          if (s.free_piece[piece]) return true;
-        return false;
+        for (first = 0; first < kPieces && !s.free_piece[first];) first++;
+        return first < kPieces;
       });
-      s.free_piece[piece] = false;
+      while (pieces < kRun && first + pieces < kPieces && s.free_piece[first + pieces] && at + pieces * kPieceBytes < bytes)
+        s.free_piece[first + pieces++] = false;
     }
-    const bool ok = cudaMemcpyAsync(s.pinned + piece * kPieceBytes, (const char*)src->data_device + at, n, cudaMemcpyDeviceToHost,
+    const size_t run = bytes - at < pieces * kPieceBytes ? bytes - at : pieces * kPieceBytes;
+    const int event = s.copied++ % kPieces;      // (its copy of kPieces copies ago has been carried: there are no more pieces)
+    const bool ok = cudaMemcpyAsync(s.pinned + first * kPieceBytes, (const char*)src->data_device + at, run, cudaMemcpyDeviceToHost,
                                     s.copies) == cudaSuccess &&
-                    cudaEventRecord(s.landed[piece], s.copies) == cudaSuccess;
+                    cudaEventRecord(s.landed[event], s.copies) == cudaSuccess;
     std::lock_guard<std::mutex> lock(s.mu);
     if (!ok) {
-      s.free_piece[piece] = true;
+      for (int i = 0; i < pieces; i++) s.free_piece[first + i] = true;
       s.failed = true;
       return set_error(cudaGetErrorString(cudaGetLastError()));
     }
-    s.jobs.push_back({piece, (float*)((char*)dst + at), n});
-    s.in_flight++;
-    s.work.notify_one();
+    const size_t part = bytes <= kPieceBytes ? kPartBytes : kPieceBytes;
+    for (size_t from = 0; from < run; from += part) {
+      const int piece = first + (int)(from / kPieceBytes);
+      s.jobs.push_back({piece, event, first * kPieceBytes + from, (float*)((char*)dst + at + from), run - from < part ? run - from : part});
+      s.parts[piece]++;
+      s.in_flight++;
+      s.work.notify_one();
+    }
+    at += run;
   }
   // the matrix of the call before has been read once this stream is past its copies
   if (s.adds > 0 && cudaStreamWaitEvent(stream(), s.done[(s.adds - 1) & 1], 0) != cudaSuccess)

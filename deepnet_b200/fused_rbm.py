@@ -142,7 +142,7 @@ class FusedRBM(LossReadback):
             self.v_samp = z(V, B)
             self.v_act = z(V, B)                  # W h + b_v before the softmax
             self.tiny = 1e-10
-        self._h_out = None                        # second buffer of representations being written out
+        self._group = None                        # states of several minibatches whose representations are written out
         self._sched = Parameter(cm, self.hyp)
         self._esched = Parameter(cm, self.ehyp)
         self.kernel_launches = 0
@@ -517,36 +517,67 @@ class FusedRBM(LossReadback):
         the inference-only positive phase of deepnet/dbm.py:340-398 (extract_rbm_representation.py)
         as one fused product per minibatch.  Returns (cases x H) host array, and with input_recon
         also the summed squared error of the input reconstructed from the hidden means."""
-        cm, B, W, P = self.cm, self.B, self.W, self.cm.split_passes
-        Wa = None if self.f16 else self.W_aux     # the bfloat16 parts exist only in that form of the aux
+        cm, B, W, Wa, P, F, E = self.cm, self.B, self.W, self.W_aux, self.cm.split_passes, self.cm.f16_passes, 14
+        V, H = self.V, self.H
         n = data.shape[1] // B
-        rep = np.empty((n * B, self.H), np.float32)
+        rep = np.empty((n * B, H), np.float32)
         err = 0.0
         soft = self.visible == REPLICATED_SOFTMAX
-        if n > 1 and self._h_out is None:
-            self._h_out = cm.empty((self.H, B))
+        # Several minibatches a product, about 1024 cases: launches and calls cost more than the products of one (8 minibatches of
+        # 250 x 1000 units, reconstruction error and 8 MB to the host: 550 us one by one).
+        g = 1 if soft else max(1, min(n, 1024 // B))
+        if n > 1 and (self._group is None or self._group[0].shape[1] != g * B):
+            z = lambda r: cm.empty((r, g * B))
+            aux = lambda r: cm.empty_aux((r, g * B)) if self.f16 else None
+            self._group = None                   # (given back first)
+            self._group = (z(H), z(H), z(V), aux(V), aux(H))
         # one small minibatch has nothing to hide its copy behind: 784 x 500 with 100 cases 53 us copied the plain way, 62 by
         # the threads; with 400 cases of 500 100 and 94
         with cm.RowsOut(n > 1 or rep.nbytes >= 1 << 19) as out:
-            for b in range(n):
-                v0 = data.slice(b * B, (b + 1) * B)
-                h = self.h_pos if (n - 1 - b) % 2 == 0 else self._h_out    # one is on its way to the host, the last stays
+            for i, b in enumerate(range(0, n, g)):
+                e = min(b + g, n)
+                v0 = data.slice(b * B, e * B)
+                if n == 1:
+                    h, v, va, ha = self.h_pos, self.v_neg, self.data_aux, self.h_pos_aux
+                else:                            # (of the two buffers for hidden states one is on its way to the host)
+                    h, v, va, ha = self._group[i % 2], self._group[2], self._group[3], self._group[4]
+                    if e - b < g:
+                        h, v, va, ha = (m.slice(0, (e - b) * B) if m is not None else None for m in (h, v, va, ha))
+                act = 1 if self.visible == LOGISTIC else 0
                 if soft:
                     v0.sum(axis=0, target=self.NN)
                     self.NN.add(self.tiny)
-                cm.fused_gemm(P(W.T, v0, exact_b=soft or self.binary_data, a_aux=Wa), out=h, bias=self.bh, activation=1,
-                              col_scale=self.NN if soft else None)
-                if input_recon:
-                    down = P(W, h, a_aux=Wa)
-                    if soft:
-                        cm.fused_gemm(down, out=self.v_act, bias=self.bv, activation=0)
-                        self.v_act.softmax_scaled(self.NN, target=self.v_neg)
-                        self.v_neg.div_by_row(self.NN, target=self.v_negn)
-                        cm._check(cm._lib.add_sq_diff(self.v_negn.p_mat, v0.p_mat, self.loss_acc.p_mat))
+                    cm.fused_gemm(P(W.T, v0, exact_b=True, a_aux=Wa), out=h, bias=self.bh, activation=1, col_scale=self.NN)
+                elif self.f16:
+                    hidden = dict(out=h, out_aux=ha if input_recon else None, bias=self.bh, activation=1, aux_f16=True, aux_exp=E)
+                    if self.v_range is None:
+                        v0.split_f16(va, None, E)
+                        cm.fused_gemm(F(W.T, Wa, v0, va, exact_b=True), scale_exp=self.W_exp, scale_exp_const=E, **hidden)
                     else:
-                        cm.fused_gemm(down, out=self.v_neg, bias=self.bv, activation=self._act(self.visible))
-                        cm._check(cm._lib.add_sq_diff(self.v_neg.p_mat, v0.p_mat, self.loss_acc.p_mat))
-                out.add(h, rep[b * B:(b + 1) * B])
+                        cm.Immediate().split_ranged(v0, va, v0, va, self.v_range, self.W_scale, 0, False)
+                        cm.fused_gemm(F(W.T, Wa, v0, va), scale_exp=self.v_range.slice(5, 6), **hidden)
+                else:
+                    cm.fused_gemm(P(W.T, v0, exact_b=self.binary_data, a_aux=Wa), out=h, bias=self.bh, activation=1)
+                if out.held:                     # on its way while the error is computed
+                    out.add(h, rep[b * B:e * B])
+                if input_recon and soft:
+                    cm.fused_gemm(P(W, h, a_aux=Wa), out=self.v_act, bias=self.bv, activation=0)
+                    self.v_act.softmax_scaled(self.NN, target=self.v_neg)
+                    self.v_neg.div_by_row(self.NN, target=self.v_negn)
+                    cm._check(cm._lib.add_sq_diff(self.v_negn.p_mat, v0.p_mat, self.loss_acc.p_mat))
+                elif input_recon:
+                    if self.f16:
+                        cm.fused_gemm(F(W, Wa, h, ha), out=v, bias=self.bv, activation=act, scale_exp=self.W_exp, scale_exp_const=E)
+                    else:
+                        cm.fused_gemm(P(W, h, a_aux=Wa), out=v, bias=self.bv, activation=act)
+                    cm._check(cm._lib.add_sq_diff(v.p_mat, v0.p_mat, self.loss_acc.p_mat))
+                if not out.held:
+                    out.add(h, rep[b * B:e * B])
+            if n > 1:                            # the engine's own states are those of the last minibatch
+                last = lambda m: m.slice((e - b - 1) * B, (e - b) * B) if m.shape[1] != B else m
+                self.h_pos.assign(last(h))
+                if input_recon and not soft:
+                    self.v_neg.assign(last(v))
         if input_recon:
             err = self.read_loss()
             return rep, err

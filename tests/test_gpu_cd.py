@@ -779,6 +779,32 @@ def test_half_precision_engine_on_real_data_matches_oracle(cm, oracle, V, H, B, 
     assert cm.read_status() == 0
 
 
+@pytest.mark.parametrize("V,H,B,n,visible,binary", [(61, 130, 90, 15, "LOGISTIC", True), (61, 130, 90, 12, "LOGISTIC", False),
+                                                    (40, 33, 1, 7, "LINEAR", False), (61, 130, 600, 3, "LOGISTIC", True), (60, 44, 250, 5, "LINEAR", False)])
+@pytest.mark.parametrize("planes", ["0", "1"])
+def test_representations_of_several_minibatches_a_product(cm, V, H, B, n, visible, binary, planes, monkeypatch):
+    """Groups of minibatches, whole and a ragged last one, in every form of the engine: representation and reconstruction error
+    against float64 (1e-5 of the largest, 1e-5 of the error), the engine's states those of the last minibatch."""
+    monkeypatch.setenv("B200_RBM_STATE_AUX", planes)
+    rng = np.random.default_rng(n)
+    w, bv, bh = (0.1 * rng.standard_normal(s).astype(np.float32) for s in ((V, H), (V, 1), (H, 1)))
+    x = (rng.random((V, n * B)) < 0.3 if binary else rng.standard_normal((V, n * B)) if visible == "LINEAR" else rng.random((V, n * B)))
+    x = x.astype(np.float32)
+    eng = FusedRBM(cm, V, H, B, w, dbm.Hyperparams(), visible=getattr(dbm, visible), binary_data=binary, bias_v=bv, bias_h=bh, seed=1)
+    data = cm.CUDAMatrix(x)
+    rep, err = eng.Inference(data, input_recon=True)
+    sig = lambda z: 1 / (1 + np.exp(-z))
+    h = sig(w.T.astype(np.float64) @ x + bh)
+    v = w.astype(np.float64) @ h + bv
+    v = v if visible == "LINEAR" else sig(v)
+    assert np.abs(rep.T - h).max() < 1e-5
+    np.testing.assert_allclose(err, ((v - x) ** 2).sum(), rtol=1e-5)
+    np.testing.assert_array_equal(get(eng.h_pos).T, rep[(n - 1) * B:])
+    assert np.abs(get(eng.v_neg) - v[:, (n - 1) * B:]).max() < 1e-5 * max(1.0, np.abs(v).max())
+    np.testing.assert_array_equal(eng.Inference(data), rep)
+    assert cm.read_status() == 0
+
+
 def test_representations_leave_while_the_next_minibatch_is_computed(cm):
     """Several pieces a minibatch and a ragged last one, an even and an odd number of minibatches, and the staging area taken by
     someone else (plain copies): the rows are the products', bit for bit."""
