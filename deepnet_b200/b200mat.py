@@ -1243,10 +1243,11 @@ class Event(object):
             pass
 
 
-def ais_binary_steps(w, w_aux, a, b, v_state, v_sample, h_pre, h_sample, weights, schedule):
-    """Every step of the annealing schedule for a binary RBM (see `ais.ais_binary_rbm`), issued from C."""
+def ais_binary_steps(w, w_aux, a, b, v_state, v_sample, h_pre, h_sample, weights, schedule, scaled_bias=None):
+    """Every step of the annealing schedule for a binary RBM (see `ais.ais_binary_rbm`), issued from C; scaled_bias: scratch
+    of the shape of b."""
     steps = np.ascontiguousarray(schedule, np.float64).reshape(-1)
-    scaled_bias = empty(b.shape)
+    scaled_bias = empty(b.shape) if scaled_bias is None else scaled_bias
     _check(_lib.ais_binary_steps(CUDAMatrix.rnd_state_p, w.p_mat, w_aux.p_mat, a.p_mat, b.p_mat, v_state.p_mat,
                                  v_sample.p_mat, h_pre.p_mat, h_sample.p_mat, scaled_bias.p_mat, weights.p_mat,
                                  steps.ctypes.data_as(ct.POINTER(ct.c_double)), ct.c_int(len(steps))))
