@@ -97,3 +97,26 @@ def test_stacked_training_on_the_device_matches_the_cpu_restatement(cm, oracle):
     Wc, lc, rc = _stack(cm, fused_top=False)
     assert np.abs(rc - ro).max() < 1e-5 and abs(lc - lo) < 1e-5 * lo
     assert cm.read_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("sizes,acts,B,exact", [((784, 500, 1000), "LL", 2048, True), ((784, 500, 1000), "LL", 2048, False),
+                                                ((61, 33, 70), "LL", 20, True), ((301, 203, 77, 45), "LNL", 333, False),
+                                                ((1001, 515, 130, 33), "LLN", 517, True)])
+def test_upward_net_on_half_precision_planes(cm, sizes, acts, B, exact):
+    """0/1 and real data, odd layers, a linear layer between logistic ones (its states have no planes): every layer's states
+    against float64, 1e-5 of the largest."""
+    rng = np.random.default_rng(B)
+    specs = [((0.1 * rng.standard_normal((sizes[i], sizes[i + 1]))).astype(np.float32), rng.standard_normal(sizes[i + 1]).astype(np.float32),
+              dbm.LOGISTIC if a == "L" else dbm.LINEAR) for i, a in enumerate(acts)]
+    net = dbn.UpwardNet(cm, specs, B)
+    x = (rng.random((sizes[0], B)) < 0.3 if exact else rng.standard_normal((sizes[0], B))).astype(np.float32)
+    for _ in range(2):
+        top = net.forward(cm.CUDAMatrix(x), exact_input=exact)
+    assert top is net.layers[-1]["state"]
+    want = x.astype(np.float64)
+    for (w, b, act), l in zip(specs, net.layers):
+        want = w.T.astype(np.float64) @ want + b[:, None]
+        want = 1 / (1 + np.exp(-want)) if act == dbm.LOGISTIC else want
+        assert np.abs(np.array(l["state"].asarray()) - want).max() < 1e-5 * max(1.0, np.abs(want).max())
+    assert cm.read_status() == 0
