@@ -824,7 +824,7 @@ def _build_fused_gemm(passes, out=None, sample=None, bias=None, col_scale=None, 
  OP_COPY, OP_SAMPLE_BERNOULLI, OP_SOFTMAX_SAMPLE, OP_MOMENTUM_UPDATE_COLUMNS, OP_ALLREDUCE_BEGIN, OP_ALLREDUCE_END,
  OP_SM_LIMIT, OP_DP_PEER_UPDATE, OP_RBM_BIAS_UPDATE, OP_SOFTMAX_RECONSTRUCTION,
  OP_DOCUMENT_LENGTHS, OP_BIAS_UPDATES, OP_UPDATE_ALL, OP_SIGMOID,
- OP_SPLIT_RANGED) = range(29)
+ OP_SPLIT_RANGED, OP_BRANCH) = range(30)
 
 
 class _Op(ct.Structure):
@@ -887,6 +887,10 @@ class Immediate(object):
 
     def split_f16(self, x, aux, exp_dev=None, exp_const=0):
         x.split_f16(aux, exp_dev, exp_const)
+
+    def branch(self, what):
+        """Work side by side: 0 fork, 1 beside, 2 back, 3 join (`b200_branch` in b200mat.h)."""
+        _check(_lib.b200_branch(ct.c_int(what)))
 
     def split_ranged(self, x, aux, data, data_aux, state, w_scale, step, last):
         """The planes of real-valued states and their common exponent (`split_ranged` in b200mat.h)."""
@@ -1036,6 +1040,9 @@ class Program(object):
 
     def split_f16(self, x, aux, exp_dev=None, exp_const=0):
         return self._add(OP_SPLIT_F16, (x, aux, exp_dev), (exp_const,))
+
+    def branch(self, what):
+        return self._add(OP_BRANCH, (), (what,))
 
     def split_ranged(self, x, aux, data, data_aux, state, w_scale, step, last):
         return self._add(OP_SPLIT_RANGED, (x, aux, data, data_aux, state, w_scale), (step, int(last)))

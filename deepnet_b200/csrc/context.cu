@@ -33,6 +33,15 @@ struct Scratch {
 };
 static Scratch g_scratch[kScratchStreams];
 static Scratch* g_ws = g_scratch;   // the current stream's
+
+// Work that needs nothing of each other, side by side (b200_branch): between fork and join the calling thread's operations go
+// to the library stream or to one beside it, each with its own scratch.  Other threads stay where they are.
+static thread_local cudaStream_t t_stream = nullptr;   // where this thread's operations go instead
+static thread_local Scratch* t_ws = nullptr;
+static thread_local bool t_forked = false;
+static cudaStream_t g_side = nullptr;
+static cudaEvent_t g_fork = nullptr, g_join = nullptr;
+static Scratch* current_scratch() { return t_ws ? t_ws : g_ws; }
 static size_t g_scratch_limit = ~(size_t)0;   // largest scratch a call gets (b200_test_limit_scratch)
 
 static int g_dependent_launch = -1;        // programmatic dependent launch of the hot kernels: -1 = read the environment
@@ -83,9 +92,9 @@ static void ensure_init() {
 
 cudaStream_t stream() {
   ensure_init();
-  return g_stream;
+  return t_stream ? t_stream : g_stream;
 }
-cudaStream_t stream_if_initialised() { return g_stream; }
+cudaStream_t stream_if_initialised() { return t_stream ? t_stream : g_stream; }
 static int g_sm_limit = 0;
 int sm_count() {
   ensure_init();
@@ -138,8 +147,8 @@ int check_launch() {
   return check_launch_any_stream();
 }
 
-// Makes the scratch of `s` the current one.
-static int select_scratch(cudaStream_t s) {
+// Makes the scratch of `s` the current one, or hands it out.
+static int select_scratch(cudaStream_t s, Scratch** only = nullptr) {
   static unsigned long clock = 0;
   const unsigned long long id = stream_id(s);
   Scratch* take = nullptr;
@@ -155,21 +164,22 @@ static int select_scratch(cudaStream_t s) {
     take->stream = id;
   }
   take->selected = ++clock;
-  g_ws = take;
+  if (only) *only = take;
+  else g_ws = take;
   return 0;
 }
 
 void* workspace(int slot, size_t bytes) {
   ensure_init();
   if (slot < 0 || slot >= kWorkspaces) return nullptr;
-  Scratch& ws = *g_ws;
+  Scratch& ws = *current_scratch();
   if (bytes > g_scratch_limit) {
     set_error("workspace allocation failed");
     return nullptr;
   }
   if (ws.bytes[slot] >= bytes && ws.p[slot]) return ws.p[slot];
   if (ws.p[slot]) {
-    cudaStreamSynchronize(g_stream);
+    cudaStreamSynchronize(stream());
     cudaFree(ws.p[slot]);
     ws.p[slot] = nullptr;
     ws.bytes[slot] = 0;
@@ -194,12 +204,13 @@ void* workspace(int slot, size_t bytes) {
 // users leave at zero between calls.
 void* workspace_zeroed(int slot, size_t bytes) {
   void* p = workspace(slot, bytes);
-  if (p && g_ws->fresh[slot]) {
-    if (cudaMemsetAsync(p, 0, g_ws->bytes[slot], g_stream) != cudaSuccess) {
+  Scratch* const ws = current_scratch();
+  if (p && ws->fresh[slot]) {
+    if (cudaMemsetAsync(p, 0, ws->bytes[slot], stream()) != cudaSuccess) {
       set_error("workspace clear failed");
       return nullptr;
     }
-    g_ws->fresh[slot] = false;
+    ws->fresh[slot] = false;
   }
   return p;
 }
@@ -274,6 +285,52 @@ int cublas_shutdown() {
       ws.fresh[i] = false;
     }
   }
+  return 0;
+}
+
+// 0: fork, 1: what follows goes beside, 2: to the library stream, 3: join (what follows waits for both).  Without the second
+// stream, or while the library stream is captured, everything stays on the library stream.
+int b200_branch(int what) {
+  ensure_init();
+  if (!g_stream) return CUDA_ERROR;
+  if (what == 0) {
+    if (t_forked || t_stream) return ERROR_GENERIC;
+    if (stream_capturing()) return 0;
+    if (!g_side) {
+      std::lock_guard<std::mutex> lock(g_mu);
+      cudaStream_t side = nullptr;
+      if (!g_side && cudaEventCreateWithFlags(&g_fork, cudaEventDisableTiming) == cudaSuccess &&
+          cudaEventCreateWithFlags(&g_join, cudaEventDisableTiming) == cudaSuccess &&
+          cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) == cudaSuccess)
+        g_side = side;
+      cudaGetLastError();
+    }
+    Scratch* ws = nullptr;
+    if (!g_side || select_scratch(g_side, &ws)) {
+      clear_error();
+      return 0;
+    }
+    if (cudaEventRecord(g_fork, g_stream) != cudaSuccess || cudaStreamWaitEvent(g_side, g_fork, 0) != cudaSuccess)
+      return set_error(cudaGetErrorString(cudaGetLastError()));
+    t_ws = ws;
+    t_forked = true;
+  }
+  if (!t_forked) return 0;
+  static thread_local Scratch* side_ws = nullptr;
+  if (what == 0) {
+    side_ws = t_ws;
+    t_ws = nullptr;
+  } else if (what == 1) {
+    t_stream = g_side;
+    t_ws = side_ws;
+  } else {
+    t_stream = nullptr;
+    t_ws = nullptr;
+  }
+  if (what != 3) return 0;
+  t_forked = false;
+  if (cudaEventRecord(g_join, g_side) != cudaSuccess || cudaStreamWaitEvent(g_stream, g_join, 0) != cudaSuccess)
+    return set_error(cudaGetErrorString(cudaGetLastError()));
   return 0;
 }
 

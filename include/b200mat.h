@@ -357,6 +357,8 @@ int update_all_scaled(b200_bias_layers* t, cudamat* w, cudamat* delta, cudamat* 
  * [visible | hidden] in one launch (deepnet/layer.py:202-213, parameter.py:80-106, logistic_layer.py:48-52). */
 int rbm_bias_update(cudamat* v_pos, cudamat* v_neg, cudamat* h_pos, cudamat* h_neg, cudamat* suff, cudamat* b, cudamat* db,
                     cudamat* sq_acc, float inv_batch, float momentum, float eps);
+/* Work side by side: 0 fork, 1 the calling thread's operations go to a second stream, 2 to the library stream again, 3 join. */
+int b200_branch(int what);
 int b200_set_gemm_path(int path);         /* 0 auto; one kernel only: 1 tcgen05, 2 CUDA cores, 3 one launch, 4 tcgen05 behind
                                            * aligned copies of its operands */
 int b200_set_dot_precision(int mode);     /* 0 fp32-grade split TF32 (default), 1 one TF32 pass */
@@ -426,7 +428,7 @@ int dp_wait(int timeout_ms);
  * 11 div_by_row_vec, 12 add_scalar, 13 assign_scalar, 14 copy_on_device, 15 sample_bernoulli,
  * 16 softmax_sample, 17 momentum_update_columns, 18 dp_allreduce_begin, 19 dp_allreduce_end,
  * 20 b200_set_sm_limit, 21 dp_peer_update, 22 rbm_bias_update,
- * 23 softmax_reconstruction, 24 document_lengths, 25 bias_updates, 26 update_all, 27 apply_sigmoid, 28 split_ranged); m[], i0.., f0.. are its arguments in declaration order (matrices, then
+ * 23 softmax_reconstruction, 24 document_lengths, 25 bias_updates, 26 update_all, 27 apply_sigmoid, 28 split_ranged, 29 b200_branch); m[], i0.., f0.. are its arguments in declaration order (matrices, then
  * integers, then floats; gemm for kind 0, whose m[0] is add or null, and pointing to the b200_bias_layers of 25 and 26).  Stops at the first failure: returns its code, *failed_at its index. */
 struct b200_fused_gemm;
 typedef struct b200_op {

@@ -805,6 +805,47 @@ def test_representations_of_several_minibatches_a_product(cm, V, H, B, n, visibl
     assert cm.read_status() == 0
 
 
+def test_work_side_by_side(cm):
+    """Two chains of products beside each other and what follows the join, recorded and call by call: the bits of one stream.  An
+    operation that fails between fork and join leaves the thread on the library stream."""
+    rng = np.random.default_rng(3)
+    f = lambda *s: rng.random(s).astype(np.float32)
+    w, xs, b = cm.CUDAMatrix(0.05 * f(2048, 2048)), [cm.CUDAMatrix(f(2048, 200)) for _ in range(2)], cm.CUDAMatrix(f(2048, 1))
+    results = []
+    for X, beside in ((cm.Immediate(), False), (cm.Immediate(), True), (cm.Program(), True)):
+        out = [[cm.empty((2048, 200)) for _ in range(4)] for _ in range(2)]
+        total = cm.empty((2048, 1))
+        if beside:
+            X.branch(0)
+        for k in range(4):
+            for side in (0, 1):
+                if beside and side:
+                    X.branch(1)
+                X.fused_gemm(cm.split_passes(w.T, out[side][k - 1] if k else xs[side]), out=out[side][k], bias=b, activation=1)
+                if beside and side:
+                    X.branch(2)
+        if beside:
+            X.branch(3)
+        X.row_sum_diff(out[0][3], out[1][3], total)
+        if isinstance(X, cm.Program):
+            X.run()
+        results.append([get(m) for o in out for m in o] + [get(total)])
+    for other in results[1:]:
+        for a, c in zip(results[0], other):
+            np.testing.assert_array_equal(a, c)
+    stream = cm._lib.b200_get_stream()
+    bad = cm.Program()
+    bad.branch(0)
+    bad.branch(1)
+    bad.copy(xs[0], b)
+    bad.branch(3)
+    with pytest.raises(cm.CUDAMatException):
+        bad.run()
+    assert cm._lib.b200_get_stream() == stream
+    np.testing.assert_array_equal(get(cm.empty((2048, 200)).assign(xs[0])), get(xs[0]))
+    assert cm.read_status() == 0
+
+
 def test_representations_leave_while_the_next_minibatch_is_computed(cm):
     """Several pieces a minibatch and a ragged last one, an even and an odd number of minibatches, and the staging area taken by
     someone else (plain copies): the rows are the products', bit for bit."""
