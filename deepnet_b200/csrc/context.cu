@@ -6,6 +6,7 @@
 #include <stdlib.h>
 #include <string.h>
 
+#include <atomic>
 #include <mutex>
 
 #include "common.cuh"
@@ -41,7 +42,9 @@ static thread_local Scratch* t_ws = nullptr;
 static thread_local bool t_forked = false;
 static cudaStream_t g_side = nullptr;
 static cudaEvent_t g_fork = nullptr, g_join = nullptr;
-static Scratch* current_scratch() { return t_ws ? t_ws : g_ws; }
+static std::atomic<int> g_forks{0};     // threads between fork and join: without one nobody looks at the thread's own
+static Scratch* current_scratch() { return g_forks.load(std::memory_order_relaxed) && t_ws ? t_ws : g_ws; }
+static cudaStream_t current_stream() { return g_forks.load(std::memory_order_relaxed) && t_stream ? t_stream : g_stream; }
 static size_t g_scratch_limit = ~(size_t)0;   // largest scratch a call gets (b200_test_limit_scratch)
 
 static int g_dependent_launch = -1;        // programmatic dependent launch of the hot kernels: -1 = read the environment
@@ -92,9 +95,9 @@ static void ensure_init() {
 
 cudaStream_t stream() {
   ensure_init();
-  return t_stream ? t_stream : g_stream;
+  return current_stream();
 }
-cudaStream_t stream_if_initialised() { return t_stream ? t_stream : g_stream; }
+cudaStream_t stream_if_initialised() { return current_stream(); }
 static int g_sm_limit = 0;
 int sm_count() {
   ensure_init();
@@ -314,6 +317,7 @@ int b200_branch(int what) {
       return set_error(cudaGetErrorString(cudaGetLastError()));
     t_ws = ws;
     t_forked = true;
+    g_forks++;
   }
   if (!t_forked) return 0;
   static thread_local Scratch* side_ws = nullptr;
@@ -329,6 +333,7 @@ int b200_branch(int what) {
   }
   if (what != 3) return 0;
   t_forked = false;
+  g_forks--;
   if (cudaEventRecord(g_join, g_side) != cudaSuccess || cudaStreamWaitEvent(g_stream, g_join, 0) != cudaSuccess)
     return set_error(cudaGetErrorString(cudaGetLastError()));
   return 0;

@@ -33,6 +33,7 @@
 #include <stdlib.h>
 #include <time.h>
 
+#include <atomic>
 #include <mutex>
 #include <type_traits>
 #include <unordered_map>
@@ -1807,13 +1808,38 @@ enum { kForms = 4 };
 static const int kFormColumns[kForms] = {256, 128, 128, 64};
 static const bool kFormTwo[kForms] = {true, true, false, false};
 
-static int resident_tiles(int form, int splits, int& clusters) {
-  switch (form) {
-    case 0: return resident_clusters<256, kEpiTile, true>(2 * splits, clusters);
-    case 1: return resident_clusters<128, kEpiTile, true>(2 * splits, clusters);
-    case 2: return resident_clusters<128, kEpiTile, false>(splits, clusters);
-    default: return resident_clusters<64, kEpiTile, false>(splits, clusters);
+// Tiles resident at once, of every form and number of splits: asked once per device (every product looks at some twenty).
+struct ResidentTiles {
+  int room[kForms][kLargestCluster + 1];
+};
+static const ResidentTiles* resident_tiles() {
+  constexpr int kMaxDev = 64;
+  static std::atomic<const ResidentTiles*> known[kMaxDev];
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= kMaxDev) {
+    set_error("cudaGetDevice failed");
+    return nullptr;
   }
+  const ResidentTiles* t = known[dev].load(std::memory_order_acquire);
+  if (t) return t;
+  static std::mutex mu;
+  std::lock_guard<std::mutex> lock(mu);
+  ResidentTiles* n = new ResidentTiles();      // (kept: one per device)
+  for (int form = 0; form < kForms; form++)
+    for (int s = 1; s * (kFormTwo[form] ? 2 : 1) <= kLargestCluster; s++) {
+      int& room = n->room[form][s];
+      const int err = form == 0   ? resident_clusters<256, kEpiTile, true>(2 * s, room)
+                      : form == 1 ? resident_clusters<128, kEpiTile, true>(2 * s, room)
+                      : form == 2 ? resident_clusters<128, kEpiTile, false>(s, room)
+                                  : resident_clusters<64, kEpiTile, false>(s, room);
+      if (err) {
+        delete n;
+        return nullptr;
+      }
+      if (s == 1 && !kFormTwo[form]) room = device_sms();
+    }
+  known[dev].store(n, std::memory_order_release);
+  return n;
 }
 
 // The layout of a product, by an estimate of all of them in us.  With one work item per CTA, tiles of 256 x 256 and 256 x 128 of
@@ -1872,6 +1898,8 @@ static int choose_plan(const GemmProblem& g, bool all16, bool pairs_allowed, TcP
   float best = 0.0f;
   int best_form = 0;
   if (!scatter && g.M > 0 && (g_split_mode == 0 || g_split_mode > 1)) {
+    const ResidentTiles* const resident = resident_tiles();
+    if (!resident) return CUDA_ERROR;
     for (int form = 0; form < kForms; form++) {
       const int per = kFormTwo[form] ? 2 : 1, columns = kFormColumns[form];
       if ((kFormTwo[form] && (g.M <= BM || !pairs_allowed)) || (columns > 64 && g.N <= columns / 2)) continue;
@@ -1880,9 +1908,7 @@ static int choose_plan(const GemmProblem& g, bool all16, bool pairs_allowed, TcP
       for (int s = 1; s * per <= kLargestCluster; s++) {
         if (s > 1 && (tiles * s * per > sms || s * 4 > min_ki)) break;
         if (g_split_mode > 1 && s != (g_split_mode < min_ki ? g_split_mode : min_ki)) continue;
-        int room = 0;
-        const int err = resident_tiles(form, s, room);
-        if (err) return err;
+        int room = resident->room[form][s];
         if (room * per * s > sms) room = sms / (per * s);     // (an SM limit in force)
         if (room < 1) continue;
         const long waves = (tiles + room - 1) / room;
