@@ -299,12 +299,12 @@ __device__ __forceinline__ void mma_commit_pair(uint32_t bar, uint16_t cta_mask)
 // costs about 0.5 us per arrive here, more than a whole k-block.  What the leader's tensor core
 // then reads from this CTA's shared memory was made visible to the async proxy by the proxy
 // fence that precedes the arrive.
-__device__ __forceinline__ void mbar_arrive_leader(uint32_t bar) {
+__device__ __forceinline__ void mbar_arrive_leader(uint32_t bar, uint32_t leader) {
   asm volatile(
       "{\n\t.reg .b32 ra;\n\t"
       "mapa.shared::cluster.u32 ra, %0, %1;\n\t"
       "mbarrier.arrive.shared::cluster.b64 _, [ra];\n\t}" ::"r"(bar),
-      "r"(cluster_ctarank() & ~1u)
+      "r"(leader)
       : "memory");
 }
 
@@ -650,6 +650,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_gemm_tc(const __grid_constant
   const int splits = (kEpi == kEpiPartial || kEpi == kEpiTile) ? p.splits : 1;
   const int num_tiles = p.tiles_m * p.tiles_n * splits;     // work items: every role walks the same list
   const uint32_t rank = kTwo ? cluster_ctarank() & 1u : 0u;   // 0 = leader of the pair
+  const uint32_t leader = kTwo && kEpi == kEpiTile ? cluster_ctarank() & ~1u : 0u;   // (its rank: a cluster holds several pairs)
   // (kEpiTile: as many CTAs or pairs as work items, the splits of a tile next to each other in one cluster)
   const int first_tile = kTwo ? (int)(blockIdx.x >> 1) : (int)blockIdx.x;
   const int tile_step = kTwo ? (int)(gridDim.x >> 1) : (int)gridDim.x;
@@ -810,7 +811,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_gemm_tc(const __grid_constant
     // issuing thread, not the tensor pipe, bounds the kernel.
     if (rank == 0) {
       const bool elected = elect_one();
-      const uint16_t pair_mask = kTwo ? (uint16_t)(3u << cluster_ctarank()) : (uint16_t)1;   // (the leader's rank is even)
+      const uint16_t pair_mask = (uint16_t)(3u << leader);
       uint32_t chunk = 0;
       int stage = 0;
       uint32_t phase = 0;
@@ -880,8 +881,9 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_gemm_tc(const __grid_constant
               // flight.  The tiles were written through the async proxy (TMA) or made visible to it by
               // the converters' proxy fence, ordered by the mbarriers.
               const uint32_t d_tmem = tmem_base + acc * BN;
-              // stage address, 16-byte units (the bits above name the CTA of the cluster: no part of a descriptor's address)
-              const uint32_t sb = ((smem_base + stage * stage_bytes) >> 4) & 0x3fffu;
+              // stage address, 16-byte units (in a larger cluster the bits above name the CTA: no part of a descriptor's address)
+              uint32_t sb = (smem_base + stage * stage_bytes) >> 4;
+              if (kEpi == kEpiTile) sb &= 0x3fffu;
 #pragma unroll
               for (int i = 0; i < kMaxMma; i++) {
                 if (i < nm) {
@@ -1045,7 +1047,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_gemm_tc(const __grid_constant
           fence_async_smem();   // the derived tiles are read through the async proxy
           __syncwarp();
           if (lane == 0) {
-            if (kTwo) mbar_arrive_leader(ready_bar(stage));
+            if (kTwo) mbar_arrive_leader(ready_bar(stage), leader);
             else mbar_arrive(ready_bar(stage));
           }
 #ifdef B200_GEMM_TIMING
@@ -1113,7 +1115,7 @@ __global__ void __launch_bounds__(kThreadsTc, 1) k_gemm_tc(const __grid_constant
         tc_fence_before();
         __syncwarp();
         if (lane == 0) {
-          if (kTwo) mbar_arrive_leader(tempty_bar(acc));   // the leader's issuer waits for both CTAs
+          if (kTwo) mbar_arrive_leader(tempty_bar(acc), leader);   // the leader's issuer waits for both CTAs
           else mbar_arrive(tempty_bar(acc));
         }
       }
@@ -1854,7 +1856,6 @@ static const ResidentTiles* resident_tiles() {
 //   512 x 100, K = 10000, W's parts from memory                 21.7 / 23.8   (few tiles: K over 32 CTAs, past what a cluster holds)
 //   784 x 500, K = 100, plain                                    8.1 /  8.8   (nothing to do but store: straight from the registers)
 //   4096 x 4096, K = 128, plain                                 33.9 / 51.5   (several waves, whose stores overlap the next)
-// What is cut along K by the classic layout only, and odd matrices' long plain sums, stay there.
 static int choose_plan(const GemmProblem& g, bool all16, bool pairs_allowed, TcPlan& plan) {
   const bool scatter = product_is_scattered(g.epi.out);
   const GemmEpilogue& e = g.epi;
@@ -1876,7 +1877,7 @@ static int choose_plan(const GemmProblem& g, bool all16, bool pairs_allowed, TcP
       }
     }
     kind[pairs] = all16 ? (terms < 3 ? kTwoPlanes : kThreePlanes) : planes < 2 ? kLightPair : planes == 2 ? kHalfPair : tf32 ? kDerivedTf32 : kDerivedBf16;
-    blocks[pairs++] = ki;
+    blocks[pairs++] = ki * ((terms + 2) / 3);      // (more terms than one product's: another over the same matrices)
     min_ki = ki < min_ki ? ki : min_ki;
   }
   auto walk = [&](const float (*us)[kForms], int form, int splits) {   // the k-blocks of one split
@@ -1948,7 +1949,7 @@ static int choose_plan(const GemmProblem& g, bool all16, bool pairs_allowed, TcP
     const float waves = (float)((ctas * splits + sms - 1) / sms), end = splits > 1 ? partial_us[form] : whole_us[form];
     if (waves > 1.0f && !plain && form == 0) {   // an activation runs beside the next tile's k-blocks
       const bool planes_only = !e.out && !e.sample;
-      const float act = planes_only ? 10.0f : 20.8f + (draw ? 13.0f : 0.0f) + (aux ? 12.7f : 0.0f);
+      const float act = planes_only ? 22.0f : 20.8f + (draw ? 13.0f : 0.0f) + (aux ? 12.7f : 0.0f);
       us = 4.3f + waves * (us > act ? us : act) + act;
     } else {
       us = 4.3f + waves * (us / splits + end);
@@ -2247,9 +2248,7 @@ int gemm_tc(const GemmProblem& g) {
     store16_mode = sv ? atoi(sv) : 1;
   }
   p.direct_store = !epi_is_plain(epi) && epi != kEpiTile &&
-                   (!tma_outputs_ok(e) || (store16_mode != 0 && !e.out && !e.sample && (e.out_aux || e.sample_aux)) ||
-                    // a CTA with one tile has no next one whose first chunk waits: 18 600 clocks against 26 500 staged
-                    (BN == 128 && g.N > 128 && (long)((g.M + BM - 1) / BM) * ((g.N + BN - 1) / BN) <= sm_count()));
+                   (!tma_outputs_ok(e) || (store16_mode != 0 && !e.out && !e.sample && (e.out_aux || e.sample_aux)));
   for (int i = 0; i < kOutArrays; i++) p.out_map[i] = -1;
   if (!epi_is_plain(epi) && epi != kEpiTile && !p.direct_store) {
     // outputs of the activation epilogues, stored as boxes of 128 rows x 4 columns: M x N floats
