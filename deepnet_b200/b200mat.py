@@ -531,6 +531,7 @@ class CUDAMatrix(object):
         correction terms of a product read: plane 0 = bf16(self - tf32(self)), plane 1 =
         bf16(self).  Returns aux."""
         _check(_lib.split_bf16(self.p_mat, aux.p_mat))
+        aux.form = "bf16"
         return aux
 
     def split_f16(self, aux, exp_dev=None, exp_const=0):
@@ -539,6 +540,7 @@ class CUDAMatrix(object):
         Returns aux."""
         _check(_lib.split_f16(self.p_mat, aux.p_mat, exp_dev.p_mat if exp_dev is not None else None,
                               ct.c_int(int(exp_const))))
+        aux.form = int(exp_const) if exp_dev is None else None
         return aux
 
     def split_tf32(self, lo, hi=None):
@@ -571,6 +573,8 @@ class AuxMatrix(CUDAMatrix):
     storage of lda x cols floats, lda = rows rounded up to 8; column c holds lda bfloat16 of
     plane 0 (bf16(x - tf32(x))) and lda of plane 1 (bf16(x)), the first `rows` of each in use.
     Passed as `a_aux` / `b_aux` of a term, written as `out_aux` / `sample_aux` / `w_aux`."""
+
+    form = None      # what it was last filled with by a call that says so: "bf16", or the exponent of the half-precision planes
 
     def __init__(self, shape):
         _require_device()

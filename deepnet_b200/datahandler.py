@@ -64,6 +64,8 @@ class DeviceFeed(object):
         if buf is None:
             cm = self.cm
             aux = cm.empty_aux((self.dims[i], count)) if (i == 0 and self.aux_mode) else None
+            if aux is not None:
+                aux.form = "bf16" if self.aux_mode == 1 else self.aux_exp
             buf = self._out[(i, count)] = (cm.empty((self.dims[i], count)), aux)
         return buf
 

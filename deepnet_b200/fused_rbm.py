@@ -235,6 +235,8 @@ class FusedRBM(LossReadback):
                 else self._issue if not self.f16 else self._issue_f16_linear if self.visible == LINEAR else self._issue_f16)
         if data_aux is not None and (self.v_range is not None or not (self.state_aux and self.visible != REPLICATED_SOFTMAX)):
             data_aux = None                      # this engine derives the parts of the data in its kernels, or finds their exponent
+        if getattr(data_aux, "form", None) not in (None, 14 if self.f16 else "bf16"):
+            data_aux = None                      # parts in another form than this engine's
         self._given_aux = data_aux
         if not self.use_program or self.timeline is not None:
             self.kernel_launches = 0

@@ -148,3 +148,27 @@ def test_bit_packed_feed_drives_the_half_precision_engine(cm, monkeypatch):
     np.testing.assert_array_equal(get(eng.W), get(ref.W))
     assert eng.read_loss() == ref.read_loss()
     assert cm.read_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode,exp", [(1, 14), (2, 14), (2, 3)])
+def test_parts_in_another_form_are_not_read(cm, mode, exp, monkeypatch):
+    """An engine on half-precision planes given bfloat16 parts, or planes of another exponent, splits the minibatch itself: the
+    bits of an update without parts."""
+    from deepnet_b200 import dbm
+    from deepnet_b200.fused_rbm import FusedRBM
+    monkeypatch.setenv("B200_RBM_STATE_AUX", "1")
+    rng = np.random.default_rng(5)
+    V, H, B = 70, 50, 20
+    x = (rng.random((B, V)) < 0.3).astype(np.float32)
+    w = (0.1 * rng.standard_normal((V, H))).astype(np.float32)
+    results = []
+    for given in (True, False):
+        eng = FusedRBM(cm, V, H, B, w, dbm.Hyperparams(base_epsilon=0.1), binary_data=True, seed=3)
+        assert eng.f16
+        feed = DeviceFeed(cm, [x], binary=[True], aux_mode=mode, aux_exp=exp)
+        batch = feed.Get(B)[0]
+        eng.TrainOneBatch(0, batch, feed.last_aux if given else None)
+        results.append(np.array(eng.W.asarray()))
+    np.testing.assert_array_equal(*results)
+    assert np.abs(results[0] - w).max() > 0
