@@ -580,7 +580,7 @@ __device__ __forceinline__ void update_weights(float* w, float* delta, float* gr
     for (long i = tid; i < (n >> 2); i += nth) {
       float4 W = reinterpret_cast<float4*>(w)[i];
       float4 D = reinterpret_cast<float4*>(delta)[i];
-      const float4 S = reinterpret_cast<const float4*>(suff)[i];
+      const float4 S = __ldcs(reinterpret_cast<const float4*>(suff) + i);   // (read for the last time: leaves the L2 first)
       float4 G = make_float4(0, 0, 0, 0);
       if (kHasGrad) G = reinterpret_cast<float4*>(grad)[i];
       update_one(W.x, D.x, G.x, S.x, ninv_batch, momentum, neps, l2, l1);
