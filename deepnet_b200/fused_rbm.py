@@ -532,7 +532,9 @@ class FusedRBM(LossReadback):
             z = lambda r: cm.empty((r, g * B))
             aux = lambda r: cm.empty_aux((r, g * B)) if self.f16 else None
             self._group = None                   # (given back first)
-            self._group = (z(H), z(H), z(V), aux(V), aux(H))
+            # (one minibatch a product: the engine's own states, and a second buffer for the hidden ones)
+            self._group = ((z(H), z(H), z(V), aux(V), aux(H)) if g > 1 else
+                           (z(H), self.h_pos, self.v_neg, self.data_aux, self.h_pos_aux))
         # one small minibatch has nothing to hide its copy behind: 784 x 500 with 100 cases 53 us copied the plain way, 62 by
         # the threads; with 400 cases of 500 100 and 94
         with cm.RowsOut(n > 1 or rep.nbytes >= 1 << 19) as out:
@@ -542,15 +544,18 @@ class FusedRBM(LossReadback):
                 if n == 1:
                     h, v, va, ha = self.h_pos, self.v_neg, self.data_aux, self.h_pos_aux
                 else:                            # (of the two buffers for hidden states one is on its way to the host)
-                    h, v, va, ha = self._group[i % 2], self._group[2], self._group[3], self._group[4]
+                    h = self._group[i % 2 if g > 1 else (n - i) % 2]
+                    v, va, ha = self._group[2:]
                     if e - b < g:
                         h, v, va, ha = (m.slice(0, (e - b) * B) if m is not None else None for m in (h, v, va, ha))
                 act = 1 if self.visible == LOGISTIC else 0
+                # (a product as small as in one launch: the call that splits the data costs more than the planes save)
+                planes = self.f16 and (e - b) * B * V * H >= 1 << 27
                 if soft:
                     v0.sum(axis=0, target=self.NN)
                     self.NN.add(self.tiny)
                     cm.fused_gemm(P(W.T, v0, exact_b=True, a_aux=Wa), out=h, bias=self.bh, activation=1, col_scale=self.NN)
-                elif self.f16:
+                elif planes:
                     hidden = dict(out=h, out_aux=ha if input_recon else None, bias=self.bh, activation=1, aux_f16=True, aux_exp=E)
                     if self.v_range is None:
                         v0.split_f16(va, None, E)
@@ -559,7 +564,7 @@ class FusedRBM(LossReadback):
                         cm.Immediate().split_ranged(v0, va, v0, va, self.v_range, self.W_scale, 0, False)
                         cm.fused_gemm(F(W.T, Wa, v0, va), scale_exp=self.v_range.slice(5, 6), **hidden)
                 else:
-                    cm.fused_gemm(P(W.T, v0, exact_b=self.binary_data, a_aux=Wa), out=h, bias=self.bh, activation=1)
+                    cm.fused_gemm(P(W.T, v0, exact_b=self.binary_data, a_aux=None if self.f16 else Wa), out=h, bias=self.bh, activation=1)
                 if out.held:                     # on its way while the error is computed
                     out.add(h, rep[b * B:e * B])
                 if input_recon and soft:
@@ -568,14 +573,14 @@ class FusedRBM(LossReadback):
                     self.v_neg.div_by_row(self.NN, target=self.v_negn)
                     cm._check(cm._lib.add_sq_diff(self.v_negn.p_mat, v0.p_mat, self.loss_acc.p_mat))
                 elif input_recon:
-                    if self.f16:
+                    if planes:
                         cm.fused_gemm(F(W, Wa, h, ha), out=v, bias=self.bv, activation=act, scale_exp=self.W_exp, scale_exp_const=E)
                     else:
-                        cm.fused_gemm(P(W, h, a_aux=Wa), out=v, bias=self.bv, activation=act)
+                        cm.fused_gemm(P(W, h, a_aux=None if self.f16 else Wa), out=v, bias=self.bv, activation=act)
                     cm._check(cm._lib.add_sq_diff(v.p_mat, v0.p_mat, self.loss_acc.p_mat))
                 if not out.held:
                     out.add(h, rep[b * B:e * B])
-            if n > 1:                            # the engine's own states are those of the last minibatch
+            if g > 1:                            # the engine's own states are those of the last minibatch
                 last = lambda m: m.slice((e - b - 1) * B, (e - b) * B) if m.shape[1] != B else m
                 self.h_pos.assign(last(h))
                 if input_recon and not soft:

@@ -780,7 +780,8 @@ def test_half_precision_engine_on_real_data_matches_oracle(cm, oracle, V, H, B, 
 
 
 @pytest.mark.parametrize("V,H,B,n,visible,binary", [(61, 130, 90, 15, "LOGISTIC", True), (61, 130, 90, 12, "LOGISTIC", False),
-                                                    (40, 33, 1, 7, "LINEAR", False), (61, 130, 600, 3, "LOGISTIC", True), (60, 44, 250, 5, "LINEAR", False)])
+                                                    (40, 33, 1, 7, "LINEAR", False), (61, 130, 600, 3, "LOGISTIC", True), (60, 44, 250, 5, "LINEAR", False),
+                                                    (785, 301, 600, 3, "LOGISTIC", True), (501, 512, 250, 5, "LINEAR", False)])
 @pytest.mark.parametrize("planes", ["0", "1"])
 def test_representations_of_several_minibatches_a_product(cm, V, H, B, n, visible, binary, planes, monkeypatch):
     """Groups of minibatches, whole and a ragged last one, in every form of the engine: representation and reconstruction error
@@ -788,6 +789,7 @@ def test_representations_of_several_minibatches_a_product(cm, V, H, B, n, visibl
     monkeypatch.setenv("B200_RBM_STATE_AUX", planes)
     rng = np.random.default_rng(n)
     w, bv, bh = (0.1 * rng.standard_normal(s).astype(np.float32) for s in ((V, H), (V, 1), (H, 1)))
+    w /= max(1.0, (V / 100) ** 0.5)
     x = (rng.random((V, n * B)) < 0.3 if binary else rng.standard_normal((V, n * B)) if visible == "LINEAR" else rng.random((V, n * B)))
     x = x.astype(np.float32)
     eng = FusedRBM(cm, V, H, B, w, dbm.Hyperparams(), visible=getattr(dbm, visible), binary_data=binary, bias_v=bv, bias_h=bh, seed=1)
