@@ -1496,7 +1496,7 @@ int g_inject_stage_bytes = 0;
 // What a kernel needs before its first launch on a device, and how many of its clusters of `ctas` CTAs the device keeps
 // resident at once (a CTA takes an SM; the clusters leave some over in every group of SMs that can share one).  Both
 // belong to a device, not to the process: kept per device ordinal for a host that drives several GPUs.
-constexpr int kLargestCluster = 8;
+constexpr int kLargestCluster = 16;     // (more than 8 is not portable: a device may hold none)
 template <int BN, int kEpi, bool kTwo>
 int resident_clusters(int ctas, int& clusters) {
   using Cfg = TcConfig<BN>;
@@ -1511,6 +1511,7 @@ int resident_clusters(int ctas, int& clusters) {
   if (!attr_set[dev]) {
     if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes) != cudaSuccess)
       return set_error("cudaFuncSetAttribute(max dynamic shared memory) failed");
+    if (kEpi == kEpiTile && cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) cudaGetLastError();
     attr_set[dev] = true;
   }
   if (ctas == 1) {
@@ -1532,7 +1533,8 @@ int resident_clusters(int ctas, int& clusters) {
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, kernel, &q) != cudaSuccess || n < 1) {
       cudaGetLastError();
-      return set_error("cudaOccupancyMaxActiveClusters failed for a tensor-core product");
+      if (ctas <= 8) return set_error("cudaOccupancyMaxActiveClusters failed for a tensor-core product");
+      n = 0;
     }
     resident[dev][ctas] = n;
   }
@@ -1845,7 +1847,7 @@ static const ResidentTiles* resident_tiles() {
 }
 
 // The layout of a product, by an estimate of all of them in us.  With one work item per CTA, tiles of 256 x 256 and 256 x 128 of
-// two CTAs and of 128 x 128 and 128 x 64 of one, each with K cut over up to 8 CTAs of a cluster: fitted to 3300 products of 35
+// two CTAs and of 128 x 128 and 128 x 64 of one, each with K cut over up to 16 CTAs of a cluster: fitted to 3300 products of 35
 // shapes and eleven term lists (64 to 10000 rows and columns, K from 64 to 10000; rms error 5 %).  With persistent CTAs: fitted
 // to 1500 of them and 1088 others.  Measured, the best persistent layout with its finishing launch / the best of one work item:
 //   500 x 2048, K = 784, draw, W's parts from memory           18.8 / 15.0
@@ -1853,7 +1855,9 @@ static const ResidentTiles* resident_tiles() {
 //   1024 x 256, K = 4096, two planes                            29.2 / 15.0
 //   1024 x 4096, K = 1024, draw, W's parts from memory          51.6 / 30.8
 //   784 x 1000, K = 256, difference of two, all parts derived   17.2 / 14.7
-//   512 x 100, K = 10000, W's parts from memory                 21.7 / 23.8   (few tiles: K over 32 CTAs, past what a cluster holds)
+//   512 x 100, K = 10000, W's parts from memory, draw           21.7 / 20.1   (few tiles, K over 16 CTAs; over 8: 24.5)
+//   128 x 128, K = 8192, the same                               19.0 / 16.3   (over 8: 21.2)
+//   512 x 200, K = 10000, all of the right operand derived      27.8 / 29.0   (K over 10: seven clusters of 16 fit, and 8 are needed)
 //   784 x 500, K = 100, plain                                    8.1 /  8.8   (nothing to do but store: straight from the registers)
 //   4096 x 4096, K = 128, plain                                 33.9 / 51.5   (several waves, whose stores overlap the next)
 static int choose_plan(const GemmProblem& g, bool all16, bool pairs_allowed, TcPlan& plan) {
@@ -1930,7 +1934,7 @@ static int choose_plan(const GemmProblem& g, bool all16, bool pairs_allowed, TcP
     }
   }
   // the persistent layouts: 256 columns shared by two CTAs, 128, 64
-  if (plan.tile && !plain && (tiles_of(best_form) <= sms / (plan.two ? 2 : 1)) && (min_ki < 64 || plan.splits * (plan.two ? 2 : 1) * tiles_of(best_form) * 2 > sms)) return 0;
+  if (plan.tile && !plain && min_ki < 64 && tiles_of(best_form) <= sms / (plan.two ? 2 : 1)) return 0;
   static const float persistent_us[kPairKinds][kForms] = {{0.53f, 0.0f, 0.49f, 0.40f}, {0.72f, 0.0f, 0.60f, 0.55f}, {0.76f, 0.0f, 0.81f, 0.82f},
                                                           {1.01f, 0.0f, 1.00f, 0.92f}, {0.62f, 0.0f, 0.53f, 0.45f}, {0.88f, 0.0f, 0.67f, 0.55f}};
   static const float plain_us[kForms] = {7.7f, 0.0f, 1.6f, 0.5f}, activation_us[kForms] = {23.1f, 0.0f, 6.2f, 3.3f}, partial_us[kForms] = {7.8f, 0.0f, 0.5f, 0.0f};

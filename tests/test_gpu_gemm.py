@@ -976,8 +976,8 @@ def test_narrow_tiles_of_products_of_few_tiles(cm, M, N, K, two_pairs, columns):
 
 
 @pytest.mark.parametrize("columns", [64, 128, 256])
-@pytest.mark.parametrize("splits", [0, 2, 3, 7])
-@pytest.mark.parametrize("M,N,K", [(130, 129, 900), (257, 260, 1024), (1001, 515, 904), (516, 1029, 900)])
+@pytest.mark.parametrize("splits", [0, 2, 3, 7, 13])
+@pytest.mark.parametrize("M,N,K", [(130, 129, 900), (257, 260, 1024), (1001, 515, 904), (516, 1029, 900), (130, 129, 1700)])
 def test_one_work_item_per_cta(cm, M, N, K, splits, columns):
     """Tiles that end in shared memory, K cut over a cluster or not: ragged rows (columns of the result that start on no
     16 bytes) and ragged columns, every output and option of the epilogue, both forms of the 16-bit planes.  Bound: sums of K
