@@ -28,30 +28,6 @@ def log_mean_exp(x):
     return offset + np.log(np.exp(x - offset).mean())
 
 
-def _carve(cm, shapes):
-    """Matrices of these shapes in few device allocations (each starts on 256 bytes), all zero.  Taking and giving back device
-    memory costs some 700 us from a megabyte on and hardly anything below: a call that needs more than that for one matrix gets
-    all of them in one allocation (784 x 500, 100 chains, 100 steps: 2660 -> 2030 us, 1100 of them steps), others stay below it
-    (300 x 200, 300 chains in one: 350 -> 1010)."""
-    need = [-(-r * c // 64) * 64 for r, c in shapes]
-    room = (1 << 18) - 4096                       # floats of an allocation that costs little
-    blocks, left = [], 0
-    for n in need:                                # where each matrix goes: (block, first float)
-        if not blocks or (max(need) <= room and n > left):
-            blocks.append([])
-            left = room
-        blocks[-1].append(n)
-        left -= n
-    out, at = [], 0
-    for block in blocks:
-        slab, first = cm.empty((sum(block), 1)), 0
-        for n in block:
-            r, c = shapes[at]
-            out.append(slab.slice(first, first + r * c).reshape((r, c)))
-            first, at = first + n, at + 1
-    return out
-
-
 def ais_binary_rbm(cm, weight, hidden_bias, visible_bias, num_chains, schedule, seed=0, fused=None):
     """log Z estimate of the RBM  E(v, h) = -v'Wh - b'v - a'h  (weight V x H, a = hidden bias,
     b = visible bias) from `num_chains` annealing runs along `schedule` (inverse temperatures
@@ -63,8 +39,8 @@ def ais_binary_rbm(cm, weight, hidden_bias, visible_bias, num_chains, schedule, 
         fused = hasattr(cm, "fused_gemm")
     B = num_chains
     if fused:
-        w, w_aux, a, b, scaled, v_state, v_sample, h_state, h_sample, w_ais = _carve(
-            cm, [(V, H), ((V + 7) // 8 * 8, H), (H, 1), (V, 1), (V, 1), (V, B), (V, B), (H, B), (H, B), (1, B)])
+        w, w_aux, a, b, scaled, v_state, v_sample, h_state, h_sample, w_ais = cm.carve(
+            [(V, H), ((V + 7) // 8 * 8, H), (H, 1), (V, 1), (V, 1), (V, B), (V, B), (H, B), (H, B), (1, B)])
         for m, host in ((w, weight), (a, hidden_bias), (b, visible_bias)):
             m.overwrite(host)
     else:

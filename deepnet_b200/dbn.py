@@ -56,7 +56,7 @@ class UpwardNet(object):
                 self._data_aux = cm.empty_aux((w.shape[0], batchsize))
             else:
                 continue
-            l["exp"] = cm.f16_scale_state(float(np.abs(w).max())).slice(0, 1)
+            l["exp"] = cm.f16_scale_state(float(np.maximum(w.max(), -w.min()))).slice(0, 1)
             l["planes"] = W.split_f16(cm.empty_aux(w.shape), exp_dev=l["exp"])
         # the pass is recorded, once for 0/1 and once for real data, and replayed with one library call on whatever minibatch the
         # handle points at

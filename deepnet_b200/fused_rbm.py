@@ -106,7 +106,7 @@ class FusedRBM(LossReadback):
         self.f16 = self.state_aux and f16_ok
         self.v_range = z(1, 8) if self.f16 and visible == LINEAR else None
         if self.f16:
-            self.W_scale = cm.f16_scale_state(float(np.abs(w).max()))
+            self.W_scale = cm.f16_scale_state(float(np.maximum(w.max(), -w.min())))
             self.W_exp = self.W_scale.slice(0, 1)
             self.W.split_f16(self.W_aux, exp_dev=self.W_exp)
         # both bias vectors, their update histories and their statistics are packed [b_v | b_h], so
@@ -128,8 +128,8 @@ class FusedRBM(LossReadback):
         self.suff_b = self.pack.slice(V * H, V * H + V + H)
         B = batchsize
         za = lambda r, c: cm.empty_aux((r, c))
-        self.h_pos, self.h_samp, self.h_samp_aux = z(H, B), z(H, B), za(H, B)
-        self.v_neg, self.v_neg_aux, self.h_neg = z(V, B), za(V, B), z(H, B)
+        self.h_pos, self.h_samp, self.v_neg, self.h_neg = cm.carve([(H, B), (H, B), (V, B), (H, B)])
+        self.h_samp_aux, self.v_neg_aux = za(H, B), za(V, B)
         self.data_aux = za(V, B)
         self.h_pos_aux, self.h_neg_aux = (za(H, B), za(H, B)) if getattr(self, "f16", False) else (None, None)
         self.v_samp = self.v_samp_aux = None      # allocated when sample_input asks for visible draws
@@ -509,7 +509,7 @@ class FusedRBM(LossReadback):
         """Rebuilds the 16-bit parts of W after W was written from outside (a loaded checkpoint)."""
         if self.f16:
             w = np.array(self.W.asarray())
-            self.W_scale.assign(self.cm.f16_scale_state(float(np.abs(w).max())))   # (in place: recorded steps name it)
+            self.W_scale.assign(self.cm.f16_scale_state(float(np.maximum(w.max(), -w.min()))))   # (in place: recorded steps name it)
             self.W.split_f16(self.W_aux, exp_dev=self.W_exp)
         else:
             self.W.split_bf16(self.W_aux)
@@ -529,12 +529,12 @@ class FusedRBM(LossReadback):
         # 250 x 1000 units, reconstruction error and 8 MB to the host: 550 us one by one).
         g = 1 if soft else max(1, min(n, 1024 // B))
         if n > 1 and (self._group is None or self._group[0].shape[1] != g * B):
-            z = lambda r: cm.empty((r, g * B))
-            aux = lambda r: cm.empty_aux((r, g * B)) if self.f16 else None
             self._group = None                   # (given back first)
-            # (one minibatch a product: the engine's own states, and a second buffer for the hidden ones)
-            self._group = ((z(H), z(H), z(V), aux(V), aux(H)) if g > 1 else
-                           (z(H), self.h_pos, self.v_neg, self.data_aux, self.h_pos_aux))
+            if g > 1:                            # (an aux matrix holds whole groups of eight rows)
+                aux = [((r + 7) // 8 * 8, g * B) for r in (V, H)] if self.f16 else []
+                self._group = (cm.carve([(H, g * B), (H, g * B), (V, g * B)] + aux) + [None, None])[:5]
+            else:                                # (one minibatch a product: the engine's own states, a second buffer for the hidden ones)
+                self._group = [cm.empty((H, B)), self.h_pos, self.v_neg, self.data_aux, self.h_pos_aux]
         # one small minibatch has nothing to hide its copy behind: 784 x 500 with 100 cases 53 us copied the plain way, 62 by
         # the threads; with 400 cases of 500 100 and 94
         with cm.RowsOut(n > 1 or rep.nbytes >= 1 << 19) as out:
