@@ -352,3 +352,21 @@ def test_scalar_reductions_after_a_squared_difference(cm, shape):
         assert abs(cm.vdot(ga, gb) - (a * b).sum()) <= 1e-6 * np.abs(a * b).sum()
         want = 2 * turn * ((a - b) ** 2).sum()
         assert abs(get(acc)[0, 0] - want) <= 1e-6 * want
+
+
+@pytest.mark.parametrize("shapes", [[(1, 1), (3, 5), (64, 1), (1, 65)], [(7, 9), (300, 800), (40, 1000), (1, 1)], [(600, 500), (1, 3), (513, 511)]])
+def test_matrices_of_one_allocation(cm, shapes):
+    """Zero-filled, each on 256 bytes, none over another, alive as long as one of them is."""
+    import ctypes
+    mats = cm.carve(shapes)
+    for i, (m, shape) in enumerate(zip(mats, shapes)):
+        assert m.shape == shape and ctypes.cast(m.mat.data_device, ctypes.c_void_p).value % 256 == 0
+        assert not np.array(m.asarray()).any()
+        m.assign(i + 1)
+    last = mats[-1]
+    for i, (m, shape) in enumerate(zip(mats, shapes)):
+        m.copy_to_host()
+        assert (m.numpy_array == i + 1).all()
+    del mats, m
+    last.copy_to_host()
+    assert (last.numpy_array == len(shapes)).all()
