@@ -855,7 +855,7 @@ def _build_fused_gemm(passes, out=None, sample=None, bias=None, col_scale=None, 
  OP_COPY, OP_SAMPLE_BERNOULLI, OP_SOFTMAX_SAMPLE, OP_MOMENTUM_UPDATE_COLUMNS, OP_ALLREDUCE_BEGIN, OP_ALLREDUCE_END,
  OP_SM_LIMIT, OP_DP_PEER_UPDATE, OP_RBM_BIAS_UPDATE, OP_SOFTMAX_RECONSTRUCTION,
  OP_DOCUMENT_LENGTHS, OP_BIAS_UPDATES, OP_UPDATE_ALL, OP_SIGMOID,
- OP_SPLIT_RANGED, OP_BRANCH) = range(30)
+ OP_BRANCH) = range(29)
 
 
 class _Op(ct.Structure):
@@ -922,11 +922,6 @@ class Immediate(object):
     def branch(self, what):
         """Work side by side: 0 fork, 1 beside, 2 back, 3 join (`b200_branch` in b200mat.h)."""
         _check(_lib.b200_branch(ct.c_int(what)))
-
-    def split_ranged(self, x, aux, data, data_aux, state, w_scale, step, last):
-        """The planes of real-valued states and their common exponent (`split_ranged` in b200mat.h)."""
-        _check(_lib.split_ranged(x.p_mat, aux.p_mat, data.p_mat, data_aux.p_mat, state.p_mat, w_scale.p_mat, ct.c_int(step),
-                                 ct.c_int(int(last))))
 
     def split_bf16(self, x, aux):
         x.split_bf16(aux)
@@ -1074,9 +1069,6 @@ class Program(object):
 
     def branch(self, what):
         return self._add(OP_BRANCH, (), (what,))
-
-    def split_ranged(self, x, aux, data, data_aux, state, w_scale, step, last):
-        return self._add(OP_SPLIT_RANGED, (x, aux, data, data_aux, state, w_scale), (step, int(last)))
 
     def split_bf16(self, x, aux):
         return self._add(OP_SPLIT_BF16, (x, aux))

@@ -222,93 +222,6 @@ __global__ void __launch_bounds__(256) k_split_f16(const float* x, uint16_t* aux
   }
 }
 
-// Planes of real-valued states whose range nobody knows beforehand: the data of a minibatch and, once they exist, the states
-// that a Gibbs step reconstructs from them.  `state` (1 x 8): {exponent in force, the data's own, largest |data|, largest |x| of
-// odd steps, of even steps, exponent in force + the weights', -, -}; the maxima as bits.  k_abs_max gathers the maximum of a
-// step, k_split_ranged reads it: the largest magnitude of both goes to (2^12, 2^13] at most, so that the statistics, which
-// take the difference of products over either, need one factor.  Step 0 splits the data; later ones x and, in the last, the
-// data once more where the exponent has moved.  Each step clears the word the next one gathers.
-__global__ void __launch_bounds__(256) k_abs_max(const float* x, long n, bool vec, float* word) {
-  grid_dependents_launch();
-  grid_dependency_wait();
-  const long tid = (long)blockIdx.x * blockDim.x + threadIdx.x, nth = (long)gridDim.x * blockDim.x;
-  float m = 0.0f;
-  auto see = [&](float v) {
-    const float a = fabsf(v);
-    m = a <= 3.4028234e38f ? fmaxf(m, a) : m;      // (infinities and NaN have no range)
-  };
-  if (vec) {
-    for (long i = tid; i < (n >> 2); i += nth) {
-      const float4 v = reinterpret_cast<const float4*>(x)[i];
-      see(v.x); see(v.y); see(v.z); see(v.w);
-    }
-  } else {
-    for (long i = tid; i < n; i += nth) see(x[i]);
-  }
-  __shared__ unsigned warp_max[8];
-  const unsigned w = __reduce_max_sync(0xffffffffu, __float_as_uint(m));
-  if ((threadIdx.x & 31) == 0) warp_max[threadIdx.x >> 5] = w;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    unsigned b = warp_max[0];
-    for (int i = 1; i < 8; i++) b = max(b, warp_max[i]);
-    atomicMax(reinterpret_cast<unsigned*>(word), b);
-  }
-}
-struct RangedSplit {
-  const float* x[2];       // x, and with the last step the data
-  uint16_t* aux[2];
-  long n;
-  int rows, lda, step, last;
-  bool vec;
-  float* state;
-  const float* w_exp;
-};
-__global__ void __launch_bounds__(256) k_split_ranged(const __grid_constant__ RangedSplit a) {
-  grid_dependents_launch();
-  grid_dependency_wait();
-  const int gathered = a.step == 0 ? 2 : 3 + ((a.step + 1) & 1);
-  const float m = a.state[gathered];
-  // an all-zero (or non-finite) matrix leaves room for what the other one holds
-  float e = m > 0.0f ? fminf(fmaxf(floorf(log2f(8192.0f / m)), -100.0f), 100.0f) : 100.0f;
-  const float own = a.step == 0 ? e : a.state[1];
-  e = fminf(e, own);
-  const float scale = exp2f(e);
-  const long tid = (long)blockIdx.x * blockDim.x + threadIdx.x, nth = (long)gridDim.x * blockDim.x;
-#pragma unroll 1
-  for (int j = 0; j < (a.last && e != own ? 2 : 1); j++) {
-    const float* const x = a.x[j];
-    uint16_t* const aux = a.aux[j];
-    if (a.vec) {   // rows % 4 == 0: four consecutive elements share a column
-      for (long i = tid; i < (a.n >> 2); i += nth) {
-        const float4 v = reinterpret_cast<const float4*>(x)[i];
-        const long at = i << 2, c = at / a.rows, r = at - c * a.rows;
-        ushort4 l, h;
-        split_f16(v.x, scale, l.x, h.x); split_f16(v.y, scale, l.y, h.y);
-        split_f16(v.z, scale, l.z, h.z); split_f16(v.w, scale, l.w, h.w);
-        uint16_t* dst = aux + c * 2 * a.lda + r;
-        *reinterpret_cast<ushort4*>(dst) = l;
-        *reinterpret_cast<ushort4*>(dst + a.lda) = h;
-      }
-    } else {
-      for (long i = tid; i < a.n; i += nth) {
-        const long c = i / a.rows, r = i - c * a.rows;
-        uint16_t l, h;
-        split_f16(x[i], scale, l, h);
-        aux[c * 2 * a.lda + r] = l;
-        aux[c * 2 * a.lda + a.lda + r] = h;
-      }
-    }
-  }
-  if (tid == 0) {          // (no block of this launch reads these words)
-    a.state[0] = e;
-    a.state[5] = e + *a.w_exp;
-    a.state[3 + (a.step & 1)] = 0.0f;
-    if (a.step > 0) a.state[2] = 0.0f;
-  }
-  if (a.step == 0 && tid == 0) a.state[1] = e;
-}
-
 // aux holds aux_rows(rows) floats per column.
 int launch_split_aux(const float* x, float* aux, int rows, long n) {
   if (n == 0) return 0;
@@ -850,30 +763,6 @@ int split_f16(cudamat* x, cudamat* aux, cudamat* exp_dev, int exp_const) {
   if (launch_dependent(k_split_f16, dim3((unsigned)blocks), dim3(256), 0, stream(), x->data_device,
                        reinterpret_cast<uint16_t*>(aux->data_device), rows, aux_rows(rows), n, vec,
                        exp_dev ? exp_dev->data_device : nullptr, exp_const, nullptr) != cudaSuccess)
-    return set_error(cudaGetErrorString(cudaGetLastError()));
-  return check_launch();
-}
-
-// Step `step` of an update on real-valued data (see k_split_ranged): the planes of x (and in the last step, where their common
-// exponent has moved, of the data) and that exponent, alone (state[0]) and with the weights' (state[5]).
-int split_ranged(cudamat* x, cudamat* aux, cudamat* data, cudamat* data_aux, cudamat* state, cudamat* w_scale, int step, int last) {
-  for (cudamat* m : {x, aux, data, data_aux, state, w_scale}) {
-    if (!m->on_device) return ERROR_NOT_ON_DEVICE;
-    if (m->is_trans) return ERROR_TRANSPOSED;
-  }
-  if (!aux_shape_ok(aux, x) || !aux_shape_ok(data_aux, data) || !same_shape(x, data) || numel(state) < 8 || numel(w_scale) < 1 || step < 0)
-    return ERROR_INCOMPATIBLE_DIMENSIONS;
-  const long n = numel(x);
-  if (n == 0) return 0;
-  RangedSplit a = {{x->data_device, data->data_device},
-                   {reinterpret_cast<uint16_t*>(aux->data_device), reinterpret_cast<uint16_t*>(data_aux->data_device)},
-                   n, x->size[0], aux_rows(x->size[0]), step, step > 0 && last, false, state->data_device, w_scale->data_device};
-  a.vec = a.rows % 4 == 0 && (((uintptr_t)a.x[0] | (uintptr_t)a.x[1]) & 15) == 0;
-  long blocks = ((a.vec ? n / 4 : n) + 255) / 256;
-  if (blocks > (long)sm_count() * 8) blocks = (long)sm_count() * 8;
-  if (launch_dependent(k_abs_max, dim3((unsigned)(blocks < sm_count() * 2 ? blocks : sm_count() * 2)), dim3(256), 0, stream(), a.x[0], n,
-                       a.vec, a.state + (step == 0 ? 2 : 3 + ((step + 1) & 1))) != cudaSuccess ||
-      launch_dependent(k_split_ranged, dim3((unsigned)blocks), dim3(256), 0, stream(), a) != cudaSuccess)
     return set_error(cudaGetErrorString(cudaGetLastError()));
   return check_launch();
 }

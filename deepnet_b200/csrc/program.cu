@@ -35,7 +35,6 @@ int update_all_scaled(b200_bias_layers* t, cudamat* w, cudamat* delta, cudamat* 
 int split_f16(cudamat* x, cudamat* aux, cudamat* exp_dev, int exp_const);
 int split_bf16(cudamat* x, cudamat* aux);
 int b200_branch(int what);
-int split_ranged(cudamat* x, cudamat* aux, cudamat* data, cudamat* data_aux, cudamat* state, cudamat* w_scale, int step, int last);
 int dp_allreduce(cudamat* mat);
 int softmax_reconstruction(cudamat* pre, cudamat* nn, cudamat* state, cudamat* norm, cudamat* data, cudamat* acc);
 int document_lengths(cudamat* counts, cudamat* nn, cudamat* norm, float tiny);
@@ -79,8 +78,7 @@ enum {
   B200_OP_BIAS_UPDATES = 25,      // gemm points to a b200_bias_layers; f0 inv_batch, f1 momentum, f2 eps
   B200_OP_UPDATE_ALL = 26,        // the same, m0 w, m1 delta, m2 suff, m3 w_aux, m4 w_scale?; f0 inv_batch, f1 mom_b, f2 eps_b, f3 mom_w, f4 eps_w, f5 l2, f6 l1
   B200_OP_SIGMOID = 27,           // m0 mat, m1 target
-  B200_OP_SPLIT_RANGED = 28,      // m0 x, m1 aux, m2 data, m3 data_aux, m4 state, m5 w_scale, i0 step, i1 last
-  B200_OP_BRANCH = 29,            // i0 what (b200_branch)
+  B200_OP_BRANCH = 28,            // i0 what (b200_branch)
   B200_OP_COUNT
 };
 
@@ -134,7 +132,6 @@ extern "C" int b200_run_program(rnd_struct* rnd_state, b200_op* ops, int n, int*
       case B200_OP_DOCUMENT_LENGTHS: err = document_lengths(o.m[0], o.m[1], o.m[2], o.f0); break;
       case B200_OP_BIAS_UPDATES: err = bias_updates(reinterpret_cast<b200_bias_layers*>(o.gemm), o.f0, o.f1, o.f2); break;
       case B200_OP_BRANCH: err = b200_branch(o.i0); break;
-      case B200_OP_SPLIT_RANGED: err = split_ranged(o.m[0], o.m[1], o.m[2], o.m[3], o.m[4], o.m[5], o.i0, o.i1); break;
       case B200_OP_SIGMOID: err = apply_sigmoid(o.m[0], o.m[1]); break;
       case B200_OP_UPDATE_ALL:
         err = update_all_scaled(reinterpret_cast<b200_bias_layers*>(o.gemm), o.m[0], o.m[1], o.m[2], o.m[3], o.m[4], o.f0, o.f1, o.f2, o.f3, o.f4, o.f5, o.f6);

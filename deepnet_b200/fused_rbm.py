@@ -97,14 +97,13 @@ class FusedRBM(LossReadback):
         env = os.environ.get("B200_RBM_STATE_AUX")
         big = V * H * batchsize >= 1 << 32
         # the half-precision form below serves every model but the small ones (and, over several ranks, the big ones)
-        f16_ok = (binary_data and visible == LOGISTIC or visible == LINEAR and world_size == 1) and os.environ.get("B200_RBM_F16", "1") != "0"
+        f16_ok = binary_data and visible == LOGISTIC and os.environ.get("B200_RBM_F16", "1") != "0"
         self.state_aux = big or (f16_ok and world_size == 1 and self._planes_pay()) if env is None else env != "0"
         # With 0/1 data and logistic units every operand's range is known, and the big products run
         # on the scaled half-precision form of W and of the states (three fp16 terms, no TF32 term,
-        # no fp32 operand read): W * 2^e with e kept by the update kernel, states * 2^14.  Linear visible units (one rank) take
-        # it too, with an exponent that every update finds for the minibatch and what is reconstructed from it.
+        # no fp32 operand read): W * 2^e with e kept by the update kernel, states * 2^14.  Real-valued data have no range: one
+        # exponent for a minibatch takes from every case what the largest of them lies above it.
         self.f16 = self.state_aux and f16_ok
-        self.v_range = z(1, 8) if self.f16 and visible == LINEAR else None
         if self.f16:
             self.W_scale = cm.f16_scale_state(float(np.maximum(w.max(), -w.min())))
             self.W_exp = self.W_scale.slice(0, 1)
@@ -176,11 +175,9 @@ class FusedRBM(LossReadback):
         with parts derived in the kernel, by what an update costs (us, CD-1 / CD-3, planes against the better of the others):
         784 x 500, 100 cases 50.3 / 49.1, 87 / 91; 250 cases 57 / 64, 97 / 117; 1000 x 200, 100 cases 48 / 44, 85 / 91; 1357 x 601,
         203 cases 62 / 114, 105 / 228; 2048 x 2048, 512 cases 123 / 135, 193 / 242; 784 x 500, 20 cases 47 / 41, 87 / 79.  The
-        split of the minibatch is what the smaller ones lose, once an update; linear units, whose range has to be found as well, lose it
-        every Gibbs step (CD-1 / CD-5): 784 x 500, 100 cases 55 / 51, 141 / 131; 250 cases 61 / 66, 157 / 162; 1024 x 4096, 256 cases
-        91 / 116."""
+        split of the minibatch is what the smaller ones lose, once an update."""
         work = self.V * self.H * self.B
-        return work >= 1 << 26 or (self.visible == LOGISTIC and self.hyp.gibbs_steps > 1 and work >= 1 << 24)
+        return work >= 1 << 26 or (self.hyp.gibbs_steps > 1 and work >= 1 << 24)
 
     def _act(self, layer_activation):
         return 1 if layer_activation == LOGISTIC else 0
@@ -197,7 +194,7 @@ class FusedRBM(LossReadback):
         return bool(self.hyp.sample_input) and self.hyp.sample_input_after <= step
 
     # launches behind one operation of the vocabulary (the draws' counts start from zero)
-    _LAUNCHES = dict(sample_multinomial=2, split_ranged=2, sm_limit=0, allreduce_end=0)
+    _LAUNCHES = dict(sample_multinomial=2, sm_limit=0, allreduce_end=0)
 
     def _op(self, X, name, flops, nbytes, method, *args, **kw):
         """Names one operation of the step to the executor X (`Immediate` or a recording `Program`);
@@ -232,9 +229,9 @@ class FusedRBM(LossReadback):
         if draw_v and self.v_samp is None:
             self.v_samp, self.v_samp_aux = cm.empty((self.V, self.B)), cm.empty_aux((self.V, self.B))
         body = (self._issue_replicated_softmax if self.visible == REPLICATED_SOFTMAX
-                else self._issue if not self.f16 else self._issue_f16_linear if self.visible == LINEAR else self._issue_f16)
-        if data_aux is not None and (self.v_range is not None or not (self.state_aux and self.visible != REPLICATED_SOFTMAX)):
-            data_aux = None                      # this engine derives the parts of the data in its kernels, or finds their exponent
+                else self._issue_f16 if self.f16 else self._issue)
+        if data_aux is not None and not (self.state_aux and self.visible != REPLICATED_SOFTMAX):
+            data_aux = None                      # this engine derives the parts of the data in its kernels
         if getattr(data_aux, "form", None) not in (None, 14 if self.f16 else "bf16"):
             data_aux = None                      # parts in another form than this engine's
         self._given_aux = data_aux
@@ -435,35 +432,6 @@ class FusedRBM(LossReadback):
         self.kernel_launches += 2
         return ub, uw
 
-    def _issue_f16_linear(self, X, data, k, draw_v, sc):
-        """`_issue_f16` for linear visible units: the minibatch and the states reconstructed from it share an exponent that is
-        found on the way (`split_ranged`), hidden states and W are as there."""
-        cm = self.cm
-        V, H, B = self.V, self.H, self.B
-        W, Wa, We, R, F = self.W, self.W_aux, self.W_exp, self.v_range, cm.f16_passes
-        E = 14
-        v0, v0a = data, self.data_aux
-        gf = 2.0 * V * H * B
-        vb, hb, wb = 4.0 * V * B, 4.0 * H * B, 4.0 * V * H
-        hidden = dict(scale_exp=R.slice(5, 6), bias=self.bh, activation=1, aux_f16=True, aux_exp=E)
-        self._op(X, "split", 0, 3 * vb, "split_ranged", v0, v0a, v0, v0a, R, self.W_scale, 0, False)
-        self._op(X, "gemm_up", gf, 2.5 * hb, "fused_gemm", F(W.T, Wa, v0, v0a), out=self.h_pos, out_aux=self.h_pos_aux,
-                 sample_aux=self.h_samp_aux, **hidden)
-        for i in range(k):
-            last = i == k - 1
-            self._op(X, "gemm_down", gf, vb, "fused_gemm", F(W, Wa, self.h_samp, self.h_samp_aux, exact_b=True), out=self.v_neg,
-                     scale_exp=We, scale_exp_const=E, bias=self.bv, activation=0)
-            if i == 0 and k > 1:
-                self._op(X, "sq_err", 0, 2 * vb, "sq_diff", self.v_neg, v0, self.loss_acc)
-            self._op(X, "split", 0, 3 * vb, "split_ranged", self.v_neg, self.v_neg_aux, v0, v0a, R, self.W_scale, i + 1, last)
-            self._op(X, "gemm_up", gf, 2.5 * hb, "fused_gemm", F(W.T, Wa, self.v_neg, self.v_neg_aux),
-                     out=self.h_neg if last else None, out_aux=self.h_neg_aux if last else None,
-                     sample=self.h_samp if last else None, sample_aux=self.h_samp_aux, **hidden)
-        pos = F(v0, v0a, self.h_pos.T, self.h_pos_aux)
-        neg = F(self.v_neg, self.v_neg_aux, self.h_neg.T, self.h_neg_aux, negate=1)
-        self._op(X, "gemm_stats", 2 * gf, wb, "fused_gemm", pos + neg, out=self.suff_W, scale_exp=R.slice(0, 1), scale_exp_const=E)
-        return self._issue_updates(X, sc, wb, w_scale=self.W_scale, bias=(v0, self.v_neg, self.loss_acc if k == 1 else None))
-
     def _issue_replicated_softmax(self, X, data, k, draw_v, sc):
         """CD-k with a replicated-softmax visible layer (word-count columns): the call sequence of
         deepnet/dbm.py:118-238 with replicated_softmax_layer.py:12-60,90-154 and edge.py:222-246, on
@@ -557,12 +525,8 @@ class FusedRBM(LossReadback):
                     cm.fused_gemm(P(W.T, v0, exact_b=True, a_aux=Wa), out=h, bias=self.bh, activation=1, col_scale=self.NN)
                 elif planes:
                     hidden = dict(out=h, out_aux=ha if input_recon else None, bias=self.bh, activation=1, aux_f16=True, aux_exp=E)
-                    if self.v_range is None:
-                        v0.split_f16(va, None, E)
-                        cm.fused_gemm(F(W.T, Wa, v0, va, exact_b=True), scale_exp=self.W_exp, scale_exp_const=E, **hidden)
-                    else:
-                        cm.Immediate().split_ranged(v0, va, v0, va, self.v_range, self.W_scale, 0, False)
-                        cm.fused_gemm(F(W.T, Wa, v0, va), scale_exp=self.v_range.slice(5, 6), **hidden)
+                    v0.split_f16(va, None, E)
+                    cm.fused_gemm(F(W.T, Wa, v0, va, exact_b=True), scale_exp=self.W_exp, scale_exp_const=E, **hidden)
                 else:
                     cm.fused_gemm(P(W.T, v0, exact_b=self.binary_data, a_aux=None if self.f16 else Wa), out=h, bias=self.bh, activation=1)
                 if out.held:                     # on its way while the error is computed

@@ -196,10 +196,6 @@ int split_bf16(cudamat* x, cudamat* aux);
  * |a||b| per term; the caller names the exponent sum in b200_fused_gemm and the kernel divides
  * it out.  e must keep the largest |xs| inside the fp16 range (65504). */
 int split_f16(cudamat* x, cudamat* aux, cudamat* exp_dev, int exp_const);
-/* Planes of real-valued states of unknown range: step 0 splits the minibatch (x = data), step i > 0 the states x reconstructed
- * from it, with one exponent for both, and in the last step the minibatch again where that exponent has moved.  state: 1 x 8,
- * zero at first: [0] the exponent, [5] with w_scale[0] added. */
-int split_ranged(cudamat* x, cudamat* aux, cudamat* data, cudamat* data_aux, cudamat* state, cudamat* w_scale, int step, int last);
 
 /* One term of a fused product: op(a) is M x k, op(b) is k x N (handles carry is_trans).
  * Both parts of a term are fp32-wide (X, LO32) or both bfloat16 (LO16, B16).  a_aux / b_aux:
@@ -428,7 +424,7 @@ int dp_wait(int timeout_ms);
  * 11 div_by_row_vec, 12 add_scalar, 13 assign_scalar, 14 copy_on_device, 15 sample_bernoulli,
  * 16 softmax_sample, 17 momentum_update_columns, 18 dp_allreduce_begin, 19 dp_allreduce_end,
  * 20 b200_set_sm_limit, 21 dp_peer_update, 22 rbm_bias_update,
- * 23 softmax_reconstruction, 24 document_lengths, 25 bias_updates, 26 update_all, 27 apply_sigmoid, 28 split_ranged, 29 b200_branch); m[], i0.., f0.. are its arguments in declaration order (matrices, then
+ * 23 softmax_reconstruction, 24 document_lengths, 25 bias_updates, 26 update_all, 27 apply_sigmoid, 28 b200_branch); m[], i0.., f0.. are its arguments in declaration order (matrices, then
  * integers, then floats; gemm for kind 0, whose m[0] is add or null, and pointing to the b200_bias_layers of 25 and 26).  Stops at the first failure: returns its code, *failed_at its index. */
 struct b200_fused_gemm;
 typedef struct b200_op {

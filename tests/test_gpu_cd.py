@@ -748,10 +748,9 @@ def test_half_precision_engine_on_odd_models_matches_oracle(cm, oracle, V, H, B,
 
 @pytest.mark.parametrize("V,H,B,gibbs,scale", [(64, 128, 40, 1, 1.0), (301, 203, 78, 3, 1.0), (130, 67, 1030, 2, 1e-3), (97, 515, 33, 1, 300.0),
                                                (60, 40, 16, 2, 0.0)])
-def test_half_precision_engine_on_real_data_matches_oracle(cm, oracle, V, H, B, gibbs, scale, monkeypatch):
-    """Linear visible units on half-precision planes, whose exponent follows the minibatch and what is reconstructed from it:
-    data of any magnitude, all zero among them (the reconstruction then sets the exponent), and one outlier of a thousand times
-    the rest; draws bit for bit, parameters and states to 1e-5 of the largest."""
+def test_engine_on_real_data_with_parts_in_memory_matches_oracle(cm, oracle, V, H, B, gibbs, scale, monkeypatch):
+    """Linear visible units on bfloat16 parts from memory: data of any magnitude, all zero among them, and one outlier of a thousand
+    times the rest; draws bit for bit, parameters and states to 1e-5 of the largest."""
     monkeypatch.setenv("B200_RBM_STATE_AUX", "1")
     rng = np.random.default_rng(V)
     hyp = dbm.Hyperparams(base_epsilon=1e-3 / max(scale, 1.0) ** 2, initial_momentum=0.5, final_momentum=0.9, momentum_change_steps=10,
@@ -763,7 +762,7 @@ def test_half_precision_engine_on_real_data_matches_oracle(cm, oracle, V, H, B, 
     layers = [dict(name="v", activation=dbm.LINEAR, numdims=V, is_input=True), dict(name="h", activation=dbm.LOGISTIC, numdims=H)]
     ref = dbm.DBM(oracle, layers, [dict(node1="v", node2="h", weight=w, hyperparams=hyp)], hyp, B, dbm.CD, seed=9)
     eng = FusedRBM(cm, V, H, B, w, hyp, visible=dbm.LINEAR, seed=9)
-    assert eng.f16
+    assert eng.state_aux and not eng.f16
     xo, xg = oracle.CUDAMatrix(x), cm.CUDAMatrix(x)
     for step in range(3):
         s = (step % 2) * B
@@ -804,6 +803,52 @@ def test_representations_of_several_minibatches_a_product(cm, V, H, B, n, visibl
     np.testing.assert_array_equal(get(eng.h_pos).T, rep[(n - 1) * B:])
     assert np.abs(get(eng.v_neg) - v[:, (n - 1) * B:]).max() < 1e-5 * max(1.0, np.abs(v).max())
     np.testing.assert_array_equal(eng.Inference(data), rep)
+    assert cm.read_status() == 0
+
+
+@pytest.mark.parametrize("scale", [1e8, 1e-3])
+def test_results_depend_on_no_data_of_earlier_calls(cm, scale):
+    """Real-valued data of another magnitude first: representations, reconstruction error and an update afterwards are a fresh
+    engine's, bit for bit."""
+    rng = np.random.default_rng(11)
+    V, H, B = 256, 512, 512
+    w = (0.05 * rng.standard_normal((V, H))).astype(np.float32)
+    x, other = (rng.standard_normal((V, 4 * B)).astype(np.float32) for _ in range(2))
+    data, first = cm.CUDAMatrix(x), cm.CUDAMatrix(other * np.float32(scale))
+    mk = lambda: FusedRBM(cm, V, H, B, w, dbm.Hyperparams(base_epsilon=1e-3), visible=dbm.LINEAR, seed=2)
+    used, fresh = mk(), mk()
+    used.Inference(first, input_recon=True)
+    for a, b in zip(used.Inference(data, input_recon=True), fresh.Inference(data, input_recon=True)):
+        np.testing.assert_array_equal(a, b)
+    weights = []
+    for used in (True, False):
+        eng = mk()                       # (the random stream starts over)
+        if used:
+            eng.Inference(first)
+        eng.TrainOneBatch(0, data.slice(0, B))
+        weights.append(get(eng.W))
+    np.testing.assert_array_equal(*weights)
+    assert cm.read_status() == 0
+
+
+@pytest.mark.parametrize("outlier", [0.0, 1e3, 1e6, 1e8, 1e12])
+def test_one_case_of_large_values_leaves_the_others_exact(cm, outlier):
+    """One entry of any size in one case of real-valued data: every other case's representation, and the statistics of every other
+    visible unit, against float64 (1e-5 of the largest)."""
+    rng = np.random.default_rng(12)
+    V, H, B = 512, 516, 512
+    w = (0.05 * rng.standard_normal((V, H))).astype(np.float32)
+    x = rng.standard_normal((V, 2 * B)).astype(np.float32)
+    x[3, 7] += np.float32(outlier)
+    eng = FusedRBM(cm, V, H, B, w, dbm.Hyperparams(base_epsilon=1e-3), visible=dbm.LINEAR, seed=2)
+    data = cm.CUDAMatrix(x)
+    sig = lambda z: 1 / (1 + np.exp(-np.clip(z, -700, 700)))
+    others, rows = np.arange(2 * B) != 7, np.arange(V) != 3
+    assert np.abs(eng.Inference(data).T - sig(w.T.astype(np.float64) @ x))[:, others].max() < 1e-5
+    eng.TrainOneBatch(0, data.slice(0, B))
+    v = get(eng.v_neg).astype(np.float64)
+    want = (x[:, :B] @ sig(w.T.astype(np.float64) @ x[:, :B]).T - v @ sig(w.T.astype(np.float64) @ v).T)[rows]
+    assert relerr(get(eng.suff_W)[rows], want) < 1e-5
     assert cm.read_status() == 0
 
 
