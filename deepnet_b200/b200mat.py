@@ -575,7 +575,17 @@ class AuxMatrix(CUDAMatrix):
     plane 0 (bf16(x - tf32(x))) and lda of plane 1 (bf16(x)), the first `rows` of each in use.
     Passed as `a_aux` / `b_aux` of a term, written as `out_aux` / `sample_aux` / `w_aux`."""
 
-    form = None      # what it was last filled with by a call that says so: "bf16", or the exponent of the half-precision planes
+    _form, _recorded = None, False
+
+    @property
+    def form(self):
+        """What it was last filled with: "bf16", the exponent of half-precision planes, or None where nobody can say (a draw's one
+        plane, an exponent in device memory, an output of a recorded step)."""
+        return None if self._recorded else self._form
+
+    @form.setter
+    def form(self, form):
+        self._form = form
 
     def __init__(self, shape):
         _require_device()
@@ -801,6 +811,10 @@ def fused_gemm(passes, out=None, sample=None, bias=None, col_scale=None, activat
     f = _build_fused_gemm(passes, out, sample, bias, col_scale, activation, alpha, beta, out_aux, sample_aux, scale_exp,
                           scale_exp_const, aux_f16, aux_exp)
     _check(_lib.fused_gemm_add(CUDAMatrix.rnd_state_p, ct.byref(f), add.p_mat if add is not None else None))
+    if out_aux is not None:
+        out_aux.form = int(aux_exp) if aux_f16 else "bf16"
+    if sample_aux is not None:
+        sample_aux.form = None
 
 
 def _build_bias_layers(layers, sq_acc):
@@ -1007,10 +1021,18 @@ class Program(object):
         self._arr = None
         return len(self._ops) - 1
 
+    @staticmethod
+    def _writes(*parts):
+        """A replay writes these whenever it runs: from here on they have no form of their own."""
+        for aux in parts:
+            if isinstance(aux, AuxMatrix):
+                aux._recorded = True
+
     def fused_gemm(self, passes, **kw):
         for p in passes:
             self._keep.extend([p[0], p[1]])
         self._keep.extend(v for v in kw.values() if isinstance(v, CUDAMatrix))
+        self._writes(kw.get("out_aux"), kw.get("sample_aux"))
         add = kw.pop("add", None)
         return self._add(OP_FUSED_GEMM, (add,), gemm=_build_fused_gemm(passes, **kw))
 
@@ -1065,12 +1087,14 @@ class Program(object):
                          (inv_batch, mom_b, eps_b, mom_w, eps_w, l2, l1))
 
     def split_f16(self, x, aux, exp_dev=None, exp_const=0):
+        self._writes(aux)
         return self._add(OP_SPLIT_F16, (x, aux, exp_dev), (exp_const,))
 
     def branch(self, what):
         return self._add(OP_BRANCH, (), (what,))
 
     def split_bf16(self, x, aux):
+        self._writes(aux)
         return self._add(OP_SPLIT_BF16, (x, aux))
 
     def allreduce(self, mat):
@@ -1158,6 +1182,8 @@ def feed_gather(src, packed, dims, key, shuffle, start, out, mean=None, std=None
                             mean.p_mat if mean is not None else None, std.p_mat if std is not None else None,
                             out.p_mat, out_aux.p_mat if out_aux is not None else None, ct.c_int(aux_mode),
                             ct.c_int(aux_exp)))
+    if out_aux is not None:
+        out_aux.form = {1: "bf16", 2: int(aux_exp)}.get(aux_mode)
     return out
 
 

@@ -64,8 +64,6 @@ class DeviceFeed(object):
         if buf is None:
             cm = self.cm
             aux = cm.empty_aux((self.dims[i], count)) if (i == 0 and self.aux_mode) else None
-            if aux is not None:
-                aux.form = "bf16" if self.aux_mode == 1 else self.aux_exp
             buf = self._out[(i, count)] = (cm.empty((self.dims[i], count)), aux)
         return buf
 
@@ -92,6 +90,8 @@ class DeviceFeed(object):
                                 aux_exp=self.aux_exp)
             if self.add_noise[i]:
                 out.sample_gaussian(mult=self.sigma)          # datahandler.py:335-337
+                if aux is not None:
+                    aux.form = None                           # (parts of the data without noise)
             batch.append(out)
         self.last_aux = self._buffers(0, end - start)[1]
         return batch

@@ -99,6 +99,7 @@ class FusedRBM(LossReadback):
         # the half-precision form below serves every model but the small ones (and, over several ranks, the big ones)
         f16_ok = binary_data and visible == LOGISTIC and os.environ.get("B200_RBM_F16", "1") != "0"
         self.state_aux = big or (f16_ok and world_size == 1 and self._planes_pay()) if env is None else env != "0"
+        self.takes_unmarked = big or env is not None     # parts that do not say what they are are the caller's word: big models take it
         # With 0/1 data and logistic units every operand's range is known, and the big products run
         # on the scaled half-precision form of W and of the states (three fp16 terms, no TF32 term,
         # no fp32 operand read): W * 2^e with e kept by the update kernel, states * 2^14.  Real-valued data have no range: one
@@ -232,7 +233,8 @@ class FusedRBM(LossReadback):
                 else self._issue_f16 if self.f16 else self._issue)
         if data_aux is not None and not (self.state_aux and self.visible != REPLICATED_SOFTMAX):
             data_aux = None                      # this engine derives the parts of the data in its kernels
-        if getattr(data_aux, "form", None) not in (None, 14 if self.f16 else "bf16"):
+        form = getattr(data_aux, "form", None)
+        if form != (14 if self.f16 else "bf16") and not (form is None and self.takes_unmarked):
             data_aux = None                      # parts in another form than this engine's
         self._given_aux = data_aux
         if not self.use_program or self.timeline is not None:

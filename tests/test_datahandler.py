@@ -172,3 +172,33 @@ def test_parts_in_another_form_are_not_read(cm, mode, exp, monkeypatch):
         results.append(np.array(eng.W.asarray()))
     np.testing.assert_array_equal(*results)
     assert np.abs(results[0] - w).max() > 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("how", ["feed_gather", "out_aux", "recorded", "own"])
+def test_parts_say_what_they_were_last_filled_with(cm, how):
+    """An engine of middling size, which chose its planes itself, given parts that a gather, a product or a recorded product wrote
+    in bfloat16 (over planes of its own form): the bits of an update without parts.  Its own form is read: parts of other data show."""
+    from deepnet_b200 import dbm
+    from deepnet_b200.fused_rbm import FusedRBM
+    rng = np.random.default_rng(5)
+    V, H, B = 512, 512, 256
+    x = (rng.random((V, B)) < 0.3).astype(np.float32)
+    w = (0.1 * rng.standard_normal((V, H))).astype(np.float32)
+    results = []
+    for given in (True, False):
+        eng = FusedRBM(cm, V, H, B, w, dbm.Hyperparams(base_epsilon=0.1), binary_data=True, seed=3)
+        assert eng.f16 and not eng.takes_unmarked
+        data, aux, eye = cm.CUDAMatrix(x), cm.empty_aux((V, B)), cm.CUDAMatrix(np.eye(V, dtype=np.float32))
+        cm.CUDAMatrix(1 - x).split_f16(aux, None, 14)
+        X = cm.Program() if how == "recorded" else cm.Immediate()
+        if how == "feed_gather":
+            cm.feed_gather(cm.feed_pack(x), True, V, (0, 0), False, 0, data, out_aux=aux, aux_mode=1)
+        elif how != "own":
+            X.fused_gemm(cm.split_passes(eye, data, exact_a=True, exact_b=True), out=cm.empty((V, B)), out_aux=aux)
+        if how == "recorded":
+            data.split_f16(aux, None, 14)
+            X.run()
+        eng.TrainOneBatch(0, data, aux if given else None)
+        results.append(np.array(eng.W.asarray()))
+    assert np.array_equal(*results) == (how != "own")
