@@ -69,7 +69,7 @@ class UpwardNet(object):
 
     def forward(self, data, exact_input=False):
         """States of the top lower layer for the minibatch `data` (dims x batch); exact_input: the
-        data are 0/1 (no low part)."""
+        data are 0/1, or whole numbers of up to eleven bits (no low part)."""
         if not self.fused:   # the reference's calls (deepnet/neuralnet.py ForwardPropagate: dot, add_col_vec, activation)
             cm, x = self.cm, data
             for l in self.layers:
@@ -87,16 +87,17 @@ class UpwardNet(object):
 
     def _issue(self, X, x, exact):
         cm, E, planes = self.cm, 14, None
+        at = E
         if exact and self._data_aux is not None:
-            planes = self._data_aux
-            X.split_f16(x, planes, None, E)
+            planes, at = self._data_aux, 0      # (whole numbers are exact as they are, up to 65504; times 2^14 no further than 3)
+            X.split_f16(x, planes, None, at)
         for l in self.layers:
             kw = dict(out=l["state"], out_aux=l["state_aux"], bias=l["b"], activation=l["act"], aux_f16=True, aux_exp=E)
             if planes is not None:
-                X.fused_gemm(cm.f16_passes(l["W"].T, l["planes"], x, planes, exact_b=exact), scale_exp=l["exp"], scale_exp_const=E, **kw)
+                X.fused_gemm(cm.f16_passes(l["W"].T, l["planes"], x, planes, exact_b=exact), scale_exp=l["exp"], scale_exp_const=at, **kw)
             else:
                 X.fused_gemm(cm.split_passes(l["W"].T, x, exact_b=exact, a_aux=l["W_aux"]), **kw)
-            x, planes, exact = l["state"], l["state_aux"], False
+            x, planes, exact, at = l["state"], l["state_aux"], False, E
 
 
 class DBN(object):

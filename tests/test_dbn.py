@@ -120,3 +120,19 @@ def test_upward_net_on_half_precision_planes(cm, sizes, acts, B, exact):
         want = 1 / (1 + np.exp(-want)) if act == dbm.LOGISTIC else want
         assert np.abs(np.array(l["state"].asarray()) - want).max() < 1e-5 * max(1.0, np.abs(want).max())
     assert cm.read_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("largest", [1, 3, 4, 255, 2047])
+def test_upward_net_takes_counts_for_exact_input(cm, largest):
+    """A net that splits its data into planes, on 0/1 data and on counts, which the weights bring back to ordinary size: the
+    logistic against float64."""
+    rng = np.random.default_rng(largest)
+    V, H, B = 1024, 2048, 512
+    w = (0.05 / largest * rng.standard_normal((V, H))).astype(np.float32)
+    net = dbn.UpwardNet(cm, [(w, np.zeros(H, np.float32), dbm.LOGISTIC)], B)
+    assert net._data_aux is not None
+    x = (rng.integers(1, largest + 1, (V, B)) * (rng.random((V, B)) < 0.1)).astype(np.float32)
+    got = np.array(net.forward(cm.CUDAMatrix(x), exact_input=True).asarray())
+    assert np.abs(got - 1 / (1 + np.exp(-(w.T.astype(np.float64) @ x)))).max() < 1e-5
+    assert cm.read_status() == 0
