@@ -58,14 +58,14 @@ class UpwardNet(object):
                 continue
             l["exp"] = cm.f16_scale_state(float(np.maximum(w.max(), -w.min()))).slice(0, 1)
             l["planes"] = W.split_f16(cm.empty_aux(w.shape), exp_dev=l["exp"])
-        # the pass is recorded, once for 0/1 and once for real data, and replayed with one library call on whatever minibatch the
+        # the pass is recorded, once for every form its data take, and replayed with one library call on whatever minibatch the
         # handle points at
         self._programs = {}
         if self.fused:
             self._batch = cm.CUDAMatrix._from_mat(cm.cudamat())
-            for exact in (False, True):
-                self._programs[exact] = cm.Program()
-                self._issue(self._programs[exact], self._batch, exact)
+            for exact, split in ((False, False), (True, False)) + (((True, True),) if self._data_aux is not None else ()):
+                self._programs[exact, split] = cm.Program()
+                self._issue(self._programs[exact, split], self._batch, exact, split)
 
     def forward(self, data, exact_input=False):
         """States of the top lower layer for the minibatch `data` (dims x batch); exact_input: the
@@ -82,13 +82,14 @@ class UpwardNet(object):
         ct.memmove(ct.byref(self._batch.mat), ct.byref(data.mat), ct.sizeof(data.mat))
         self._batch.mat.owns_data = 0
         self._batch_owner = data
-        self._programs[bool(exact_input)].run()
+        # (what is split is read in its own order: a transposed handle goes the other way)
+        self._programs[bool(exact_input), bool(exact_input) and self._data_aux is not None and not data.mat.is_trans].run()
         return self.layers[-1]["state"]
 
-    def _issue(self, X, x, exact):
+    def _issue(self, X, x, exact, split):
         cm, E, planes = self.cm, 14, None
         at = E
-        if exact and self._data_aux is not None:
+        if split:
             planes, at = self._data_aux, 0      # (whole numbers are exact as they are, up to 65504; times 2^14 no further than 3)
             X.split_f16(x, planes, None, at)
         for l in self.layers:

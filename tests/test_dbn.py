@@ -136,3 +136,19 @@ def test_upward_net_takes_counts_for_exact_input(cm, largest):
     got = np.array(net.forward(cm.CUDAMatrix(x), exact_input=True).asarray())
     assert np.abs(got - 1 / (1 + np.exp(-(w.T.astype(np.float64) @ x)))).max() < 1e-5
     assert cm.read_status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("V,H,B", [(1024, 2048, 512), (70, 40, 20)])
+def test_upward_net_takes_a_transposed_minibatch(cm, V, H, B):
+    """Whether or not the net splits its data into planes."""
+    rng = np.random.default_rng(V)
+    w = (0.05 * rng.standard_normal((V, H))).astype(np.float32)
+    net = dbn.UpwardNet(cm, [(w, np.zeros(H, np.float32), dbm.LOGISTIC)], B)
+    assert (net._data_aux is not None) == (V == 1024)
+    x = (rng.random((V, B)) < 0.3).astype(np.float32)
+    want = 1 / (1 + np.exp(-(w.T.astype(np.float64) @ x)))
+    for exact in (True, False):
+        for m in (cm.CUDAMatrix(np.ascontiguousarray(x.T)).T, cm.CUDAMatrix(x)):
+            assert np.abs(np.array(net.forward(m, exact_input=exact).asarray()) - want).max() < 1e-5
+    assert cm.read_status() == 0
