@@ -79,6 +79,8 @@ class UpwardNet(object):
                     cm.sigmoid(l["state"])
                 x = l["state"]
             return x
+        if not self.layers:
+            return data
         ct.memmove(ct.byref(self._batch.mat), ct.byref(data.mat), ct.sizeof(data.mat))
         self._batch.mat.owns_data = 0
         self._batch_owner = data

@@ -152,3 +152,11 @@ def test_upward_net_takes_a_transposed_minibatch(cm, V, H, B):
         for m in (cm.CUDAMatrix(np.ascontiguousarray(x.T)).T, cm.CUDAMatrix(x)):
             assert np.abs(np.array(net.forward(m, exact_input=exact).asarray()) - want).max() < 1e-5
     assert cm.read_status() == 0
+
+
+@pytest.mark.gpu
+def test_upward_net_without_layers_hands_the_data_on(cm):
+    """A deep belief network whose top model sees the data itself."""
+    data = cm.CUDAMatrix(np.ones((6, 4), np.float32))
+    for exact in (False, True):
+        assert dbn.UpwardNet(cm, [], 4).forward(data, exact_input=exact) is data
