@@ -663,6 +663,17 @@ def f16_scale_state(max_abs):
     return CUDAMatrix(np.array([[e, e, 0.0, 0.0]], np.float32))
 
 
+# Half-precision planes have one exponent a matrix: whatever its size, an element is kept to 2^-38 of the largest.  That does no
+# harm where the logistic of a sum is wanted and the largest weight is one a model can use: with one weight of 100 among 784 x 512
+# of 0.05 the other units' logistics are as exact as without it (1.3e-7), with 10^4 they are off by 6e-7, with 10^6 by 4e-5.
+F16_LARGEST_WEIGHT = 64.0
+
+
+def f16_holds(max_abs):
+    """Whether weights of this largest magnitude may be multiplied as half-precision planes."""
+    return bool(max_abs <= F16_LARGEST_WEIGHT)     # (a NaN may not)
+
+
 def split_passes(a, b, negate=0, exact_a=False, exact_b=False, terms="bf16", a_aux=None, b_aux=None, a_rows=None,
                  b_rows=None):
     """The terms of a . b at fp32 grade, small terms first.  terms="bf16": the corrections are

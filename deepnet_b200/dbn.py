@@ -37,8 +37,8 @@ class UpwardNet(object):
         self.cm, self.B = cm, batchsize
         self.layers = []
         self.fused = hasattr(cm, "fused_gemm") if fused is None else bool(fused)
-        # Logistic states are read as scaled half-precision planes, which the layer below leaves beside them (no fp32 operand,
-        # the most exact form), and so are 0/1 data where splitting them costs less than it saves (2048 x 512, 2048 units: 4 us
+        # A logistic layer reads logistic states as scaled half-precision planes, which the layer below leaves beside them (no fp32
+        # operand, the most exact form), and so it does 0/1 data where splitting them costs less than it saves (2048 x 512, 2048 units: 4 us
         # of 7; 784 x 2048, 500 units: 4.5 of 2.5; 784 x 700, 500 units, which go in one launch otherwise: 3 of 9).
         self._data_aux = None
         specs = [(np.asarray(w, np.float32), b, 1 if act == LOGISTIC else 0) for w, b, act in specs]
@@ -48,7 +48,8 @@ class UpwardNet(object):
                      b=cm.CUDAMatrix(np.asarray(b, np.float32).reshape(-1, 1)), act=act, state=cm.empty((w.shape[1], batchsize)),
                      planes=None, state_aux=None)
             self.layers.append(l)
-            if not self.fused or not np.isfinite(w).all():
+            # (a linear layer's units keep their own precision however far their weights lie apart)
+            if not self.fused or not act or not w.size or not cm.f16_holds(np.maximum(w.max(), -w.min())):
                 continue
             if i > 0 and specs[i - 1][2]:
                 self.layers[i - 1]["state_aux"] = cm.empty_aux((w.shape[0], batchsize))

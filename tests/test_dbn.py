@@ -160,3 +160,27 @@ def test_upward_net_without_layers_hands_the_data_on(cm):
     data = cm.CUDAMatrix(np.ones((6, 4), np.float32))
     for exact in (False, True):
         assert dbn.UpwardNet(cm, [], 4).forward(data, exact_input=exact) is data
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("act,largest", [(dbm.LINEAR, 0.0), (dbm.LOGISTIC, 0.0), (dbm.LOGISTIC, 1e4), (dbm.LOGISTIC, 1e8)])
+def test_units_of_an_upward_net_do_not_share_their_precision(cm, act, largest):
+    """Weights of a linear layer's units ten orders apart: every unit against float64, 1e-5 of its own largest state.  One
+    weight of any size in a logistic layer: every other unit's logistic to 1e-6."""
+    rng = np.random.default_rng(6)
+    V, H, H2, B = 300, 200, 100, 64
+    w = (0.1 * rng.standard_normal((V, H))).astype(np.float32)
+    w2 = (0.1 * rng.standard_normal((H, H2))).astype(np.float32)
+    if act == dbm.LINEAR:
+        w2 *= (10.0 ** -np.linspace(0, 10, H2)).astype(np.float32)
+    w2[5, 9] += np.float32(largest)
+    net = dbn.UpwardNet(cm, [(w, np.zeros(H, np.float32), dbm.LOGISTIC), (w2, np.zeros(H2, np.float32), act)], B)
+    x = rng.standard_normal((V, B)).astype(np.float32)
+    got = np.array(net.forward(cm.CUDAMatrix(x)).asarray())
+    want = w2.T.astype(np.float64) @ (1 / (1 + np.exp(-(w.T.astype(np.float64) @ x))))
+    if act == dbm.LINEAR:
+        assert (np.abs(got - want).max(axis=1) < 1e-5 * np.abs(want).max(axis=1)).all()
+    else:
+        others = np.arange(H2) != 9
+        assert np.abs(got - 1 / (1 + np.exp(-np.clip(want, -700, 700))))[others].max() < 1e-6
+    assert cm.read_status() == 0
