@@ -720,13 +720,17 @@ def carve(shapes):
     room = small if builtins.max(need) <= small else 1 << 30
     blocks, left = [], 0
     for n in need:                                # the sizes that share an allocation
-        if not blocks or n > left:
+        if not blocks or n > left or n > 1 << 30:
             blocks.append([])
             left = room
         blocks[-1].append(n)
         left -= n
     out, at = [], 0
     for block in blocks:
+        if block[0] > 1 << 30:                    # (alone, and of more elements than a column holds rows)
+            out.append(empty(shapes[at]))
+            at += 1
+            continue
         slab, first = empty((builtins.sum(block), 1)), 0
         for n in block:
             r, c = shapes[at]

@@ -73,3 +73,28 @@ def test_product_does_not_import_the_oracle():
             if f.endswith((".py", ".cu", ".cuh", ".h")):
                 text = open(os.path.join(dirpath, f)).read()
                 assert "eigenmat_oracle" not in text and "liboracle" not in text, f
+
+
+@pytest.mark.parametrize("shapes", [[(46341, 46341), (4, 4), (100000, 21475), (5, 1)], [(1 << 15, 1 << 15), (1, 64)], [(3, 5), (7, 7)]])
+def test_matrices_beyond_a_column_get_an_allocation_of_their_own_shape(shapes, monkeypatch):
+    """Matrices of 2^30 elements and more that share device memory: no allocation has a dimension beyond 2^31, every matrix lies
+    inside one and over no other (on a stand-in that records what would be allocated)."""
+    from deepnet_b200 import b200mat as cm
+
+    class Stand(object):
+        def __init__(self, shape, slab=None, first=0):
+            assert 0 < shape[0] < 1 << 31 and 0 < shape[1] < 1 << 31
+            self.shape, self.slab, self.first = shape, slab or self, first
+
+        def slice(self, first, last):
+            assert self.shape[1] == 1 and last <= self.shape[0]
+            return Stand((last - first, 1), self, first)
+
+        def reshape(self, shape):
+            assert shape[0] * shape[1] == self.shape[0] * self.shape[1]
+            return Stand(shape, self.slab, self.first)
+    monkeypatch.setattr(cm, "empty", Stand)
+    mats = cm.carve(shapes)
+    assert [m.shape for m in mats] == shapes
+    spans = sorted((id(m.slab), m.first, m.first + m.shape[0] * m.shape[1]) for m in mats)
+    assert all(a[0] != b[0] or a[2] <= b[1] for a, b in zip(spans, spans[1:]))
