@@ -89,26 +89,11 @@ class FusedRBM(LossReadback):
         w = np.asarray(weight, np.float32)
         assert w.shape == (V, H)
         self.W = cm.CUDAMatrix(w)
-        # bfloat16 parts of W kept in memory (rewritten by every update): the big products read
+        # 16-bit parts of W kept in memory (rewritten by every update): the big products read
         # them instead of deriving them, as they do for the states that feed the next product
-        self.W_aux = self.W.split_bf16(cm.empty_aux((V, H)))
-        # ... and for the states only when the products are big: a small model is bound by launch
-        # latency, where the extra split launch and the wider epilogue cost more than they save
-        env = os.environ.get("B200_RBM_STATE_AUX")
-        big = V * H * batchsize >= 1 << 32
-        # the half-precision form below serves every model but the small ones (and, over several ranks, the big ones)
-        f16_ok = binary_data and visible == LOGISTIC and os.environ.get("B200_RBM_F16", "1") != "0"
-        self.state_aux = big or (f16_ok and world_size == 1 and self._planes_pay()) if env is None else env != "0"
-        self.takes_unmarked = big or env is not None     # parts that do not say what they are are the caller's word: big models take it
-        # With 0/1 data and logistic units every operand's range is known, and the big products run
-        # on the scaled half-precision form of W and of the states (three fp16 terms, no TF32 term,
-        # no fp32 operand read): W * 2^e with e kept by the update kernel, states * 2^14.  Real-valued data have no range: one
-        # exponent for a minibatch takes from every case what the largest of them lies above it.
-        self.f16 = self.state_aux and f16_ok
-        if self.f16:
-            self.W_scale = cm.f16_scale_state(float(np.maximum(w.max(), -w.min())))
-            self.W_exp = self.W_scale.slice(0, 1)
-            self.W.split_f16(self.W_aux, exp_dev=self.W_exp)
+        self.W_aux = cm.empty_aux((V, H))
+        self.W_scale = self.W_exp = self.h_pos_aux = self.h_neg_aux = None
+        self._choose_form(w)
         # both bias vectors, their update histories and their statistics are packed [b_v | b_h], so
         # one kernel updates them
         b0 = np.zeros((V + H, 1), np.float32)
@@ -131,7 +116,6 @@ class FusedRBM(LossReadback):
         self.h_pos, self.h_samp, self.v_neg, self.h_neg = cm.carve([(H, B), (H, B), (V, B), (H, B)])
         self.h_samp_aux, self.v_neg_aux = za(H, B), za(V, B)
         self.data_aux = za(V, B)
-        self.h_pos_aux, self.h_neg_aux = (za(H, B), za(H, B)) if getattr(self, "f16", False) else (None, None)
         self.v_samp = self.v_samp_aux = None      # allocated when sample_input asks for visible draws
         self.loss_acc = z(1, 1)
         if visible == REPLICATED_SOFTMAX:
@@ -142,7 +126,6 @@ class FusedRBM(LossReadback):
             self.v_samp = z(V, B)
             self.v_act = z(V, B)                  # W h + b_v before the softmax
             self.tiny = 1e-10
-        self._group = None                        # states of several minibatches whose representations are written out
         self._sched = Parameter(cm, self.hyp)
         self._esched = Parameter(cm, self.ehyp)
         self.kernel_launches = 0
@@ -150,7 +133,6 @@ class FusedRBM(LossReadback):
         # the step is recorded once per (Gibbs steps, visible draw) and replayed with one library call;
         # B200_RBM_PROGRAM=0 issues every operation through its own call instead
         self.use_program = os.environ.get("B200_RBM_PROGRAM", "1") != "0"
-        self._programs = {}
         # data parallel, big model: the all-reduce and the update (and with B200_DP_PANEL_PRODUCTS the
         # statistics product, which then leaves the all-reduce some SMs) can run in column panels of W,
         # the all-reduce on a side stream.  Measured on two B200s neither form changed the time of an
@@ -170,6 +152,41 @@ class FusedRBM(LossReadback):
         self._batch = cm.CUDAMatrix._from_mat(cm.cudamat())   # the recorded step's view of the current minibatch
         self._batch_aux = cm.CUDAMatrix._from_mat(cm.cudamat())   # ... and of its 16-bit parts, when the caller has them
         self._given_aux = None
+
+    def _choose_form(self, w):
+        """The form of the products for weights w (host; None: read back where they decide), and W's parts in it."""
+        cm, V, H, B = self.cm, self.V, self.H, self.B
+        # parts of the states, too, only when the products are big: a small model is bound by launch
+        # latency, where the extra split launch and the wider epilogue cost more than they save
+        env = os.environ.get("B200_RBM_STATE_AUX")
+        big = V * H * B >= 1 << 32
+        # With 0/1 data and logistic units every operand's range is known, and the big products run
+        # on the scaled half-precision form of W and of the states (three fp16 terms, no TF32 term,
+        # no fp32 operand read): W * 2^e with e kept by the update kernel, states * 2^14.  Real-valued data have no range: one
+        # exponent for a minibatch takes from every case what the largest of them lies above it.  It serves every model but the
+        # small ones (and, over several ranks, the big ones) and those whose weights it does not hold.
+        f16_ok = self.binary_data and self.visible == LOGISTIC and os.environ.get("B200_RBM_F16", "1") != "0"
+        pays = f16_ok and self.world_size == 1 and self._planes_pay()
+        largest = 0.0
+        if f16_ok and (pays or big or env is not None):
+            w = np.array(self.W.asarray()) if w is None else w
+            largest = float(np.maximum(w.max(), -w.min()))
+        self.planes_hold = cm.f16_holds(largest)
+        self.state_aux = big or (pays and self.planes_hold) if env is None else env != "0"
+        self.takes_unmarked = big or env is not None     # parts that do not say what they are are the caller's word: big models take it
+        self.f16 = self.state_aux and f16_ok
+        self._programs = {}
+        self._group = None                               # states of several minibatches whose representations are written out
+        if not self.f16:
+            self.W.split_bf16(self.W_aux)
+            return
+        if self.W_scale is None:
+            self.W_scale = cm.f16_scale_state(largest)
+            self.W_exp = self.W_scale.slice(0, 1)
+            self.h_pos_aux, self.h_neg_aux = cm.empty_aux((H, B)), cm.empty_aux((H, B))
+        else:
+            self.W_scale.assign(cm.f16_scale_state(largest))
+        self.W.split_f16(self.W_aux, exp_dev=self.W_exp)
 
     def _planes_pay(self):
         """Whether the products come off better on half-precision planes (tcgen05, no fp32 operand read) than in one launch or
@@ -476,13 +493,8 @@ class FusedRBM(LossReadback):
         return self._issue_updates(X, sc, wb)
 
     def refresh_weight_aux(self):
-        """Rebuilds the 16-bit parts of W after W was written from outside (a loaded checkpoint)."""
-        if self.f16:
-            w = np.array(self.W.asarray())
-            self.W_scale.assign(self.cm.f16_scale_state(float(np.maximum(w.max(), -w.min()))))   # (in place: recorded steps name it)
-            self.W.split_f16(self.W_aux, exp_dev=self.W_exp)
-        else:
-            self.W.split_bf16(self.W_aux)
+        """Rebuilds the 16-bit parts of W after W was written from outside (a loaded checkpoint), in the form that suits it."""
+        self._choose_form(None)
 
     def Inference(self, data, input_recon=False):
         """Hidden representation of `data` (V x cases device matrix), minibatch by minibatch:
@@ -520,7 +532,7 @@ class FusedRBM(LossReadback):
                         h, v, va, ha = (m.slice(0, (e - b) * B) if m is not None else None for m in (h, v, va, ha))
                 act = 1 if self.visible == LOGISTIC else 0
                 # (a product as small as in one launch: the call that splits the data costs more than the planes save)
-                planes = self.f16 and (e - b) * B * V * H >= 1 << 27
+                planes = self.f16 and self.planes_hold and (e - b) * B * V * H >= 1 << 27
                 if soft:
                     v0.sum(axis=0, target=self.NN)
                     self.NN.add(self.tiny)

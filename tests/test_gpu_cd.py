@@ -852,6 +852,41 @@ def test_one_case_of_large_values_leaves_the_others_exact(cm, outlier):
     assert cm.read_status() == 0
 
 
+@pytest.mark.parametrize("largest", [0.0, 10.0, 1e4, 1e8])
+def test_one_large_weight_leaves_the_other_units_exact(cm, largest):
+    """One weight of any size, in a model that would go on half-precision planes: every other unit's representation against float64
+    to 3e-7 (1.3e-7 without it), whether the engine was made with it or loads it, and planes again once it is gone."""
+    rng = np.random.default_rng(0)
+    V, H, B = 784, 512, 256
+    w = (0.05 * rng.standard_normal((V, H))).astype(np.float32)
+    x = (rng.random((V, 4 * B)) < 0.3).astype(np.float32)
+    plain, odd = w.copy(), w.copy()
+    odd[3, 7] += np.float32(largest)
+    sig = lambda z: 1 / (1 + np.exp(-np.clip(z, -700, 700)))
+    others, data = np.arange(H) != 7, cm.CUDAMatrix(x)
+    made = FusedRBM(cm, V, H, B, odd, dbm.Hyperparams(), binary_data=True, seed=1)
+    loads = FusedRBM(cm, V, H, B, plain, dbm.Hyperparams(), binary_data=True, seed=1)
+    assert loads.f16
+    loads.W.overwrite(np.asfortranarray(odd))
+    loads.refresh_weight_aux()
+    for eng in (made, loads):
+        assert eng.f16 == (largest < 64)
+        assert np.abs(eng.Inference(data).T - sig(odd.T.astype(np.float64) @ x))[others].max() < 3e-7
+    results = []
+    for eng in (made, loads):
+        cm.CUDAMatrix.init_random(1)
+        eng.TrainOneBatch(0, data.slice(0, B))
+        results.append(get(eng.W))
+        eng.W.overwrite(np.asfortranarray(plain))
+        eng.refresh_weight_aux()
+        assert eng.f16
+        assert np.abs(eng.Inference(data).T - sig(plain.T.astype(np.float64) @ x + get(eng.bh))).max() < 3e-7
+        eng.TrainOneBatch(1, data.slice(0, B))
+        assert np.isfinite(get(eng.W)).all()
+    np.testing.assert_array_equal(*results)
+    assert cm.read_status() == 0
+
+
 def test_work_side_by_side(cm):
     """Two chains of products beside each other and what follows the join, recorded and call by call: the bits of one stream.  An
     operation that fails between fork and join leaves the thread on the library stream."""
