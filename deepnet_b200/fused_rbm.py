@@ -381,7 +381,7 @@ class FusedRBM(LossReadback):
             self._op(X, "gemm_down", gf, 2 * vb, "fused_gemm", F(W, Wa, self.h_samp, self.h_samp_aux, exact_b=True),
                      out=self.v_neg if (i == 0 or last) else None,
                      out_aux=self.v_neg_aux if (last or not draw_v) else None,
-                     sample=self.v_samp if draw_v and last and tail else None, sample_aux=self.v_samp_aux if draw_v else None,
+                     sample=self.v_samp if draw_v and last else None, sample_aux=self.v_samp_aux if draw_v else None,
                      bias=self.bv, activation=1, **act)
             if i == 0 and not (tail and k == 1):
                 self._op(X, "sq_err", 0, 2 * vb, "sq_diff", self.v_neg, v0, self.loss_acc)
