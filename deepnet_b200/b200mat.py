@@ -656,10 +656,10 @@ def f16_passes(a, a_aux, b, b_aux, negate=0, exact_a=False, exact_b=False, a_row
 
 def f16_scale_state(max_abs):
     """The 1 x 4 device matrix `momentum_update` keeps for a parameter in scaled half-precision
-    form: {exponent, -, max |w| of the running update (bits), -}; the exponent puts the largest
+    form: {exponent, the one a fresh start would take, max |w| of the running update (bits), -}; the exponent puts the largest
     magnitude at or below 2^13.  `.slice(0, 1)` is the `scale_exp` of a product."""
     m = float(max_abs) if np.isfinite(max_abs) else 1.0         # (weights that are not finite have no exponent that fits)
-    e = float(np.floor(np.log2(8192.0 / max(m, 1e-30))))
+    e = min(float(np.floor(np.log2(8192.0 / max(m, 1e-30)))), 100.0)
     return CUDAMatrix(np.array([[e, e, 0.0, 0.0]], np.float32))
 
 

@@ -208,6 +208,12 @@ __device__ __forceinline__ void split_f16(float x, float scale, uint16_t& lo, ui
   hi = __half_as_ushort(h);
   lo = __half_as_ushort(l);
 }
+// The exponent for a matrix whose largest magnitude is m > 0: m * 2^e in (2^12, 2^13].
+__device__ __forceinline__ float f16_exponent(float m) {
+  int x;
+  const float f = frexpf(m, &x);          // m = f * 2^x, f in [1/2, 1)
+  return (float)min(max((f == 0.5f ? 14 : 13) - x, -100), 100);
+}
 __device__ __forceinline__ float f16_to_float(uint16_t h) { return __half2float(__ushort_as_half(h)); }
 
 #endif

@@ -195,16 +195,16 @@ __global__ void k_peer_finish(PeerPtrs pp, int nranks, int rank, int epoch, floa
     f[kMaxBits + q] = 0u;      // (the owners write their next maximum only after the next `ready` round)
   }
   const float m = __uint_as_float(mb);
-  float redo = 0.0f;
+  float redo = 0.0f, want = scale_state[0];
   if (m > 0.0f && m < 3.0e38f) {
-    const float want = fminf(fmaxf(floorf(log2f(8192.0f / m)), -100.0f), 100.0f);
+    want = f16_exponent(m);
     const float d = scale_state[0] - want;
     if (d < -1.0f || d > 2.0f) {
       scale_state[0] = want;
       redo = 1.0f;
     }
   }
-  scale_state[1] = scale_state[0];
+  scale_state[1] = want;
   scale_state[3] = redo;
   reinterpret_cast<unsigned*>(scale_state)[2] = 0u;
 }

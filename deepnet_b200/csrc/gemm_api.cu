@@ -589,15 +589,16 @@ struct UpdateArgs {
 __device__ __forceinline__ bool update_scale(float* scale) {
   const float m = __uint_as_float(__ldcg(reinterpret_cast<unsigned*>(scale) + 2));
   bool redo = false;
+  float want = scale[0];
   if (m > 0.0f && m < 3.0e38f) {
-    const float want = fminf(fmaxf(floorf(log2f(8192.0f / m)), -100.0f), 100.0f);
+    want = f16_exponent(m);
     const float d = scale[0] - want;
     if (d < -1.0f || d > 2.0f) {
       scale[0] = want;
       redo = true;
     }
   }
-  scale[1] = scale[0];
+  scale[1] = want;
   reinterpret_cast<unsigned*>(scale)[2] = 0u;
   return redo;
 }
@@ -655,7 +656,7 @@ __global__ void __launch_bounds__(256) k_update_all(const __grid_constant__ Tail
 // After an update in scaled half-precision form.  The exponent wanted for the new parameter puts
 // the largest |w| * 2^e in (2^12, 2^13] (the fp16 limit is just under 2^16).  The aux was written
 // with the exponent carried so far; it stands while the largest scaled magnitude stays within
-// (2^11, 2^15].  Otherwise the wanted exponent is stored and scale[3] tells the second pass to
+// (2^11, 2^15].  Otherwise the wanted exponent, which scale[1] names in any case, is stored and scale[3] tells the second pass to
 // rewrite the aux.  The maximum starts over.  A parameter that is all zero (or not finite) keeps
 // its exponent.
 __global__ void k_update_scale(float* scale) {
@@ -931,7 +932,7 @@ int dot(cudamat* mat1, cudamat* mat2, cudamat* target, float beta, float alpha) 
 // deepnet/dbm.py:242,254 + deepnet/parameter.py:80-106 in one pass over the parameter:
 //   grad += suff * (-inv_batch); delta = momentum*delta + l2*w + l1*sign(w) + grad;
 //   w -= eps * delta; grad = 0; and, when w_aux is given, the aux matrix of the new w: its
-//   bfloat16 parts, or with w_scale (1 x 4 device matrix {exponent, -, max |w| bits, -}) its
+//   bfloat16 parts, or with w_scale (1 x 4 device matrix {exponent, the one a fresh start would take, max |w| bits, -}) its
 //   scaled half-precision form, written in the same pass with the exponent carried so far; a
 //   second pass rewrites it only when the new w no longer fits that exponent.
 // grad may be null (treated as zero and not written).  20 bytes of traffic per element

@@ -176,6 +176,8 @@ class FusedRBM(LossReadback):
         self.takes_unmarked = big or env is not None     # parts that do not say what they are are the caller's word: big models take it
         self.f16 = self.state_aux and f16_ok
         self._programs = {}
+        self._updated = False                            # since W's planes were made from W as a whole
+        self._w_planes = None
         self._group = None                               # states of several minibatches whose representations are written out
         if not self.f16:
             self.W.split_bf16(self.W_aux)
@@ -254,6 +256,7 @@ class FusedRBM(LossReadback):
         if form != (14 if self.f16 else "bf16") and not (form is None and self.takes_unmarked):
             data_aux = None                      # parts in another form than this engine's
         self._given_aux = data_aux
+        self._updated = True
         if not self.use_program or self.timeline is not None:
             self.kernel_launches = 0
             return body(cm.Immediate(), data, k, draw_v, sc)
@@ -496,6 +499,21 @@ class FusedRBM(LossReadback):
         """Rebuilds the 16-bit parts of W after W was written from outside (a loaded checkpoint), in the form that suits it."""
         self._choose_form(None)
 
+    def _representation_planes(self):
+        """W's planes and their exponent as an engine made with the weights of this moment has them (updates keep an exponent while it
+        serves, and it shows in the last bits: a representation follows from the weights alone), or None where planes do not hold W."""
+        cm = self.cm
+        if not self._updated:
+            return (self.W_aux, self.W_exp) if self.planes_hold else None
+        now, fresh = np.array(self.W_scale.asarray())[0, :2]
+        if not cm.f16_holds(2.0 ** (13 - fresh)):
+            return None
+        if now == fresh:
+            return self.W_aux, self.W_exp
+        if self._w_planes is None:
+            self._w_planes = cm.empty_aux((self.V, self.H))
+        return self.W.split_f16(self._w_planes, exp_dev=self.W_scale.slice(1, 2)), self.W_scale.slice(1, 2)
+
     def Inference(self, data, input_recon=False):
         """Hidden representation of `data` (V x cases device matrix), minibatch by minibatch:
         the inference-only positive phase of deepnet/dbm.py:340-398 (extract_rbm_representation.py)
@@ -517,6 +535,8 @@ class FusedRBM(LossReadback):
                 self._group = (cm.carve([(H, g * B), (H, g * B), (V, g * B)] + aux) + [None, None])[:5]
             else:                                # (one minibatch a product: the engine's own states, a second buffer for the hidden ones)
                 self._group = [cm.empty((H, B)), self.h_pos, self.v_neg, self.data_aux, self.h_pos_aux]
+        # (a product as small as in one launch: the call that splits the data costs more than the planes save)
+        w_planes = self._representation_planes() if self.f16 and g * B * V * H >= 1 << 27 else None
         # one small minibatch has nothing to hide its copy behind: 784 x 500 with 100 cases 53 us copied the plain way, 62 by
         # the threads; with 400 cases of 500 100 and 94
         with cm.RowsOut(n > 1 or rep.nbytes >= 1 << 19) as out:
@@ -531,8 +551,7 @@ class FusedRBM(LossReadback):
                     if e - b < g:
                         h, v, va, ha = (m.slice(0, (e - b) * B) if m is not None else None for m in (h, v, va, ha))
                 act = 1 if self.visible == LOGISTIC else 0
-                # (a product as small as in one launch: the call that splits the data costs more than the planes save)
-                planes = self.f16 and self.planes_hold and (e - b) * B * V * H >= 1 << 27
+                planes = w_planes is not None and (e - b) * B * V * H >= 1 << 27
                 if soft:
                     v0.sum(axis=0, target=self.NN)
                     self.NN.add(self.tiny)
@@ -540,7 +559,7 @@ class FusedRBM(LossReadback):
                 elif planes:
                     hidden = dict(out=h, out_aux=ha if input_recon else None, bias=self.bh, activation=1, aux_f16=True, aux_exp=E)
                     v0.split_f16(va, None, E)
-                    cm.fused_gemm(F(W.T, Wa, v0, va, exact_b=True), scale_exp=self.W_exp, scale_exp_const=E, **hidden)
+                    cm.fused_gemm(F(W.T, w_planes[0], v0, va, exact_b=True), scale_exp=w_planes[1], scale_exp_const=E, **hidden)
                 else:
                     cm.fused_gemm(P(W.T, v0, exact_b=self.binary_data, a_aux=None if self.f16 else Wa), out=h, bias=self.bh, activation=1)
                 if out.held:                     # on its way while the error is computed
@@ -552,7 +571,7 @@ class FusedRBM(LossReadback):
                     cm._check(cm._lib.add_sq_diff(self.v_negn.p_mat, v0.p_mat, self.loss_acc.p_mat))
                 elif input_recon:
                     if planes:
-                        cm.fused_gemm(F(W, Wa, h, ha), out=v, bias=self.bv, activation=act, scale_exp=self.W_exp, scale_exp_const=E)
+                        cm.fused_gemm(F(W, w_planes[0], h, ha), out=v, bias=self.bv, activation=act, scale_exp=w_planes[1], scale_exp_const=E)
                     else:
                         cm.fused_gemm(P(W, h, a_aux=None if self.f16 else Wa), out=v, bias=self.bv, activation=act)
                     cm._check(cm._lib.add_sq_diff(v.p_mat, v0.p_mat, self.loss_acc.p_mat))

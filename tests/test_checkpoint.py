@@ -152,3 +152,33 @@ def test_trained_rbm_survives_a_checkpoint(cm, tmp_path):
         np.testing.assert_array_equal(np.array(a.asarray()), np.array(b.asarray()))
     # the restored engine computes the same hidden representation
     np.testing.assert_array_equal(eng.Inference(data.slice(0, B)), other.Inference(data.slice(0, B)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("edge,moves", [(15.99, 1), (16.01, -1), (63.9, 1)])
+def test_representations_follow_from_the_weights_alone(cm, tmp_path, edge, moves):
+    """A mid-sized model on half-precision planes whose largest weight crosses a power of two (and the size that planes hold) while
+    the exponent in force stays: trained and restored engine give the same bits.  Weights over many orders, where an exponent shows."""
+    from deepnet_b200 import dbm
+    from deepnet_b200.fused_rbm import FusedRBM
+    rng = np.random.default_rng(8)
+    V, H, B = 784, 512, 256
+    w = 1e-3 * rng.standard_normal((V, H)) * np.exp(2 * rng.standard_normal((V, H)))
+    w = np.clip(w, -10, 10).astype(np.float32)
+    w[5, :20] = edge
+    hyp = dbm.Hyperparams(base_epsilon=1e-2, l2_decay=-2.0 * moves, apply_l2_decay=True)
+    mk = lambda w: FusedRBM(cm, V, H, B, w, hyp, binary_data=True, seed=9)
+    data = cm.CUDAMatrix((rng.random((V, 4 * B)) < 0.3).astype(np.float32))
+    eng = mk(w)
+    now = []
+    for step in range(3):
+        eng.TrainOneBatch(step, data.slice(step * B, (step + 1) * B))
+        other = mk(np.zeros((V, H), np.float32))
+        ck.load_into_rbm(other, ck.model_from_rbm(eng, "rbm"))
+        now.append(np.array(eng.W_scale.asarray())[0, :2])
+        eng.read_loss()                  # (of the update)
+        for a, b in zip(eng.Inference(data, input_recon=True), other.Inference(data, input_recon=True)):
+            np.testing.assert_array_equal(a, b)
+    assert any(a != b for a, b in now), now
+    assert (np.abs(np.array(eng.W.asarray())).max() > 64) == (not other.f16) == (edge > 60)
+    assert cm.read_status() == 0
