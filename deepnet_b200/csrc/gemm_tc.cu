@@ -1515,12 +1515,12 @@ int resident_clusters(int ctas, int& clusters) {
     attr_set[dev] = true;
   }
   if (ctas == 1) {
-    clusters = sm_count();
+    clusters = device_sms();
     return 0;
   }
   if (!resident[dev][ctas]) {
     cudaLaunchConfig_t q = {};
-    q.gridDim = dim3((unsigned)(ctas * (sm_count() / ctas)));
+    q.gridDim = dim3((unsigned)(ctas * (device_sms() / ctas)));   // (kept: not what a limit in force leaves of it)
     q.blockDim = dim3(kThreadsTc);
     q.dynamicSmemBytes = Cfg::kSmemBytes;
     cudaLaunchAttribute at[1];
@@ -1533,8 +1533,8 @@ int resident_clusters(int ctas, int& clusters) {
     int n = 0;
     if (cudaOccupancyMaxActiveClusters(&n, kernel, &q) != cudaSuccess || n < 1) {
       cudaGetLastError();
-      if (ctas <= 8) return set_error("cudaOccupancyMaxActiveClusters failed for a tensor-core product");
-      n = 0;
+      if (kEpi != kEpiTile) return set_error("cudaOccupancyMaxActiveClusters failed for a tensor-core product");
+      n = 0;                                    // (the product goes on persistent CTAs)
     }
     resident[dev][ctas] = n;
   }
@@ -1794,7 +1794,7 @@ static int splits_of(int ctas, int min_ki) {
   return want > 32 ? 32 : (want < 1 ? 1 : want);
 }
 
-static int g_tile_columns = 0, g_last_columns = 0;   // b200_test_tile_columns
+static int g_tile_columns = 0, g_last_columns = 0, g_last_plan = 0;   // b200_test_tile_columns, b200_test_plan
 
 // How a product is laid out.  tile: one work item per CTA (pair), the splits of a tile in one cluster (TileEpilogue); else
 // persistent CTAs, and a finishing launch behind the splits.
@@ -2011,6 +2011,7 @@ int gemm_tc(const GemmProblem& g) {
   const bool two = plan.two;
   const int BN_LOCAL = two ? BN / 2 : BN;      // rows of B staged per CTA
   g_last_columns = BN;
+  g_last_plan = plan.tile ? BN + (two ? 1000 : 0) + 10000 * plan.splits : 0;
   TcParams p;
   p.M = g.M;
   p.N = g.N;
@@ -2321,6 +2322,8 @@ extern "C" int b200_test_tile_columns(int columns) {
   if (columns == 0 || columns == 64 || columns == 128 || columns == 256) b200::g_tile_columns = columns;
   return b200::g_last_columns;
 }
+// Test hook: the last product's layout, see b200mat.h.
+extern "C" int b200_test_plan(void) { return b200::g_last_plan; }
 
 #ifdef B200_GEMM_TIMING
 // Debug build only: copies the per-CTA cycle counters of the last launch (8 words per CTA).

@@ -323,6 +323,9 @@ int b200_test_limit_scratch(size_t bytes);
 /* Test hook: columns of the tensor-core tiles (64, 128 or 256; 0 by the estimate) of products where the estimate has the choice.
  * Returns those of the last product. */
 int b200_test_tile_columns(int columns);
+/* Test hook: the layout of the last tensor-core product with one work item per CTA: its tiles' columns, 1000 more where two CTAs
+ * share a tile, 10000 for each part of K; 0 where CTAs were persistent. */
+int b200_test_plan(void);
 /* Test hooks: the form of ais_binary_steps (0 the faster one, 1 all steps in one launch or an error, 2 three launches a step); whether
  * n inverse temperatures of B chains take one launch. */
 int b200_test_ais_form(int form);

@@ -5,6 +5,9 @@ and the fused epilogue (bias, logistic, Bernoulli draw, TF32 split, negated pass
 Tolerance: 1e-5 of the largest magnitude of the exact result (the bound the path must
 meet on activations and gradients); the single-pass TF32 mode is checked at 2e-3."""
 import ctypes as ct
+import os
+import subprocess
+import sys
 
 import numpy as np
 import pytest
@@ -1023,6 +1026,35 @@ def test_one_work_item_per_cta(cm, M, N, K, splits, columns):
     np.testing.assert_array_equal(lo, (got * np.float32(2.0 ** 14) - want_hi).astype(np.float16).astype(np.float32))
     np.testing.assert_array_equal(f16_planes(smp_aux)[1], get(smp) * 2.0 ** 14)
     assert cm.read_status() == 0
+
+
+@pytest.mark.parametrize("limit", [2, 4, 12])
+def test_first_product_of_a_process_under_a_limit_of_sms(limit):
+    """The layouts of a product are looked up once: under a limit that leaves room for no large cluster, and after it is lifted, the
+    product is right (512 x 128, K = 8192: 1e-5 of the largest) and the layout the one of a process without a limit."""
+    code = """if True:
+        import numpy as np, sys
+        from deepnet_b200 import b200mat as cm
+        cm.cublas_init()
+        rng = np.random.default_rng(0)
+        a, b = rng.standard_normal((512, 8192)).astype(np.float32), rng.standard_normal((8192, 128)).astype(np.float32)
+        A, B, out, bias = cm.CUDAMatrix(a), cm.CUDAMatrix(b), cm.empty((512, 128)), cm.empty((512, 1))
+        want = a.astype(np.float64) @ b
+        cm.set_gemm_path(1)
+        for limit in (int(sys.argv[1]), 0):
+            cm.set_sm_limit(limit)
+            cm.fused_gemm(cm.split_passes(A, B), out=out, bias=bias)
+            assert np.abs(np.array(out.asarray()) - want).max() < 1e-5 * np.abs(want).max()
+        assert cm.read_status() == 0
+        print(cm._lib.b200_test_plan())
+    """
+    root = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+    plans = []
+    for first in (limit, 0):
+        r = subprocess.run([sys.executable, "-c", code, str(first)], cwd=root, capture_output=True, text=True, timeout=120)
+        assert r.returncode == 0, r.stderr[-2000:]
+        plans.append(r.stdout)
+    assert plans[0] == plans[1]
 
 
 @pytest.mark.parametrize("M,N,K,columns", [(784, 1000, 1024, 256), (4096, 132, 1024, 256), (512, 1024, 2048, 256), (500, 500, 500, 64)])
