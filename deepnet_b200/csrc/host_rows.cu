@@ -35,6 +35,7 @@ namespace {
 // 65 us; parts of 64 KB cost large results up to a third).
 constexpr int kPieces = 16, kRun = 4, kCarriers = 4, kBusy = 2;
 constexpr size_t kPieceBytes = 256 * 1024, kPartBytes = 64 * 1024;
+static_assert((1ull << 32) % kPieces == 0, "the counter of copies wraps to the same turn");
 
 struct RowsStaging {
   std::mutex mu;
@@ -52,7 +53,8 @@ struct RowsStaging {
   cudaStream_t copies = nullptr;
   bool free_piece[kPieces];
   int parts[kPieces] = {0};      // of a piece, still to be carried
-  int device = 0, in_flight = 0, adds = 0, copied = 0;    // copied: copies so far; each has the next event in turn
+  int device = 0, in_flight = 0, adds = 0;
+  unsigned copied = 0;           // copies so far; each has the next event in turn
   std::atomic<long> taken{0}, seen{0};     // pieces carriers have taken, and seen land
   bool held = false, stop = false, made = false, failed = false;
 
@@ -182,7 +184,9 @@ int b200_rows_add(cudamat* src, float* dst) {
         s.free_piece[first + pieces++] = false;
     }
     const size_t run = bytes - at < pieces * kPieceBytes ? bytes - at : pieces * kPieceBytes;
-    const int event = s.copied++ % kPieces;      // (its copy of kPieces copies ago has been carried: there are no more pieces)
+    // A job may still wait for this event, that of a copy kPieces copies ago: all copies are on one stream, so what it then waits
+    // for landed later than its own.
+    const int event = (int)(s.copied++ % kPieces);
     const bool ok = cudaMemcpyAsync(s.pinned + first * kPieceBytes, (const char*)src->data_device + at, run, cudaMemcpyDeviceToHost,
                                     s.copies) == cudaSuccess &&
                     cudaEventRecord(s.landed[event], s.copies) == cudaSuccess;
