@@ -511,7 +511,10 @@ class FusedRBM(LossReadback):
         if now == fresh:
             return self.W_aux, self.W_exp
         if self._w_planes is None:
-            self._w_planes = cm.empty_aux((self.V, self.H))
+            try:
+                self._w_planes = cm.empty_aux((self.V, self.H))
+            except cm.CUDAMatException:          # a device that is nearly full
+                return None
         return self.W.split_f16(self._w_planes, exp_dev=self.W_scale.slice(1, 2)), self.W_scale.slice(1, 2)
 
     def Inference(self, data, input_recon=False):
@@ -532,8 +535,11 @@ class FusedRBM(LossReadback):
             self._group = None                   # (given back first)
             if g > 1:                            # (an aux matrix holds whole groups of eight rows)
                 aux = [((r + 7) // 8 * 8, g * B) for r in (V, H)] if self.f16 else []
-                self._group = (cm.carve([(H, g * B), (H, g * B), (V, g * B)] + aux) + [None, None])[:5]
-            else:                                # (one minibatch a product: the engine's own states, a second buffer for the hidden ones)
+                try:
+                    self._group = (cm.carve([(H, g * B), (H, g * B), (V, g * B)] + aux) + [None, None])[:5]
+                except cm.CUDAMatException:      # a device that is nearly full
+                    g = 1
+            if g == 1:                           # (one minibatch a product: the engine's own states, a second buffer for the hidden ones)
                 self._group = [cm.empty((H, B)), self.h_pos, self.v_neg, self.data_aux, self.h_pos_aux]
         # (a product as small as in one launch: the call that splits the data costs more than the planes save)
         w_planes = self._representation_planes() if self.f16 and g * B * V * H >= 1 << 27 else None

@@ -888,6 +888,31 @@ def test_one_large_weight_leaves_the_other_units_exact(cm, largest):
     assert cm.read_status() == 0
 
 
+def test_representations_on_a_device_that_is_nearly_full(cm, monkeypatch):
+    """Without memory for states of several minibatches, or for planes of a fresh exponent, they go one by one, from fp32 operands."""
+    rng = np.random.default_rng(1)
+    V, H, B = 784, 512, 256
+    w = (0.05 * rng.standard_normal((V, H))).astype(np.float32)
+    w[0, 0] = 0.9999                       # (grows past 1: another exponent would be fresh)
+    x = (rng.random((V, 4 * B)) < 0.3).astype(np.float32)
+    x[0] = 1
+    eng = FusedRBM(cm, V, H, B, w, dbm.Hyperparams(base_epsilon=0.1), binary_data=True, seed=1)
+    data = cm.CUDAMatrix(x)
+    eng.TrainOneBatch(0, data.slice(0, B))
+    now, fresh = get(eng.W_scale)[0, :2]
+    assert eng.f16 and now != fresh
+
+    def full(*_):
+        raise cm.CUDAMatException("no memory")
+    for name in ("carve", "empty_aux"):
+        monkeypatch.setattr(cm, name, full)
+    w, b = get(eng.W).astype(np.float64), get(eng.bh)
+    assert np.abs(eng.Inference(data).T - 1 / (1 + np.exp(-(w.T @ x + b)))).max() < 1e-5
+    monkeypatch.undo()
+    assert np.abs(eng.Inference(data).T - 1 / (1 + np.exp(-(w.T @ x + b)))).max() < 1e-5
+    assert cm.read_status() == 0
+
+
 def test_work_side_by_side(cm):
     """Two chains of products beside each other and what follows the join, recorded and call by call: the bits of one stream.  An
     operation that fails between fork and join leaves the thread on the library stream."""
