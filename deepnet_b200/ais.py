@@ -39,8 +39,8 @@ def ais_binary_rbm(cm, weight, hidden_bias, visible_bias, num_chains, schedule, 
         fused = hasattr(cm, "fused_gemm")
     B = num_chains
     if fused:
-        w, w_aux, a, b, scaled, v_state, v_sample, h_state, h_sample, w_ais = cm.carve(
-            [(V, H), ((V + 7) // 8 * 8, H), (H, 1), (V, 1), (V, 1), (V, B), (V, B), (H, B), (H, B), (1, B)])
+        w, a, b, scaled, v_state, v_sample, h_state, h_sample, w_ais, w_aux = cm.carve(
+            [(V, H), (H, 1), (V, 1), (V, 1), (V, B), (V, B), (H, B), (H, B), (1, B)], aux=[(V, H)])
         for m, host in ((w, weight), (a, hidden_bias), (b, visible_bias)):
             m.overwrite(host)
     else:

@@ -595,6 +595,17 @@ class AuxMatrix(CUDAMatrix):
         self.p_mat = ct.pointer(self.mat)
         self.numpy_array = None
 
+    @classmethod
+    def _over(cls, storage, shape):
+        """The parts of a matrix of this shape in `storage` (a matrix of whole groups of eight rows)."""
+        new = cls.__new__(cls)
+        new.rows, new.cols = int(shape[0]), int(shape[1])
+        new.mat = cudamat()
+        ct.memmove(ct.pointer(new.mat), storage.p_mat, ct.sizeof(new.mat))
+        new.mat.owns_data = 0
+        new.p_mat, new.numpy_array, new._parent = ct.pointer(new.mat), None, storage
+        return new
+
     def planes(self):
         """Host copy of the two planes as float32 arrays (rows x cols each)."""
         raw = np.array(self.asarray(), copy=True)                       # lda x cols floats
@@ -709,15 +720,17 @@ def empty(shape):
     return CUDAMatrix._from_mat(mat)
 
 
-def carve(shapes):
-    """Matrices of these shapes in few device allocations (each starts on 256 bytes), all zero.  Taking device memory costs some
-    340 us from a megabyte on, whatever its size, and giving it back 270; below, hardly anything.  So what needs more than that for
-    one matrix is taken in one allocation (annealing 784 x 500, 100 chains, 100 steps: 2660 -> 2030 us a call, 1100 of them steps;
-    the five matrices of an engine's first `Inference` of 8 x 250 cases, 1000 x 1000: 2300 -> 900), the rest stays below it
-    (annealing 300 x 200, 300 chains in one: 350 -> 1010)."""
+def carve(shapes, aux=()):
+    """Matrices of these shapes, and behind them aux matrices for matrices of the shapes in `aux`, in few device allocations (each
+    matrix starts on 256 bytes), all zero.  Taking device memory costs some 340 us from a megabyte on, whatever its size, and giving
+    it back 270; below, hardly anything while there are few.  So what needs more than that for one matrix, or for four altogether,
+    is taken in one allocation (annealing 784 x 500, 100 chains, 100 steps: 2660 -> 2030 us a call, 1100 of them steps; 500 x 500,
+    400 chains, 20 steps: 2650 -> 1400; the five matrices of an engine's first `Inference` of 8 x 250 cases, 1000 x 1000: 2300 ->
+    900), the rest stays below it (annealing 300 x 200, 300 chains in one: 350 -> 1010)."""
+    shapes = list(shapes) + [((r + 7) // 8 * 8, c) for r, c in aux]
     need = [-(-r * c // 64) * 64 for r, c in shapes]
     small = (1 << 18) - 4096                      # floats of an allocation that costs little
-    room = small if builtins.max(need) <= small else 1 << 30
+    room = small if builtins.max(need) <= small and builtins.sum(need) <= 4 * small else 1 << 30
     blocks, left = [], 0
     for n in need:                                # the sizes that share an allocation
         if not blocks or n > left or n > 1 << 30:
@@ -736,7 +749,8 @@ def carve(shapes):
             r, c = shapes[at]
             out.append(slab.slice(first, first + r * c).reshape((r, c)))
             first, at = first + n, at + 1
-    return out
+    plain = len(out) - len(aux)
+    return out[:plain] + [AuxMatrix._over(m, shape) for m, shape in zip(out[plain:], aux)]
 
 
 def reformat(array):

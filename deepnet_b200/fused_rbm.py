@@ -113,9 +113,13 @@ class FusedRBM(LossReadback):
         self.suff_b = self.pack.slice(V * H, V * H + V + H)
         B = batchsize
         za = lambda r, c: cm.empty_aux((r, c))
-        self.h_pos, self.h_samp, self.v_neg, self.h_neg = cm.carve([(H, B), (H, B), (V, B), (H, B)])
-        self.h_samp_aux, self.v_neg_aux = za(H, B), za(V, B)
-        self.data_aux = za(V, B)
+        states, aux = [(H, B), (H, B), (V, B), (H, B)], [(H, B), (V, B), (V, B)]
+        if self.f16:
+            made = cm.carve(states, aux=aux + [(H, B), (H, B)])
+            self.h_pos_aux, self.h_neg_aux = made[7:]
+        else:                                     # (the parts of small states fit in beside other allocations: 784 x 500 1.5 ms, 1.8 in one)
+            made = cm.carve(states) + [za(*s) for s in aux]
+        self.h_pos, self.h_samp, self.v_neg, self.h_neg, self.h_samp_aux, self.v_neg_aux, self.data_aux = made[:7]
         self.v_samp = self.v_samp_aux = None      # allocated when sample_input asks for visible draws
         self.loss_acc = z(1, 1)
         if visible == REPLICATED_SOFTMAX:
@@ -169,8 +173,8 @@ class FusedRBM(LossReadback):
         pays = f16_ok and self.world_size == 1 and self._planes_pay()
         largest = 0.0
         if f16_ok and (pays or big or env is not None):
-            w = np.array(self.W.asarray()) if w is None else w
-            largest = float(np.maximum(w.max(), -w.min()))
+            host = np.array(self.W.asarray()) if w is None else w
+            largest = float(np.maximum(host.max(), -host.min()))
         self.planes_hold = cm.f16_holds(largest)
         self.state_aux = big or (pays and self.planes_hold) if env is None else env != "0"
         self.takes_unmarked = big or env is not None     # parts that do not say what they are are the caller's word: big models take it
@@ -185,10 +189,11 @@ class FusedRBM(LossReadback):
         if self.W_scale is None:
             self.W_scale = cm.f16_scale_state(largest)
             self.W_exp = self.W_scale.slice(0, 1)
-            self.h_pos_aux, self.h_neg_aux = cm.empty_aux((H, B)), cm.empty_aux((H, B))
         else:
             self.W_scale.assign(cm.f16_scale_state(largest))
         self.W.split_f16(self.W_aux, exp_dev=self.W_exp)
+        if w is None and self.h_pos_aux is None:         # (an engine made for weights that planes do not hold)
+            self.h_pos_aux, self.h_neg_aux = cm.carve((), aux=[(H, B), (H, B)])
 
     def _planes_pay(self):
         """Whether the products come off better on half-precision planes (tcgen05, no fp32 operand read) than in one launch or
@@ -533,10 +538,10 @@ class FusedRBM(LossReadback):
         g = 1 if soft else max(1, min(n, 1024 // B))
         if n > 1 and (self._group is None or self._group[0].shape[1] != g * B):
             self._group = None                   # (given back first)
-            if g > 1:                            # (an aux matrix holds whole groups of eight rows)
-                aux = [((r + 7) // 8 * 8, g * B) for r in (V, H)] if self.f16 else []
+            if g > 1:
                 try:
-                    self._group = (cm.carve([(H, g * B), (H, g * B), (V, g * B)] + aux) + [None, None])[:5]
+                    aux = [(V, g * B), (H, g * B)] if self.f16 else []
+                    self._group = (cm.carve([(H, g * B), (H, g * B), (V, g * B)], aux=aux) + [None, None])[:5]
                 except cm.CUDAMatException:      # a device that is nearly full
                     g = 1
             if g == 1:                           # (one minibatch a product: the engine's own states, a second buffer for the hidden ones)

@@ -902,7 +902,7 @@ def test_representations_on_a_device_that_is_nearly_full(cm, monkeypatch):
     now, fresh = get(eng.W_scale)[0, :2]
     assert eng.f16 and now != fresh
 
-    def full(*_):
+    def full(*_, **__):
         raise cm.CUDAMatException("no memory")
     for name in ("carve", "empty_aux"):
         monkeypatch.setattr(cm, name, full)

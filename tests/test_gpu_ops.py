@@ -370,3 +370,25 @@ def test_matrices_of_one_allocation(cm, shapes):
     del mats, m
     last.copy_to_host()
     assert (last.numpy_array == len(shapes)).all()
+
+
+@pytest.mark.parametrize("shapes,aux", [([], [(5, 3)]), ([(7, 9)], [(61, 40), (8, 300)]), ([(600, 500)], [(513, 511), (1, 1)]),
+                                        ([(500, 500)] * 5, [(499, 500)])])
+def test_aux_matrices_of_one_allocation(cm, shapes, aux):
+    """The parts of a matrix in storage of their own and carved: the same planes, nothing else touched, shared by few matrices and many."""
+    rng = np.random.default_rng(1)
+    made = cm.carve(shapes, aux=aux)
+    plain, parts = made[:len(shapes)], made[len(shapes):]
+    assert [m.shape for m in plain] == list(shapes)
+    for shape, a in zip(aux, parts):
+        x = cm.CUDAMatrix(rng.standard_normal(shape).astype(np.float32))
+        own = x.split_bf16(cm.empty_aux(shape))
+        assert x.split_bf16(a) is a and a.form == "bf16"
+        for p, q in zip(a.planes(), own.planes()):
+            np.testing.assert_array_equal(p, q)
+    assert not any(np.array(m.asarray()).any() for m in plain)
+    last = parts[-1]
+    planes = [p.copy() for p in last.planes()]
+    del made, plain, parts, a
+    for p, q in zip(planes, last.planes()):
+        np.testing.assert_array_equal(p, q)
