@@ -62,9 +62,8 @@ class DeviceFeed(object):
     def _buffers(self, i, count):
         buf = self._out.get((i, count))
         if buf is None:
-            cm = self.cm
-            aux = cm.empty_aux((self.dims[i], count)) if (i == 0 and self.aux_mode) else None
-            buf = self._out[(i, count)] = (cm.empty((self.dims[i], count)), aux)
+            cm, shape = self.cm, (self.dims[i], count)
+            buf = self._out[(i, count)] = tuple(cm.carve([shape], aux=[shape])) if i == 0 and self.aux_mode else (cm.empty(shape), None)
         return buf
 
     def Get(self, batchsize, get_last_piece=False):
