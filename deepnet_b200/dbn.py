@@ -42,23 +42,37 @@ class UpwardNet(object):
         # of 7; 784 x 2048, 500 units: 4.5 of 2.5; 784 x 700, 500 units, which go in one launch otherwise: 3 of 9).
         self._data_aux = None
         specs = [(np.asarray(w, np.float32), b, 1 if act == LOGISTIC else 0) for w, b, act in specs]
+        largest = [float(np.maximum(w.max(), -w.min())) if self.fused and w.size else 0.0 for w, _, _ in specs]
+        aux = {}                 # (what, layer): the matrix whose 16-bit parts it holds
         for i, (w, b, act) in enumerate(specs):
-            W = cm.CUDAMatrix(w)
-            l = dict(W=W, W_aux=W.split_bf16(cm.empty_aux(w.shape)) if hasattr(cm, "empty_aux") else None,
-                     b=cm.CUDAMatrix(np.asarray(b, np.float32).reshape(-1, 1)), act=act, state=cm.empty((w.shape[1], batchsize)),
-                     planes=None, state_aux=None)
-            self.layers.append(l)
             # (a linear layer's units keep their own precision however far their weights lie apart)
-            if not self.fused or not act or not w.size or not cm.f16_holds(np.maximum(w.max(), -w.min())):
-                continue
-            if i > 0 and specs[i - 1][2]:
-                self.layers[i - 1]["state_aux"] = cm.empty_aux((w.shape[0], batchsize))
-            elif i == 0 and (w.size * batchsize >= 1 << 30 or w.size * batchsize >= 1 << 27 and w.shape[0] * batchsize <= 1 << 20):
-                self._data_aux = cm.empty_aux((w.shape[0], batchsize))
+            planes = self.fused and act and w.size and cm.f16_holds(largest[i])
+            if planes and i > 0 and specs[i - 1][2]:
+                aux["state_aux", i - 1] = (w.shape[0], batchsize)
+            elif planes and i == 0 and (w.size * batchsize >= 1 << 30 or w.size * batchsize >= 1 << 27 and w.shape[0] * batchsize <= 1 << 20):
+                aux["data_aux", 0] = (w.shape[0], batchsize)
             else:
-                continue
-            l["exp"] = cm.f16_scale_state(float(np.maximum(w.max(), -w.min()))).slice(0, 1)
-            l["planes"] = W.split_f16(cm.empty_aux(w.shape), exp_dev=l["exp"])
+                planes = False
+            if planes:
+                aux["planes", i] = w.shape
+            if self.fused and (i == 0 or not planes):        # (the first layer's data may be real)
+                aux["W_aux", i] = w.shape
+        states = [(w.shape[1], batchsize) for w, _, _ in specs]
+        if self.fused and specs:
+            made = cm.carve(states, aux=list(aux.values()))
+            states, aux = made[:len(specs)], dict(zip(aux, made[len(specs):]))
+            self._data_aux = aux.get(("data_aux", 0))
+        else:
+            states = [cm.empty(s) for s in states]
+        for i, (w, b, act) in enumerate(specs):
+            l = dict(W=cm.CUDAMatrix(w), b=cm.CUDAMatrix(np.asarray(b, np.float32).reshape(-1, 1)), act=act, state=states[i])
+            l.update((what, aux.get((what, i))) for what in ("W_aux", "planes", "state_aux"))
+            if l["W_aux"] is not None:
+                l["W"].split_bf16(l["W_aux"])
+            if l["planes"] is not None:
+                l["exp"] = cm.f16_scale_state(largest[i]).slice(0, 1)
+                l["W"].split_f16(l["planes"], exp_dev=l["exp"])
+            self.layers.append(l)
         # the pass is recorded, once for every form its data take, and replayed with one library call on whatever minibatch the
         # handle points at
         self._programs = {}
