@@ -299,6 +299,8 @@ class FusedRBM(LossReadback):
             u = self._op(X, "update", 0, 8.0 * (V + H) * self.B + 6 * wb, "update_all", layers, self.W, self.dW, self.suff_W,
                          self.W_aux, sc["inv_b"], sc["mom"], sc["eps"], sc["emom"], sc["eeps"], l2=sc["l2"], l1=sc["l1"],
                          sq_acc=bias[2], w_scale=w_scale)
+            if w_scale is not None and V * H > 1 << 19:      # (beyond what one block rewrites: a launch that returns at once unless it has to)
+                self.kernel_launches += 1
             if self.B > 1024:      # past that the operation is made of its separate launches
                 self.kernel_launches += 5 if bias[2] is not None else 4
             return ("update", u), None

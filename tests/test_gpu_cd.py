@@ -913,6 +913,53 @@ def test_representations_on_a_device_that_is_nearly_full(cm, monkeypatch):
     assert cm.read_status() == 0
 
 
+def _launches(cm, step):
+    """Kernels of an update, recorded as a graph behind two that were not."""
+    import torch
+    from cuda.bindings import runtime
+    stream, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph(keep_graph=True)
+    cm.cuda_sync_threads()
+    cm._lib.b200_set_stream(stream.cuda_stream)
+    try:
+        for n in range(2):
+            step(n)
+        cm.cuda_sync_threads()
+        with torch.cuda.graph(graph, stream=stream):
+            step(2)
+    finally:
+        cm._lib.b200_set_stream(None)
+    raw = runtime.cudaGraph_t(graph.raw_cuda_graph())
+    _, nodes, _ = runtime.cudaGraphGetNodes(raw, runtime.cudaGraphGetNodes(raw, 0)[2])
+    assert all(runtime.cudaGraphNodeGetType(x)[1] == runtime.cudaGraphNodeType.cudaGraphNodeTypeKernel for x in nodes)
+    return len(nodes)
+
+
+@pytest.mark.parametrize("config,launches", [(0, 5), (1, 5), (2, 9), (3, 44)])
+def test_launches_of_an_update_are_counted(cm, config, launches):
+    """The configurations at their full size: what the engine says, what the library issues, what the launch lists hold."""
+    from deepnet_b200.fused_dbm import FusedDBM
+    cfg = configs.build(config, cases=256)
+    B, dims, weights = cfg["batchsize"], [l["numdims"] for l in cfg["layers"]], [e["weight"] for e in cfg["edges"]]
+    if config == 3:
+        eng = FusedDBM(cm, dims, B, weights, cfg["hyperparams"], seed=1)
+    else:
+        eng = FusedRBM(cm, dims[0], dims[1], B, weights[0], cfg["hyperparams"], visible=cfg["layers"][0]["activation"],
+                       binary_data=config != 1, seed=1)
+    data = cm.CUDAMatrix(cfg["data"][:, :B])
+    assert _launches(cm, lambda n: eng.TrainOneBatch(n, data)) == eng.kernel_launches == launches
+
+
+@pytest.mark.parametrize("V,H,B,k,sample", [(1024, 512, 256, 1, False), (1024, 513, 300, 3, True), (1001, 777, 1100, 2, True),
+                                            (100, 100, 20, 1, False), (1000, 100, 1100, 1, False)])
+def test_launches_on_either_side_of_the_lines_are_counted(cm, V, H, B, k, sample):
+    """Weights whose planes one block rewrites and more, up to 1024 cases and more, planes and fp32 operands."""
+    rng = np.random.default_rng(0)
+    eng = FusedRBM(cm, V, H, B, (0.01 * rng.standard_normal((V, H))).astype(np.float32),
+                   dbm.Hyperparams(gibbs_steps=k, sample_input=sample), binary_data=True, seed=1)
+    data = cm.CUDAMatrix((rng.random((V, B)) < 0.3).astype(np.float32))
+    assert _launches(cm, lambda n: eng.TrainOneBatch(n, data)) == eng.kernel_launches
+
+
 def test_work_side_by_side(cm):
     """Two chains of products beside each other and what follows the join, recorded and call by call: the bits of one stream.  An
     operation that fails between fork and join leaves the thread on the library stream."""
