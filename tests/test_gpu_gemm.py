@@ -978,15 +978,20 @@ def test_narrow_tiles_of_products_of_few_tiles(cm, M, N, K, two_pairs, columns):
     assert cm.read_status() == 0
 
 
-@pytest.mark.parametrize("columns", [64, 128, 256])
-@pytest.mark.parametrize("splits", [0, 2, 3, 7, 13])
-@pytest.mark.parametrize("M,N,K", [(130, 129, 900), (257, 260, 1024), (1001, 515, 904), (516, 1029, 900), (130, 129, 1700)])
+@pytest.mark.parametrize("M,N,K,columns,splits", [
+    (130, 129, 900, 64, 0), (130, 129, 900, 128, 0), (130, 129, 900, 256, 0), (1001, 515, 904, 0, 0), (516, 1029, 900, 0, 0),
+    (130, 129, 4100, 64, 2), (130, 129, 4100, 64, 7), (130, 129, 4100, 64, 13), (130, 129, 4100, 64, 16),
+    (130, 129, 4100, 128, 3), (130, 129, 4100, 128, 8), (130, 129, 4100, 128, 13), (130, 129, 4100, 128, 16),
+    (130, 129, 4100, 256, 2), (130, 129, 4100, 256, 7), (130, 129, 4100, 256, 8),
+    (257, 260, 2308, 64, 3), (257, 260, 2308, 64, 9), (257, 260, 2308, 128, 2), (257, 260, 2308, 128, 7), (257, 260, 2308, 256, 3),
+    (257, 260, 2308, 256, 8), (1001, 515, 904, 64, 2), (1001, 515, 904, 128, 2), (1001, 515, 904, 128, 3), (1001, 515, 904, 256, 2),
+    (1001, 515, 904, 256, 3), (516, 1029, 900, 128, 3), (516, 1029, 900, 256, 2), (516, 1029, 900, 256, 3), (100, 129, 4100, 128, 16)])
 def test_one_work_item_per_cta(cm, M, N, K, splits, columns):
-    """Tiles that end in shared memory, K cut over a cluster or not: ragged rows (columns of the result that start on no
+    """Tiles that end in shared memory, K cut over a cluster (of up to 16 CTAs, single ones and pairs) or not: ragged rows (columns of the result that start on no
     16 bytes) and ragged columns, every output and option of the epilogue, both forms of the 16-bit planes.  Bound: sums of K
     products in chunks of 128 at 2^-18 a term, 1e-5 of the largest result; draws and planes follow from the result exactly."""
     rng = np.random.default_rng(M + K + splits)
-    w = (rng.standard_normal((K, M)) * 0.05).astype(np.float32)
+    w = (rng.standard_normal((K, M)) * 0.05 * min(1.0, (1000 / K) ** 0.5)).astype(np.float32)
     x = rng.random((K, N)).astype(np.float32)
     b, c = rng.standard_normal((M, 1)).astype(np.float32), rng.random((1, N)).astype(np.float32)
     add = rng.standard_normal((M, N)).astype(np.float32)
@@ -1003,12 +1008,19 @@ def test_one_work_item_per_cta(cm, M, N, K, splits, columns):
     try:
         cm.fused_gemm(cm.f16_passes(W.T, wf, X, xf), out=out, out_aux=aux, sample=smp, sample_aux=smp_aux, bias=bias, activation=1,
                       scale_exp=scale.slice(0, 1), scale_exp_const=14, aux_f16=True, aux_exp=14)
+        plans = [cm._lib.b200_test_plan()]
         cm.fused_gemm(cm.split_passes(W.T, X, terms="tf32"), out=plain, add=cm.CUDAMatrix(add))
+        plans.append(cm._lib.b200_test_plan())
         cm.fused_gemm(cm.split_passes(W.T, X), out=scaled, sample=draw, bias=bias, col_scale=cm.CUDAMatrix(c), activation=1)
+        plans.append(cm._lib.b200_test_plan())
     finally:
         cm.set_gemm_path(0)
         cm.set_split_k(0)
         cm._lib.b200_test_tile_columns(0)
+    if splits:
+        assert all(p // 10000 == splits and p % 1000 == columns for p in plans), plans
+    else:
+        assert plans[0] and (not columns or plans[0] % 1000 == columns), plans
     pre = w.T.astype(np.float64) @ x
     sig = lambda z: 1 / (1 + np.exp(-z))
     got = get(out)
