@@ -1860,6 +1860,16 @@ static const ResidentTiles* resident_tiles() {
 //   512 x 200, K = 10000, all of the right operand derived      27.8 / 29.0   (K over 10: seven clusters of 16 fit, and 8 are needed)
 //   784 x 500, K = 100, plain                                    8.1 /  8.8   (nothing to do but store: straight from the registers)
 //   4096 x 4096, K = 128, plain                                 33.9 / 51.5   (several waves, whose stores overlap the next)
+// What the rules beside the estimate are worth, on 584 products that nothing was fitted to (73 shapes of 4 to 10000 rows and
+// columns, K up to 10000, eight term lists; two runs of one side differ by 0.8 %, at most 5 % in nineteen of twenty), as the time
+// without a rule over the time with it where the layout changes:
+//   several waves of one work item behind an activation          22 products, 1.00 to 3.53, mean 1.77
+//   ... up to four of them (nine instead)                         2 products, 1.00 and 1.12
+//   ... but not where the result is plain                         4 products, 1.09 to 1.13
+//   no look at persistent CTAs below 64 k-blocks                 23 products, 1.00 to 1.10, mean 1.05 (at any K instead: 4, 0.84 to 0.97)
+//   a draw (5 %) goes to persistent CTAs                         16 products, 0.64 to 1.06, mean 0.95: costs more than it keeps
+//   12 % on narrow tiles behind derived TF32 parts                4 products, 0.84 to 0.95: the same
+//   3 % on narrower persistent tiles                              none
 static int choose_plan(const GemmProblem& g, bool all16, bool pairs_allowed, TcPlan& plan) {
   const bool scatter = product_is_scattered(g.epi.out);
   const GemmEpilogue& e = g.epi;
