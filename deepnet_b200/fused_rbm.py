@@ -158,19 +158,22 @@ class FusedRBM(LossReadback):
         self._given_aux = None
 
     def _choose_form(self, w):
-        """The form of the products for weights w (host; None: read back where they decide), and W's parts in it."""
+        """The form of the products for weights w (host; None: those the engine has now, read back where they decide), and W's parts
+        in it."""
         cm, V, H, B = self.cm, self.V, self.H, self.B
         # parts of the states, too, only when the products are big: a small model is bound by launch
         # latency, where the extra split launch and the wider epilogue cost more than they save
-        env = os.environ.get("B200_RBM_STATE_AUX")
         big = V * H * B >= 1 << 32
         # With 0/1 data and logistic units every operand's range is known, and the big products run
         # on the scaled half-precision form of W and of the states (three fp16 terms, no TF32 term,
         # no fp32 operand read): W * 2^e with e kept by the update kernel, states * 2^14.  Real-valued data have no range: one
         # exponent for a minibatch takes from every case what the largest of them lies above it.  It serves every model but the
         # small ones (and, over several ranks, the big ones) and those whose weights it does not hold.
-        f16_ok = self.binary_data and self.visible == LOGISTIC and os.environ.get("B200_RBM_F16", "1") != "0"
-        pays = f16_ok and self.world_size == 1 and self._planes_pay()
+        if w is not None:
+            f16_ok = self.binary_data and self.visible == LOGISTIC and os.environ.get("B200_RBM_F16", "1") != "0"
+            self._form = (os.environ.get("B200_RBM_STATE_AUX"), f16_ok, f16_ok and self.world_size == 1 and self._planes_pay())
+            self.f16 = None
+        (env, f16_ok, pays), had = self._form, self.f16
         largest = 0.0
         if f16_ok and (pays or big or env is not None):
             host = np.array(self.W.asarray()) if w is None else w
@@ -179,10 +182,11 @@ class FusedRBM(LossReadback):
         self.state_aux = big or (pays and self.planes_hold) if env is None else env != "0"
         self.takes_unmarked = big or env is not None     # parts that do not say what they are are the caller's word: big models take it
         self.f16 = self.state_aux and f16_ok
-        self._programs = {}
         self._updated = False                            # since W's planes were made from W as a whole
         self._w_planes = None
-        self._group = None                               # states of several minibatches whose representations are written out
+        if self.f16 != had:
+            self._programs = {}
+            self._group = None                           # states of several minibatches whose representations are written out
         if not self.f16:
             self.W.split_bf16(self.W_aux)
             return
