@@ -58,8 +58,8 @@ class LossReadback(object):
 class FusedRBM(LossReadback):
     def __init__(self, cm, V, H, batchsize, weight, hyperparams, edge_hyperparams=None, visible=LOGISTIC,
                  binary_data=False, bias_v=None, bias_h=None, seed=0, world_size=1, rank=0, group=None):
-        """binary_data: the caller states that every input is exactly 0 or 1 (or, for word counts, a
-        small integer): such data have no low part, so the products over them run one term shorter
+        """binary_data: the caller states that every input is exactly 0 or 1 (for the replicated-softmax
+        model, whose inputs are word counts, a small integer): such data have no low part, so the products over them run one term shorter
         and, for a logistic model that is not small (`_planes_pay`), on the scaled half-precision form.  Real-valued inputs
         (grey levels in [0, 1], standardised features) must leave it False: with it set their low
         parts would be dropped without notice.
